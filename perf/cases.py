@@ -183,7 +183,9 @@ def prepare(case, seed):
         if not case["full"]:
             masks = _packed([_image_flags(gen, -(-n // q_tokens), case["kv_heads"], -(-n // BLOCK), case["density"],
                                           case["text"], q_tokens) for n in lens])
-        return {"case": case, "wrapper": wrapper, "q": q, "k": k, "v": v, "masks": masks}
+        # the log-sum-exp buffer is the caller's: rows of inactive q-blocks are not written
+        lse = torch.zeros(total, case["heads"], device=_dev()) if case["lse"] else None
+        return {"case": case, "wrapper": wrapper, "q": q, "k": k, "v": v, "masks": masks, "lse": lse}
     if kind in ("gemm_q", "gemm_o"):
         dt, n, hid = _DTYPES[case["dtype"]], case["heads"] * case["dim"], case["hidden"]
         nb = case["rows"] // BLOCK
@@ -239,7 +241,7 @@ def run(state):
     kind = case["kind"]
     if kind == "attention":
         return state["wrapper"].run(state["q"], state["k"], state["v"], *state["masks"], case["full"],
-                                    return_lse=case["lse"])
+                                    lse=state["lse"], return_lse=case["lse"])
     if kind == "gemm_q":
         return fo.flashomni_gemm(state["x"], state["w"], case["heads"], *state["masks"], 0, state["bias"],
                                  out=state["out"])
