@@ -217,8 +217,16 @@ def _prepare(kind: str, batch: int, M: int, N: int, K: int, num_qo_heads: int, h
         wl = into
     else:
         wl = GemmWorklist(kind, key, torch.zeros(max(nbytes, 256), dtype=torch.uint8, device=dev))
+        if stream is not None:
+            # The workspace is zeroed (and its memory was perhaps last used) on the current stream: the list must not
+            # be built before that, or the zeros land on top of it, in the middle of the build at worst.
+            stream.wait_stream(torch.cuda.current_stream(dev))
+            wl.ws.record_stream(stream)
     if indptr.dtype != torch.int32:
         indptr = indptr.to(torch.int32)
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream(dev))
+            indptr.record_stream(stream)
     st = torch.cuda.current_stream(dev) if stream is None else stream
     with torch.cuda.device(dev):
         if kind == "q":

@@ -152,3 +152,22 @@ def test_prepared_worklists_give_the_same_result(cuda_device):
     assert ql2 is ql
     with pytest.raises(ValueError):
         fo.flashomni_gemm_reduction(x, w, H, None, None, 0, cache, worklist=ql)
+
+
+def test_list_storage_made_behind_pending_work_is_not_wiped(cuda_device):
+    """The workspace of a new list is zeroed on the current stream; a list built on another stream has to wait for that,
+    even when the current stream has work in front of it."""
+    from flashomni_b200.gemm import prepare_gemm_o_list, prepare_gemm_q_list
+    B, H, S = 2, 6, 1024
+    m = wl.flux_masks(B, H, S // 128, S // 128, 0.5, seed=71, text_blocks=1)
+    si, _, ip, _ = masks_to_device(m, cuda_device)
+    busy = torch.randn(4096, 4096, device=cuda_device)
+    side = torch.cuda.Stream(cuda_device)
+    for prepare in (prepare_gemm_q_list, prepare_gemm_o_list):   # the Q list first: its build reads nothing back
+        want = prepare(B, S, H * 128, H, si, ip, 0)
+        torch.cuda.synchronize()
+        for _ in range(20):
+            busy @ busy
+        got = prepare(B, S, H * 128, H, si, ip, 0, stream=side)
+        torch.cuda.synchronize()
+        assert torch.equal(want.ws, got.ws)
