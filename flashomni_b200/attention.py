@@ -239,6 +239,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         self._mask_num_heads = mask_num_heads
         self._mask_head_begin = mask_head_begin
         self._total_q = total_num_rows
+        self._rows_from_0 = int(qo_indptr_host[0]) == 0
         self._total_kv = int(kv_indptr_host[-1])
         self._causal = causal
         # Custom mask (reference: flashomni/attention.py:524-533): per request a [q_len, kv_len] matrix of flags,
@@ -359,6 +360,13 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         self._ws_words = words
         self._ws_offs = offs
         self._scratch_bytes = scratch_bytes
+        # the arguments of fo_attn_lists that only depend on the plan
+        ptrs = {k: v.data_ptr() for k, v in self._ws.items()}
+        self._list_args = (
+            self._batch_size, self._mask_num_heads, self._mask_head_begin, self._num_kv_heads, self._q_block_tokens,
+            128, self._n_cand, self._max_nkv, n, kept, ptrs["items"], ptrs["kv_ptr"], ptrs["kv_idx"], ptrs["order"],
+            ptrs["counters"], ptrs["scratch"], scratch_bytes, self._min_items, self._num_streams, self._min_chunk,
+            self._max_units, self._partial_slots, ptrs["units"], ptrs["unit_counters"], ptrs["arrive"])
         pbytes = lib.fo_attn_partial_bytes(self._partial_slots)
         fw = self._float_workspace_buffer
         self._partials = None
@@ -408,9 +416,8 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 lse = torch.empty((q.size(0), q.size(1)), dtype=torch.float32, device=q.device)
             else:
                 _check_shape_dtype_device(lse, (q.size(0), q.size(1)), torch.float32, q.device, "lse")
-        if out is None:
-            out = torch.zeros(q.shape[:-1] + v.shape[-1:], dtype=q.dtype, device=q.device)
-        else:
+        fresh_out = out is None
+        if not fresh_out:
             _check_shape_dtype_device(out, q.shape[:-1] + v.shape[-1:], q.dtype, q.device, "out")
         if not is_full:
             # the reference dereferences null masks here (csrc/batch_sparseFA.cu:123-131); raise instead
@@ -434,21 +441,35 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             total_kv, hkv = k.size(1), k.size(0)
         if total_kv != self._total_kv or hkv != self._num_kv_heads:
             raise ValueError("k/v shape does not match the plan")
-        if q.stride(2) != 1 or k.stride(2) != 1 or v.stride(2) != 1 or out.stride(2) != 1:
+        if q.stride(2) != 1 or k.stride(2) != 1 or v.stride(2) != 1 or (out is not None and out.stride(2) != 1):
             raise ValueError("the head dimension of q/k/v/out must be contiguous")
-        if out.stride(1) % 8 != 0 or out.stride(0) % 8 != 0:
+        if out is not None and (out.stride(1) % 8 != 0 or out.stride(0) % 8 != 0):
             raise ValueError("out strides must be multiples of 8 elements")
 
         lib = _native.load()
         ws = self._ws
         stream = _native.current_stream(self.device)
         with torch.cuda.device(self.device):
-            key = self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full)
-            if self._prepared_key is not None and self._prepared_key == key:
+            prepared = False
+            if self._prepared_key is not None:
+                prepared = self._prepared_key == self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr,
+                                                                sparse_kv_info_indptr, is_full)
+            # An output allocated here reads as zero in q-blocks that are not computed. When this call builds the lists,
+            # and the requests' rows start at row 0, the list builder zeroes exactly those blocks.
+            zero_out = None
+            if fresh_out:
+                alloc = torch.zeros
+                if not prepared and self._rows_from_0 and v.size(2) == self._head_dim:
+                    alloc = torch.empty
+                out = alloc(q.shape[:-1] + v.shape[-1:], dtype=q.dtype, device=q.device)
+                if alloc is torch.empty:
+                    zero_out = out
+            if prepared:
                 # the lists were built by prepare_masks() on the side stream: just order after it
                 torch.cuda.current_stream(self.device).wait_event(self._prepared_event)
             else:
-                self._compact(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream)
+                self._compact(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream,
+                              zero_out)
             self._prepared_key = None
             head = (_native.ptr(q), _native.ptr(k), _native.ptr(v), _native.ptr(out), _native.ptr(lse),
                     native_dtype(q.dtype), self._total_q, self._total_kv, self._num_qo_heads, self._num_kv_heads,
@@ -485,28 +506,22 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         return tuple((t.data_ptr(), t._version) for t in (sparse_info, sparse_kv_info, sparse_info_indptr,
                                                           sparse_kv_info_indptr))
 
-    def _compact(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream):
-        ws = self._ws
-        rc = _native.load().fo_mask_compact(
-            _native.ptr(sparse_info), 0 if sparse_info is None else sparse_info.numel(),
-            _native.ptr(sparse_kv_info), 0 if sparse_kv_info is None else sparse_kv_info.numel(),
-            _native.ptr(sparse_info_indptr), _native.ptr(sparse_kv_info_indptr),
-            _native.ptr(self._qo_indptr_buf), _native.ptr(self._kv_indptr_buf),
-            self._batch_size, self._mask_num_heads, self._mask_head_begin, self._num_kv_heads,
-            self._q_block_tokens, self._sparse_block_size_for_kv, 1 if is_full else 0,
-            self._n_cand, self._max_nkv, max(self._n_cand, 1), max(self._max_kept, 1),
-            _native.ptr(ws["items"]), _native.ptr(ws["kv_ptr"]), _native.ptr(ws["kv_idx"]),
-            _native.ptr(ws["order"]), _native.ptr(ws["counters"]), _native.ptr(ws["scratch"]),
-            self._scratch_bytes, stream)
-        _native.check(rc, "BatchFlashOmniFAWithRaggedKVWrapper (mask compaction)")
-        rc = _native.load().fo_attn_units(
-            _native.ptr(ws["items"]), _native.ptr(ws["kv_ptr"]), _native.ptr(ws["kv_idx"]), _native.ptr(ws["order"]),
-            _native.ptr(ws["counters"]), _native.ptr(self._qo_indptr_buf), _native.ptr(self._kv_indptr_buf),
-            max(self._n_cand, 1), self._max_nkv, self._q_block_tokens, self._sparse_block_size_for_kv,
-            self._min_items, self._num_streams, self._min_chunk, self._max_units, self._partial_slots,
-            _native.ptr(ws["units"]),
-            _native.ptr(ws["unit_counters"]), _native.ptr(ws["arrive"]), stream)
-        _native.check(rc, "BatchFlashOmniFAWithRaggedKVWrapper (work units)")
+    def _compact(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream,
+                 zero_out=None):
+        """Work lists and unit records on `stream`; the rows of inactive q-blocks of `zero_out` (contiguous, laid out like
+        the planned q) are zeroed in the same pass."""
+        p = _native.ptr
+        zero = (None, 0, 0, 0)
+        if zero_out is not None:
+            isz = zero_out.element_size()
+            zero = (zero_out.data_ptr(), zero_out.stride(0) * isz,
+                    self._num_qo_heads // self._num_kv_heads * self._head_dim * isz, zero_out.numel() * isz)
+        rc = _native.load().fo_attn_lists(
+            p(sparse_info), 0 if sparse_info is None else sparse_info.numel(),
+            p(sparse_kv_info), 0 if sparse_kv_info is None else sparse_kv_info.numel(),
+            p(sparse_info_indptr), p(sparse_kv_info_indptr), 1 if is_full else 0, *zero, p(self._qo_indptr_buf),
+            p(self._kv_indptr_buf), *self._list_args, stream)
+        _native.check(rc, "BatchFlashOmniFAWithRaggedKVWrapper (work lists)")
 
     def build_work_lists(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
                          is_full: bool = False) -> None:

@@ -172,13 +172,15 @@ size_t fo_mask_compact_scratch_bytes(int64_t n_cand, int32_t max_nkv) {
   return b + 16;
 }
 
-int fo_mask_compact(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
-                    int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr,
-                    const int32_t* sparse_kv_info_indptr, const int32_t* qo_indptr, const int32_t* kv_indptr,
-                    int32_t batch, int32_t num_heads, int32_t head_begin, int32_t head_count, int32_t sbq,
-                    int32_t sbkv, int32_t is_full, int64_t n_cand, int32_t max_nkv, int64_t max_items,
-                    int64_t max_kept, int32_t* items, int32_t* kv_ptr, int32_t* kv_idx, int32_t* order,
-                    int32_t* counters, void* scratch, size_t scratch_bytes, void* stream) {
+namespace {
+// Checks the arguments of a compaction and fills `a` from them.
+int make_compact_args(CompactArgs& a, const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                      int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr, const int32_t*
+                      sparse_kv_info_indptr, const int32_t* qo_indptr, const int32_t* kv_indptr, int32_t batch,
+                      int32_t num_heads, int32_t head_begin, int32_t head_count, int32_t sbq, int32_t sbkv,
+                      int32_t is_full, int64_t n_cand, int32_t max_nkv, int64_t max_items, int64_t max_kept,
+                      int32_t* items, int32_t* kv_ptr, int32_t* kv_idx, int32_t* order, int32_t* counters,
+                      void* scratch, size_t scratch_bytes) {
   if (batch <= 0 || num_heads <= 0 || head_count <= 0 || head_begin < 0 || head_begin + head_count > num_heads)
     return fail(FO_ERR_INVALID_ARG, "fo_mask_compact: bad batch / head window");
   if (sbq <= 0 || sbkv <= 0) return fail(FO_ERR_INVALID_ARG, "fo_mask_compact: block sizes must be positive");
@@ -195,7 +197,6 @@ int fo_mask_compact(const uint8_t* sparse_info, int64_t sparse_info_bytes, const
   if (num_heads > 65535) return fail(FO_ERR_UNSUPPORTED, "fo_mask_compact: more than 65535 heads");
   if (scratch == nullptr || scratch_bytes < fo_mask_compact_scratch_bytes(n_cand, max_nkv) || !aligned16(scratch))
     return fail(FO_ERR_WORKSPACE, "fo_mask_compact: scratch too small or misaligned");
-  CompactArgs a;
   memset(&a, 0, sizeof(a));
   a.sparse_info = sparse_info;
   a.sparse_kv_info = sparse_kv_info;
@@ -230,19 +231,13 @@ int fo_mask_compact(const uint8_t* sparse_info, int64_t sparse_info_bytes, const
   a.kv_off = reinterpret_cast<long long*>(p);
   p += (n * 8 + 15) & ~static_cast<size_t>(15);
   a.hist = reinterpret_cast<int32_t*>(p);
-  const cudaError_t e = launch_attn_compact(a, static_cast<cudaStream_t>(stream));
-  count_launches(a.n_cand > 0 ? 3 : 0);
-  return e == cudaSuccess ? FO_OK : fail_cuda("fo_mask_compact", e);
+  return FO_OK;
 }
-
-size_t fo_attn_partial_bytes(int64_t partial_slots) {
-  return partial_slots > 0 ? static_cast<size_t>(partial_slots) * kPartialFloats * sizeof(float) : 0;
-}
-
-int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int32_t* kv_idx, const int32_t* order,
-                  const int32_t* counters, const int32_t* qo_indptr, const int32_t* kv_indptr, int64_t max_items,
-                  int32_t max_nkv, int32_t sbq, int32_t sbkv, int32_t min_items, int32_t num_streams, int32_t min_chunk, int64_t max_units,
-                  int64_t max_slots, int32_t* units, int32_t* unit_counters, int32_t* arrive, void* stream) {
+int make_unit_args(UnitArgs& a, const int32_t* items, const int32_t* kv_ptr, const int32_t* kv_idx, const int32_t* order,
+                   const int32_t* counters, const int32_t* qo_indptr, const int32_t* kv_indptr, int64_t
+                   max_items, int32_t max_nkv, int32_t sbq, int32_t sbkv, int32_t min_items, int32_t
+                   num_streams, int32_t min_chunk, int64_t max_units, int64_t max_slots, int32_t* units,
+                   int32_t* unit_counters, int32_t* arrive) {
   if (items == nullptr || kv_ptr == nullptr || kv_idx == nullptr || order == nullptr || counters == nullptr ||
       qo_indptr == nullptr || kv_indptr == nullptr || units == nullptr || unit_counters == nullptr ||
       (max_slots > 0 && arrive == nullptr))
@@ -251,7 +246,6 @@ int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int32_t* kv
       sbq <= 0 || sbkv <= 0)
     return fail(FO_ERR_INVALID_ARG, "fo_attn_units: max_units must cover max_items; sizes must be positive");
   if (!aligned16(units)) return fail(FO_ERR_INVALID_ARG, "fo_attn_units: units must be 16-byte aligned");
-  UnitArgs a;
   memset(&a, 0, sizeof(a));
   a.items = items;
   a.kv_ptr = kv_ptr;
@@ -272,9 +266,91 @@ int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int32_t* kv
   a.units = units;
   a.unit_counters = unit_counters;
   a.arrive = arrive;
+  return FO_OK;
+}
+}  // namespace
+
+int fo_mask_compact(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                    int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr,
+                    const int32_t* sparse_kv_info_indptr, const int32_t* qo_indptr, const int32_t* kv_indptr,
+                    int32_t batch, int32_t num_heads, int32_t head_begin, int32_t head_count, int32_t sbq,
+                    int32_t sbkv, int32_t is_full, int64_t n_cand, int32_t max_nkv, int64_t max_items,
+                    int64_t max_kept, int32_t* items, int32_t* kv_ptr, int32_t* kv_idx, int32_t* order,
+                    int32_t* counters, void* scratch, size_t scratch_bytes, void* stream) {
+  CompactArgs a;
+  const int rc = make_compact_args(a, sparse_info, sparse_info_bytes, sparse_kv_info, sparse_kv_info_bytes,
+                                   sparse_info_indptr, sparse_kv_info_indptr, qo_indptr, kv_indptr, batch,
+                                   num_heads, head_begin, head_count, sbq, sbkv, is_full, n_cand, max_nkv,
+                                   max_items, max_kept, items, kv_ptr, kv_idx, order, counters, scratch,
+                                   scratch_bytes);
+  if (rc != FO_OK) return rc;
+  const cudaError_t e = launch_attn_compact(a, static_cast<cudaStream_t>(stream));
+  count_launches(a.n_cand > 0 ? 3 : 0);
+  return e == cudaSuccess ? FO_OK : fail_cuda("fo_mask_compact", e);
+}
+
+size_t fo_attn_partial_bytes(int64_t partial_slots) {
+  return partial_slots > 0 ? static_cast<size_t>(partial_slots) * kPartialFloats * sizeof(float) : 0;
+}
+
+int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int32_t* kv_idx, const int32_t* order,
+                  const int32_t* counters, const int32_t* qo_indptr, const int32_t* kv_indptr, int64_t max_items,
+                  int32_t max_nkv, int32_t sbq, int32_t sbkv, int32_t min_items, int32_t num_streams, int32_t min_chunk, int64_t max_units,
+                  int64_t max_slots, int32_t* units, int32_t* unit_counters, int32_t* arrive, void* stream) {
+  UnitArgs a;
+  const int rc = make_unit_args(a, items, kv_ptr, kv_idx, order, counters, qo_indptr, kv_indptr, max_items,
+                                max_nkv, sbq, sbkv, min_items, num_streams, min_chunk, max_units, max_slots,
+                                units, unit_counters, arrive);
+  if (rc != FO_OK) return rc;
   const cudaError_t e = launch_attn_units(a, static_cast<cudaStream_t>(stream));
   count_launches(1);
   return e == cudaSuccess ? FO_OK : fail_cuda("fo_attn_units", e);
+}
+
+int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                  int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr, const int32_t* sparse_kv_info_indptr,
+                  int32_t is_full, void* zero_out, int64_t zero_token_bytes, int32_t zero_head_bytes,
+                  int64_t zero_total_bytes, const int32_t* qo_indptr, const int32_t* kv_indptr, int32_t batch,
+                  int32_t num_heads, int32_t head_begin, int32_t head_count, int32_t sbq, int32_t sbkv, int64_t n_cand,
+                  int32_t max_nkv, int64_t max_items, int64_t max_kept, int32_t* items, int32_t* kv_ptr,
+                  int32_t* kv_idx, int32_t* order, int32_t* counters, void* scratch, size_t scratch_bytes,
+                  int32_t min_items, int32_t num_streams, int32_t min_chunk, int64_t max_units, int64_t max_slots,
+                  int32_t* units, int32_t* unit_counters, int32_t* arrive, void* stream) {
+  CompactArgs a;
+  int rc = make_compact_args(a, sparse_info, sparse_info_bytes, sparse_kv_info, sparse_kv_info_bytes,
+                             sparse_info_indptr, sparse_kv_info_indptr, qo_indptr, kv_indptr, batch, num_heads,
+                             head_begin, head_count, sbq, sbkv, is_full, n_cand, max_nkv, max_items, max_kept,
+                             items, kv_ptr, kv_idx, order, counters, scratch, scratch_bytes);
+  if (rc != FO_OK) return rc;
+  UnitArgs u;
+  rc = make_unit_args(u, items, kv_ptr, kv_idx, order, counters, qo_indptr, kv_indptr, max_items, max_nkv, sbq,
+                      sbkv, min_items, num_streams, min_chunk, max_units, max_slots, units, unit_counters,
+                      arrive);
+  if (rc != FO_OK) return rc;
+  if (zero_out != nullptr && (!aligned16(zero_out) || zero_token_bytes <= 0 || zero_token_bytes % 16 != 0 ||
+                              zero_head_bytes <= 0 || zero_head_bytes % 16 != 0 || zero_total_bytes < 0))
+    return fail(FO_ERR_INVALID_ARG, "fo_attn_lists: zero_out and its strides must be multiples of 16 bytes");
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  ZeroArgs z;
+  z.out = static_cast<uint8_t*>(zero_out);
+  z.token_bytes = zero_token_bytes;
+  z.head_bytes = zero_head_bytes;
+  if (attn_lists_small_applies(a, u)) {
+    const cudaError_t e = launch_attn_lists_small(a, u, z, st);
+    count_launches(1);
+    return e == cudaSuccess ? FO_OK : fail_cuda("fo_attn_lists", e);
+  }
+  if (zero_out != nullptr && !is_full && zero_total_bytes > 0) {
+    const cudaError_t e = cudaMemsetAsync(zero_out, 0, static_cast<size_t>(zero_total_bytes), st);
+    if (e != cudaSuccess) return fail_cuda("fo_attn_lists (zero)", e);
+  }
+  cudaError_t e = launch_attn_compact(a, st);
+  count_launches(a.n_cand > 0 ? 3 : 0);
+  if (e == cudaSuccess) {
+    e = launch_attn_units(u, st);
+    count_launches(1);
+  }
+  return e == cudaSuccess ? FO_OK : fail_cuda("fo_attn_lists", e);
 }
 
 // ------------------------------------------------------------------------------------------ attention

@@ -73,6 +73,13 @@ struct UnitArgs {
   int32_t* arrive;           // [max_slots]
 };
 cudaError_t launch_attn_units(const UnitArgs& a, cudaStream_t stream);
+struct ZeroArgs {            // output rows of inactive q-blocks that the list builder zeroes (out null: none)
+  uint8_t* out;              // first byte of token 0, first head of the mask window
+  int64_t token_bytes;       // bytes between tokens
+  int head_bytes;            // contiguous bytes of one token that belong to one mask head, a multiple of 16
+};
+bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u);
+cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream);
 cudaError_t launch_cast_fp8(const void* src, int64_t n, int e5m2, int is_bf16, void* dst, int sm_count, cudaStream_t stream);
 cudaError_t launch_gemm_q_tiles(const GemmListArgs& a, cudaStream_t stream);
 cudaError_t launch_gemm_o_rows(const GemmListArgs& a, cudaStream_t stream);

@@ -132,6 +132,22 @@ FO_API int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int3
                          int64_t max_items, int32_t max_nkv, int32_t sbq, int32_t sbkv, int32_t min_items,
                          int32_t num_streams, int32_t min_chunk, int64_t max_units, int64_t max_slots, int32_t* units,
                          int32_t* unit_counters, int32_t* arrive, void* stream);
+/* fo_mask_compact followed by fo_attn_units (same arguments, same lists) in one call; a mask of at most 4096 candidates
+ * (and 2^18 kv bits, uncut lists) takes a single launch. With zero_out != NULL the output rows of the q-blocks that are
+ * not active are set to zero on the way: zero_out is the output at token 0 and the first head of the window,
+ * zero_token_bytes the distance of two tokens, zero_head_bytes the contiguous bytes of a token that belong to one mask
+ * head (both multiples of 16), zero_total_bytes the size of the whole contiguous output (larger masks zero all of it;
+ * nothing is zeroed when is_full != 0: every block is active then). */
+FO_API int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                         int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr,
+                         const int32_t* sparse_kv_info_indptr, int32_t is_full, void* zero_out, int64_t zero_token_bytes,
+                         int32_t zero_head_bytes, int64_t zero_total_bytes, const int32_t* qo_indptr,
+                         const int32_t* kv_indptr, int32_t batch, int32_t num_heads, int32_t head_begin,
+                         int32_t head_count, int32_t sbq, int32_t sbkv, int64_t n_cand, int32_t max_nkv,
+                         int64_t max_items, int64_t max_kept, int32_t* items, int32_t* kv_ptr, int32_t* kv_idx,
+                         int32_t* order, int32_t* counters, void* scratch, size_t scratch_bytes, int32_t min_items,
+                         int32_t num_streams, int32_t min_chunk, int64_t max_units, int64_t max_slots, int32_t* units,
+                         int32_t* unit_counters, int32_t* arrive, void* stream);
 /* Bytes of partial-result scratch for `partial_slots` slots (fp32 O of a 128-row q-block plus row maxima and sums). */
 FO_API size_t fo_attn_partial_bytes(int64_t partial_slots);
 

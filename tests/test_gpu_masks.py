@@ -126,6 +126,68 @@ def test_attention_compaction_random_ragged_cases(cuda_device):
         _assert_lists_equal(got, ref)
 
 
+# (request lengths q, kv, mask heads, head window, density): one candidate; a remainder of the 16 candidates per CTA;
+# ragged with a request of no rows; a window; kv rows of more than one 64-bit word; more (group, length) buckets than
+# lengths are ordered for (single heads, q-blocks ascending); the largest candidate count and the first one past it
+@pytest.mark.parametrize("lens_q,lens_kv,H,hb,hc,density", [
+    ([100], [77], 1, 0, 1, 1.0), ([17 * 128], [300], 1, 0, 1, 0.5), ([300, 0, 1000, 77], [256, 128, 1300, 129], 5, 0, 5, 0.4),
+    ([4608, 4608], [4608, 4608], 24, 6, 3, 0.5), ([700], [64 * 128 + 1], 3, 0, 3, 0.3), ([512], [102400], 40, 0, 40, 0.4),
+    ([128 * 128], [512], 32, 0, 32, 0.5), ([128 * 128 + 1], [512], 32, 0, 32, 0.5)])
+@pytest.mark.parametrize("is_full", [False, True])
+def test_attention_lists_in_one_call_match_the_oracle(cuda_device, lens_q, lens_kv, H, hb, hc, density, is_full):
+    rng = np.random.default_rng(len(lens_q) * 100 + H)
+    qa = [(rng.random((-(-a // 128), H)) < density).astype(np.uint8) for a in lens_q]
+    kk = [(rng.random((-(-a // 128), H, -(-b // 128))) < density).astype(np.uint8) for a, b in zip(lens_q, lens_kv)]
+    qo = np.concatenate([[0], np.cumsum(lens_q)]); kv = np.concatenate([[0], np.cumsum(lens_kv)])
+    m = wl.pack_masks(qa, kk)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device))
+    w.plan(dev(qo.astype(np.int32), cuda_device), dev(kv.astype(np.int32), cuda_device), hc, hc, 128,
+           q_data_type=torch.bfloat16, mask_num_heads=H, mask_head_begin=hb)
+    w.build_work_lists(*masks_to_device(m, cuda_device), is_full=is_full)
+    torch.cuda.synchronize()
+    got = w.work_lists()
+    ref = om.compact(m.sparse_info, m.sparse_kv_info, m.info_indptr, m.kv_info_indptr, qo, kv, H, 128, 128, hb, hc,
+                     is_full=is_full)
+    _assert_lists_equal(got, ref)
+    assert got["n_units"] == got["n_items"] and got["unit_status"] == 0
+    for pos, it in enumerate(got["order"]):   # one record per item, in processing order
+        b, h, qb, n = (int(x) for x in got["items"][it])
+        ends = n > 0 and lens_kv[b] % 128 != 0 and int(got["kv_idx"][got["kv_indptr"][it] + n - 1]) == lens_kv[b] // 128
+        valid = min(128, lens_q[b] - 128 * qb) | ((lens_kv[b] % 128) << 16 if ends else 0)
+        want = [n, int(got["kv_indptr"][it]), h | b << 16, int(qo[b]) + 128 * qb, valid, int(kv[b]),
+                128 * qb + lens_kv[b] - lens_q[b], -65535]
+        assert got["units"][pos].tolist() == want
+
+
+@pytest.mark.parametrize("H,group,D,lens", [(2, 1, 64, [300]), (4, 2, 128, [65, 700]), (24, 1, 128, [128 * 180])])
+def test_allocated_output_is_zero_in_skipped_blocks(cuda_device, H, group, D, lens):
+    """An output that run() allocates itself, over memory that held other values; the last case is past the one-launch
+    builder's size."""
+    rng = np.random.default_rng(3)
+    toks = 128 // group
+    qa = [(rng.random((-(-n // toks), H)) < 0.5).astype(np.uint8) for n in lens]
+    kk = [(rng.random((-(-n // toks), H, -(-n // 128))) < 0.1).astype(np.uint8) for n in lens]
+    m = wl.pack_masks(qa, kk)
+    ip = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=cuda_device)
+    total = sum(lens)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device))
+    w.plan(ip, ip, H * group, H, D, q_data_type=torch.bfloat16)
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    q = torch.randn(total, H * group, D, generator=g, device=cuda_device).bfloat16()
+    k, v = (torch.randn(total, H, D, generator=g, device=cuda_device).bfloat16() for _ in range(2))
+    masks = masks_to_device(m, cuda_device)
+    junk = torch.full_like(q, 7.0)
+    del junk
+    got = w.run(q, k, v, *masks)
+    want = w.run(q, k, v, *masks, out=torch.zeros_like(q))
+    w.check_status()
+    on = torch.cat([dev(a, cuda_device).bool().repeat_interleave(toks, 0)[:n] for a, n in zip(qa, lens)])
+    off = ~on.repeat_interleave(group, 1)
+    assert not got[off].any() and not want[off].any()
+    # the order in which a q-block's row sums are added depends on the CTA that draws it: one bf16 step of values below 4
+    assert (got.float() - want.float()).abs().max() <= 2 ** -6
+
+
 def test_gemm_worklists_bit_exact(cuda_device):
     lib = _native.load()
     B, H, nq = 2, 24, 36
