@@ -29,6 +29,8 @@ SIGNATURES = {
     "fo_select_blocks_scratch_bytes": (c_size_t, [c_int32, c_int32]),
     "fo_select_blocks": (c_int32, [_P, c_int32, c_int32, c_int32, c_int32, _P, _P, c_int32, _P, c_int64, _P, c_int64,
                                    _P, _P, _P, c_size_t, _P]),
+    "fo_select_blocks_uniform": (c_int32, [_P, c_int32, c_int32, c_int32, c_int32, c_float, c_float, c_int32, _P, c_int64,
+                                           _P, c_int64, _P, _P, _P, c_size_t, _P]),
     "fo_abi_version": (c_int32, []),
     "fo_launch_count": (ctypes.c_longlong, []),
     "fo_reduce_rows": (c_int32, [c_int32, _P, c_int64, _P, c_int64, _P, c_int64, c_int64, c_int64, c_int32, _P]),

@@ -831,15 +831,18 @@ size_t fo_select_blocks_scratch_bytes(int32_t batch, int32_t num_blocks) {
   return ((n * 4 + 15) & ~static_cast<size_t>(15)) + ((n + 15) & ~static_cast<size_t>(15)) + 16;
 }
 
-int32_t fo_select_blocks(const float* pooled_score, int32_t batch, int32_t num_heads, int32_t num_blocks,
-                         int32_t num_text_blocks, const float* q_threshold, const float* kv_threshold,
+namespace {
+// Thresholds: device arrays, or (both null) one value each.
+int select_blocks_impl(const float* pooled_score, int32_t batch, int32_t num_heads, int32_t num_blocks,
+                         int32_t num_text_blocks, const float* q_threshold, const float* kv_threshold, float q_all,
+                         float kv_all,
                          int32_t zero_inactive, uint8_t* sparse_info, int64_t sparse_info_bytes,
                          uint8_t* sparse_kv_info, int64_t sparse_kv_info_bytes, int32_t* info_indptr,
                          int32_t* kv_info_indptr, void* scratch, size_t scratch_bytes, void* stream) {
   if (batch <= 0 || num_heads <= 0 || num_blocks <= 0 || num_text_blocks < 0 || num_text_blocks > num_blocks)
     return fail(FO_ERR_INVALID_ARG, "fo_select_blocks: bad sizes");
   if (num_blocks > 2048) return fail(FO_ERR_UNSUPPORTED, "fo_select_blocks: at most 2048 blocks per request");
-  if (pooled_score == nullptr || q_threshold == nullptr || kv_threshold == nullptr || sparse_info == nullptr ||
+  if (pooled_score == nullptr || sparse_info == nullptr ||
       sparse_kv_info == nullptr || info_indptr == nullptr || kv_info_indptr == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_select_blocks: null pointer");
   SelectArgs a;
@@ -858,6 +861,8 @@ int32_t fo_select_blocks(const float* pooled_score, int32_t batch, int32_t num_h
   a.score = pooled_score;
   a.q_thr = q_threshold;
   a.kv_thr = kv_threshold;
+  a.q_thr_all = q_all;
+  a.kv_thr_all = kv_all;
   a.batch = batch;
   a.heads = num_heads;
   a.n = num_blocks;
@@ -867,12 +872,32 @@ int32_t fo_select_blocks(const float* pooled_score, int32_t batch, int32_t num_h
   a.sparse_kv_info = sparse_kv_info;
   a.info_indptr = info_indptr;
   a.kv_info_indptr = kv_info_indptr;
-  const size_t n = static_cast<size_t>(batch) * static_cast<size_t>(num_blocks);
-  a.t2i = static_cast<float*>(scratch);
-  a.q_keep = static_cast<uint8_t*>(scratch) + ((n * 4 + 15) & ~static_cast<size_t>(15));
+  a.q_keep = static_cast<uint8_t*>(scratch);
   const cudaError_t e = launch_select_blocks(a, static_cast<cudaStream_t>(stream));
-  count_launches(3);
+  count_launches(2);
   return e == cudaSuccess ? FO_OK : fail_cuda("fo_select_blocks", e);
+}
+}  // namespace
+
+int32_t fo_select_blocks(const float* pooled_score, int32_t batch, int32_t num_heads, int32_t num_blocks,
+                         int32_t num_text_blocks, const float* q_threshold, const float* kv_threshold,
+                         int32_t zero_inactive, uint8_t* sparse_info, int64_t sparse_info_bytes,
+                         uint8_t* sparse_kv_info, int64_t sparse_kv_info_bytes, int32_t* info_indptr,
+                         int32_t* kv_info_indptr, void* scratch, size_t scratch_bytes, void* stream) {
+  if (q_threshold == nullptr || kv_threshold == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_select_blocks: null pointer");
+  return select_blocks_impl(pooled_score, batch, num_heads, num_blocks, num_text_blocks, q_threshold, kv_threshold, 0.f, 0.f,
+                            zero_inactive, sparse_info, sparse_info_bytes, sparse_kv_info, sparse_kv_info_bytes, info_indptr,
+                            kv_info_indptr, scratch, scratch_bytes, stream);
+}
+
+int32_t fo_select_blocks_uniform(const float* pooled_score, int32_t batch, int32_t num_heads, int32_t num_blocks,
+                                 int32_t num_text_blocks, float q_threshold, float kv_threshold, int32_t zero_inactive,
+                                 uint8_t* sparse_info, int64_t sparse_info_bytes, uint8_t* sparse_kv_info,
+                                 int64_t sparse_kv_info_bytes, int32_t* info_indptr, int32_t* kv_info_indptr, void* scratch,
+                                 size_t scratch_bytes, void* stream) {
+  return select_blocks_impl(pooled_score, batch, num_heads, num_blocks, num_text_blocks, nullptr, nullptr, q_threshold,
+                            kv_threshold, zero_inactive, sparse_info, sparse_info_bytes, sparse_kv_info, sparse_kv_info_bytes,
+                            info_indptr, kv_info_indptr, scratch, scratch_bytes, stream);
 }
 
 int32_t fo_strided_gather(int32_t n_src, const void* const* src, const int64_t* src_row_stride_bytes,

@@ -117,17 +117,17 @@ cudaError_t launch_gemm_tall(const GemmArgs& a, int max_ctas, cudaStream_t strea
 // ------------------------------------------------------------------ block selection
 struct SelectArgs {
   const float* score;        // [batch, heads, n, n]
-  const float* q_thr;        // [batch]
-  const float* kv_thr;       // [heads]
+  const float* q_thr;        // [batch], or null: q_thr_all for every request
+  const float* kv_thr;       // [heads], or null: kv_thr_all for every head
+  float q_thr_all, kv_thr_all;
   int batch, heads, n, t2t, zero_inactive;
   int64_t info_seg_bytes;    // ceil(n * heads / 8)
   int64_t kv_seg_bytes;      // ceil(n * heads * n / 8)
-  int64_t kv_words;          // 32-bit words of sparse_kv_info that are zeroed first
+  int64_t kv_words;          // 32-bit words of sparse_kv_info (zeroed by the first launch)
   uint8_t* sparse_info;
   uint8_t* sparse_kv_info;
   int32_t* info_indptr;      // [batch + 1]
   int32_t* kv_info_indptr;   // [batch + 1]
-  float* t2i;                // scratch [batch, n]
   uint8_t* q_keep;           // scratch [batch, n]
 };
 cudaError_t launch_select_blocks(const SelectArgs& a, cudaStream_t stream);

@@ -42,8 +42,7 @@ def select_blocks(pooled_score: torch.Tensor, num_text_blocks: int, q_threshold:
         raise ValueError("num_text_blocks out of range")
     dev = s.device
     lib = _native.load()
-    qthr = _threshold(q_threshold, B, dev, "q_threshold")
-    kthr = _threshold(kv_threshold, H, dev, "kv_threshold")
+    uniform = not isinstance(q_threshold, torch.Tensor) and not isinstance(kv_threshold, torch.Tensor)
     info_seg = (n * H + 7) // 8
     kv_seg = (n * H * n + 7) // 8
     kv_alloc = (B * kv_seg + 3) // 4 * 4
@@ -52,9 +51,14 @@ def select_blocks(pooled_score: torch.Tensor, num_text_blocks: int, q_threshold:
     ip = torch.empty(B + 1, dtype=torch.int32, device=dev)
     kp = torch.empty(B + 1, dtype=torch.int32, device=dev)
     scratch = torch.empty(lib.fo_select_blocks_scratch_bytes(B, n), dtype=torch.uint8, device=dev)
-    rc = lib.fo_select_blocks(_native.ptr(s), B, H, n, int(num_text_blocks), _native.ptr(qthr), _native.ptr(kthr),
-                              int(bool(zero_inactive)), _native.ptr(sparse_info), sparse_info.numel(),
-                              _native.ptr(sparse_kv), sparse_kv.numel(), _native.ptr(ip), _native.ptr(kp),
-                              _native.ptr(scratch), scratch.numel(), _native.current_stream(dev))
+    if uniform:   # passed by value: no threshold arrays to fill
+        qthr, kthr, op = float(q_threshold), float(kv_threshold), lib.fo_select_blocks_uniform
+        thr = (qthr, kthr)
+    else:
+        qthr, kthr = _threshold(q_threshold, B, dev, "q_threshold"), _threshold(kv_threshold, H, dev, "kv_threshold")
+        thr, op = (_native.ptr(qthr), _native.ptr(kthr)), lib.fo_select_blocks
+    rc = op(_native.ptr(s), B, H, n, int(num_text_blocks), *thr, int(bool(zero_inactive)), _native.ptr(sparse_info),
+            sparse_info.numel(), _native.ptr(sparse_kv), sparse_kv.numel(), _native.ptr(ip), _native.ptr(kp),
+            _native.ptr(scratch), scratch.numel(), _native.current_stream(dev))
     _native.check(rc, "select_blocks")
     return sparse_info, sparse_kv[:B * kv_seg], ip, kp

@@ -331,6 +331,13 @@ FO_API int32_t fo_select_blocks(const float* pooled_score, int32_t batch, int32_
                                 uint8_t* sparse_kv_info, int64_t sparse_kv_info_bytes, int32_t* info_indptr,
                                 int32_t* kv_info_indptr, void* scratch, size_t scratch_bytes, void* stream);
 
+/* The same with one threshold for all requests and one for all heads, given by value. */
+FO_API int32_t fo_select_blocks_uniform(const float* pooled_score, int32_t batch, int32_t num_heads, int32_t num_blocks,
+                                        int32_t num_text_blocks, float q_threshold, float kv_threshold,
+                                        int32_t zero_inactive, uint8_t* sparse_info, int64_t sparse_info_bytes,
+                                        uint8_t* sparse_kv_info, int64_t sparse_kv_info_bytes, int32_t* info_indptr,
+                                        int32_t* kv_info_indptr, void* scratch, size_t scratch_bytes, void* stream);
+
 /* ---- strided row gather (sequence-parallel exchange) -----------------------------------------------
  * No counterpart in the reference (it has no multi-GPU code). For source i < n_src (at most 16), copies
  * n_rows[i] rows of row_bytes bytes from src[i] (rows src_row_stride_bytes[i] apart) to dst[i] (rows

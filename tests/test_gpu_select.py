@@ -43,6 +43,31 @@ def test_ties_and_extremes(cuda_device):
         assert np.array_equal(info, rinfo) and np.array_equal(kv, rkv)
 
 
+# row lengths at the edges of the per-lane entry counts (4, 20 and 64), one threshold for all; scores that spread,
+# that differ by less than a float step of their mass, that take three values (more than 32 equal masses), and with
+# infinities of both signs
+@pytest.mark.parametrize("n", [1, 2, 31, 128, 129, 640, 641])
+@pytest.mark.parametrize("kind", ["normal", "flat", "three", "inf"])
+@pytest.mark.parametrize("thr", [0.0, 0.3, 0.97])
+def test_one_threshold_for_all(cuda_device, n, kind, thr):
+    rng = np.random.default_rng(n)
+    H, t2t = (2 if n < 600 else 1), min(2, n)
+    s = rng.standard_normal((1, H, n, n)).astype(np.float32)
+    if kind == "flat":
+        s *= np.float32(1e-6)
+    elif kind == "three":
+        s = rng.integers(0, 3, s.shape).astype(np.float32)
+    elif kind == "inf":
+        s[rng.random(s.shape) < 0.5] = -np.inf
+        s[:, :, :, 0] = np.where(s[:, :, :, 0] == -np.inf, 0, s[:, :, :, 0])
+    info, kv, ip, kp = _run(s, t2t, thr, thr, True, cuda_device)
+    with np.errstate(invalid="ignore"):
+        qa, kk = osel.select_blocks(s, t2t, thr, thr)
+    rinfo, rkv, rip, rkp = osel.pack_selection(qa, kk)
+    assert np.array_equal(ip, rip) and np.array_equal(kp, rkp)
+    assert np.array_equal(info, rinfo) and np.array_equal(kv, rkv)
+
+
 def test_feeds_the_hot_path(cuda_device):
     """The emitted tensors go straight into the attention wrapper; the result equals the run on masks packed
     from the CPU statement."""
