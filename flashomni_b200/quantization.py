@@ -45,6 +45,25 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
     including its one host synchronisation to size the output)."""
     little = _little(bitorder)
     _native.require_cuda(x)
+    n_seg = len(indptr) - 1
+    # The usual call: the byte indptr, its total and the packed bytes in one launch and one wait. The output is allocated
+    # for the most that these segments can need and shortened; anything else takes the general path below.
+    if (indptr.dim() == 1 and 1 <= n_seg <= 1024 and indptr.dtype in (torch.int32, torch.int64)
+            and indptr.device == x.device and 0 < x.numel() < 1 << 33):
+        device = x.device
+        xb, ip = _as_bytes(x), indptr.contiguous()
+        capacity = (xb.numel() + 7 * n_seg) // 8
+        y = torch.empty(capacity, dtype=torch.uint8, device=device)
+        indptr_new = torch.empty(n_seg + 1, dtype=torch.int32, device=device)
+        total = torch.empty(1, dtype=torch.int64, pin_memory=True)
+        with torch.cuda.device(device):
+            rc = _native.load().fo_segment_packbits_sized(
+                xb.data_ptr(), ip.data_ptr(), int(ip.dtype == torch.int64), n_seg, capacity, little, y.data_ptr(),
+                indptr_new.data_ptr(), total.data_ptr(), _native.current_stream(device))
+        _native.check(rc, "segment_packbits")
+        nbytes = int(total[0])
+        if nbytes >= 0:
+            return y.narrow(0, 0, nbytes), indptr_new
     seglen = indptr[1:] - indptr[:-1]
     packed_len = (seglen + 7) // 8
     indptr_new = torch.zeros(len(indptr), dtype=indptr.dtype, device=indptr.device)

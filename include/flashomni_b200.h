@@ -74,6 +74,13 @@ FO_API int fo_packbits(const uint8_t* x, int64_t n, int little, uint8_t* y, void
  * as known to the host (flashomni/quantization.py:148-152). */
 FO_API int fo_segment_packbits(const uint8_t* x, const int32_t* indptr, const int32_t* new_indptr,
                         int32_t num_segments, int64_t out_bytes, int little, uint8_t* y, void* stream);
+/* The same from the element indptr alone (int32, or int64 with indptr_is_64), at most 1024 segments: also writes the
+ * byte indptr (int32 [num_segments + 1]) and the number of packed bytes, and waits for the stream so that the host can
+ * read it. total_bytes is pinned host memory. y has room for `capacity` bytes; a decreasing or negative indptr, or one
+ * that needs more, gives total_bytes = -1 and packs nothing. */
+FO_API int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                                     int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
+                                     int64_t* total_bytes, void* stream);
 
 /* ---- attention mask compaction (new step; no counterpart op in the reference, which re-reads
  * the bits in the kernel: prefill.cuh:1284-1294,1380-1460) -------------------------------------

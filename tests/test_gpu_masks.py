@@ -46,6 +46,23 @@ def test_segment_packbits_ragged(cuda_device, order):
     assert np.array_equal(y2.cpu().numpy(), ry)
 
 
+# one empty segment; an indptr that starts past zero; the most segments of the one-launch path and one more;
+# more inputs than the segments cover
+@pytest.mark.parametrize("lens,start,extra", [([0], 0, 5), ([3, 40], 17, 0), ([13] * 1024, 0, 3), ([13] * 1025, 0, 0),
+                                              ([0, 31, 32, 33, 0, 257], 1, 300), ([70001], 0, 0)])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("indptr_device", ["cuda", "cpu"])
+def test_segment_packbits_sizes(cuda_device, lens, start, extra, dtype, indptr_device):
+    indptr = start + np.concatenate([[0], np.cumsum(lens)])
+    rng = np.random.default_rng(len(lens) + start)
+    x = rng.integers(0, 2, int(indptr[-1]) + extra).astype(np.uint8)
+    ip = torch.from_numpy(indptr).to(dtype)
+    y, nip = fo.segment_packbits(dev(x, cuda_device), ip.to(cuda_device) if indptr_device == "cuda" else ip, bitorder="little")
+    ry, rip = om.segment_packbits(x[start:], indptr - start, "little")
+    assert nip.dtype == torch.int32 and nip.device == y.device and y.is_contiguous()
+    assert np.array_equal(nip.cpu().numpy(), rip) and np.array_equal(y.cpu().numpy(), ry)
+
+
 def _compact_gpu(device, m, qo, kv, H, head_begin=0, head_count=None, is_full=False):
     hc = H - head_begin if head_count is None else head_count
     w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=device))
