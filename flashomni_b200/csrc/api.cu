@@ -428,7 +428,6 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     if (r == 0) r = encode_tmap_16bit(&a.tmap_k, k, 3, kd, ks, box);
     if (r == 0) r = encode_tmap_16bit(&a.tmap_v, v, 3, kd, vs, box);
     const uint64_t os[3] = {0, static_cast<uint64_t>(o_stride_h) * 2, static_cast<uint64_t>(o_stride_n) * 2};
-    if (r == 0) r = encode_tmap_16bit(&a.tmap_o, o, 3, qd, os, qbox);  // stores of 64 columns x 128 rows
     const uint32_t obox16[3] = {32, group, 16 / group};
     if (r == 0) r = encode_tmap_16bit(&a.tmap_o16, o, 3, qd, os, obox16, false);
     if (r != 0) {

@@ -1,5 +1,4 @@
-// Block-sparse prefill attention on tcgen05 / TMEM / TMA, driven by compacted work lists: the kernel for launches
-// with MANY work units (several per SM). Launches with few units take attention_streams.cu instead.
+// Block-sparse prefill attention on tcgen05 / TMEM / TMA, driven by compacted work lists.
 //
 // What it computes (reference: include/flashomni/attention/prefill.cuh:1203-1531): for every work
 // item (b, h, qb) -- an active 128-row q-block of one head -- and its ascending list of kept
@@ -25,11 +24,15 @@
 // reduces and hands over. S is read twice (row maximum, then exponentials) instead of being held in
 // registers across the exchanges; the two halves of a row meet through shared memory; the running
 // maximum passes from block to block through shared memory (m_pub / m_ready); each thread keeps its
-// own partial row sum, and the four of a row are merged, with the output, in the epilogue (whole
+// own partial row sum, and the four of a row are merged, with the output, by the epilogue warps (whole
 // q-blocks leave through a per-warp staging area and TMA box stores).
-// Warps: 0-7 softmax group 0, 8-15 softmax group 1 (TMEM lane = q row; `setmaxnreg` gives them 112
+// Warps: 0-7 softmax group 0, 8-15 softmax group 1 (TMEM lane = q row; `setmaxnreg` gives them 104
 // registers), 16 TMA producer of Q (double-buffered) and K (two-slot FIFO of 32 KB tiles) and drawer of
-// work-list positions, 17 QK issuer, 18 PV issuer, 19 TMA producer of V (its own two-slot FIFO).
+// work-list positions, 17 QK issuer, 18 PV issuer, 19 TMA producer of V (its own two-slot FIFO), 20-23 epilogue.
+// Registers: a softmax thread holds 64 columns of S; a spill inside the block loop goes through L2 (213 KB of shared
+// memory leave hardly any L1) and costs far more than the instruction: the same code with 104 and 96 instead of 112
+// registers (112 and 144 spilled bytes) took 278 and 314 us instead of 246 on the 4608-token layer, all blocks kept.
+// With the warp index read through a shuffle the role state lives in uniform registers and the block loop fits in 104.
 // Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
 
@@ -55,18 +58,20 @@ constexpr int kWarpQK = kSoftmaxWarps + 1;      // issues S = Q K^T
 constexpr int kWarpPV = kSoftmaxWarps + 2;      // issues O += P V
 constexpr int kWarpProducerV = kSoftmaxWarps + 3;
 constexpr int kWarpMma = kWarpQK;               // owner of the TMEM allocation
-constexpr int kThreads = (kSoftmaxWarps + 4) * 32;  // 640: four softmax warpgroups and the producer / issuer warpgroup
-constexpr int kRegsSoftmax = 112, kRegsOther = 32;  // register split between the warpgroups (setmaxnreg)
+constexpr int kWarpEpilogue = kSoftmaxWarps + 4;  // first of the four epilogue warps (TMEM lane quadrant = warp % 4)
+constexpr int kEpilogueWarps = 4;
+constexpr int kThreads = (kSoftmaxWarps + 4 + kEpilogueWarps) * 32;  // 768: four softmax warpgroups, producers / issuers, epilogue
+constexpr int kRegsSoftmax = 104, kRegsOther = 32, kRegsEpilogue = 32;  // register split between the warpgroups (setmaxnreg)
 // setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with (threads x the
 // per-thread count the compiler settles on for this block size): a split that asks for more never returns.
 constexpr int kRegsAtLaunch = (65536 / kThreads) / 8 * 8;
-static_assert(kSoftmaxWarps * 32 * kRegsSoftmax + (kThreads - kSoftmaxWarps * 32) * kRegsOther <= kThreads * kRegsAtLaunch,
+static_assert(kSoftmaxWarps * 32 * kRegsSoftmax + 4 * 32 * kRegsOther + kEpilogueWarps * 32 * kRegsEpilogue <= kThreads * kRegsAtLaunch,
               "register split exceeds the CTA's register pool");
 constexpr int kTmemCols = 512;
 constexpr uint32_t kColS = 0, kColO = 256, kColP = 384;
 constexpr int kRotStep = FO_ROT_STEP;       // q-block qb starts its kv list at entry (qb * kRotStep) mod length
 constexpr int kItemQ = 8;                   // entries of the item queue
-constexpr int kItemReaders = kSoftmaxWarps + 3;  // softmax warps, V producer, the two MMA issuers
+constexpr int kItemReaders = kSoftmaxWarps + 3 + kEpilogueWarps;  // softmax warps, V producer, the two MMA issuers, epilogue warps
 constexpr float kRescaleThreshold = 8.0f;  // lazy rescale: keep the old max while exp2 stays <= 2^8
 
 struct Tail {
@@ -76,9 +81,10 @@ struct Tail {
   uint64_t p_full[2], pv_done[2];  // indexed by block parity, so that no waiter can fall two phases behind
   uint64_t m_ready[2];             // running maximum after a block of this parity has been published
   uint64_t stats_ready[2];         // indexed by item parity: both groups have published (m, l) of the item
+  uint64_t stats_free[2];          // indexed by item parity: the epilogue has read them
   uint64_t o_full, o_free;
   uint64_t iq_full[kItemQ], iq_empty[kItemQ];  // item queue: the K producer draws work-list positions for the CTA
-  uint64_t ep_bar;                 // all softmax warps, in the epilogue of a part of a split item
+  uint64_t ep_bar;                 // the epilogue warps, in the epilogue of a part of a split item
   int item_q[kItemQ];
   uint32_t tmem_base;
   int abort_flag;
@@ -92,8 +98,9 @@ struct Tail {
 
 
 
-constexpr int kOutStageBytes = 16 * 64;  // per softmax warp: 16 rows x 32 output columns
-constexpr int kSmemBytes = (kQBufs + kRing) * kTileBytes + kSoftmaxWarps * kOutStageBytes + 1024 +
+constexpr int kOutSlabBytes = 32 * 64;            // 32 rows x 32 output columns
+constexpr int kOutStageBytes = 2 * kOutSlabBytes;  // per epilogue warp: two of them
+constexpr int kSmemBytes = (kQBufs + kRing) * kTileBytes + kEpilogueWarps * kOutStageBytes + 1024 +
                            static_cast<int>(sizeof(Tail));
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
@@ -324,17 +331,16 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
   constexpr int kTB = kWide ? 2 * kTileBytes : kTileBytes;                               // bytes of a tile slot
   constexpr int kQB = kWide ? 1 : kQBufs, kRK = kWide ? 1 : kRingK, kRV = kWide ? 1 : kRingV;   // slots of Q, K, V
   static_assert((kQB + kRK + kRV) * kTB <= (kQBufs + kRing) * kTileBytes, "tile slots");
-  constexpr int kOW = kWide ? 64 : 32;       // columns of O per softmax thread in the epilogue
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* smem_q = smem;                           // kQBufs tiles
   uint8_t* smem_ring = smem + kQB * kTB;  // K slots, then V slots
-  uint8_t* smem_ostage = smem + (kQBufs + kRing) * kTileBytes;  // output staging of the softmax warps
-  Tail* tail = reinterpret_cast<Tail*>(smem_ostage + kSoftmaxWarps * kOutStageBytes);
+  uint8_t* smem_ostage = smem + (kQBufs + kRing) * kTileBytes;  // output staging of the epilogue warps
+  Tail* tail = reinterpret_cast<Tail*>(smem_ostage + kEpilogueWarps * kOutStageBytes);
   volatile int* abort_flag = &tail->abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform: role state in uniform registers
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -350,10 +356,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
       mbar_init(&tail->pv_done[i], 1);
       mbar_init(&tail->m_ready[i], kGroupWarps);
       mbar_init(&tail->stats_ready[i], kSoftmaxWarps);
+      mbar_init(&tail->stats_free[i], kEpilogueWarps);
     }
     mbar_init(&tail->o_full, 1);
-    mbar_init(&tail->o_free, kSoftmaxWarps);
-    mbar_init(&tail->ep_bar, kSoftmaxWarps);
+    mbar_init(&tail->o_free, kEpilogueWarps);
+    mbar_init(&tail->ep_bar, kEpilogueWarps);
     for (int i = 0; i < kItemQ; ++i) { mbar_init(&tail->iq_full[i], 1); mbar_init(&tail->iq_empty[i], kItemReaders); }
     for (int i = 0; i < 8; ++i) mbar_init(&tail->pair_bar[i >> 2][i & 3], 2);
     tail->abort_flag = 0;
@@ -383,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
   auto ignore_empty = [](int, int, int) {};
 
   // The softmax warps take the registers that the producer / issuer warpgroup does not need.
-  if (warp >= kSoftmaxWarps) {
+  if (warp >= kSoftmaxWarps && warp < kWarpEpilogue) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
   if (warp == kWarpProducer) {
     // ------------------------------------------------------------------ TMA producer of Q and K tiles
@@ -541,13 +548,200 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
       }
     }
   }
+  } else if (warp >= kWarpEpilogue) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+    // ------------------------------------------------------------------ epilogue warps: O / l to global memory
+    // One thread per q row, 16 columns at a time. O has ONE accumulator, so the next unit's first PV waits until it has
+    // been read out: that is on the pipeline's critical path and is all these warps do. (The softmax warps used to do it
+    // after their next block; the first PV of a unit then started about 3 600 clocks after its P was ready.) 4608 tokens,
+    // 24 heads of 128 on a B200: 113.0 -> 108.3 us at density 0.5, 243.5 -> 230.4 us with all blocks. Chunks of 16 columns
+    // because two of them in registers would take them from the softmax warps (32 columns and 64 / 96 registers: 110.0 and
+    // 236.9 us; 8 columns: 111.1 and 234.4 us).
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t tmem_o = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kColO;
+    uint8_t* stg = smem_ostage + (warp - kWarpEpilogue) * kOutStageBytes;
+    const int grp = a.group_size;
+    uint32_t slab = 0;      // slabs handed to TMA stores so far (selects the staging half)
+    uint32_t item = 0;
+    [[maybe_unused]] uint32_t ep_phase = 0;
+    // bounded barrier of the epilogue warps (parts of split items)
+    [[maybe_unused]] auto ep_sync = [&]() -> bool {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->ep_bar);
+      const bool r = __all_sync(0xffffffffu, mbar_wait(&tail->ep_bar, ep_phase, abort_flag) ? 1 : 0) != 0;
+      ep_phase ^= 1u;
+      return r;
+    };
+    ItemRead<true> src;
+    src.init(tail, abort_flag);
+    while (true) {
+      const int pos = src.next();
+      if (pos < 0) break;
+      const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
+      const int4 u0 = up[0], u1 = up[1];
+      const int q_row0 = u0.w, q_valid = u1.x & 0xffff, h = (u0.z & 0xffff) - a.head_begin;
+      // Row r of a tile is token q_row0 + r / group, q head h * group + r % group (group = 1: the row itself).
+      const bool row_ok = row < q_valid * grp;
+      const int64_t grow = static_cast<int64_t>(q_row0) + row / grp;
+      const int hq = h * grp + row % grp;
+      uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + grow * a.o_stride_n + static_cast<int64_t>(hq) * a.o_stride_h;
+      float* lse = a.lse != nullptr ? a.lse + grow * a.lse_stride_n + hq : nullptr;
+      if (u0.x <= 0) {  // active q-block that keeps nothing: zeros, lse = -5e4
+        if (row_ok) {
+#pragma unroll 1
+          for (int i = 0; i < kD / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (lse != nullptr) *lse = -5e4f;
+        }
+        continue;
+      }
+      const uint32_t ip = item & 1u;
+      if (!mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag)) break;
+      float l_out = 0.f, m_out = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m_out = fmaxf(m_out, tail->stats_m[ip][i][row]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float mi = tail->stats_m[ip][i][row];
+        const float ci = (mi == m_out) ? 1.f : ex2_approx(mi - m_out);
+        l_out = fmaf(tail->stats_l[ip][i][row], ci, l_out);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->stats_free[ip]);
+      if (!mbar_wait(&tail->o_full, item & 1u, abort_flag)) break;
+      ++item;
+      tc_fence_after_sync();
+      auto release_o = [&]() {  // O may be overwritten by the next unit
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tail->o_free);
+      };
+      float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
+      const bool whole = q_valid * grp == kBQ;  // no row of the q-block is past the request
+      auto emit = [&](int col, const uint32_t* v) {  // 16 columns of this thread's row
+        uint4 out[2];
+        uint32_t* w = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const float x0 = __uint_as_float(v[2 * t]) * inv_out, x1 = __uint_as_float(v[2 * t + 1]) * inv_out;
+          w[t] = kBf16 ? pack_bf16x2(x0, x1) : pack_f16x2(x0, x1);
+        }
+        if (whole) {
+          // Through a staging area per warp (32 rows x 32 columns, plain row-major, two of them) and TMA stores of 16-row x
+          // 32-column boxes: a store instruction of a warp would otherwise write 32 scattered 16-byte pieces.
+          uint8_t* half = stg + (slab & 1u) * kOutSlabBytes;
+          if ((col & 16) == 0) {
+            if (lane == 0) tma_store_wait_read<1>();  // this half is free once the stores before the last ones have read it
+            __syncwarp();
+          }
+          uint4* dst = reinterpret_cast<uint4*>(half + lane * 64 + (col & 16) * 2);
+          dst[0] = out[0];
+          dst[1] = out[1];
+          if ((col & 16) != 0) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              const int t0 = q_row0 + (quad * 32) / grp;
+              tma_store_3d(&a.tmap_o16, half, col - 16, h * grp, t0);
+              tma_store_3d(&a.tmap_o16, half + kOutSlabBytes / 2, col - 16, h * grp, t0 + 16 / grp);
+              tma_store_commit();
+            }
+            ++slab;
+          }
+        } else if (row_ok) {
+          uint4* dst = reinterpret_cast<uint4*>(orow + col);
+          dst[0] = out[0];
+          dst[1] = out[1];
+        }
+      };
+      const int nparts = u1.w & 0xff;
+      bool merged = false;
+      if constexpr (kParts) {
+        if (nparts > 1) {
+          // ---- a part of a split item: the fp32 O (relative to m_out), m_out and the row sum go to the part's slot
+          // as [column group of 4][row][4] (a warp's store covers 512 contiguous bytes); the part that delivers last
+          // merges all of them, in ascending order whichever part it is (the result does not depend on it):
+          // O = sum_p O_p 2^(m_p - m) / sum_p l_p 2^(m_p - m), m = max_p m_p.
+          const int slot = static_cast<int>(static_cast<uint32_t>(u1.w) >> 16), part = (u1.w >> 8) & 0xff;
+          float* ps = a.partials + static_cast<size_t>(slot) * kPartialFloats;
+#pragma unroll 1
+          for (int col = 0; col < kD; col += 16) {
+            uint32_t v[16];
+            tmem_ld_x16(tmem_o + col, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              *reinterpret_cast<uint4*>(ps + (static_cast<size_t>(col / 4 + q) * 128 + row) * 4) =
+                  make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          }
+          release_o();
+          ps[128 * 128 + row] = m_out;
+          ps[128 * 128 + 128 + row] = l_out;
+          __threadfence();
+          if (!ep_sync()) break;
+          if (warp == kWarpEpilogue && lane == 0) {
+            int* cnt = a.arrive + (slot - part);  // a split item counts at its first slot
+            const int old = atomicAdd(cnt, 1);
+            const int mine = old == nparts - 1 ? 1 : 0;
+            if (mine) *cnt = 0;  // the counter is back at zero for the next launch
+            __threadfence();
+            tail->merge_go = mine;
+          }
+          if (!ep_sync()) break;
+          if (tail->merge_go == 0) continue;  // another part will merge
+          const float* base = a.partials + static_cast<size_t>(slot - part) * kPartialFloats;
+          m_out = -INFINITY;
+          for (int pp = 0; pp < nparts; ++pp)
+            m_out = fmaxf(m_out, __ldcg(base + static_cast<size_t>(pp) * kPartialFloats + 128 * 128 + row));
+          l_out = 0.f;
+          for (int pp = 0; pp < nparts; ++pp) {
+            const float mp = __ldcg(base + static_cast<size_t>(pp) * kPartialFloats + 128 * 128 + row);
+            const float wgt = (mp == -INFINITY) ? 0.f : ex2_approx(mp - m_out);
+            l_out = fmaf(__ldcg(base + static_cast<size_t>(pp) * kPartialFloats + 128 * 128 + 128 + row), wgt, l_out);
+          }
+          inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
+#pragma unroll 1
+          for (int col = 0; col < kD; col += 16) {
+            uint32_t v[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = 0u;  // the accumulator (fp32 bit patterns)
+            for (int pp = 0; pp < nparts; ++pp) {
+              const float* pq = base + static_cast<size_t>(pp) * kPartialFloats;
+              const float mp = __ldcg(pq + 128 * 128 + row);
+              const float wgt = (mp == -INFINITY) ? 0.f : ex2_approx(mp - m_out);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(pq + (static_cast<size_t>(col / 4 + q) * 128 + row) * 4));
+                v[4 * q] = __float_as_uint(fmaf(x.x, wgt, __uint_as_float(v[4 * q])));
+                v[4 * q + 1] = __float_as_uint(fmaf(x.y, wgt, __uint_as_float(v[4 * q + 1])));
+                v[4 * q + 2] = __float_as_uint(fmaf(x.z, wgt, __uint_as_float(v[4 * q + 2])));
+                v[4 * q + 3] = __float_as_uint(fmaf(x.w, wgt, __uint_as_float(v[4 * q + 3])));
+              }
+            }
+            emit(col, v);
+          }
+          merged = true;
+        }
+      }
+      if (!merged) {
+#pragma unroll 1
+        for (int col = 0; col < kD; col += 16) {
+          uint32_t v[16];
+          tmem_ld_x16(tmem_o + col, v);
+          tmem_wait_ld();
+          if (col == kD - 16) release_o();
+          emit(col, v);
+        }
+      }
+      if (row_ok && lse != nullptr) *lse = (l_out > 0.f) ? (log2f(l_out) + m_out) : -5e4f;
+    }
+    if (lane == 0) tma_store_wait_all<0>();
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
-    // ------------------------------------------------------------------ softmax / epilogue warps 0..15
+    // ------------------------------------------------------------------ softmax warps 0..15
     // Group X = warp / 8 takes the blocks with g & 1 == X. Two threads per q row: thread
     // (quadrant = warp & 3, half ch = (warp >> 2) & 1, lane) owns row 32 * quadrant + lane (its TMEM lane)
-    // and the columns [64 ch, 64 ch + 64) of S[X], P[X] and (in a rescale) O; in the epilogue the 16 warps
-    // cover O in 32-column quarters.
+    // and the columns [64 ch, 64 ch + 64) of S[X], P[X] and (in a rescale) O.
     const uint32_t X = static_cast<uint32_t>(warp >> 3), Y = X ^ 1u;
     const uint32_t ch = static_cast<uint32_t>((warp >> 2) & 1);
     const int quad = warp & 3;
@@ -555,39 +749,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     const uint32_t tmem_s = tmem_base + lane_base + kColS + X * 128u + ch * 64u;
     const uint32_t tmem_p = tmem_base + lane_base + (kWide ? kColS + X * 128u : kColP + X * 64u) + ch * 32u;
     const uint32_t tmem_o = tmem_base + lane_base + kColO;
-    const uint32_t ocol = static_cast<uint32_t>(kOW) * (2u * X + ch);  // this thread's quarter of O in the epilogue
-    const bool has_cols = ocol < static_cast<uint32_t>(kD);  // head_dim 64: the second group's threads own no column of O
     const int row = quad * 32 + lane;
     uint64_t* pair_bar = &tail->pair_bar[X][quad];
     uint32_t pair_phase = 0;
-    uint16_t* o16 = reinterpret_cast<uint16_t*>(a.o);
     bool ok = true;
-
-    struct RowCtx {  // where an item's row lives in global memory (this thread's 32-column quarter)
-      uint16_t* orow;
-      float* lse;
-      bool row_ok;
-    };
-    // Row r of a tile is token q_row0 + r / group, q head h * group + r % group (group = 1: the row itself).
-    const int grp = a.group_size;
-    auto row_ctx = [&](int q_row0, int q_valid, int h) -> RowCtx {
-      RowCtx c;
-      c.row_ok = static_cast<int>(row) < q_valid * grp;
-      const int64_t grow = static_cast<int64_t>(q_row0) + static_cast<int>(row) / grp;
-      const int hq = h * grp + static_cast<int>(row) % grp;
-      c.orow = o16 + grow * a.o_stride_n + static_cast<int64_t>(hq) * a.o_stride_h + ocol;
-      c.lse = (a.lse != nullptr && ocol == 0u) ? a.lse + grow * a.lse_stride_n + hq : nullptr;
-      return c;
-    };
-    auto on_empty = [&](int q_row0, int q_valid, int hq) {  // active q-block that keeps nothing: zeros, lse = -5e4
-      const RowCtx c = row_ctx(q_row0, q_valid, hq);
-      if (c.row_ok && has_cols) {
-        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int i = 0; i < kOW / 8; ++i) reinterpret_cast<uint4*>(c.orow)[i] = z;
-        if (c.lse != nullptr) *c.lse = -5e4f;
-      }
-    };
+    [[maybe_unused]] const int grp = a.group_size;
 
     GroupSeq<kMask != 0> seq;
     seq.init(tail, abort_flag);
@@ -596,166 +762,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     uint32_t items_seen = 0; // items whose last block has been passed
     float m_ref = -INFINITY; // the maximum this thread's partial sum refers to
     uint64_t l2a = 0, l2b = 0;  // partial row sum over this thread's columns of the group's blocks
-    // an item whose statistics have been published and whose O is still being accumulated
-    int cm_kv_len = 0, cm_base = 0;   // custom mask: the request's kv length, byte offset of its matrix,
-    int64_t cm_row_bit = 0;           // and the bit offset of this thread's row inside it
-    bool pend = false;
-    uint32_t pend_item = 0;
-    int pend_q_row0 = 0, pend_q_valid = 0, pend_h = 0, pend_parts = 1;
-    uint32_t ep_phase = 0;
-    // bounded barrier of the softmax warps (only the epilogue of a part of a split item uses it)
-    auto ep_sync = [&]() -> bool {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tail->ep_bar);
-      const bool r = __all_sync(0xffffffffu, mbar_wait(&tail->ep_bar, ep_phase, abort_flag) ? 1 : 0) != 0;
-      ep_phase ^= 1u;
-      return r;
-    };
+    [[maybe_unused]] int cm_kv_len = 0, cm_base = 0;   // custom mask: the request's kv length, byte offset of its matrix,
+    [[maybe_unused]] int64_t cm_row_bit = 0;           // and the bit offset of this thread's row inside it
 
-    auto epilogue = [&]() -> bool {
-      const uint32_t ip = pend_item & 1u;
-      if (!mbar_wait(&tail->stats_ready[ip], (pend_item >> 1) & 1u, abort_flag)) return false;
-      float lsum = 0.f, m_fin = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) m_fin = fmaxf(m_fin, tail->stats_m[ip][i][row]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float mi = tail->stats_m[ip][i][row];
-        const float ci = (mi == m_fin) ? 1.f : ex2_approx(mi - m_fin);
-        lsum = fmaf(tail->stats_l[ip][i][row], ci, lsum);
-      }
-      if (!mbar_wait(&tail->o_full, pend_item & 1u, abort_flag)) return false;
-      tc_fence_after_sync();
-      uint32_t v[32];
-      [[maybe_unused]] uint32_t v_hi[kWide ? 32 : 1];  // head dimension 256: the thread's second 32 columns
-      if (has_cols) {
-        tmem_ld_x32(tmem_o + ocol, v);
-        if constexpr (kWide) tmem_ld_x32(tmem_o + ocol + 32u, v_hi);
-        tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (int t = 0; t < 32; ++t) v[t] = 0u;
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tail->o_free);  // O may be overwritten by the next item
-      const RowCtx pend_ctx = row_ctx(pend_q_row0, pend_q_valid, pend_h);
-      const int nparts = pend_parts & 0xff;
-      float m_out = m_fin, l_out = lsum;
-      if constexpr (kParts) {
-        if (nparts > 1) {
-          // ---- a part of a split item: the fp32 O (relative to m_fin), m_fin and the row sum go to the part's slot
-          // as [column group of 4][row][4] (a warp's store covers 512 contiguous bytes); the part that delivers last
-          // merges all of them, in ascending order whichever part it is (the result does not depend on it):
-          // O = sum_p O_p 2^(m_p - m) / sum_p l_p 2^(m_p - m), m = max_p m_p.
-          const int slot = static_cast<int>(static_cast<uint32_t>(pend_parts) >> 16), part = (pend_parts >> 8) & 0xff;
-          float* ps = a.partials + static_cast<size_t>(slot) * kPartialFloats;
-          if (has_cols) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              *reinterpret_cast<uint4*>(ps + (static_cast<size_t>(ocol / 4u + q) * 128 + row) * 4) =
-                  make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-          }
-          if (ocol == 0u) {
-            ps[128 * 128 + row] = m_fin;
-            ps[128 * 128 + 128 + row] = lsum;
-          }
-          __threadfence();
-          if (!ep_sync()) return false;
-          if (warp == 0 && lane == 0) {
-            int* cnt = a.arrive + (slot - part);  // a split item counts at its first slot
-            const int old = atomicAdd(cnt, 1);
-            const int mine = old == nparts - 1 ? 1 : 0;
-            if (mine) *cnt = 0;  // the counter is back at zero for the next launch
-            __threadfence();
-            tail->merge_go = mine;
-          }
-          if (!ep_sync()) return false;
-          if (tail->merge_go == 0) {  // another part will merge
-            pend = false;
-            return true;
-          }
-          const float* base = a.partials + static_cast<size_t>(slot - part) * kPartialFloats;
-          float m_all = -INFINITY;
-          for (int pp = 0; pp < nparts; ++pp)
-            m_all = fmaxf(m_all, __ldcg(base + static_cast<size_t>(pp) * kPartialFloats + 128 * 128 + row));
-          float l_all = 0.f;
-#pragma unroll
-          for (int t = 0; t < 32; ++t) v[t] = 0u;  // v becomes the accumulator (fp32 bit patterns)
-          for (int pp = 0; pp < nparts; ++pp) {
-            const float* pq = base + static_cast<size_t>(pp) * kPartialFloats;
-            const float mp = __ldcg(pq + 128 * 128 + row);
-            const float wgt = (mp == -INFINITY) ? 0.f : ex2_approx(mp - m_all);
-            l_all = fmaf(__ldcg(pq + 128 * 128 + 128 + row), wgt, l_all);
-            if (!has_cols) continue;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const float4 x = __ldcg(reinterpret_cast<const float4*>(pq + (static_cast<size_t>(ocol / 4u + q) * 128 + row) * 4));
-              v[4 * q] = __float_as_uint(fmaf(x.x, wgt, __uint_as_float(v[4 * q])));
-              v[4 * q + 1] = __float_as_uint(fmaf(x.y, wgt, __uint_as_float(v[4 * q + 1])));
-              v[4 * q + 2] = __float_as_uint(fmaf(x.z, wgt, __uint_as_float(v[4 * q + 2])));
-              v[4 * q + 3] = __float_as_uint(fmaf(x.w, wgt, __uint_as_float(v[4 * q + 3])));
-            }
-          }
-          m_out = m_all;
-          l_out = l_all;
-        }
-      }
-      const float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
-      const bool whole = pend_q_valid * grp == kBQ;  // no row of the q-block is past the request
-#pragma unroll
-      for (int hh = 0; hh < kOW / 32; ++hh) {  // 32 columns at a time
-        uint4 outv[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint32_t w[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t r0 = v[8 * q + 2 * t], r1 = v[8 * q + 2 * t + 1];
-            if constexpr (kWide) {
-              if (hh == 1) { r0 = v_hi[8 * q + 2 * t]; r1 = v_hi[8 * q + 2 * t + 1]; }
-            }
-            const float x0 = __uint_as_float(r0) * inv_out;
-            const float x1 = __uint_as_float(r1) * inv_out;
-            w[t] = kBf16 ? pack_bf16x2(x0, x1) : pack_f16x2(x0, x1);
-          }
-          outv[q] = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        if (!has_cols) {
-          // head_dim 64: this thread's quarter of O does not exist
-        } else if (whole) {
-          // Through a 1 KB staging area per warp (16 rows x 64 bytes, plain row-major) and a TMA store of one
-          // 16-row x 32-column box: a store instruction of a warp would otherwise write 32 scattered 16-byte pieces.
-          uint8_t* stg = smem_ostage + warp * kOutStageBytes;
-          const int grow0 = pend_q_row0 + (quad * 32) / grp;
-#pragma unroll
-          for (int ph = 0; ph < 2; ++ph) {
-            if (lane == 0) tma_store_wait_read<0>();  // the staging area is free once its last store has read it
-            __syncwarp();
-            if ((lane >> 4) == ph) {
-              const int r = lane & 15;
-#pragma unroll
-              for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(stg + r * 64 + c * 16) = outv[c];
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_3d(&a.tmap_o16, stg, static_cast<int>(ocol) + 32 * hh, pend_h * grp, grow0 + (ph * 16) / grp);
-              tma_store_commit();
-            }
-          }
-        } else if (pend_ctx.row_ok) {
-          uint4* dst = reinterpret_cast<uint4*>(pend_ctx.orow) + 4 * hh;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) dst[q] = outv[q];
-        }
-      }
-      if (pend_ctx.row_ok && pend_ctx.lse != nullptr) *pend_ctx.lse = (l_out > 0.f) ? (log2f(l_out) + m_out) : -5e4f;
-      pend = false;
-      return true;
-    };
-
-    while (ok && seq.next(a, on_empty)) {
+    while (ok && seq.next(a, ignore_empty)) {
       if (seq.first()) {
         if constexpr (kMask == 2) {  // both groups: the row's bit offset inside the request's matrix
           const int q0 = a.qo_indptr[seq.req];
@@ -872,9 +882,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
         tmem_wait_st();
         if (rescale) {
           // (after the exponentials, when S has left the registers, and before P is handed over: the PV of this
-          // block must see the rescaled O) O is rescaled only after the PV of block g-1 has completed; that PV may be the first of
-          // its item and wait for the previous item's epilogue, so this thread's share of it goes first
-          if (pend && !epilogue()) { ok = false; break; }
+          // block must see the rescaled O) O is rescaled only after the PV of block g-1 has completed
           if (!mbar_wait(&tail->pv_done[Y], ((g - 1u) >> 1) & 1u, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
           const float alpha = need ? ex2_approx(m_prev - m_new) : 1.0f;
@@ -893,15 +901,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive(&tail->p_full[X]);
         ++my_blocks;
-        // the previous item's epilogue runs after this group's first block of the next item, so that
-        // the item's last PV overlaps a softmax step (running it before the block, in the wait for S,
-        // frees O earlier for the next item's first PV but measured 9 % slower: it delays the group's
-        // own chain, which is the longer one)
-        if (pend && !epilogue()) { ok = false; break; }
       }
       if (seq.last()) {
-        if (pend && !epilogue()) { ok = false; break; }
         const uint32_t ip = items_seen & 1u;
+        // the statistics of the item before the last one must have been read
+        if (items_seen >= 2u && !mbar_wait(&tail->stats_free[ip], ((items_seen >> 1) - 1u) & 1u, abort_flag)) { ok = false; break; }
         float la, lb, lc, ld;
         unpack_f32x2(l2a, la, lb);
         unpack_f32x2(l2b, lc, ld);
@@ -909,15 +913,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
         tail->stats_l[ip][2u * X + ch][row] = (la + lb) + (lc + ld);
         __syncwarp();
         if (lane == 0) mbar_arrive(&tail->stats_ready[ip]);
-        pend = true;
-        pend_item = items_seen;
-        pend_q_row0 = seq.q_row0; pend_q_valid = seq.q_valid; pend_h = seq.h; pend_parts = seq.parts;
         ++items_seen;
       }
       ++g;
     }
-    if (ok && pend) epilogue();
-    if (lane == 0) tma_store_wait_all<0>();
   }
 
   // ------------------------------------------------------------------ common exit
