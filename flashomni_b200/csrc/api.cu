@@ -57,6 +57,12 @@ int sm_count() {
   return cached[dev];
 }
 
+// Set by fo_attn_lists when its single launch was the last thing this thread put on a stream through this library: the
+// attention launch that follows on the same stream may then set itself up while the lists are built. Any other work in
+// between only makes the launch an ordinary one.
+thread_local bool t_lists_pending = false;
+thread_local cudaStream_t t_lists_stream = nullptr;
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -353,6 +359,8 @@ int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const u
   if (attn_lists_small_applies(a, u)) {
     const cudaError_t e = launch_attn_lists_small(a, u, z, st);
     count_launches(1);
+    t_lists_pending = e == cudaSuccess;
+    t_lists_stream = st;
     return e == cudaSuccess ? FO_OK : fail_cuda("fo_attn_lists", e);
   }
   if (zero_out != nullptr && !is_full && zero_total_bytes > 0) {
@@ -466,6 +474,8 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     a.sm_scale_log2 = sm_scale * 1.4426950408889634f;
   }
   a.status = status;
+  a.after_lists = t_lists_pending && t_lists_stream == static_cast<cudaStream_t>(stream);
+  t_lists_pending = false;
   int64_t ctas = static_cast<int64_t>(sm_count());  // one persistent CTA per SM
   if (ctas > max_units) ctas = max_units;
   const cudaError_t e = launch_attention(a, static_cast<int>(ctas), static_cast<cudaStream_t>(stream));
@@ -720,6 +730,7 @@ int gemm_q_impl(const void* x, const void* w, void* y, const void* bias, int32_t
     // (set only when a bounded wait runs out) stays as it is until the next list is built.
     e = prepared ? cudaSuccess : launch_gemm_q_tiles(la, st);
     if (e != cudaSuccess) return fail_cuda("fo_gemm_q (work list)", e);
+    g.after_list = prepared ? 0 : 1;
     count_launches(prepared ? 0 : 1);
     g.tiles = la.tiles;
     g.n_tiles_ptr = la.counters;
@@ -801,6 +812,7 @@ int gemm_o_impl(const void* x, const void* w, void* y, const void* init, int32_t
   la.is_for_cache = is_for_cache;
   cudaError_t e = prepared ? cudaSuccess : launch_gemm_o_rows(la, st);
   if (e != cudaSuccess) return fail_cuda("fo_gemm_o (work list)", e);
+  g.after_list = prepared ? 0 : 1;
   count_launches(prepared ? 1 : 2);
   g.y = y;
   g.init = init;

@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  if (a.after_lists) asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the lists in front of it were built
 
   // The list may be shorter than counters[0] says: a compaction that ran out of room records it in counters[2]
   // and leaves records unwritten. Nothing of such a list is dereferenced; the launch only reports it.
@@ -953,8 +954,8 @@ cudaError_t launch_one(const AttnArgs& a, int ctas, cudaStream_t stream) {
   const cudaError_t e = cudaFuncSetAttribute(attention_kernel<kBf16, kSoftCap, kParts, kD, kMask>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return e;
-  attention_kernel<kBf16, kSoftCap, kParts, kD, kMask><<<ctas, kThreads, kSmemBytes, stream>>>(a);
-  return cudaGetLastError();
+  return launch_dependent(attention_kernel<kBf16, kSoftCap, kParts, kD, kMask>, ctas, kThreads, kSmemBytes, stream,
+                          a.after_lists != 0, a);
 }
 template <bool kBf16, bool kSoftCap>
 cudaError_t launch_two(const AttnArgs& a, int ctas, cudaStream_t stream) {

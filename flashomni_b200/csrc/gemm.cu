@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  if (a.after_list) asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the list in front of it was built
 
   const int n_tiles = num_tiles(a);
   // Tiles are handed out in list order through a device-wide cursor (the GEMM-O rows are sorted
@@ -463,17 +464,10 @@ cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream) {
   const int cap = a.batch * (a.m / kBM) * ((a.mode == kGemmQ && a.tiles != nullptr) ? a.n / kBNH : (a.n / kBNH + 1) / 2);
   if (cap <= 0) return cudaSuccess;
   const int grid = cap < max_ctas ? cap : max_ctas;
-  cudaError_t e;
-  if (a.is_bf16) {
-    e = cudaFuncSetAttribute(gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    gemm_kernel<true><<<grid, kThreads, kSmemBytes, stream>>>(a);
-  } else {
-    e = cudaFuncSetAttribute(gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    gemm_kernel<false><<<grid, kThreads, kSmemBytes, stream>>>(a);
-  }
-  return cudaGetLastError();
+  const auto kernel = a.is_bf16 ? gemm_kernel<true> : gemm_kernel<false>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(kernel, grid, kThreads, kSmemBytes, stream, a.after_list != 0, a);
 }
 
 }  // namespace fo

@@ -10,6 +10,24 @@
 
 namespace fo {
 
+// Launches a kernel whose arguments struct is `args`; with `dependent` it may start while the kernel in front of it in the
+// stream still runs (programmatic dependent launch): it must then wait (griddepcontrol.wait) before it touches memory.
+template <class Args>
+inline cudaError_t launch_dependent(void (*kernel)(Args), int grid, int threads, size_t smem, cudaStream_t stream, bool dependent,
+                                    const Args& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 // ------------------------------------------------------------------ mask path
 struct CompactArgs {
   const uint8_t* sparse_info;
@@ -110,6 +128,7 @@ struct GemmArgs {
   const int32_t* row_order;
   int32_t* status;                 // device status word (DevStatus)
   int32_t* cursor;                 // device-wide tile cursor, zero when the kernel starts
+  int after_list;                  // the launch in front of this one builds the list (dependent launch)
 };
 cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream);
 // dense projections whose shape divides into 256x256 tiles take the tall-tile kernel (gemm_tall.cu)
@@ -196,6 +215,7 @@ struct AttnArgs {
   int group_size;                  // H / Hkv
   int is_bf16;
   float sm_scale_log2;             // sm_scale * log2(e); with a soft cap: cap * log2(e)
+  int after_lists;                 // the launch in front of this one builds the lists (dependent launch)
   float soft_cap_pre;              // 0: no soft cap; else sm_scale / cap (logits = cap * tanh(q.k * sm_scale / cap))
   int32_t* status;
 };

@@ -973,6 +973,7 @@ constexpr int64_t kSmallCand = 4096, kSmallBits = 1 << 18;
 
 __global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(CompactArgs a, UnitArgs u, ZeroArgs z, int by_length,
                                                                          int heads_per_group) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention kernel may set itself up meanwhile
   extern __shared__ __align__(16) uint32_t s_dyn[];   // [n_cand] keys, then [n_cand] counts
   __shared__ int s_first[kSmallBatch + 1];            // first candidate of a request
   __shared__ int s_q0[kSmallBatch], s_ql[kSmallBatch], s_k0[kSmallBatch], s_kl[kSmallBatch];
@@ -1162,7 +1163,10 @@ cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, con
 // are cut into two single-block records each, k chosen so that the launch ends earliest when `n_ctas` CTAs draw
 // the records in list order (gemm_q_split_rule: a two-block tile costs 20 time units, a single-block tile 13).
 // counters[0] = number of records, counters[1] = number of active 128x128 tiles, counters[3] = number
-// of two-block records. The kernel walks the row blocks twice: totals first, then the records.
+// of two-block records. The kernel walks the row blocks twice: totals first, then the records; with at most one row block
+// per thread (the usual case) the second walk has everything in registers.
+// Both list kernels are all latency and sit in front of the GEMM when the caller did not prepare the list: they let it
+// start its set-up at once (programmatic dependent launch; the GEMM waits for the list before reading it).
 constexpr int kPairCost = 20, kSingleCost = 13;
 
 // Time at which the last CTA ends when `n` CTAs draw `pairs` two-block tiles and then `singles` single-block tiles
@@ -1192,8 +1196,15 @@ __global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
   __shared__ int s_warp_t[32];
   __shared__ int s_carry, s_carry_t, s_pairs_total, s_best;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int mt = a.m / 128, nt = a.n / 128;
   const int rows = a.batch * mt;
+  const bool one_walk = rows <= static_cast<int>(blockDim.x);
+  int cnt = 0, x = 0, xt = 0;
+  const uint8_t* seg = nullptr;
+  int64_t limit = 0, bit0 = 0;
+  uint64_t rowbits = 0;
+  bool fast = false;
   for (int pass = 0; pass < 2; ++pass) {
     if (tid == 0) { s_carry = 0; s_carry_t = 0; }
     __syncthreads();
@@ -1202,12 +1213,9 @@ __global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
     const int pairs_kept = pairs_total - n_split;
     for (int base = 0; base < rows; base += blockDim.x) {
       const int r = base + tid;
-      int cnt = 0;
-      const uint8_t* seg = nullptr;
-      int64_t limit = 0, bit0 = 0;
-      uint64_t rowbits = 0;
-      bool fast = false;
-      if (r < rows) {
+      const bool have = pass == 1 && one_walk;   // s_warp / s_warp_t still hold the scan, too
+      if (!have) cnt = 0;
+      if (r < rows && !have) {
         const int b = r / mt, iy = r % mt;
         if (a.is_full) {
           cnt = nt;
@@ -1228,36 +1236,42 @@ __global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
       }
       // x: two-block records, xt: single-block records (inclusive scans over the CTA)
       const int npair = cnt >> 1, nsingle = cnt & 1;
-      int x = npair, xt = nsingle;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        const int yt = __shfl_up_sync(0xffffffffu, xt, o);
-        if (lane >= o) { x += y; xt += yt; }
-      }
-      if (lane == 31) { s_warp[warp] = x; s_warp_t[warp] = xt; }
-      __syncthreads();
-      if (warp == 0) {
-        int w = s_warp[lane], wt = s_warp_t[lane];
+      if (!have) {
+        x = npair; xt = nsingle;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, w, o);
-          const int yt = __shfl_up_sync(0xffffffffu, wt, o);
-          if (lane >= o) { w += y; wt += yt; }
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          const int yt = __shfl_up_sync(0xffffffffu, xt, o);
+          if (lane >= o) { x += y; xt += yt; }
         }
-        s_warp[lane] = w;
-        s_warp_t[lane] = wt;
+        if (lane == 31) { s_warp[warp] = x; s_warp_t[warp] = xt; }
+        __syncthreads();
+        if (warp == 0) {
+          int w = s_warp[lane], wt = s_warp_t[lane];
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            const int yt = __shfl_up_sync(0xffffffffu, wt, o);
+            if (lane >= o) { w += y; wt += yt; }
+          }
+          s_warp[lane] = w;
+          s_warp_t[lane] = wt;
+        }
+        __syncthreads();
       }
-      __syncthreads();
       if (pass == 1 && r < rows && cnt > 0) {
         int pos = s_carry + (warp ? s_warp[warp - 1] : 0) + x - npair;
         const int spos = pairs_total + n_split + s_carry_t + (warp ? s_warp_t[warp - 1] : 0) + xt - nsingle;
         const int b = r / mt, iy = r % mt;
         int first = -1;
         for (int ix = 0; ix < nt; ++ix) {
-          const int on = a.is_full ? 1 : (fast ? static_cast<int>((rowbits >> ix) & 1ull)
-                                                 : get_bit(seg, bit0 + (ix * 128) / a.head_dim, limit));
-          if (!on) continue;
+          if (fast) {   // straight to the next active block
+            if (rowbits == 0) break;
+            ix = __ffsll(static_cast<long long>(rowbits)) - 1;
+            rowbits &= rowbits - 1;
+          } else if (!a.is_full && !get_bit(seg, bit0 + (ix * 128) / a.head_dim, limit)) {
+            continue;
+          }
           if (first < 0) {
             first = ix;
           } else {
@@ -1316,8 +1330,13 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mt = a.m / 128;
   const int rows = a.batch * mt;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int local_heads = a.k / a.head_dim;
   const int want = a.is_for_cache ? 0 : 1;
+  // At most one row block per thread: a row's place in the order is the number of longer rows (and of equal ones in front
+  // of it), counted over the lengths in shared memory. More rows: counting sort by length.
+  const bool by_rank = rows <= static_cast<int>(blockDim.x);
+  __shared__ int s_len[1024];
   if (tid == 0) s_carry = 0;
   for (int i = tid; i <= local_heads; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
@@ -1340,6 +1359,7 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
       }
     }
     int x = cnt;
+    if (by_rank && r < rows) s_len[r] = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1347,6 +1367,14 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
+    if (by_rank && r < rows) {
+      int rank = 0;
+      for (int o = 0; o < rows; ++o) {
+        const int len = s_len[o];
+        rank += (len > cnt || (len == cnt && o < r)) ? 1 : 0;
+      }
+      a.row_order[rank] = r;
+    }
     if (warp == 0) {
       int w = s_warp[lane];
 #pragma unroll
@@ -1360,7 +1388,7 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
     const int off = s_carry + (warp ? s_warp[warp - 1] : 0) + x - cnt;
     if (r < rows) {
       a.row_indptr[r] = off;
-      atomicAdd(&s_hist[cnt], 1);
+      if (!by_rank) atomicAdd(&s_hist[cnt], 1);
       const int b = r / mt, iy = r % mt;
       const int64_t ioff = a.info_indptr[b];
       const int64_t qb = (static_cast<int64_t>(a.num_text_tokens) + static_cast<int64_t>(iy) * 128) / a.sparse_q_size;
@@ -1389,10 +1417,12 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
     a.counters[4] = kDevOk;  // status word of the GEMM kernel that follows
     a.counters[5] = 0;       // its tile cursor
     a.counters[6] = 0;       // and the count of CTAs that have finished
-    // bucket starts, descending count
-    int acc = 0;
-    for (int k = local_heads; k >= 0; --k) { const int v = s_hist[k]; s_hist[k] = acc; acc += v; }
+    if (!by_rank) {  // bucket starts, descending count
+      int acc = 0;
+      for (int k = local_heads; k >= 0; --k) { const int v = s_hist[k]; s_hist[k] = acc; acc += v; }
+    }
   }
+  if (by_rank) return;
   __syncthreads();
   if (warp == 0) {
     for (int base = 0; base < rows; base += 32) {

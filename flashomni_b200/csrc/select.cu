@@ -18,7 +18,6 @@
 // Measured on a B200 at 40 heads x 604 blocks, thresholds 0.2 / 0.3 (the text-to-image scores switch most q-blocks off):
 // whole call 82.4 us with four launches, a memset and threshold arrays, 25.5 us with these two launches.
 #include <cooperative_groups.h>
-#include <string.h>
 
 #include "internal.h"
 
@@ -381,17 +380,7 @@ static cudaError_t launch_kv(const SelectArgs& a, cudaStream_t stream) {
   const int64_t rows = static_cast<int64_t>(a.batch) * a.heads * a.n;
   int64_t ctas = (rows + kSelWarps - 1) / kSelWarps;
   if (ctas > 148 * 3) ctas = 148 * 3;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
-  cfg.blockDim = dim3(kSelWarps * 32);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, select_kv_kernel<kPer>, a);
+  return launch_dependent(select_kv_kernel<kPer>, static_cast<int>(ctas), kSelWarps * 32, 0, stream, true, a);
 }
 
 cudaError_t launch_select_blocks(const SelectArgs& a, cudaStream_t stream) {
