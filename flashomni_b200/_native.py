@@ -86,6 +86,8 @@ SIGNATURES = {
                                    _P, c_int64, _P, _P]),
     "fo_gemm_q_worklist": (c_int32, [c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                      c_int32, _P, c_int64, _P, _P, c_size_t, _P]),
+    "fo_layer_lists": (c_int32, [_P, c_int64, _P, c_int64, _P, _P, _P, c_int32, c_int32, c_int32, c_int32, _P, c_size_t, _P,
+                                 c_size_t, _P]),
     "fo_gemm_o_worklist": (c_int32, [c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                      c_int32, _P, c_int64, _P, _P, c_size_t, _P]),
 }

@@ -8,6 +8,7 @@ the tcgen05 attention kernel over those lists. Nothing in `run()` synchronises o
 
 from __future__ import annotations
 
+import ctypes
 import functools
 import logging
 import math
@@ -367,6 +368,9 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             128, self._n_cand, self._max_nkv, n, kept, ptrs["items"], ptrs["kv_ptr"], ptrs["kv_idx"], ptrs["order"],
             ptrs["counters"], ptrs["scratch"], scratch_bytes, self._min_items, self._num_streams, self._min_chunk,
             self._max_units, self._partial_slots, ptrs["units"], ptrs["unit_counters"], ptrs["arrive"])
+        # ... and the same as the host array that fo_layer_lists reads
+        fixed = (self._qo_indptr_buf.data_ptr(), self._kv_indptr_buf.data_ptr()) + self._list_args
+        self._layer_plan = (ctypes.c_int64 * len(fixed))(*fixed)
         pbytes = lib.fo_attn_partial_bytes(self._partial_slots)
         fw = self._float_workspace_buffer
         self._partials = None
@@ -566,6 +570,29 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             self._prepared_event.record(side)
         self._prepared_key = self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
                                             is_full)
+
+    def prepare_layer_lists(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, q_list, o_list,
+                            m: int, n_local: int, stream: torch.cuda.Stream, after: torch.cuda.Event) -> None:
+        """Extension: `prepare_masks()` together with the GEMM-Q and GEMM-O lists of the same masks (rebuilt in the storage of
+        `q_list` / `o_list`, made by `prepare_gemm_q_list` / `prepare_gemm_o_list` for the same shapes), in one call
+        and, for small masks, one launch on `stream`, ordered after the event `after`. int32 indptrs only."""
+        if not self._planned:
+            raise RuntimeError("plan() must be called before prepare_layer_lists()")
+        q_list.check("q", self._batch_size, m, n_local, self._head_dim, self.device)
+        o_list.check("o", self._batch_size, m, n_local, self._head_dim, self.device)
+        p = _native.ptr
+        with torch.cuda.device(self.device):
+            if self._prepared_event is None:
+                self._prepared_event = torch.cuda.Event()
+            stream.wait_event(after)
+            rc = _native.load().fo_layer_lists(
+                p(sparse_info), sparse_info.numel(), p(sparse_kv_info), sparse_kv_info.numel(), p(sparse_info_indptr),
+                p(sparse_kv_info_indptr), self._layer_plan, m, n_local, self._head_dim, 0, p(q_list.ws), q_list.ws.numel(),
+                p(o_list.ws), o_list.ws.numel(), stream.cuda_stream)
+            _native.check(rc, "prepare_layer_lists")
+            self._prepared_event.record(stream)
+        q_list.event = o_list.event = self._prepared_event
+        self._prepared_key = self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, False)
 
     # ------------------------------------------------------------------------------------------ extras
     def check_status(self) -> None:

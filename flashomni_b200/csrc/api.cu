@@ -675,6 +675,47 @@ int fo_gemm_o_worklist(int32_t batch, int32_t m, int32_t k, int32_t num_heads, i
   return e == cudaSuccess ? FO_OK : fail_cuda("fo_gemm_o_worklist", e);
 }
 
+int fo_layer_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                   int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr, const int32_t* sparse_kv_info_indptr,
+                   const int64_t* plan, int32_t m, int32_t n_local, int32_t head_dim, int32_t num_text_tokens,
+                   void* q_workspace, size_t q_workspace_bytes, void* o_workspace, size_t o_workspace_bytes, void* stream) {
+  if (plan == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_layer_lists: null plan");
+  auto i32 = [&](int i) { return static_cast<int32_t>(plan[i]); };
+  auto ptr = [&](int i) { return reinterpret_cast<int32_t*>(plan[i]); };
+  CompactArgs a;
+  int rc = make_compact_args(a, sparse_info, sparse_info_bytes, sparse_kv_info, sparse_kv_info_bytes, sparse_info_indptr,
+                             sparse_kv_info_indptr, ptr(0), ptr(1), i32(2), i32(3), i32(4), i32(5), i32(6), i32(7), 0,
+                             plan[8], i32(9), plan[10], plan[11], ptr(12), ptr(13), ptr(14), ptr(15), ptr(16),
+                             reinterpret_cast<void*>(plan[17]), static_cast<size_t>(plan[18]));
+  if (rc != FO_OK) return rc;
+  UnitArgs u;
+  rc = make_unit_args(u, ptr(12), ptr(13), ptr(14), ptr(15), ptr(16), ptr(0), ptr(1), plan[10], i32(9), i32(6), i32(7),
+                      i32(19), i32(20), i32(21), plan[22], plan[23], ptr(24), ptr(25), ptr(26));
+  if (rc != FO_OK) return rc;
+  const GemmShape sq = {i32(2), m, n_local, head_dim > 0 ? head_dim : 1, i32(3), i32(4), head_dim, 128, num_text_tokens};
+  const GemmShape so = {i32(2), m, 128, n_local, i32(3), i32(4), head_dim, 128, num_text_tokens};
+  rc = check_lists_common("fo_layer_lists", sq, true, sparse_info, sparse_info_indptr, q_workspace, q_workspace_bytes);
+  if (rc == FO_OK) rc = check_lists_common("fo_layer_lists", so, true, sparse_info, sparse_info_indptr, o_workspace, o_workspace_bytes);
+  if (rc != FO_OK) return rc;
+  if ((128 % head_dim != 0 && head_dim % 128 != 0) || n_local % head_dim != 0)
+    return fail(FO_ERR_UNSUPPORTED, "fo_layer_lists: head_dim must divide or be a multiple of 128, and divide n_local");
+  const GemmListArgs q = make_list_args(sq, sparse_info, sparse_info_bytes, sparse_info_indptr, q_workspace);
+  const GemmListArgs o = make_list_args(so, sparse_info, sparse_info_bytes, sparse_info_indptr, o_workspace);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e;
+  if (attn_lists_small_applies(a, u)) {
+    e = launch_layer_lists(a, u, q, o, st);
+    count_launches(1);
+  } else {
+    e = launch_gemm_q_tiles(q, st);
+    if (e == cudaSuccess) e = launch_attn_compact(a, st);
+    if (e == cudaSuccess) e = launch_attn_units(u, st);
+    if (e == cudaSuccess) e = launch_gemm_o_rows(o, st);
+    count_launches(a.n_cand > 0 ? 6 : 3);
+  }
+  return e == cudaSuccess ? FO_OK : fail_cuda("fo_layer_lists", e);
+}
+
 namespace {
 
 int encode_gemm_maps(const char* who, GemmArgs& g, const void* x, const void* w, const void* y, int64_t rows_a,

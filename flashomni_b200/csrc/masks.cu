@@ -971,9 +971,8 @@ cudaError_t launch_attn_units(const UnitArgs& a, cudaStream_t stream) {
 constexpr int kSmallThreads = 512, kSmallBatch = 64;
 constexpr int64_t kSmallCand = 4096, kSmallBits = 1 << 18;
 
-__global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(CompactArgs a, UnitArgs u, ZeroArgs z, int by_length,
-                                                                         int heads_per_group) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention kernel may set itself up meanwhile
+__device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, int by_length,
+                                                      int heads_per_group, int cta) {
   extern __shared__ __align__(16) uint32_t s_dyn[];   // [n_cand] keys, then [n_cand] counts
   __shared__ int s_first[kSmallBatch + 1];            // first candidate of a request
   __shared__ int s_q0[kSmallBatch], s_ql[kSmallBatch], s_k0[kSmallBatch], s_kl[kSmallBatch];
@@ -1042,7 +1041,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(Compact
     s_key[c] = key;
   }
   __syncthreads();
-  const int c = blockIdx.x * (kSmallThreads / 32) + warp;
+  const int c = cta * (kSmallThreads / 32) + warp;
   if (c >= n) return;
   const int kept = s_cnt[c];
   const uint32_t key = s_key[c];
@@ -1137,6 +1136,12 @@ __global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(Compact
   }
 }
 
+__global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(CompactArgs a, UnitArgs u, ZeroArgs z, int by_length,
+                                                                         int heads_per_group) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention kernel may set itself up meanwhile
+  attn_lists_small_body(a, u, z, by_length, heads_per_group, static_cast<int>(blockIdx.x));
+}
+
 // The line lies where the redundant work stays below the launches it saves: keys have 12 bits for the candidate, and
 // every CTA reads the whole mask (kSmallBits = 32 KB). Cut lists and larger masks take the chain above.
 bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u) {
@@ -1191,12 +1196,12 @@ __device__ __forceinline__ int gemm_q_makespan(int pairs, int singles, int n) {
   return end;
 }
 
-__global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
+__device__ __forceinline__ void gemm_q_tiles_body(const GemmListArgs& a) {
   __shared__ int s_warp[32];
   __shared__ int s_warp_t[32];
   __shared__ int s_carry, s_carry_t, s_pairs_total, s_best;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid < 32) s_warp[tid] = s_warp_t[tid] = 0;   // (a CTA may have fewer warps)
   const int mt = a.m / 128, nt = a.n / 128;
   const int rows = a.batch * mt;
   const bool one_walk = rows <= static_cast<int>(blockDim.x);
@@ -1321,16 +1326,21 @@ __global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(1024) gemm_q_tiles_kernel(GemmListArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  gemm_q_tiles_body(a);
+}
+
 // GEMM-O: per 128-row block the ascending list of selected local heads, plus the row blocks sorted
 // by descending list length (stable). counters[0] = number of row blocks, counters[1] = total heads.
-__global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
+__device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
   __shared__ int s_warp[32];
   __shared__ int s_carry;
   extern __shared__ int s_hist[];  // local_heads + 2 buckets
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mt = a.m / 128;
   const int rows = a.batch * mt;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid < 32) s_warp[tid] = 0;   // (a CTA may have fewer warps)
   const int local_heads = a.k / a.head_dim;
   const int want = a.is_for_cache ? 0 : 1;
   // At most one row block per thread: a row's place in the order is the number of longer rows (and of equal ones in front
@@ -1439,6 +1449,42 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
       __syncwarp();
     }
   }
+}
+
+__global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  gemm_o_rows_body(a);
+}
+
+// The lists of a whole layer step (GEMM-Q tiles, GEMM-O rows, attention items and units) in one launch: they only share
+// the masks, so each kind has CTAs of its own. In front of a small layer three launches in a row, each a few
+// microseconds of latency, were as long as the projection they ran beside.
+__global__ void __launch_bounds__(kSmallThreads) layer_lists_kernel(CompactArgs a, UnitArgs u, int by_length, int heads_per_group,
+                                                                    GemmListArgs q, GemmListArgs o) {
+  if (blockIdx.x == 0) {
+    gemm_q_tiles_body(q);
+  } else if (blockIdx.x == 1) {
+    gemm_o_rows_body(o);
+  } else {
+    ZeroArgs z;
+    z.out = nullptr;
+    z.token_bytes = 0;
+    z.head_bytes = 16;
+    attn_lists_small_body(a, u, z, by_length, heads_per_group, static_cast<int>(blockIdx.x) - 2);
+  }
+}
+
+cudaError_t launch_layer_lists(const CompactArgs& a, const UnitArgs& u, const GemmListArgs& q, const GemmListArgs& o,
+                               cudaStream_t stream) {
+  int by_length, hpg;
+  order_rule(a, &by_length, &hpg);
+  const int wpb = kSmallThreads / 32;
+  const int blocks = static_cast<int>((a.n_cand + wpb - 1) / wpb) + 2;
+  size_t smem = static_cast<size_t>(a.n_cand) * 8;
+  const size_t hist = static_cast<size_t>(o.k / o.head_dim + 2) * sizeof(int);
+  if (smem < hist) smem = hist;
+  layer_lists_kernel<<<blocks, kSmallThreads, smem, stream>>>(a, u, by_length, hpg, q, o);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_gemm_q_tiles(const GemmListArgs& a, cudaStream_t stream) {

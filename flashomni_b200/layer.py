@@ -127,13 +127,14 @@ class SparseDiTAttentionBlock:
             flashomni_gemm(x, self.wkv, H, is_full=True, out=self.kv, head_dim=D)
         else:
             flashomni_gemm(x, self.w.wk, H, is_full=True, out=self.k, head_dim=D)
-        self._side.wait_event(self._start)
-        self._q_list = prepare_gemm_q_list(self.B, self.S, n_local, H, sparse_info, sparse_info_indptr, 0,
-                                           head_begin=hb, head_dim=D, into=self._q_list, stream=self._side)
-        self.wrapper.prepare_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
-                                   stream=self._side, after=self._start)
-        self._o_list = prepare_gemm_o_list(self.B, self.S, n_local, H, sparse_info, sparse_info_indptr, 0,
-                                           head_begin=hb, head_dim=D, into=self._o_list, stream=self._side)
+        key = (self.B, self.S, n_local, D, False)
+        if all(wl is not None and wl.key == key and wl.ws.device == self.wrapper.device for wl in (self._q_list, self._o_list)) \
+                and sparse_info_indptr.dtype == torch.int32 and sparse_kv_info_indptr.dtype == torch.int32:
+            # from the second step on the three lists go into the storage they have, with one call
+            self.wrapper.prepare_layer_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
+                                             self._q_list, self._o_list, self.S, n_local, self._side, self._start)
+        else:
+            self._first_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, n_local)
         if self.fuse_kv:
             kv = self.kv.view(T, 2 * self.hc, D)
             k, v = kv[:, :self.hc], kv[:, self.hc:]
@@ -149,6 +150,17 @@ class SparseDiTAttentionBlock:
                                  self.cache if self.add_cache else None,
                                  is_for_cache=False, head_begin=hb, head_dim=D, out=y, worklist=self._o_list)
         return y
+
+    def _first_lists(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, n_local):
+        """The three lists one by one, in new storage for the GEMM lists if there is none."""
+        H, D, hb = self.H, self.D, self.hb
+        self._side.wait_event(self._start)
+        self._q_list = prepare_gemm_q_list(self.B, self.S, n_local, H, sparse_info, sparse_info_indptr, 0,
+                                           head_begin=hb, head_dim=D, into=self._q_list, stream=self._side)
+        self.wrapper.prepare_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
+                                   stream=self._side, after=self._start)
+        self._o_list = prepare_gemm_o_list(self.B, self.S, n_local, H, sparse_info, sparse_info_indptr, 0,
+                                           head_begin=hb, head_dim=D, into=self._o_list, stream=self._side)
 
 
 class UlyssesSparseDiTAttentionBlock:

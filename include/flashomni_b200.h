@@ -304,6 +304,19 @@ FO_API int fo_gemm_o_worklist(int32_t batch, int32_t m, int32_t k, int32_t num_h
                        const int32_t* sparse_info_indptr, void* workspace, size_t workspace_bytes,
                        void* stream);
 
+/* ---- every list of a layer step ------------------------------------------------------------------------
+ * fo_gemm_q_worklist (m x n_local, head_dim) into q_workspace, fo_attn_lists (not full, nothing zeroed) and
+ * fo_gemm_o_worklist (k = n_local, active heads) into o_workspace from the same masks, in one launch when the mask is
+ * small (see fo_attn_lists). `plan` is a host array with the arguments of fo_attn_lists that do not change from step to
+ * step, in its order: [0] qo_indptr, kv_indptr, [2] batch, num_heads, head_begin, head_count, [6] sbq, sbkv, [8] n_cand,
+ * max_nkv, max_items, max_kept, [12] items, kv_ptr, kv_idx, order, counters, scratch, scratch_bytes, [19] min_items,
+ * num_streams, min_chunk, max_units, max_slots, [24] units, unit_counters, arrive. */
+FO_API int fo_layer_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
+                          int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr,
+                          const int32_t* sparse_kv_info_indptr, const int64_t* plan, int32_t m, int32_t n_local,
+                          int32_t head_dim, int32_t num_text_tokens, void* q_workspace, size_t q_workspace_bytes,
+                          void* o_workspace, size_t o_workspace_bytes, void* stream);
+
 /* ---- GEMM-Q / GEMM-O over a work list built earlier -------------------------------------------------
  * No counterpart in the reference. Same computation as fo_gemm_q (sparse) / fo_gemm_o, but the work list is
  * taken from `workspace` as fo_gemm_q_worklist / fo_gemm_o_worklist left it (same batch, m, n / k, head_dim),

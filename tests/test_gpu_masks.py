@@ -243,6 +243,57 @@ def test_gemm_worklists_bit_exact(cuda_device):
             assert np.array_equal(w[o0:o0 + R], rorder)
 
 
+@pytest.mark.parametrize("rows", [1, 31, 33, 1024, 1025])   # one row block per thread of the list kernels, and one more
+def test_gemm_worklists_row_counts(cuda_device, rows):
+    lib = _native.load()
+    H, rng = 5, np.random.default_rng(rows)
+    m = wl.pack_masks([(rng.random((rows, H)) < 0.5).astype(np.uint8)], [np.zeros((rows, H, 1), np.uint8)])
+    si, _, ip, _ = masks_to_device(m, cuda_device)
+    ws = torch.zeros(lib.fo_gemm_workspace_bytes(1, rows * 128, H * 128, H * 128, 128), dtype=torch.uint8, device=cuda_device)
+    st = torch.cuda.current_stream(cuda_device).cuda_stream
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    mask = (_native.ptr(si), si.numel(), _native.ptr(ip), _native.ptr(ws), ws.numel(), st)
+    _native.check(lib.fo_gemm_q_worklist(1, rows * 128, H * 128, H, 0, 128, 128, 0, 0, *mask), "fo_gemm_q_worklist")
+    w = ws.view(torch.int32).cpu().numpy()
+    ref = om.gemm_q_tile_pairs(m.sparse_info, m.info_indptr, 1, rows * 128, H * 128, H, 128, 0, head_dim=128, num_ctas=sms)
+    assert w[0] == len(ref) and w[2] == 0 and np.array_equal(w[8:8 + 4 * len(ref)].reshape(-1, 4), ref)
+    for cache in (0, 1):
+        _native.check(lib.fo_gemm_o_worklist(1, rows * 128, H * 128, H, 0, 128, 128, 0, cache, *mask), "fo_gemm_o_worklist")
+        w = ws.view(torch.int32).cpu().numpy()
+        rip, rheads, rorder = om.gemm_o_rows(m.sparse_info, m.info_indptr, 1, rows * 128, H * 128, H, 128, 0, bool(cache))
+        o0 = 8 + rows + 1 + rows * H
+        assert np.array_equal(w[8:8 + rows + 1], rip) and np.array_equal(w[8 + rows + 1:8 + rows + 1 + len(rheads)], rheads)
+        assert np.array_equal(w[o0:o0 + rows], rorder)
+
+
+# smallest; the image layer with a head window; past the one-launch size
+@pytest.mark.parametrize("B,nb,H,hb,hc", [(1, 1, 1, 0, 1), (2, 36, 24, 6, 5), (1, 180, 23, 0, 23)])
+def test_layer_lists_in_one_call_match_the_separate_ones(cuda_device, B, nb, H, hb, hc):
+    from flashomni_b200.gemm import prepare_gemm_o_list, prepare_gemm_q_list
+    masks = masks_to_device(wl.flux_masks(B, H, nb, nb, 0.5, seed=5, text_blocks=min(4, nb)), cuda_device)
+    S, n = nb * 128, hc * 128
+    indptr = torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * S
+    side, ev = torch.cuda.Stream(cuda_device), torch.cuda.Event()
+    got = []
+    for together in (False, True):
+        w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device))
+        w.plan(indptr, indptr, hc, hc, 128, q_data_type=torch.bfloat16, mask_num_heads=H, mask_head_begin=hb)
+        lists = [f(B, S, n, H, masks[0], masks[2], 0, head_begin=hb, head_dim=128) for f in (prepare_gemm_q_list, prepare_gemm_o_list)]
+        if together:
+            for wlist in lists:
+                wlist.ws.zero_()
+            ev.record()
+            w.prepare_layer_lists(*masks, *lists, S, n, side, ev)
+        else:
+            w.build_work_lists(*masks)
+        torch.cuda.synchronize()
+        got.append((w.work_lists(), [wlist.ws.cpu() for wlist in lists]))
+    _assert_lists_equal(got[1][0], dict(got[0][0], items=got[0][0]["items"]))
+    assert np.array_equal(got[0][0]["units"], got[1][0]["units"])
+    for a, b in zip(got[0][1], got[1][1]):
+        assert torch.equal(a, b)
+
+
 def test_strided_gather_matches_torch(cuda_device):
     """fo_strided_gather on local buffers: the two layouts of the sequence-parallel exchange."""
     from flashomni_b200.parallel import PeerExchange
