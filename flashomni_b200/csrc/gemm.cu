@@ -64,7 +64,8 @@ struct TileInfo {
   const int32_t* heads;  // GEMM-O: selected heads of the row block (null for GEMM-Q)
 };
 
-__device__ __forceinline__ int pairs_per_row(const GemmArgs& a) { return (a.n / kBNH + 1) / 2; }
+// tiles per row block where the launch has no tile list: pairs of column blocks, or single blocks (launch_gemm)
+__device__ __forceinline__ int tiles_per_row(const GemmArgs& a) { return a.single ? a.n / kBNH : (a.n / kBNH + 1) / 2; }
 
 __device__ __forceinline__ int num_tiles(const GemmArgs& a) {
   if (a.mode == kGemmQ && a.tiles != nullptr) {
@@ -72,7 +73,7 @@ __device__ __forceinline__ int num_tiles(const GemmArgs& a) {
     const int n = *a.n_tiles_ptr;
     return n < cap ? (n < 0 ? 0 : n) : cap;
   }
-  return a.batch * (a.m / kBM) * pairs_per_row(a);
+  return a.batch * (a.m / kBM) * tiles_per_row(a);
 }
 
 __device__ __forceinline__ TileInfo get_tile(const GemmArgs& a, int t) {
@@ -87,11 +88,11 @@ __device__ __forceinline__ TileInfo get_tile(const GemmArgs& a, int t) {
     ti.heads = nullptr;
     return ti;
   }
-  const int npr = pairs_per_row(a);
+  const int npr = tiles_per_row(a);
   const int j = t % npr;
   const int rr = t / npr;
-  ti.w_row0 = (2 * j) * kBNH;
-  ti.w_row1 = (2 * j + 1 < nct) ? (2 * j + 1) * kBNH : -1;
+  ti.w_row0 = (a.single ? j : 2 * j) * kBNH;
+  ti.w_row1 = (!a.single && 2 * j + 1 < nct) ? (2 * j + 1) * kBNH : -1;
   if (a.mode == kGemmQ) {  // dense: row blocks in natural order
     ti.a_row = rr * kBM;
     ti.nkb = (a.k + kBK - 1) / kBK;  // a last partial K block reads zeros past k (TMA fill)
@@ -461,13 +462,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 
 
 cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream) {
-  const int cap = a.batch * (a.m / kBM) * ((a.mode == kGemmQ && a.tiles != nullptr) ? a.n / kBNH : (a.n / kBNH + 1) / 2);
+  // Without a tile list (GEMM-O, dense): when even the single 128 x 128 tiles fit the CTAs in one round, they are the
+  // tiles. A pair tile moves 25 % fewer operand bytes per FLOP, which is what counts once the SMs are full, but here it
+  // would leave half of them idle and take twice the MMAs and the epilogue on the others. GEMM-O kernel
+  // on a B200, 24 heads of 128: 24, 96 and 144 single tiles 24.3, 22.9 and 23.3 us, as 12, 48 and 72 pairs 29.3, 27.8 and 28.2
+  // us; dense with K = 1024: 10.9-11.8 against 12.8-13.3 us. With one tile more than CTAs a second round would cost
+  // more than that.
+  GemmArgs g = a;
+  const bool listed = a.mode == kGemmQ && a.tiles != nullptr;
+  const int blocks = a.batch * (a.m / kBM) * (a.n / kBNH);
+  g.single = !listed && blocks <= max_ctas ? 1 : 0;
+  const int cap = listed || g.single ? blocks : a.batch * (a.m / kBM) * ((a.n / kBNH + 1) / 2);
   if (cap <= 0) return cudaSuccess;
   const int grid = cap < max_ctas ? cap : max_ctas;
   const auto kernel = a.is_bf16 ? gemm_kernel<true> : gemm_kernel<false>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return e;
-  return launch_dependent(kernel, grid, kThreads, kSmemBytes, stream, a.after_list != 0, a);
+  return launch_dependent(kernel, grid, kThreads, kSmemBytes, stream, g.after_list != 0, g);
 }
 
 }  // namespace fo

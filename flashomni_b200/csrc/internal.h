@@ -131,6 +131,7 @@ struct GemmArgs {
   const int32_t* row_order;
   int32_t* status;                 // device status word (DevStatus)
   int32_t* cursor;                 // device-wide tile cursor, zero when the kernel starts
+  int single;                      // no tile list: tiles of one column block instead of two (set by launch_gemm)
   int after_list;                  // the launch in front of this one builds the list (dependent launch)
 };
 cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream);

@@ -171,3 +171,62 @@ def test_list_storage_made_behind_pending_work_is_not_wiped(cuda_device):
         got = prepare(B, S, H * 128, H, si, ip, 0, stream=side)
         torch.cuda.synchronize()
         assert torch.equal(want.ws, got.ws)
+
+
+# one column block; an odd count; as many 128 x 128 tiles as CTAs of a B200 (148: single tiles), one row block more (pairs)
+@pytest.mark.parametrize("nb,hid", [(1, 128), (3, 640), (4, 37 * 128), (37, 512), (38, 512)])
+@pytest.mark.parametrize("for_cache", [False, True])
+def test_gemm_o_tile_width_by_launch_size(cuda_device, nb, hid, for_cache):
+    H = 3
+    m = wl.flux_masks(1, H, nb, nb, 0.5, seed=nb, text_blocks=1)
+    si, _, ip, _ = masks_to_device(m, cuda_device)
+    x = wl.randn_bf16((1, nb * 128, H * 128), 4); w = wl.randn_bf16((hid, H * 128), 5, std=(H * 128) ** -0.5)
+    init = wl.randn_bf16((hid,) if for_cache else (1, nb * 128, hid), 6)
+    y = fo.flashomni_gemm_reduction(dev(x, cuda_device), dev(w, cuda_device), H, si, ip, 0, dev(init, cuda_device),
+                                    is_for_cache=for_cache, head_dim=128)
+    ref = og.gemm_o(x, w, H, m.sparse_info, m.info_indptr, 0, init, for_cache)
+    _status_ok()
+    assert_close_bf16(y, ref, f"gemm_o {nb} x {hid}", allow_ulp=1.0)
+
+
+def test_calls_that_build_their_own_lists_replay_from_a_graph(cuda_device):
+    """List kernel and dependent launch as a captured pair: GEMM-Q, attention and GEMM-O in a row, on masks selected in
+    the same graph, twice, the second time with other inputs."""
+    H, nb, D = 4, 6, 128
+    S, hid = nb * 128, 512
+    indptr = torch.tensor([0, S], dtype=torch.int32, device=cuda_device)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device))
+    w.plan(indptr, indptr, H, H, D, q_data_type=torch.bfloat16)
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda_device)
+    x, wq, wo = rnd(1, S, hid).bfloat16(), (rnd(H * D, hid) * hid ** -0.5).bfloat16(), (rnd(hid, H * D) * 0.04).bfloat16()
+    k, v, cache, score = rnd(S, H, D).bfloat16(), rnd(S, H, D).bfloat16(), rnd(1, S, hid).bfloat16(), rnd(1, H, nb, nb)
+    q, attn = torch.zeros(1, S, H * D, dtype=torch.bfloat16, device=cuda_device), torch.zeros_like(k)
+
+    def step():
+        m = fo.select_blocks(score, 1, 0.3, 0.4)
+        fo.flashomni_gemm(x, wq, H, m[0], m[2], 0, None, out=q)
+        w.run(q.view(S, H, D), k, v, *m, out=attn)
+        return fo.flashomni_gemm_reduction(attn.view(1, S, H * D), wo, H, m[0], m[2], 0, cache, head_dim=D)
+
+    side = torch.cuda.Stream(cuda_device)
+    side.wait_stream(torch.cuda.current_stream(cuda_device))
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        y = step()
+    for _ in range(2):
+        x.copy_(rnd(*x.shape))
+        score.copy_(rnd(*score.shape))
+        q.zero_(), attn.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        got = y.clone()
+        q.zero_(), attn.zero_()
+        want = step()
+        torch.cuda.synchronize()
+        w.check_status()
+        # the order in which a q-block's row sums are added depends on the CTA that draws it: bf16 steps of O, through GEMM-O
+        assert (got.float() - want.float()).abs().max() <= 2 ** -5
