@@ -58,6 +58,20 @@ def _cast_fp8(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return out
 
 
+def _cast_fp8_pair(k: torch.Tensor, v: torch.Tensor, dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor]:
+    """`_cast_fp8` of both, in one launch when their sizes match."""
+    if k.shape != v.shape or k.numel() % 8 != 0:   # (the second copy starts on a 16-byte boundary)
+        return _cast_fp8(k, dtype), _cast_fp8(v, dtype)
+    k, v = k.contiguous(), v.contiguous()
+    out = torch.empty((2, *k.shape), dtype=dtype, device=k.device)
+    kc, vc = out[0], out[1]
+    with torch.cuda.device(k.device):
+        _native.check(_native.load().fo_cast_fp8_pair(
+            k.data_ptr(), v.data_ptr(), k.numel(), _FP8_KINDS[k.dtype], native_dtype(dtype), kc.data_ptr(), vc.data_ptr(),
+            _native.current_stream(k.device)), "fo_cast_fp8_pair")
+    return kc, vc
+
+
 class BatchFlashOmniFAWithRaggedKVWrapper:
     r"""Prefill attention over ragged q/k/v with two bit-packed block masks: `sparse_info` selects the
     (q-block, head) pairs that are computed at all, `sparse_kv_info` the kv-blocks each of them attends
@@ -409,7 +423,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if v.dtype != k.dtype:
             raise ValueError(f"v has dtype {v.dtype}, k has {k.dtype}")
         if k.dtype in _FP8_KINDS:
-            k, v = _cast_fp8(k, q.dtype), _cast_fp8(v, q.dtype)
+            k, v = _cast_fp8_pair(k, v, q.dtype)
         sm_scale = self._sm_scale
         if sm_scale is None:
             sm_scale = 1.0 / math.sqrt(q.size(-1))

@@ -541,16 +541,30 @@ int fo_sparse_attn_fwd_custom_mask(const void* q, const void* k, const void* v, 
                           stream);
 }
 
-int fo_cast_fp8(const void* src, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst, void* stream) {
-  if (n < 0) return fail(FO_ERR_INVALID_ARG, "fo_cast_fp8: n < 0");
+namespace {
+int cast_fp8_impl(const char* who, const void* src0, const void* src1, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst0,
+                  void* dst1, bool pair, void* stream) {
+  if (n < 0) return fail(FO_ERR_INVALID_ARG, std::string(who) + ": n < 0");
   if (n == 0) return FO_OK;
-  if (src == nullptr || dst == nullptr || !aligned16(src) || !aligned16(dst))
-    return fail(FO_ERR_INVALID_ARG, "fo_cast_fp8: null or misaligned pointer (16 bytes)");
+  if (src0 == nullptr || dst0 == nullptr || !aligned16(src0) || !aligned16(dst0) ||
+      (pair && (src1 == nullptr || dst1 == nullptr || !aligned16(src1) || !aligned16(dst1))))
+    return fail(FO_ERR_INVALID_ARG, std::string(who) + ": null or misaligned pointer (16 bytes)");
   if ((fp8_kind != 0 && fp8_kind != 1) || (dtype != FO_DTYPE_F16 && dtype != FO_DTYPE_BF16))
-    return fail(FO_ERR_INVALID_ARG, "fo_cast_fp8: fp8_kind must be 0 (e4m3) or 1 (e5m2), dtype f16 or bf16");
-  const cudaError_t e = launch_cast_fp8(src, n, fp8_kind, dtype == FO_DTYPE_BF16, dst, sm_count(), static_cast<cudaStream_t>(stream));
+    return fail(FO_ERR_INVALID_ARG, std::string(who) + ": fp8_kind must be 0 (e4m3) or 1 (e5m2), dtype f16 or bf16");
+  const cudaError_t e = launch_cast_fp8(src0, src1, n, fp8_kind, dtype == FO_DTYPE_BF16, dst0, dst1, sm_count(),
+                                        static_cast<cudaStream_t>(stream));
   count_launches(1);
-  return e == cudaSuccess ? FO_OK : fail_cuda("fo_cast_fp8", e);
+  return e == cudaSuccess ? FO_OK : fail_cuda(who, e);
+}
+}  // namespace
+
+int fo_cast_fp8(const void* src, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst, void* stream) {
+  return cast_fp8_impl("fo_cast_fp8", src, nullptr, n, fp8_kind, dtype, dst, nullptr, false, stream);
+}
+
+int fo_cast_fp8_pair(const void* src0, const void* src1, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst0, void* dst1,
+                     void* stream) {
+  return cast_fp8_impl("fo_cast_fp8_pair", src0, src1, n, fp8_kind, dtype, dst0, dst1, true, stream);
 }
 
 // ------------------------------------------------------------------------------------------ GEMMs

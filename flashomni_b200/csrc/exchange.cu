@@ -120,7 +120,10 @@ __global__ void __launch_bounds__(64) peer_barrier_kernel(const __grid_constant_
 // fp8 K / V fragments before the MMA (a plain cast, no scales; include/flashomni/attention/prefill.cuh:602-612),
 // done once per tensor here. Every fp8 value is exactly representable in f16 and in bf16.
 template <bool kE5m2, bool kBf16>
-__global__ void __launch_bounds__(256) cast_fp8_kernel(const uint8_t* __restrict__ src, int64_t n, uint16_t* __restrict__ dst) {
+__global__ void __launch_bounds__(256) cast_fp8_kernel(const uint8_t* __restrict__ src0, const uint8_t* __restrict__ src1, int64_t n,
+                                                       uint16_t* __restrict__ dst0, uint16_t* __restrict__ dst1) {
+  const uint8_t* __restrict__ src = blockIdx.y == 0 ? src0 : src1;   // K and V of a call go through one launch
+  uint16_t* __restrict__ dst = blockIdx.y == 0 ? dst0 : dst1;
   const int64_t nvec = n / 16;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -151,20 +154,21 @@ __global__ void __launch_bounds__(256) cast_fp8_kernel(const uint8_t* __restrict
 
 }  // namespace
 
-cudaError_t launch_cast_fp8(const void* src, int64_t n, int e5m2, int is_bf16, void* dst, int sm_count, cudaStream_t stream) {
+cudaError_t launch_cast_fp8(const void* src0, const void* src1, int64_t n, int e5m2, int is_bf16, void* dst0, void* dst1,
+                            int sm_count, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   int64_t blocks = (n / 16 + 255) / 256;
-  const int64_t cap = static_cast<int64_t>(sm_count) * 8;
+  const int64_t cap = static_cast<int64_t>(sm_count) * (src1 != nullptr ? 4 : 8);
   blocks = blocks > cap ? cap : (blocks < 1 ? 1 : blocks);
-  const uint8_t* s = static_cast<const uint8_t*>(src);
-  uint16_t* d = static_cast<uint16_t*>(dst);
-  const unsigned g = static_cast<unsigned>(blocks);
+  const uint8_t *s0 = static_cast<const uint8_t*>(src0), *s1 = static_cast<const uint8_t*>(src1);
+  uint16_t *d0 = static_cast<uint16_t*>(dst0), *d1 = static_cast<uint16_t*>(dst1);
+  const dim3 g(static_cast<unsigned>(blocks), src1 != nullptr ? 2 : 1);
   if (e5m2) {
-    if (is_bf16) cast_fp8_kernel<true, true><<<g, 256, 0, stream>>>(s, n, d);
-    else cast_fp8_kernel<true, false><<<g, 256, 0, stream>>>(s, n, d);
+    if (is_bf16) cast_fp8_kernel<true, true><<<g, 256, 0, stream>>>(s0, s1, n, d0, d1);
+    else cast_fp8_kernel<true, false><<<g, 256, 0, stream>>>(s0, s1, n, d0, d1);
   } else {
-    if (is_bf16) cast_fp8_kernel<false, true><<<g, 256, 0, stream>>>(s, n, d);
-    else cast_fp8_kernel<false, false><<<g, 256, 0, stream>>>(s, n, d);
+    if (is_bf16) cast_fp8_kernel<false, true><<<g, 256, 0, stream>>>(s0, s1, n, d0, d1);
+    else cast_fp8_kernel<false, false><<<g, 256, 0, stream>>>(s0, s1, n, d0, d1);
   }
   return cudaGetLastError();
 }

@@ -101,7 +101,9 @@ struct ZeroArgs {            // output rows of inactive q-blocks that the list b
 };
 bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u);
 cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream);
-cudaError_t launch_cast_fp8(const void* src, int64_t n, int e5m2, int is_bf16, void* dst, int sm_count, cudaStream_t stream);
+// src1 / dst1: a second tensor of the same size, or null
+cudaError_t launch_cast_fp8(const void* src0, const void* src1, int64_t n, int e5m2, int is_bf16, void* dst0, void* dst1,
+                            int sm_count, cudaStream_t stream);
 // the lists of a layer step in one launch (attn_lists_small_applies must hold)
 cudaError_t launch_layer_lists(const CompactArgs& a, const UnitArgs& u, const GemmListArgs& q, const GemmListArgs& o,
                                cudaStream_t stream);

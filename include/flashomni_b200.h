@@ -235,6 +235,9 @@ FO_API int fo_sparse_attn_fwd_custom_mask(const void* q, const void* k, const vo
  * are cast to dtype (exact: every fp8 value is representable in f16 and bf16) into dst; the attention then runs on
  * the 16-bit copy. src and dst 16-byte aligned. */
 FO_API int fo_cast_fp8(const void* src, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst, void* stream);
+/* The same for two tensors of n values each, in one launch. */
+FO_API int fo_cast_fp8_pair(const void* src0, const void* src1, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst0,
+                            void* dst1, void* stream);
 
 /* ---- GEMM-Q / GEMM-O ---------------------------------------------------------------------------
  * Workspace (device, caller-owned, 16-byte aligned) of fo_gemm_workspace_bytes(...) bytes, laid out
