@@ -1201,7 +1201,7 @@ __device__ __forceinline__ void gemm_q_tiles_body(const GemmListArgs& a) {
   __shared__ int s_warp_t[32];
   __shared__ int s_carry, s_carry_t, s_pairs_total, s_best;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 32) s_warp[tid] = s_warp_t[tid] = 0;   // (a CTA may have fewer warps)
+  const int warps = static_cast<int>(blockDim.x) >> 5;   // 32, or the 16 of layer_lists_kernel: only their sums are scanned
   const int mt = a.m / 128, nt = a.n / 128;
   const int rows = a.batch * mt;
   const bool one_walk = rows <= static_cast<int>(blockDim.x);
@@ -1252,7 +1252,7 @@ __device__ __forceinline__ void gemm_q_tiles_body(const GemmListArgs& a) {
         if (lane == 31) { s_warp[warp] = x; s_warp_t[warp] = xt; }
         __syncthreads();
         if (warp == 0) {
-          int w = s_warp[lane], wt = s_warp_t[lane];
+          int w = lane < warps ? s_warp[lane] : 0, wt = lane < warps ? s_warp_t[lane] : 0;
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, w, o);
@@ -1340,7 +1340,7 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mt = a.m / 128;
   const int rows = a.batch * mt;
-  if (tid < 32) s_warp[tid] = 0;   // (a CTA may have fewer warps)
+  const int warps = static_cast<int>(blockDim.x) >> 5;   // as in gemm_q_tiles_body
   const int local_heads = a.k / a.head_dim;
   const int want = a.is_for_cache ? 0 : 1;
   // At most one row block per thread: a row's place in the order is the number of longer rows (and of equal ones in front
@@ -1386,7 +1386,7 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
       a.row_order[rank] = r;
     }
     if (warp == 0) {
-      int w = s_warp[lane];
+      int w = lane < warps ? s_warp[lane] : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, w, o);

@@ -294,6 +294,41 @@ def test_layer_lists_in_one_call_match_the_separate_ones(cuda_device, B, nb, H, 
         assert torch.equal(a, b)
 
 
+# (batch, row blocks a request, mask heads, head window): as many row blocks as the one-launch kernel has threads (512), more,
+# and more than twice as many (three passes of its scans), all within the one-launch size
+@pytest.mark.parametrize("B,nb,H,hb,hc", [(16, 32, 3, 0, 3), (16, 36, 5, 1, 3), (64, 9, 7, 0, 7), (64, 17, 4, 2, 2)])
+def test_layer_lists_of_many_row_blocks_match_the_oracle(cuda_device, B, nb, H, hb, hc):
+    from flashomni_b200.gemm import prepare_gemm_o_list, prepare_gemm_q_list
+    lib, rng = _native.load(), np.random.default_rng(nb)
+    m = wl.pack_masks([(rng.random((nb, H)) < 0.6).astype(np.uint8) for _ in range(B)],
+                      [(rng.random((nb, H, nb)) < 0.5).astype(np.uint8) for _ in range(B)])
+    masks = masks_to_device(m, cuda_device)
+    S, n, R = nb * 128, hc * 128, B * nb
+    indptr = torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * S
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device))
+    w.plan(indptr, indptr, hc, hc, 128, q_data_type=torch.bfloat16, mask_num_heads=H, mask_head_begin=hb)
+    ql, ol = (f(B, S, n, H, masks[0], masks[2], 0, head_begin=hb, head_dim=128) for f in (prepare_gemm_q_list, prepare_gemm_o_list))
+    ql.ws.zero_(), ol.ws.zero_()
+    side, ev = torch.cuda.Stream(cuda_device), torch.cuda.Event()
+    ev.record()
+    before = lib.fo_launch_count()
+    w.prepare_layer_lists(*masks, ql, ol, S, n, side, ev)
+    assert lib.fo_launch_count() == before + 1
+    torch.cuda.synchronize()
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    got = ql.ws.view(torch.int32).cpu().numpy()
+    ref = om.gemm_q_tile_pairs(m.sparse_info, m.info_indptr, B, S, n, H, 128, 0, head_begin=hb, head_dim=128, num_ctas=sms)
+    assert got[0] == len(ref) and got[2] == 0 and np.array_equal(got[8:8 + 4 * len(ref)].reshape(-1, 4), ref)
+    got = ol.ws.view(torch.int32).cpu().numpy()
+    rip, rheads, rorder = om.gemm_o_rows(m.sparse_info, m.info_indptr, B, S, n, H, 128, 0, False, head_begin=hb, head_dim=128)
+    assert got[0] == R and got[1] == len(rheads) and np.array_equal(got[8:8 + R + 1], rip)
+    assert np.array_equal(got[9 + R:9 + R + len(rheads)], rheads)
+    assert np.array_equal(got[9 + R + R * hc:9 + R + R * hc + R], rorder)
+    qo = np.arange(B + 1) * S
+    _assert_lists_equal(w.work_lists(), om.compact(m.sparse_info, m.sparse_kv_info, m.info_indptr, m.kv_info_indptr, qo, qo, H,
+                                                   128, 128, hb, hc))
+
+
 def test_strided_gather_matches_torch(cuda_device):
     """fo_strided_gather on local buffers: the two layouts of the sequence-parallel exchange."""
     from flashomni_b200.parallel import PeerExchange
