@@ -19,6 +19,8 @@
 // whole call 82.4 us with four launches, a memset and threshold arrays, 25.5 us with these two launches.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "internal.h"
 
 namespace fo {
@@ -211,6 +213,8 @@ __device__ __forceinline__ void select_row(const float* __restrict__ x, int len,
 // sequential fp32: a CTA fetches the values of its eighth of the blocks with every thread into shared memory, one thread
 // per block adds them up. The scores then go to all eight CTAs (distributed shared memory), which compute the masses
 // redundantly and rank an eighth of the blocks each, eight lanes per block, against all of them: no sort, no search.
+// Shared memory of another CTA may only be touched once that CTA runs: each announces itself at the cluster barrier on
+// entry and waits there just in front of its first remote store, so that the barrier's latency lies under the score loads.
 constexpr int kSelQThreads = 1024, kSelCluster = 8;
 constexpr int kT2iFloats = 16384;      // values in flight per pass and CTA (64 KB)
 __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelQThreads) select_q_kernel(SelectArgs a) {
@@ -233,6 +237,7 @@ __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelQThrea
   cg::cluster_group cluster = cg::this_cluster();
   const int n_img = a.n - a.t2t;
   if (n_img > 0 && a.t2t > 0) {
+    auto running = cluster.barrier_arrive();
     const int share = (n_img + kSelCluster - 1) / kSelCluster, j0 = rank * share;
     const int cols = n_img - j0 < share ? (n_img - j0 > 0 ? n_img - j0 : 0) : share;
     const int pairs = a.heads * a.t2t, per_pass = kT2iFloats / share;
@@ -253,6 +258,7 @@ __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelQThrea
       }
       __syncthreads();
     }
+    cluster.barrier_wait(std::move(running));
     if (tid < cols) {
 #pragma unroll
       for (int r = 0; r < kSelCluster; ++r) cluster.map_shared_rank(s_t2i, r)[j0 + tid] = acc;

@@ -68,6 +68,19 @@ def test_one_threshold_for_all(cuda_device, n, kind, thr):
     assert np.array_equal(info, rinfo) and np.array_equal(kv, rkv)
 
 
+# few text rows and more requests than fit on the GPU at once: the CTAs of a request reach the exchange of their scores right
+# after they start, at different times
+@pytest.mark.parametrize("B,n", [(1, 2), (3, 9), (200, 9)])
+def test_scores_meet_across_the_cluster(cuda_device, B, n):
+    rng = np.random.default_rng(B)
+    s = (rng.standard_normal((B, 1, n, n)) * 2).astype(np.float32)
+    want = osel.pack_selection(*osel.select_blocks(s, 1, 0.4, 0.3))
+    x = torch.from_numpy(s).to(cuda_device)
+    for got in [fo.select_blocks(x, 1, 0.4, 0.3) for _ in range(50)]:
+        for g, r in zip(got, (want[0], want[1], want[2], want[3])):
+            assert np.array_equal(g.cpu().numpy(), r)
+
+
 def test_feeds_the_hot_path(cuda_device):
     """The emitted tensors go straight into the attention wrapper; the result equals the run on masks packed
     from the CPU statement."""
