@@ -438,15 +438,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if not fresh_out:
             _check_shape_dtype_device(out, q.shape[:-1] + v.shape[-1:], q.dtype, q.device, "out")
         if not is_full:
-            # the reference dereferences null masks here (csrc/batch_sparseFA.cu:123-131); raise instead
-            if sparse_info is None or sparse_kv_info is None or sparse_info_indptr is None \
-                    or sparse_kv_info_indptr is None:
-                raise ValueError("sparse_info, sparse_kv_info and their indptrs are required unless is_full=True")
-            for name, t in (("sparse_info", sparse_info), ("sparse_kv_info", sparse_kv_info)):
-                if t.dtype != torch.uint8 or not t.is_cuda or not t.is_contiguous():
-                    raise ValueError(f"{name} must be a contiguous uint8 CUDA tensor")
-            if len(sparse_info_indptr) != self._batch_size + 1 or len(sparse_kv_info_indptr) != self._batch_size + 1:
-                raise ValueError("mask indptr length must be batch_size + 1")
+            self._check_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr)
             if sparse_info_indptr.dtype != torch.int32:
                 sparse_info_indptr = sparse_info_indptr.to(torch.int32)
             if sparse_kv_info_indptr.dtype != torch.int32:
@@ -524,6 +516,17 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         return tuple((t.data_ptr(), t._version) for t in (sparse_info, sparse_kv_info, sparse_info_indptr,
                                                           sparse_kv_info_indptr))
 
+    def _check_masks(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr) -> None:
+        # the reference dereferences null masks (csrc/batch_sparseFA.cu:123-131); raise instead
+        if sparse_info is None or sparse_kv_info is None or sparse_info_indptr is None \
+                or sparse_kv_info_indptr is None:
+            raise ValueError("sparse_info, sparse_kv_info and their indptrs are required unless is_full=True")
+        for name, t in (("sparse_info", sparse_info), ("sparse_kv_info", sparse_kv_info)):
+            if t.dtype != torch.uint8 or not t.is_cuda or not t.is_contiguous():
+                raise ValueError(f"{name} must be a contiguous uint8 CUDA tensor")
+        if len(sparse_info_indptr) != self._batch_size + 1 or len(sparse_kv_info_indptr) != self._batch_size + 1:
+            raise ValueError("mask indptr length must be batch_size + 1")
+
     def _compact(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream,
                  zero_out=None):
         """Work lists and unit records on `stream`; the rows of inactive q-blocks of `zero_out` (contiguous, laid out like
@@ -567,6 +570,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if not is_full:
             if sparse_info_indptr.dtype != torch.int32 or sparse_kv_info_indptr.dtype != torch.int32:
                 return  # run() will convert and compact itself
+            self._check_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr)
         with torch.cuda.device(self.device):
             if self._prepared_event is None:
                 self._prepared_event = torch.cuda.Event()
@@ -589,9 +593,27 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                             m: int, n_local: int, stream: torch.cuda.Stream, after: torch.cuda.Event) -> None:
         """Extension: `prepare_masks()` together with the GEMM-Q and GEMM-O lists of the same masks (rebuilt in the storage of
         `q_list` / `o_list`, made by `prepare_gemm_q_list` / `prepare_gemm_o_list` for the same shapes), in one call
-        and, for small masks, one launch on `stream`, ordered after the event `after`. int32 indptrs only."""
+        and, for small masks, one launch on `stream`, ordered after the event `after`. Masks as `run()` takes them,
+        contiguous int32 indptrs, all on the wrapper's device."""
         if not self._planned:
             raise RuntimeError("plan() must be called before prepare_layer_lists()")
+        if not self._takes_layer_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr):
+            _native.require_cuda(sparse_info, sparse_info_indptr, sparse_kv_info_indptr)
+            self._check_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr)
+            raise ValueError(f"prepare_layer_lists takes masks and contiguous int32 indptrs on {self.device}")
+        self._layer_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, q_list, o_list, m, n_local,
+                          stream, after)
+
+    def _takes_layer_masks(self, si, skv, ip, kp) -> bool:
+        """Whether these go through `_layer_lists` as they are (once per step of a layer: plain attribute reads)."""
+        dev, n = self.device.index, self._batch_size + 1
+        return (si.get_device() == dev and skv.get_device() == dev and ip.get_device() == dev and kp.get_device() == dev
+                and si.dtype == torch.uint8 and skv.dtype == torch.uint8 and ip.dtype == torch.int32 and kp.dtype == torch.int32
+                and ip.dim() == 1 and kp.dim() == 1 and ip.numel() == n and kp.numel() == n
+                and si.is_contiguous() and skv.is_contiguous() and ip.is_contiguous() and kp.is_contiguous())
+
+    def _layer_lists(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, q_list, o_list, m, n_local,
+                     stream, after) -> None:
         q_list.check("q", self._batch_size, m, n_local, self._head_dim, self.device)
         o_list.check("o", self._batch_size, m, n_local, self._head_dim, self.device)
         p = _native.ptr

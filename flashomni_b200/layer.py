@@ -15,6 +15,7 @@ from typing import Optional
 
 import torch
 
+from . import _native
 from .attention import BatchFlashOmniFAWithRaggedKVWrapper
 from .gemm import flashomni_gemm, flashomni_gemm_reduction, prepare_gemm_o_list, prepare_gemm_q_list
 
@@ -129,10 +130,10 @@ class SparseDiTAttentionBlock:
             flashomni_gemm(x, self.w.wk, H, is_full=True, out=self.k, head_dim=D)
         key = (self.B, self.S, n_local, D, False)
         if all(wl is not None and wl.key == key and wl.ws.device == self.wrapper.device for wl in (self._q_list, self._o_list)) \
-                and sparse_info_indptr.dtype == torch.int32 and sparse_kv_info_indptr.dtype == torch.int32:
+                and self.wrapper._takes_layer_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr):
             # from the second step on the three lists go into the storage they have, with one call
-            self.wrapper.prepare_layer_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
-                                             self._q_list, self._o_list, self.S, n_local, self._side, self._start)
+            self.wrapper._layer_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
+                                      self._q_list, self._o_list, self.S, n_local, self._side, self._start)
         else:
             self._first_lists(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, n_local)
         if self.fuse_kv:
@@ -152,7 +153,10 @@ class SparseDiTAttentionBlock:
         return y
 
     def _first_lists(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, n_local):
-        """The three lists one by one, in new storage for the GEMM lists if there is none."""
+        """The three lists one by one, in new storage for the GEMM lists if there is none. Raises for masks that run() refuses
+        before any of them is read."""
+        _native.require_cuda(sparse_info, sparse_info_indptr)
+        self.wrapper._check_masks(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr)
         H, D, hb = self.H, self.D, self.hb
         self._side.wait_event(self._start)
         self._q_list = prepare_gemm_q_list(self.B, self.S, n_local, H, sparse_info, sparse_info_indptr, 0,

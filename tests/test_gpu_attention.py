@@ -201,6 +201,29 @@ def test_block_forward_is_cuda_graph_capturable(cuda_device, monkeypatch):
     _block_graph_capture(cuda_device)
 
 
+def test_block_refuses_on_every_step_what_it_refuses_on_the_first(cuda_device):
+    """Masks on the host, of another type or length: the later steps take another route to the lists than the first. int64
+    indptrs are taken on every step."""
+    from flashomni_b200.layer import BlockWeights, SparseDiTAttentionBlock
+    H, S, hid = 2, 512, 256
+    masks = masks_to_device(wl.flux_masks(1, H, 4, 4, 0.6, seed=5, text_blocks=1), cuda_device)
+    ws = [dev(wl.randn_bf16((hid, hid), 7 + i, std=hid ** -0.5), cuda_device) for i in range(4)]
+    x = dev(wl.randn_bf16((1, S, hid), 6), cuda_device)
+    blk = SparseDiTAttentionBlock(BlockWeights(*ws), H, 128, 1, S, device=cuda_device)
+    want = blk.forward(x, *masks).clone()
+    bad = [(0, lambda t: t.cpu()), (1, lambda t: t.cpu()), (2, lambda t: t.cpu()), (1, lambda t: t.int()),
+           (1, lambda t: torch.stack([t, t], 1)[:, 0]), (2, lambda t: t[:1]), (3, lambda t: t[:1])]
+    for i, f in bad:
+        m = list(masks)
+        m[i] = f(m[i])
+        with pytest.raises((RuntimeError, ValueError)):
+            blk.forward(x, *m)
+    good = [lambda t: t, lambda t: t.long()]
+    for f in good + [good[0]]:
+        assert torch.equal(blk.forward(x, *masks[:2], f(masks[2]), f(masks[3])), want)
+    blk.wrapper.check_status()
+
+
 def _block_graph_capture(cuda_device):
     """The whole block (projections, side-stream mask compaction, attention, GEMM-O) captured in one CUDA graph
     and replayed gives the eager result (the reference supports graph capture of run(), attention.py:353-377)."""

@@ -70,6 +70,32 @@ def test_cpu_tensors_are_rejected_not_silently_computed():
         fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.zeros(16, dtype=torch.uint8))
 
 
+@pytest.mark.parametrize("which", range(4))
+def test_layer_lists_refuse_host_masks_before_any_native_call(monkeypatch, which):
+    """What would hand a host pointer to a kernel raises first: each mask tensor on the host in turn, the others passing for
+    device tensors."""
+    from flashomni_b200 import _native
+
+    class OnDevice(torch.Tensor):
+        is_cuda = property(lambda self: True)
+
+    class List:
+        def check(self, *a):
+            pass
+
+    def called():
+        raise AssertionError("a native call before the masks were looked at")
+
+    monkeypatch.setattr(_native, "load", called)
+    w = object.__new__(fo.BatchFlashOmniFAWithRaggedKVWrapper)
+    w._planned, w._batch_size, w._head_dim, w.device, w._prepared_event = True, 1, 128, torch.device("cuda:0"), None
+    masks = [torch.zeros(8, dtype=torch.uint8), torch.zeros(8, dtype=torch.uint8), torch.zeros(2, dtype=torch.int32),
+             torch.zeros(2, dtype=torch.int32)]
+    masks = [t if i == which else t.as_subclass(OnDevice) for i, t in enumerate(masks)]
+    with pytest.raises((RuntimeError, ValueError), match="CUDA"):
+        w.prepare_layer_lists(*masks, List(), List(), 128, 128, None, None)
+
+
 def test_bitorder_and_shape_validation():
     with pytest.raises(ValueError):
         fo.packbits(torch.zeros(8, dtype=torch.bool), bitorder="middle")
