@@ -465,11 +465,13 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 prepared = self._prepared_key == self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr,
                                                                 sparse_kv_info_indptr, is_full)
             # An output allocated here reads as zero in q-blocks that are not computed. When this call builds the lists,
-            # and the requests' rows start at row 0, the list builder zeroes exactly those blocks.
+            # and the requests' rows start at row 0, the list builder zeroes exactly those blocks. Not with the caller's
+            # indptr buffers of the graph mode: a captured call may be replayed after a plan() that wrote other requests
+            # into them, whose blocks need not cover the rows of the captured output.
             zero_out = None
             if fresh_out:
                 alloc = torch.zeros
-                if not prepared and self._rows_from_0 and v.size(2) == self._head_dim:
+                if not prepared and self._rows_from_0 and v.size(2) == self._head_dim and not self._use_cuda_graph:
                     alloc = torch.empty
                 out = alloc(q.shape[:-1] + v.shape[-1:], dtype=q.dtype, device=q.device)
                 if alloc is torch.empty:

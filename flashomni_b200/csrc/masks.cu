@@ -964,8 +964,8 @@ cudaError_t launch_attn_units(const UnitArgs& a, cudaStream_t stream) {
 // and of kept blocks in front of it (its item and its offset in kv_idx) and the number of smaller sort keys (its
 // position in the processing order). No scan, no sort, no second pass.
 // A key is (bucket << 12 | candidate): the buckets of the counting sort above, ties by candidate, so the lists are
-// the same word for word. With `zero_out` a warp whose q-block is not active zeroes that block of the output, which
-// saves the caller a pass over the whole tensor.
+// the same word for word. With `zero_out` a warp whose q-block is not active (or whose lists do not fit) zeroes that
+// block of the output, which saves the caller a pass over the whole tensor.
 // Measured on a B200, whole attention call, against the chain and a zeroed allocation: 36 q-blocks x 24 heads x 36
 // kv-blocks at density 0.5 134.8 -> 112.2 us, all blocks 302.2 -> 280.3 us; 3 x 4 x 3 blocks 56.6 -> 36.2 us.
 constexpr int kSmallThreads = 512, kSmallBatch = 64;
@@ -1059,8 +1059,8 @@ __device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, cons
   rank = __reduce_add_sync(0xffffffffu, rank);
   tot_items = __reduce_add_sync(0xffffffffu, tot_items);
   tot_kept = __reduce_add_sync(0xffffffffu, tot_kept);
+  const int status = (tot_kept > a.max_kept || tot_items > a.max_items) ? kDevBadIndex : kDevOk;
   if (c == 0 && lane == 0) {
-    const int status = (tot_kept > a.max_kept || tot_items > a.max_items) ? kDevBadIndex : kDevOk;
     a.counters[0] = tot_items;
     a.counters[1] = tot_kept;
     a.counters[2] = status;
@@ -1076,17 +1076,16 @@ __device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, cons
   const int local = c - s_first[b], qb = local / H, hl = local - qb * H;
   int q_valid = s_ql[b] - qb * a.sbq;
   q_valid = q_valid > a.sbq ? a.sbq : q_valid;
-  if (kept < 0) {
-    if (z.out != nullptr) {
-      const int vecs = z.head_bytes >> 4;   // 16-byte words of one token's share of this mask head
-      uint8_t* dst = z.out + static_cast<int64_t>(s_q0[b] + qb * a.sbq) * z.token_bytes + static_cast<int64_t>(hl) * z.head_bytes;
-      for (int i = lane; i < q_valid * vecs; i += 32) {
-        const int t = i / vecs;
-        *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(t) * z.token_bytes + 16 * (i - t * vecs)) = make_uint4(0u, 0u, 0u, 0u);
-      }
+  // a q-block that nobody computes: not active, or in lists that do not fit (the attention ignores all of those)
+  if (z.out != nullptr && (kept < 0 || status != kDevOk || tot_items > u.max_units)) {
+    const int vecs = z.head_bytes >> 4;   // 16-byte words of one token's share of this mask head
+    uint8_t* dst = z.out + static_cast<int64_t>(s_q0[b] + qb * a.sbq) * z.token_bytes + static_cast<int64_t>(hl) * z.head_bytes;
+    for (int i = lane; i < q_valid * vecs; i += 32) {
+      const int t = i / vecs;
+      *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(t) * z.token_bytes + 16 * (i - t * vecs)) = make_uint4(0u, 0u, 0u, 0u);
     }
-    return;
   }
+  if (kept < 0) return;
   if (off + static_cast<int64_t>(kept) > a.max_kept || pos >= a.max_items || rank >= u.max_units) return;  // flagged above
   const int nkv = s_kl[b] > 0 ? (s_kl[b] + a.sbkv - 1) / a.sbkv : 0;
   const int64_t koff = a.is_full ? 0 : a.kv_info_indptr[b];

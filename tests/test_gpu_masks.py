@@ -205,6 +205,56 @@ def test_allocated_output_is_zero_in_skipped_blocks(cuda_device, H, group, D, le
     assert (got.float() - want.float()).abs().max() <= 2 ** -6
 
 
+def test_allocated_output_is_zero_where_the_lists_do_not_fit(cuda_device):
+    """Lists that outgrow their room are reported and not run; the output is zeros, as ever."""
+    H, D, S = 2, 64, 384
+    ip = torch.tensor([0, S], dtype=torch.int32, device=cuda_device)
+    masks = masks_to_device(wl.pack_masks([np.ones((3, H), np.uint8)], [np.ones((3, H, 3), np.uint8)]), cuda_device)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device))
+    w.plan(ip, ip, H, H, D, q_data_type=torch.bfloat16)
+    args = list(w._list_args)
+    assert args[9] == 3 * 3 * H   # room for the kept kv-blocks
+    args[9] -= 1
+    w._list_args = tuple(args)
+    q = torch.randn(S, H, D, device=cuda_device).bfloat16()
+    junk = torch.full_like(q, 7.0)
+    del junk
+    got = w.run(q, q, q, *masks)
+    assert not got.any()
+    with pytest.raises(RuntimeError):
+        w.check_status()
+
+
+def test_captured_output_is_zero_past_the_rows_of_a_later_plan(cuda_device):
+    """Graph mode: the captured call is replayed with fewer rows than it was captured with; the rest of its output is zeros."""
+    H, D = 2, 128
+    sizes = [torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (300, 200)]
+    bufs = [sizes[0].clone() for _ in range(2)]
+    # every bit set, whatever the block counts
+    masks = masks_to_device(wl.pack_masks([np.ones((3, H), np.uint8)], [np.ones((3, H, 3), np.uint8)]), cuda_device)
+    masks[0].fill_(255), masks[1].fill_(255)
+    q = torch.randn(300, H, D, device=cuda_device).bfloat16()
+    new = lambda *a: fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=cuda_device), "NHD", *a)
+    w = new(True, *bufs)
+    w.plan(sizes[0], sizes[0], H, H, D, q_data_type=torch.bfloat16)
+    side = torch.cuda.Stream(cuda_device)
+    side.wait_stream(torch.cuda.current_stream(cuda_device))
+    with torch.cuda.stream(side):
+        w.run(q, q, q, *masks)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        out = w.run(q, q, q, *masks)
+    w.plan(sizes[1], sizes[1], H, H, D, q_data_type=torch.bfloat16)
+    out.fill_(7.0)
+    g.replay()
+    ref = new()
+    ref.plan(sizes[1], sizes[1], H, H, D, q_data_type=torch.bfloat16)
+    want = ref.run(q[:200], q[:200], q[:200], *masks)
+    torch.cuda.synchronize()
+    assert torch.equal(out[:200], want) and not out[200:].any()
+
+
 def test_gemm_worklists_bit_exact(cuda_device):
     lib = _native.load()
     B, H, nq = 2, 24, 36
