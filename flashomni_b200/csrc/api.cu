@@ -167,12 +167,19 @@ int fo_segment_packbits(const uint8_t* x, const int32_t* indptr, const int32_t* 
 int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
                               int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
                               void* stream) {
-  if (num_segments < 0 || capacity < 0) return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: negative size");
+  return fo_segment_packbits_within(x, INT64_MAX, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr,
+                                    total_bytes, stream);
+}
+
+int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                               int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
+                               void* stream) {
+  if (n < 0 || num_segments < 0 || capacity < 0) return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: negative size");
   if (num_segments > 1024) return fail(FO_ERR_UNSUPPORTED, "fo_segment_packbits_sized: at most 1024 segments");
   if (x == nullptr || y == nullptr || indptr == nullptr || new_indptr == nullptr || total_bytes == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: null pointer");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = launch_segment_packbits_sized(x, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr,
+  cudaError_t e = launch_segment_packbits_sized(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr,
                                                 reinterpret_cast<long long*>(total_bytes), st);
   count_launches(1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

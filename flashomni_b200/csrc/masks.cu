@@ -135,13 +135,13 @@ cudaError_t launch_segment_packbits(const uint8_t* x, const int32_t* indptr, con
 
 // The same without a byte indptr in hand: every CTA derives it from the element indptr (a few segments: one scan in shared
 // memory) and packs its share; CTA 0 also writes the byte indptr and, to host memory that the device can write, the
-// total (-1: an indptr that decreases, nothing is packed). What bounds the step is the caller's wait for that total; the
-// byte indptr, its last element and the packing used to be ten launches and a copy: two calls for the masks of 2 x 36
-// q-blocks x 24 heads took 191.5 us on a B200, 66.0 us now.
+// total (-1: an indptr that decreases or leaves the n values of x, nothing is packed). What bounds the step is the
+// caller's wait for that total; the byte indptr, its last element and the packing used to be ten launches and a copy:
+// two calls for the masks of 2 x 36 q-blocks x 24 heads took 191.5 us on a B200, 66.0 us now.
 constexpr int kPackSegs = 1024;
 template <typename Idx>
-__global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8_t* __restrict__ x, const Idx* __restrict__ indptr,
-                                                                     int num_segments, int64_t capacity, int little,
+__global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8_t* __restrict__ x, int64_t n,
+                                                                     const Idx* __restrict__ indptr, int num_segments, int64_t capacity, int little,
                                                                      uint8_t* __restrict__ y, int32_t* __restrict__ new_indptr,
                                                                      long long* __restrict__ total_out) {
   __shared__ int64_t s_in[kPackSegs + 1];
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8
       if (i < num_segments) s_new[i + 1] = static_cast<int32_t>(carry + v);
       carry += __shfl_sync(0xffffffffu, v, 31);
     }
-    bad = __any_sync(0xffffffffu, bad) || carry > 0x7fffffffLL || carry > capacity || s_in[0] < 0;
+    bad = __any_sync(0xffffffffu, bad) || carry > 0x7fffffffLL || carry > capacity || s_in[0] < 0 || s_in[num_segments] > n;
     if (tid == 0) {
       s_new[0] = 0;
       s_bad = bad ? 1 : 0;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8
   }
 }
 
-cudaError_t launch_segment_packbits_sized(const uint8_t* x, const void* indptr, int indptr_is_64, int num_segments,
+cudaError_t launch_segment_packbits_sized(const uint8_t* x, int64_t n, const void* indptr, int indptr_is_64, int num_segments,
                                           int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, long long* total_out,
                                           cudaStream_t stream) {
   if (num_segments > kPackSegs) return cudaErrorInvalidValue;
@@ -209,10 +209,10 @@ cudaError_t launch_segment_packbits_sized(const uint8_t* x, const void* indptr, 
   if (blocks < 1) blocks = 1;
   if (indptr_is_64)
     segment_packbits_sized_kernel<int64_t><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        x, static_cast<const int64_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
+        x, n, static_cast<const int64_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
   else
     segment_packbits_sized_kernel<int32_t><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        x, static_cast<const int32_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
+        x, n, static_cast<const int32_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
   return cudaGetLastError();
 }
 

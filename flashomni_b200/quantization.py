@@ -46,6 +46,7 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
     little = _little(bitorder)
     _native.require_cuda(x)
     n_seg = len(indptr) - 1
+    refused = False
     # The usual call: the byte indptr, its total and the packed bytes in one launch and one wait. The output is allocated
     # for the most that these segments can need and shortened; anything else takes the general path below.
     if (indptr.dim() == 1 and 1 <= n_seg <= 1024 and indptr.dtype in (torch.int32, torch.int64)
@@ -57,18 +58,29 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
         indptr_new = torch.empty(n_seg + 1, dtype=torch.int32, device=device)
         total = torch.empty(1, dtype=torch.int64, pin_memory=True)
         with torch.cuda.device(device):
-            rc = _native.load().fo_segment_packbits_sized(
-                xb.data_ptr(), ip.data_ptr(), int(ip.dtype == torch.int64), n_seg, capacity, little, y.data_ptr(),
+            rc = _native.load().fo_segment_packbits_within(
+                xb.data_ptr(), xb.numel(), ip.data_ptr(), int(ip.dtype == torch.int64), n_seg, capacity, little, y.data_ptr(),
                 indptr_new.data_ptr(), total.data_ptr(), _native.current_stream(device))
         _native.check(rc, "segment_packbits")
         nbytes = int(total[0])
         if nbytes >= 0:
             return y.narrow(0, 0, nbytes), indptr_new
+        refused = True
     seglen = indptr[1:] - indptr[:-1]
     packed_len = (seglen + 7) // 8
     indptr_new = torch.zeros(len(indptr), dtype=indptr.dtype, device=indptr.device)
-    indptr_new[1:] = torch.cumsum(packed_len, 0)
-    output_nnzs = int(indptr_new[-1].item())
+    torch.cumsum(packed_len, 0, dtype=indptr.dtype, out=indptr_new[1:])
+    # No segment may leave x. An indptr on the device is taken to ascend here, as its ends come with the size at no further
+    # wait; every entry is looked at on the host, and after the kernel above has found something wrong.
+    if indptr.is_cuda and not refused:
+        output_nnzs, lo, hi = (int(v) for v in torch.cat((indptr_new[-1:], indptr[:1], indptr[-1:])).tolist())
+    else:
+        output_nnzs = int(indptr_new[-1].item())
+        ends = (indptr.numpy() if indptr.dtype in (torch.int32, torch.int64) and not indptr.is_cuda else indptr)
+        lo, hi = int(ends.min()), int(ends.max())
+    if lo < 0 or hi > x.numel():   # (an empty segment may lie anywhere)
+        if bool(((seglen > 0) & ((indptr[:-1] < 0) | (indptr[1:] > x.numel()))).any()):
+            raise ValueError(f"segment_packbits: a segment leaves the {x.numel()} values of x")
     device = x.device
     indptr32 = indptr.to(device=device, dtype=torch.int32).contiguous()
     indptr_new = indptr_new.to(device=device, dtype=torch.int32).contiguous()

@@ -81,6 +81,10 @@ FO_API int fo_segment_packbits(const uint8_t* x, const int32_t* indptr, const in
 FO_API int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
                                      int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
                                      int64_t* total_bytes, void* stream);
+/* The same with the number n of values in x: an indptr that ends past them also gives -1 (above, it is read as it is). */
+FO_API int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64,
+                                      int32_t num_segments, int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
+                                      int64_t* total_bytes, void* stream);
 
 /* ---- attention mask compaction (new step; no counterpart op in the reference, which re-reads
  * the bits in the kernel: prefill.cuh:1284-1294,1380-1460) -------------------------------------

@@ -63,6 +63,23 @@ def test_segment_packbits_sizes(cuda_device, lens, start, extra, dtype, indptr_d
     assert np.array_equal(nip.cpu().numpy(), rip) and np.array_equal(y.cpu().numpy(), ry)
 
 
+# a start and an end past the values, an end of few more, a negative start; on the one-launch path and past its segment count
+@pytest.mark.parametrize("indptr", [[1000000, 1000100], [0, 50, 107], [-8, 100], [0] * 1100 + [101]])
+@pytest.mark.parametrize("indptr_device", ["cuda", "cpu"])
+def test_segments_outside_the_input_are_refused(cuda_device, indptr, indptr_device):
+    x = torch.ones(100, dtype=torch.uint8, device=cuda_device)
+    with pytest.raises(ValueError):
+        fo.segment_packbits(x, torch.tensor(indptr, dtype=torch.int32, device=indptr_device))
+    torch.cuda.synchronize()
+
+
+def test_segments_that_read_nothing_may_lie_anywhere(cuda_device):
+    x = torch.ones(100, dtype=torch.uint8, device=cuda_device)
+    for indptr, want in (([500, 500], []), ([96, 100, 97, 100], [240, 224])):   # (a step back of less than 8 packs nothing)
+        y, ip = fo.segment_packbits(x, torch.tensor(indptr, dtype=torch.int32, device=cuda_device))
+        assert y.tolist() == want and int(ip[-1]) == len(want)
+
+
 def _compact_gpu(device, m, qo, kv, H, head_begin=0, head_count=None, is_full=False):
     hc = H - head_begin if head_count is None else head_count
     w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1024, dtype=torch.uint8, device=device))
