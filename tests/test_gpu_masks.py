@@ -73,6 +73,12 @@ def test_segments_outside_the_input_are_refused(cuda_device, indptr, indptr_devi
     torch.cuda.synchronize()
 
 
+def test_packed_bytes_of_a_few_segments_hold_no_memory_for_the_rest(cuda_device):
+    x = torch.ones(1 << 24, dtype=torch.uint8, device=cuda_device)
+    y, _ = fo.segment_packbits(x, torch.tensor([5, 5 + 16], dtype=torch.int32, device=cuda_device))
+    assert y.tolist() == [255, 255] and y.untyped_storage().nbytes() <= 1 << 20
+
+
 def test_segments_that_read_nothing_may_lie_anywhere(cuda_device):
     x = torch.ones(100, dtype=torch.uint8, device=cuda_device)
     for indptr, want in (([500, 500], []), ([96, 100, 97, 100], [240, 224])):   # (a step back of less than 8 packs nothing)
