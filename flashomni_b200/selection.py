@@ -7,6 +7,7 @@ The reference builds its masks with torch ops and Triton fill kernels on an unpa
 
 from __future__ import annotations
 
+import math
 from typing import Tuple, Union
 
 import torch
@@ -14,6 +15,7 @@ import torch
 from . import _native
 
 Threshold = Union[float, torch.Tensor]
+_FLT_MAX = torch.finfo(torch.float32).max
 
 
 def _threshold(t: Threshold, n: int, device, what: str) -> torch.Tensor:
@@ -53,6 +55,8 @@ def select_blocks(pooled_score: torch.Tensor, num_text_blocks: int, q_threshold:
     scratch = torch.empty(lib.fo_select_blocks_scratch_bytes(B, n), dtype=torch.uint8, device=dev)
     if uniform:   # passed by value: no threshold arrays to fill
         qthr, kthr, op = float(q_threshold), float(kv_threshold), lib.fo_select_blocks_uniform
+        if _FLT_MAX < abs(qthr) < math.inf or _FLT_MAX < abs(kthr) < math.inf:   # as filling an fp32 array would
+            raise RuntimeError("a threshold cannot be converted to fp32 without overflow")
         thr = (qthr, kthr)
     else:
         qthr, kthr = _threshold(q_threshold, B, dev, "q_threshold"), _threshold(kv_threshold, H, dev, "kv_threshold")

@@ -68,6 +68,14 @@ def test_one_threshold_for_all(cuda_device, n, kind, thr):
     assert np.array_equal(info, rinfo) and np.array_equal(kv, rkv)
 
 
+@pytest.mark.parametrize("thr", [(1e39, 0.3), (0.3, -1e300)])
+def test_thresholds_past_fp32_are_refused(cuda_device, thr):
+    s = torch.zeros(1, 1, 4, 4, device=cuda_device)
+    fo.select_blocks(s, 1, float("inf"), float("nan"))
+    with pytest.raises(RuntimeError, match="overflow"):
+        fo.select_blocks(s, 1, *thr)
+
+
 # few text rows and more requests than fit on the GPU at once: the CTAs of a request reach the exchange of their scores right
 # after they start, at different times
 @pytest.mark.parametrize("B,n", [(1, 2), (3, 9), (200, 9)])
