@@ -1342,10 +1342,6 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
   const int warps = static_cast<int>(blockDim.x) >> 5;   // as in gemm_q_tiles_body
   const int local_heads = a.k / a.head_dim;
   const int want = a.is_for_cache ? 0 : 1;
-  // At most one row block per thread: a row's place in the order is the number of longer rows (and of equal ones in front
-  // of it), counted over the lengths in shared memory. More rows: counting sort by length.
-  const bool by_rank = rows <= static_cast<int>(blockDim.x);
-  __shared__ int s_len[1024];
   if (tid == 0) s_carry = 0;
   for (int i = tid; i <= local_heads; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
@@ -1368,7 +1364,6 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
       }
     }
     int x = cnt;
-    if (by_rank && r < rows) s_len[r] = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1376,14 +1371,6 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    if (by_rank && r < rows) {
-      int rank = 0;
-      for (int o = 0; o < rows; ++o) {
-        const int len = s_len[o];
-        rank += (len > cnt || (len == cnt && o < r)) ? 1 : 0;
-      }
-      a.row_order[rank] = r;
-    }
     if (warp == 0) {
       int w = lane < warps ? s_warp[lane] : 0;
 #pragma unroll
@@ -1397,7 +1384,7 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
     const int off = s_carry + (warp ? s_warp[warp - 1] : 0) + x - cnt;
     if (r < rows) {
       a.row_indptr[r] = off;
-      if (!by_rank) atomicAdd(&s_hist[cnt], 1);
+      atomicAdd(&s_hist[cnt], 1);
       const int b = r / mt, iy = r % mt;
       const int64_t ioff = a.info_indptr[b];
       const int64_t qb = (static_cast<int64_t>(a.num_text_tokens) + static_cast<int64_t>(iy) * 128) / a.sparse_q_size;
@@ -1426,12 +1413,10 @@ __device__ __forceinline__ void gemm_o_rows_body(const GemmListArgs& a) {
     a.counters[4] = kDevOk;  // status word of the GEMM kernel that follows
     a.counters[5] = 0;       // its tile cursor
     a.counters[6] = 0;       // and the count of CTAs that have finished
-    if (!by_rank) {  // bucket starts, descending count
-      int acc = 0;
-      for (int k = local_heads; k >= 0; --k) { const int v = s_hist[k]; s_hist[k] = acc; acc += v; }
-    }
+    // bucket starts, descending count
+    int acc = 0;
+    for (int k = local_heads; k >= 0; --k) { const int v = s_hist[k]; s_hist[k] = acc; acc += v; }
   }
-  if (by_rank) return;
   __syncthreads();
   if (warp == 0) {
     for (int base = 0; base < rows; base += 32) {
