@@ -317,10 +317,11 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         return self._bases()[1]
 
     # Cutting kv lists into parts (split-KV with a merge of partial results) is built and tested but OFF by default:
-    # on a B200 it measured slower at every shape tried (a GPU's share of 3, 6 or 12 heads of the 4608-token layer:
-    # 35 -> 43, 70 -> 79 and 113 -> 138 microseconds). The part is power-capped: SMs that end early leave their share
-    # of the budget to the SMs with long lists, so an even spread of the blocks gains little, and every part pays
-    # an epilogue (fp32 partial result, a CTA-wide hand-over, the merge).
+    # on a B200 it measured slower at every shape tried (3, 6, 12 and 24 heads of two 4608-token requests at density 0.5,
+    # whole call replayed from a graph: 35 -> 51, 58 -> 91, 80 -> 150 and 143 -> 302 microseconds at 2, 4, 8 and 16 units
+    # per SM). The part is power-capped: SMs that end early leave their share of the budget to the SMs with long
+    # lists, so an even spread of the blocks gains little, and every part pays an epilogue (fp32 partial result, a
+    # hand-over between warps, the merge) and its lists take the general path.
     UNITS_PER_SM = 0      # > 0: kv lists are cut when the launch has more than one and at most this many items per SM
     MIN_CHUNK = 16        # shortest part (kv blocks) a kv list is cut into
     FORCE_SPLIT = False   # cut every list into parts of two blocks (tests: every case then runs the merge path)

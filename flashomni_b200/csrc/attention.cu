@@ -62,11 +62,18 @@ constexpr int kWarpEpilogue = kSoftmaxWarps + 4;  // first of the four epilogue 
 constexpr int kEpilogueWarps = 4;
 constexpr int kThreads = (kSoftmaxWarps + 4 + kEpilogueWarps) * 32;  // 768: four softmax warpgroups, producers / issuers, epilogue
 constexpr int kRegsSoftmax = 104, kRegsOther = 32, kRegsEpilogue = 32;  // register split between the warpgroups (setmaxnreg)
+// Where the epilogue also merges the parts of split items, it gets registers for the loads of two parts: with 32 it spilled
+// 412 bytes and waited for one part at a time, and since an item's O is free for the next one only behind it, the launch
+// waited with it. Graph replays on a B200, 2 x 4608 tokens at density 0.5, lists cut at 4 / 8 / 16 units per SM for 6 / 12 / 24
+// heads: 110 / 200 / 369 -> 90.6 / 150 / 302 us (91 / 157 / 312 when the 16 softmax warps merged).
+constexpr int kRegsSoftmaxParts = 96, kRegsEpilogueParts = 64;
 // setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with (threads x the
 // per-thread count the compiler settles on for this block size): a split that asks for more never returns.
 constexpr int kRegsAtLaunch = (65536 / kThreads) / 8 * 8;
 static_assert(kSoftmaxWarps * 32 * kRegsSoftmax + 4 * 32 * kRegsOther + kEpilogueWarps * 32 * kRegsEpilogue <= kThreads * kRegsAtLaunch,
               "register split exceeds the CTA's register pool");
+static_assert(kSoftmaxWarps * 32 * kRegsSoftmaxParts + 4 * 32 * kRegsOther + kEpilogueWarps * 32 * kRegsEpilogueParts <=
+              kThreads * kRegsAtLaunch, "register split exceeds the CTA's register pool");
 constexpr int kTmemCols = 512;
 constexpr uint32_t kColS = 0, kColO = 256, kColP = 384;
 constexpr int kRotStep = FO_ROT_STEP;       // q-block qb starts its kv list at entry (qb * kRotStep) mod length
@@ -550,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     }
   }
   } else if (warp >= kWarpEpilogue) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kParts ? kRegsEpilogueParts : kRegsEpilogue));
     // ------------------------------------------------------------------ epilogue warps: O / l to global memory
     // One thread per q row, 16 columns at a time. O has ONE accumulator, so the next unit's first PV waits until it has
     // been read out: that is on the pipeline's critical path and is all these warps do. (The softmax warps used to do it
@@ -706,18 +713,32 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
             uint32_t v[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t) v[t] = 0u;  // the accumulator (fp32 bit patterns)
-            for (int pp = 0; pp < nparts; ++pp) {
-              const float* pq = base + static_cast<size_t>(pp) * kPartialFloats;
-              const float mp = __ldcg(pq + 128 * 128 + row);
+            auto add = [&](const float4* x, float mp) {
               const float wgt = (mp == -INFINITY) ? 0.f : ex2_approx(mp - m_out);
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                const float4 x = __ldcg(reinterpret_cast<const float4*>(pq + (static_cast<size_t>(col / 4 + q) * 128 + row) * 4));
-                v[4 * q] = __float_as_uint(fmaf(x.x, wgt, __uint_as_float(v[4 * q])));
-                v[4 * q + 1] = __float_as_uint(fmaf(x.y, wgt, __uint_as_float(v[4 * q + 1])));
-                v[4 * q + 2] = __float_as_uint(fmaf(x.z, wgt, __uint_as_float(v[4 * q + 2])));
-                v[4 * q + 3] = __float_as_uint(fmaf(x.w, wgt, __uint_as_float(v[4 * q + 3])));
+                v[4 * q] = __float_as_uint(fmaf(x[q].x, wgt, __uint_as_float(v[4 * q])));
+                v[4 * q + 1] = __float_as_uint(fmaf(x[q].y, wgt, __uint_as_float(v[4 * q + 1])));
+                v[4 * q + 2] = __float_as_uint(fmaf(x[q].z, wgt, __uint_as_float(v[4 * q + 2])));
+                v[4 * q + 3] = __float_as_uint(fmaf(x[q].w, wgt, __uint_as_float(v[4 * q + 3])));
               }
+            };
+            // the loads of two parts in flight at a time: the round trips to L2 are what a merge costs
+            const float* pq = base + (static_cast<size_t>(col / 4) * 128 + row) * 4;
+            const float* pm = base + 128 * 128 + row;
+#pragma unroll 1
+            for (int pp = 0; pp < nparts; pp += 2) {
+              const size_t next = pp + 1 < nparts ? kPartialFloats : 0;
+              float4 x0[4], x1[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) x0[q] = __ldcg(reinterpret_cast<const float4*>(pq + q * 512));
+#pragma unroll
+              for (int q = 0; q < 4; ++q) x1[q] = __ldcg(reinterpret_cast<const float4*>(pq + next + q * 512));
+              const float m0 = __ldcg(pm), m1 = __ldcg(pm + next);
+              add(x0, m0);
+              if (next != 0) add(x1, m1);
+              pq += 2 * static_cast<size_t>(kPartialFloats);
+              pm += 2 * static_cast<size_t>(kPartialFloats);
             }
             emit(col, v);
           }
@@ -738,7 +759,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     }
     if (lane == 0) tma_store_wait_all<0>();
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kParts ? kRegsSoftmaxParts : kRegsSoftmax));
     // ------------------------------------------------------------------ softmax warps 0..15
     // Group X = warp / 8 takes the blocks with g & 1 == X. Two threads per q row: thread
     // (quadrant = warp & 3, half ch = (warp >> 2) & 1, lane) owns row 32 * quadrant + lane (its TMEM lane)
