@@ -363,7 +363,7 @@ int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const u
   z.out = static_cast<uint8_t*>(zero_out);
   z.token_bytes = zero_token_bytes;
   z.head_bytes = zero_head_bytes;
-  if (attn_lists_small_applies(a, u)) {
+  if (attn_lists_small_applies(a, u, z)) {
     const cudaError_t e = launch_attn_lists_small(a, u, z, st);
     count_launches(1);
     t_lists_pending = e == cudaSuccess;
@@ -724,7 +724,7 @@ int fo_layer_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const 
   const GemmListArgs o = make_list_args(so, sparse_info, sparse_info_bytes, sparse_info_indptr, o_workspace);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e;
-  if (attn_lists_small_applies(a, u)) {
+  if (attn_lists_small_fits(a, u)) {
     e = launch_layer_lists(a, u, q, o, st);
     count_launches(1);
   } else {

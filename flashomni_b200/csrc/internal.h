@@ -99,12 +99,13 @@ struct ZeroArgs {            // output rows of inactive q-blocks that the list b
   int64_t token_bytes;       // bytes between tokens
   int head_bytes;            // contiguous bytes of one token that belong to one mask head, a multiple of 16
 };
-bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u);
+bool attn_lists_small_fits(const CompactArgs& a, const UnitArgs& u);
+bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z);
 cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream);
 // src1 / dst1: a second tensor of the same size, or null
 cudaError_t launch_cast_fp8(const void* src0, const void* src1, int64_t n, int e5m2, int is_bf16, void* dst0, void* dst1,
                             int sm_count, cudaStream_t stream);
-// the lists of a layer step in one launch (attn_lists_small_applies must hold)
+// the lists of a layer step in one launch (attn_lists_small_fits must hold)
 cudaError_t launch_layer_lists(const CompactArgs& a, const UnitArgs& u, const GemmListArgs& q, const GemmListArgs& o,
                                cudaStream_t stream);
 cudaError_t launch_gemm_q_tiles(const GemmListArgs& a, cudaStream_t stream);

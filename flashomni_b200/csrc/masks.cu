@@ -1141,11 +1141,21 @@ __global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(Compact
   attn_lists_small_body(a, u, z, by_length, heads_per_group, static_cast<int>(blockIdx.x));
 }
 
-// The line lies where the redundant work stays below the launches it saves: keys have 12 bits for the candidate, and
-// every CTA reads the whole mask (kSmallBits = 32 KB). Cut lists and larger masks take the chain above.
-bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u) {
+// What the kernel can take: keys have 12 bits for the candidate, and every CTA reads the whole mask (kSmallBits = 32 KB).
+// Cut lists and larger masks take the chain above. The lists of a layer step go this way up to here: the chain is six
+// launches for them.
+bool attn_lists_small_fits(const CompactArgs& a, const UnitArgs& u) {
   return a.n_cand > 0 && a.n_cand <= kSmallCand && a.batch <= kSmallBatch && u.max_slots <= 0 && a.max_nkv < (1 << 18) &&
          (a.is_full || a.n_cand * a.max_nkv <= kSmallBits);
+}
+
+// The line lies where the redundant work stays below the launches it saves: it doubles where the CTAs (one per SM, 16
+// candidates each) need a second round. Lists alone, graph replays on a B200, chain against one launch: 2048 candidates
+// 22-26 and 12-14.5 us, 2560 23.3-24.2 and 20.3-22.1, 3072 21-27 and 23-30, 4096 23-29 and 29-31. To the limit of the
+// kernel it goes where the chain has more to do: many requests (4096 candidates of 16 requests 34-35 and 33-34 us, of 64
+// 55-59 and 39), all blocks (21-23 and 20.5), and an output to zero, which the chain zeroes whole.
+bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z) {
+  return attn_lists_small_fits(a, u) && (a.n_cand <= 2560 || a.batch >= 16 || a.is_full || z.out != nullptr);
 }
 
 cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream) {

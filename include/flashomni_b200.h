@@ -143,12 +143,13 @@ FO_API int fo_attn_units(const int32_t* items, const int32_t* kv_ptr, const int3
                          int64_t max_items, int32_t max_nkv, int32_t sbq, int32_t sbkv, int32_t min_items,
                          int32_t num_streams, int32_t min_chunk, int64_t max_units, int64_t max_slots, int32_t* units,
                          int32_t* unit_counters, int32_t* arrive, void* stream);
-/* fo_mask_compact followed by fo_attn_units (same arguments, same lists) in one call; a mask of at most 4096 candidates
- * (and 2^18 kv bits, uncut lists) takes a single launch. With zero_out != NULL the output rows of the q-blocks that are
- * not active are set to zero on the way: zero_out is the output at token 0 and the first head of the window,
- * zero_token_bytes the distance of two tokens, zero_head_bytes the contiguous bytes of a token that belong to one mask
- * head (both multiples of 16), zero_total_bytes the size of the whole contiguous output (larger masks zero all of it;
- * nothing is zeroed when is_full != 0: every block is active then). */
+/* fo_mask_compact followed by fo_attn_units (same arguments, same lists) in one call; a mask of at most 2560 candidates
+ * (4096 with is_full, zero_out or at least 16 requests; 2^18 kv bits, 64 requests, uncut lists) takes a single launch. With
+ * zero_out != NULL the output rows of the q-blocks that are not active are set to zero on the way (all rows when the
+ * lists do not fit): zero_out is the output at token 0 and the first head of the window, zero_token_bytes the distance of
+ * two tokens, zero_head_bytes the contiguous bytes of a token that belong to one mask head (both multiples of 16),
+ * zero_total_bytes the size of the whole contiguous output (larger masks zero all of it; nothing is zeroed there when
+ * is_full != 0: every block is active then). */
 FO_API int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const uint8_t* sparse_kv_info,
                          int64_t sparse_kv_info_bytes, const int32_t* sparse_info_indptr,
                          const int32_t* sparse_kv_info_indptr, int32_t is_full, void* zero_out, int64_t zero_token_bytes,
@@ -313,8 +314,8 @@ FO_API int fo_gemm_o_worklist(int32_t batch, int32_t m, int32_t k, int32_t num_h
 
 /* ---- every list of a layer step ------------------------------------------------------------------------
  * fo_gemm_q_worklist (m x n_local, head_dim) into q_workspace, fo_attn_lists (not full, nothing zeroed) and
- * fo_gemm_o_worklist (k = n_local, active heads) into o_workspace from the same masks, in one launch when the mask is
- * small (see fo_attn_lists). `plan` is a host array with the arguments of fo_attn_lists that do not change from step to
+ * fo_gemm_o_worklist (k = n_local, active heads) into o_workspace from the same masks, in one launch when the mask has at
+ * most 4096 candidates, 2^18 kv bits and 64 requests. `plan` is a host array with the arguments of fo_attn_lists that do not change from step to
  * step, in its order: [0] qo_indptr, kv_indptr, [2] batch, num_heads, head_begin, head_count, [6] sbq, sbkv, [8] n_cand,
  * max_nkv, max_items, max_kept, [12] items, kv_ptr, kv_idx, order, counters, scratch, scratch_bytes, [19] min_items,
  * num_streams, min_chunk, max_units, max_slots, [24] units, unit_counters, arrive. */

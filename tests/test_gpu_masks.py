@@ -168,11 +168,13 @@ def test_attention_compaction_random_ragged_cases(cuda_device):
 
 # (request lengths q, kv, mask heads, head window, density): one candidate; a remainder of the 16 candidates per CTA;
 # ragged with a request of no rows; a window; kv rows of more than one 64-bit word; more (group, length) buckets than
-# lengths are ordered for (single heads, q-blocks ascending); the largest candidate count and the first one past it
+# lengths are ordered for (single heads, q-blocks ascending); the largest candidate count of one launch and the first one past
+# it, for a few requests (2560), for many and with all blocks (4096)
 @pytest.mark.parametrize("lens_q,lens_kv,H,hb,hc,density", [
     ([100], [77], 1, 0, 1, 1.0), ([17 * 128], [300], 1, 0, 1, 0.5), ([300, 0, 1000, 77], [256, 128, 1300, 129], 5, 0, 5, 0.4),
     ([4608, 4608], [4608, 4608], 24, 6, 3, 0.5), ([700], [64 * 128 + 1], 3, 0, 3, 0.3), ([512], [102400], 40, 0, 40, 0.4),
-    ([128 * 128], [512], 32, 0, 32, 0.5), ([128 * 128 + 1], [512], 32, 0, 32, 0.5)])
+    ([128 * 128], [512], 32, 0, 32, 0.5), ([128 * 128 + 1], [512], 32, 0, 32, 0.5), ([80 * 128], [512], 32, 0, 32, 0.5),
+    ([80 * 128 + 1], [512], 32, 0, 32, 0.5), ([2048] * 16, [512] * 16, 16, 0, 16, 0.5), ([2048] * 15 + [2049], [512] * 16, 16, 0, 16, 0.5)])
 @pytest.mark.parametrize("is_full", [False, True])
 def test_attention_lists_in_one_call_match_the_oracle(cuda_device, lens_q, lens_kv, H, hb, hc, density, is_full):
     rng = np.random.default_rng(len(lens_q) * 100 + H)
