@@ -32,7 +32,9 @@
 // Registers: a softmax thread holds 64 columns of S; a spill inside the block loop goes through L2 (213 KB of shared
 // memory leave hardly any L1) and costs far more than the instruction: the same code with 104 and 96 instead of 112
 // registers (112 and 144 spilled bytes) took 278 and 314 us instead of 246 on the 4608-token layer, all blocks kept.
-// With the warp index read through a shuffle the role state lives in uniform registers and the block loop fits in 104.
+// With the warp index read through a shuffle the role state lives in uniform registers, which made room for four epilogue
+// warps at 104 registers for the softmax. 44 / 52 bytes of spill stores / loads are left (36 / 16 before those warps);
+// with 96 registers for the softmax and 64 for the epilogue it is 20 / 32, so most of them are the epilogue's.
 // Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
 
@@ -562,9 +564,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     // One thread per q row, 16 columns at a time. O has ONE accumulator, so the next unit's first PV waits until it has
     // been read out: that is on the pipeline's critical path and is all these warps do. (The softmax warps used to do it
     // after their next block; the first PV of a unit then started about 3 600 clocks after its P was ready.) 4608 tokens,
-    // 24 heads of 128 on a B200: 113.0 -> 108.3 us at density 0.5, 243.5 -> 230.4 us with all blocks. Chunks of 16 columns
-    // because two of them in registers would take them from the softmax warps (32 columns and 64 / 96 registers: 110.0 and
-    // 236.9 us; 8 columns: 111.1 and 234.4 us).
+    // 24 heads of 128 on a B200, a loop over one set of inputs: 113.0 -> 108.3 us at density 0.5 (no gain with inputs that
+    // change from call to call), 243.5 -> 230.4 us with all blocks. It pays where lists are long: 4096 units of one kv
+    // block each lose 3 % (98 -> 102 us), of two and four gain 2 %. Chunks of 16 columns because two of them in registers
+    // would take them from the softmax warps (32 columns and 64 / 96 registers: 110.0 and 236.9 us; 8 columns: 111.1 and
+    // 234.4 us).
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t tmem_o = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kColO;

@@ -1452,7 +1452,8 @@ __global__ void __launch_bounds__(1024) gemm_o_rows_kernel(GemmListArgs a) {
 
 // The lists of a whole layer step (GEMM-Q tiles, GEMM-O rows, attention items and units) in one launch: they only share
 // the masks, so each kind has CTAs of its own. In front of a small layer three launches in a row, each a few
-// microseconds of latency, were as long as the projection they ran beside.
+// microseconds of latency, were as long as the projection they ran beside. With 512 threads the GEMM list bodies take a
+// second pass past 512 row blocks, where 1024 would do with one.
 __global__ void __launch_bounds__(kSmallThreads) layer_lists_kernel(CompactArgs a, UnitArgs u, int by_length, int heads_per_group,
                                                                     GemmListArgs q, GemmListArgs o) {
   if (blockIdx.x == 0) {

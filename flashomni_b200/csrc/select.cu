@@ -399,6 +399,10 @@ cudaError_t launch_select_blocks(const SelectArgs& a, cudaStream_t stream) {
   select_q_kernel<<<static_cast<int>((a.batch + zero_clusters) * kSelCluster), kSelQThreads, kT2iFloats * 4, stream>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
+  // Entries per lane: image layers, video layers, and whatever else is allowed. The masses of a row live in registers, so a
+  // wider instantiation costs occupancy and idle lanes: every row computed, whole call on a B200, 40 heads x 604 / 640 blocks
+  // 94 / 102 us (522 / 546 with the search in shared memory that this replaced), 641 blocks 301 (584), 24 heads x 2048
+  // 661 (2878). A step between 640 and 2048 would help the sizes just past 640; none is built.
   if (a.n <= 128) return launch_kv<4>(a, stream);
   if (a.n <= 640) return launch_kv<20>(a, stream);
   return launch_kv<64>(a, stream);
