@@ -79,8 +79,8 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
         output_nnzs, lo, hi = (int(v) for v in torch.cat((indptr_new[-1:], indptr[:1], indptr[-1:])).tolist())
     else:
         output_nnzs = int(indptr_new[-1].item())
-        ends = (indptr.numpy() if indptr.dtype in (torch.int32, torch.int64) and not indptr.is_cuda else indptr)
-        lo, hi = int(ends.min()), int(ends.max())
+        v = indptr.tolist() if n_seg <= 64 else indptr.aminmax()   # (a few entries: cheaper than a tensor op)
+        lo, hi = int(min(v)), int(max(v))
     if lo < 0 or hi > x.numel():   # (an empty segment may lie anywhere)
         if bool(((seglen > 0) & ((indptr[:-1] < 0) | (indptr[1:] > x.numel()))).any()):
             raise ValueError(f"segment_packbits: a segment leaves the {x.numel()} values of x")
