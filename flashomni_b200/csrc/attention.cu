@@ -33,8 +33,8 @@
 // memory leave hardly any L1) and costs far more than the instruction: the same code with 104 and 96 instead of 112
 // registers (112 and 144 spilled bytes) took 278 and 314 us instead of 246 on the 4608-token layer, all blocks kept.
 // With the warp index read through a shuffle the role state lives in uniform registers, which made room for four epilogue
-// warps at 104 registers for the softmax. 44 / 52 bytes of spill stores / loads are left (36 / 16 before those warps);
-// with 96 registers for the softmax and 64 for the epilogue it is 20 / 32, so most of them are the epilogue's.
+// warps at 104 registers for the softmax. 44 / 52 bytes of spill stores / loads are left (36 / 16 before those warps), outside
+// the block loop: a launch of 958 units and 19 535 blocks executes 27 local loads and stores per unit.
 // Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
 
