@@ -431,6 +431,9 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     return fail(FO_ERR_UNSUPPORTED, "fo_sparse_attn_fwd: num_qo_heads / num_kv_heads must be 1, 2, 4, 8 or 16");
   AttnArgs a;
   memset(&a, 0, sizeof(a));
+  a.head_dim = head_dim;
+  a.mask_mode = mask_mode;
+  a.partial_slots = static_cast<int>(partial_slots > 0x7fffffffLL ? 0x7fffffffLL : partial_slots);
   {
     const uint32_t box[3] = {64, 1, 128};
     const uint32_t qbox[3] = {64, group, 128 / group};
@@ -443,8 +446,10 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     if (r == 0) r = encode_tmap_16bit(&a.tmap_k, k, 3, kd, ks, box);
     if (r == 0) r = encode_tmap_16bit(&a.tmap_v, v, 3, kd, vs, box);
     const uint64_t os[3] = {0, static_cast<uint64_t>(o_stride_h) * 2, static_cast<uint64_t>(o_stride_n) * 2};
-    const uint32_t obox16[3] = {32, group, 16 / group};
-    if (r == 0) r = encode_tmap_16bit(&a.tmap_o16, o, 3, qd, os, obox16, false);
+    // the output boxes of the kernel that will run (see AttnArgs)
+    const bool streams = attention_streams_applies(a);
+    const uint32_t obox[3] = {streams ? 64u : 32u, group, (streams ? 32u : 16u) / group};
+    if (r == 0) r = encode_tmap_16bit(&a.tmap_o, o, 3, qd, os, obox, streams);
     if (r != 0) {
       char buf[96];
       snprintf(buf, sizeof(buf), "fo_sparse_attn_fwd: cuTensorMapEncodeTiled failed (%d)", r);
@@ -462,10 +467,7 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
   a.max_units = static_cast<int>(max_units > 0x7fffffffLL ? 0x7fffffffLL : max_units);
   a.arrive = arrive;
   a.partials = partials;
-  a.partial_slots = static_cast<int>(partial_slots > 0x7fffffffLL ? 0x7fffffffLL : partial_slots);
   a.head_begin = head_begin;
-  a.head_dim = head_dim;
-  a.mask_mode = mask_mode;
   a.custom_mask = custom_mask;
   a.custom_mask_bytes = custom_mask_bytes;
   a.mask_indptr = mask_indptr;

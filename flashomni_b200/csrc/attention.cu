@@ -1,4 +1,5 @@
-// Block-sparse prefill attention on tcgen05 / TMEM / TMA, driven by compacted work lists.
+// Block-sparse prefill attention on tcgen05 / TMEM / TMA, driven by compacted work lists: the kernel of launches with a causal
+// or custom mask, with cut kv lists or with head dimension 256 (all others: attention_streams.cu).
 //
 // What it computes (reference: include/flashomni/attention/prefill.cuh:1203-1531): for every work
 // item (b, h, qb) -- an active 128-row q-block of one head -- and its ascending list of kept
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
     tma_prefetch_desc(&a.tmap_q);
     tma_prefetch_desc(&a.tmap_k);
     tma_prefetch_desc(&a.tmap_v);
-    tma_prefetch_desc(&a.tmap_o16);
+    tma_prefetch_desc(&a.tmap_o);
   }
   if (warp == kWarpMma) {
     tmem_alloc(&tail->tmem_base, kTmemCols);
@@ -654,8 +655,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
             __syncwarp();
             if (lane == 0) {
               const int t0 = q_row0 + (quad * 32) / grp;
-              tma_store_3d(&a.tmap_o16, half, col - 16, h * grp, t0);
-              tma_store_3d(&a.tmap_o16, half + kOutSlabBytes / 2, col - 16, h * grp, t0 + 16 / grp);
+              tma_store_3d(&a.tmap_o, half, col - 16, h * grp, t0);
+              tma_store_3d(&a.tmap_o, half + kOutSlabBytes / 2, col - 16, h * grp, t0 + 16 / grp);
               tma_store_commit();
             }
             ++slab;
@@ -998,17 +999,15 @@ cudaError_t launch_two(const AttnArgs& a, int ctas, cudaStream_t stream) {
     return a.head_dim == 64 ? launch_one<kBf16, kSoftCap, false, 64, 2>(a, ctas, stream)
                             : launch_one<kBf16, kSoftCap, false, 128, 2>(a, ctas, stream);
   }
-  // room for partial results means that the unit builder may have cut lists: the instantiation with the merge
-  if (a.head_dim == 64)
-    return a.partial_slots > 0 ? launch_one<kBf16, kSoftCap, true, 64>(a, ctas, stream)
-                               : launch_one<kBf16, kSoftCap, false, 64>(a, ctas, stream);
-  return a.partial_slots > 0 ? launch_one<kBf16, kSoftCap, true, 128>(a, ctas, stream)
-                             : launch_one<kBf16, kSoftCap, false, 128>(a, ctas, stream);
+  // what is left: room for partial results (the unit builder may have cut lists), the instantiation with the merge
+  return a.head_dim == 64 ? launch_one<kBf16, kSoftCap, true, 64>(a, ctas, stream)
+                          : launch_one<kBf16, kSoftCap, true, 128>(a, ctas, stream);
 }
 }  // namespace
 
 cudaError_t launch_attention(const AttnArgs& a, int max_ctas, cudaStream_t stream) {
   if (max_ctas <= 0) return cudaSuccess;
+  if (attention_streams_applies(a)) return launch_attention_streams(a, max_ctas, stream);
   const bool cap = a.soft_cap_pre > 0.f;
   if (a.is_bf16) return cap ? launch_two<true, true>(a, max_ctas, stream) : launch_two<true, false>(a, max_ctas, stream);
   return cap ? launch_two<false, true>(a, max_ctas, stream) : launch_two<false, false>(a, max_ctas, stream);

@@ -1,0 +1,748 @@
+// Block-sparse prefill attention, two independent streams of kv blocks per SM (tcgen05 / TMEM / TMA).
+//
+// Same result and same work lists as attention.cu (reference: include/flashomni/attention/prefill.cuh:1203-1531); this is
+// the kernel of every launch of whole items without a causal or custom mask at head dimension 64 and 128. Every CTA walks
+// its units as one sequence of kv blocks g = 0, 1, 2, ...; block g belongs to stream g & 1, and each stream has its own S
+// (fp32, 128 TMEM columns, its P is written over it), its own O (fp32, 128 columns), its own running maximum and row sum.
+// Nothing passes between the two streams until the end of a unit, where the epilogue adds the two O, each scaled to the
+// common maximum.
+//
+//   issuer of a stream    QK(0) | PV(0) QK(1) | PV(1) QK(2) | ...      one batch of 16 MMAs, one commit
+//   softmax of a stream   S -> registers (one q row per thread) -> maximum -> P = exp2 -> TMEM
+//
+// The MMAs of one thread execute in order: QK(i) may write over the P that PV(i - 1) reads, and the commit behind QK(i) also
+// says that PV(i - 1) is done and that the stream's K and V slots are free.
+//
+// What bounds it: the chain of one stream, S visible -> P complete -> PV and QK -> next S visible, during which the other
+// stream has the tensor pipe; on long launches the power cap (1.44 GHz instead of 1.77). By a clock trace of a step (one
+// block on each stream, 3 300 clocks): loads and maximum 450, exponentials 1 300 (1 160 in a loop of their own, 1 024 at the
+// MUFU's rate), P handed over to MMAs issued 150, sixteen MMAs 1 040, their completion seen by the softmax 250-300. What the
+// structure was tuned by, us of a call on a B200, 4608 tokens, 24 heads of 128, density 0.5 / all blocks, back to back:
+//   attention.cu (two groups of eight softmax warps on alternate blocks of one O, running maximum passed on)     111 / 266
+//   one issuer thread for both streams (its waits and commits fall between the batches)                          117 / 300
+//   an issuer per stream, batches as they come (both streams end up in phase)                                    122 / 313
+//   batches in turns                                                                                             111 / 264
+//   + half of P handed over early, conversions and sums some pairs behind the exponentials                       108 / 258
+//   + next unit's record and Q fetched ahead, O read out in full before it is stored (this kernel)               107 / 256
+//   a quarter (an eighth) of the exponentials as polynomials on the FMA pipe                                     112 / 275 (- / 265)
+//   P handed over after three quarters (a quarter) instead of half                                               109 / 263 (109 / 258)
+//   each stream with units of its own instead of alternate blocks of one unit                                    125 / 261
+// Other shapes, device time of a call from a graph, attention.cu -> here: one request of 4608 tokens with 12 heads 76 -> 68, at
+// density 0.2 67 -> 59; 64 requests of 128 tokens 60 -> 50, 32 of 256 60 -> 50, 8 of 1024 118 -> 108; only 64
+// requests of 77 tokens are slower, 55 -> 64 (one masked block and one partial store per unit).
+//
+// Warps: 0-3 softmax stream 0, 4-7 softmax stream 1 (TMEM lane = q row), 8-11 epilogue, 12 TMA producer and drawer of
+// work-list positions, 13 and 14 MMA issuers; 15 only takes part in the register split.
+// Every mbarrier wait is bounded.
+#include <cuda_fp16.h>
+
+#include "internal.h"
+
+namespace fo {
+namespace {
+
+constexpr int kBQ = 128, kBKV = 128;
+constexpr int kTileBytes = 128 * 128 * 2;   // slot of a 128-row tile of Q, K or V (head dimension 64 fills half of it)
+constexpr int kHalfBytes = kTileBytes / 2;  // one 64-column half (one swizzle-atom column)
+constexpr int kQBufs = 2;
+constexpr int kRing = 4;
+constexpr int kStreamWarps = 4;
+constexpr int kSoftmaxWarps = 2 * kStreamWarps;
+constexpr int kWarpEpilogue = kSoftmaxWarps;      // first of four (TMEM lane quadrant = warp % 4)
+constexpr int kEpilogueWarps = 4;
+constexpr int kWarpProducer = kWarpEpilogue + kEpilogueWarps;
+constexpr int kWarpMma = kWarpProducer + 1;
+constexpr int kThreads = (kWarpProducer + 4) * 32;   // 512
+constexpr int kRegsSoftmax = 184, kRegsEpilogue = 88, kRegsOther = 56;  // setmaxnreg split
+// setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with: a split that asks for more
+// never returns.
+constexpr int kRegsAtLaunch = (65536 / kThreads) / 8 * 8;
+static_assert(kSoftmaxWarps * 32 * kRegsSoftmax + kEpilogueWarps * 32 * kRegsEpilogue + 4 * 32 * kRegsOther <= kThreads * kRegsAtLaunch,
+              "register split exceeds the CTA's register pool");
+constexpr int kTmemCols = 512;
+constexpr uint32_t kColS = 0, kColO = 256;  // stream s: + 128 s
+constexpr int kRotStep = 5;                 // q-block qb starts its kv list at entry (qb * kRotStep) mod length
+constexpr int kItemQ = 8;
+constexpr int kItemReaders = kSoftmaxWarps + kEpilogueWarps + 2;  // softmax and epilogue warps, the two issuers
+constexpr int kEarly = 4;                   // MMAs of a PV (16 kv rows each) that may start before the whole P is there
+constexpr int kLag = 4;                     // pairs of columns between an exponential and its use
+constexpr float kRescaleThreshold = 8.0f;   // lazy rescale: keep the old maximum while exp2 stays <= 2^8
+
+struct Tail {
+  uint64_t q_full[kQBufs], q_empty[kQBufs];
+  uint64_t full[kRing];            // K of stream 0, K of stream 1, V of stream 0, V of stream 1
+  uint64_t batch[2];               // a stream's batch of MMAs (PV of block i - 1, QK of block i) is done
+  uint64_t p_most[2], p_full[2];   // the first kEarly * 16 columns of a stream's P are in TMEM (and O is rescaled); all of them
+  uint64_t turn[2];                // a stream's issuer may issue its next batch
+  uint64_t stats_ready[2];         // indexed by unit parity: both streams have published (m, l)
+  uint64_t stats_free[2];          // the epilogue has read them
+  uint64_t o_full[2];              // the last PV of a unit on a stream is done
+  uint64_t o_free[2];              // the epilogue has read a stream's O
+  uint64_t iq_full[kItemQ], iq_empty[kItemQ];  // unit queue: the producer draws work-list positions for the CTA
+  int item_q[kItemQ];
+  uint32_t tmem_base;
+  int abort_flag;
+  float stats_m[2][2][128];        // [unit parity][stream][row]: the maximum the sum refers to
+  float stats_l[2][2][128];
+};
+
+constexpr int kOutSlabBytes = 32 * 128;            // 32 rows x 64 output columns: staging of an epilogue warp
+constexpr int kSmemBytes = (kQBufs + kRing) * kTileBytes + kEpilogueWarps * kOutSlabBytes + 1024 + static_cast<int>(sizeof(Tail));
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+
+__device__ __forceinline__ int rot_of(int qb, int n) {
+  return static_cast<int>(static_cast<unsigned>(qb * kRotStep) % static_cast<unsigned>(n));
+}
+
+// Work-list positions: position i < gridDim.x goes to CTA i, the following ones are drawn from a device-wide cursor by
+// the producer and passed to the other roles through a small shared-memory queue (-1 ends the sequence).
+struct ItemDraw {
+  Tail* tail;
+  int32_t* cursor;
+  volatile int* abort_flag;
+  int n_items, n_pub;
+  int p0, p1, p2;  // current, published next, drawn (still in flight) after next: the atomic never sits between two units
+  bool started, ended;
+  __device__ __forceinline__ int draw() {
+    const int p = atomicAdd(cursor, 1) + static_cast<int>(gridDim.x);
+    return p < n_items ? p : -1;
+  }
+  __device__ __forceinline__ bool publish(int v) {
+    if (ended) return true;
+    const int slot = n_pub % kItemQ;
+    if (!mbar_wait(&tail->iq_empty[slot], (static_cast<uint32_t>(n_pub / kItemQ) & 1u) ^ 1u, abort_flag)) return false;
+    tail->item_q[slot] = v;
+    mbar_arrive(&tail->iq_full[slot]);
+    ++n_pub;
+    if (v < 0) ended = true;
+    return true;
+  }
+  __device__ __forceinline__ void init(Tail* t, int32_t* cur, volatile int* ab, int n) {
+    tail = t; cursor = cur; abort_flag = ab; n_items = n; n_pub = 0; started = false; ended = false;
+    p0 = static_cast<int>(blockIdx.x) < n ? static_cast<int>(blockIdx.x) : -1;
+    p1 = p2 = -1;
+    bool ok = publish(p0);
+    if (ok && p0 >= 0) {
+      p1 = draw();
+      ok = publish(p1);
+      if (ok && p1 >= 0) p2 = draw();
+    }
+    if (!ok) p0 = -1;
+  }
+  __device__ __forceinline__ int next() {
+    if (!started) { started = true; return p0; }
+    p0 = p1;
+    if (p0 < 0) return -1;
+    p1 = p2;
+    if (!publish(p1)) return -1;
+    p2 = p1 >= 0 ? draw() : -1;
+    return p0;
+  }
+};
+
+template <bool kWholeWarp>
+struct ItemRead {  // the reading roles: one thread, or all lanes of a warp
+  Tail* tail;
+  volatile int* abort_flag;
+  int k;
+  __device__ __forceinline__ void init(Tail* t, volatile int* ab) { tail = t; abort_flag = ab; k = 0; }
+  __device__ __forceinline__ int next() {
+    const int slot = k % kItemQ;
+    if (!mbar_wait(&tail->iq_full[slot], static_cast<uint32_t>(k / kItemQ) & 1u, abort_flag)) return -1;
+    const int v = tail->item_q[slot];
+    if (kWholeWarp) {
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(&tail->iq_empty[slot]);
+    } else {
+      mbar_arrive(&tail->iq_empty[slot]);
+    }
+    ++k;
+    return v;
+  }
+};
+
+// Waits for the TMEM loads issued so far; naming the 32 registers keeps their uses behind the wait.
+__device__ __forceinline__ void tmem_wait_ld_32(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]),
+                 "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
+                 "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+template <bool kBf16, bool kSoftCap, int kD>
+__global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __grid_constant__ AttnArgs a) {
+  static_assert(kD == 128 || kD == 64, "head dimension");
+  constexpr int kLoadBytes = 128 * kD * 2;   // bytes of one tile load
+  constexpr int kHalves = kD / 64;           // 64-column boxes per tile
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  uint8_t* smem_q = smem;
+  uint8_t* smem_ring = smem + kQBufs * kTileBytes;
+  uint8_t* smem_stage = smem_ring + kRing * kTileBytes;
+  Tail* tail = reinterpret_cast<Tail*>(smem_stage + kEpilogueWarps * kOutSlabBytes);
+  volatile int* abort_flag = &tail->abort_flag;
+
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // uniform: role state in uniform registers
+  const int lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kQBufs; ++i) { mbar_init(&tail->q_full[i], 1); mbar_init(&tail->q_empty[i], 2); }
+    for (int i = 0; i < kRing; ++i) mbar_init(&tail->full[i], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tail->batch[i], 1);
+      mbar_init(&tail->o_full[i], 1);
+      mbar_init(&tail->o_free[i], kEpilogueWarps);
+      mbar_init(&tail->p_most[i], kStreamWarps);
+      mbar_init(&tail->p_full[i], kStreamWarps);
+      mbar_init(&tail->turn[i], 1);
+      mbar_init(&tail->stats_ready[i], kSoftmaxWarps);
+      mbar_init(&tail->stats_free[i], kEpilogueWarps);
+    }
+    for (int i = 0; i < kItemQ; ++i) { mbar_init(&tail->iq_full[i], 1); mbar_init(&tail->iq_empty[i], kItemReaders); }
+    tail->abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == kWarpProducer && lane == 0) {
+    tma_prefetch_desc(&a.tmap_q);
+    tma_prefetch_desc(&a.tmap_k);
+    tma_prefetch_desc(&a.tmap_v);
+    tma_prefetch_desc(&a.tmap_o);
+  }
+  if (warp == kWarpMma) {
+    tmem_alloc(&tail->tmem_base, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tail->tmem_base;
+  if (a.after_lists) asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the lists in front of it were built
+
+  // A list that ran out of room is not dereferenced; the launch only reports it. Parts of split lists are not for this kernel.
+  const bool list_bad = a.unit_counters[3] != kDevOk || a.unit_counters[1] > 0;
+  int n_items = a.unit_counters[0];
+  if (list_bad || n_items < 0) n_items = 0;
+  if (n_items > a.max_units) n_items = a.max_units;
+
+  if (warp >= kWarpProducer) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+  if (warp == kWarpProducer) {
+    // ------------------------------------------------------------------ TMA producer, in the order the issuers read
+    if (lane == 0) {
+      ItemDraw src;
+      src.init(tail, a.status + 1, abort_flag, n_items);
+      uint32_t g = 0;
+      int unit_no = 0;
+      int vh0 = 0, vrow0 = -1, vh1 = 0, vrow1 = -1;   // V tiles still to be loaded: of block g - 2 and of block g - 1
+      bool ok = true;
+      auto load = [&](uint32_t slot, const CUtensorMap* map, int h, int row) {
+        uint8_t* dst = smem_ring + slot * kTileBytes;
+        mbar_expect_tx(&tail->full[slot], kLoadBytes);
+#pragma unroll
+        for (int i = 0; i < kHalves; ++i) tma_load_3d(dst + i * kHalfBytes, map, &tail->full[slot], 64 * i, h, row);
+      };
+      // V of block b goes to slot 2 + (b & 1) once batch b >> 1 of its stream, which read the V before it, is done
+      auto push_v = [&](uint32_t b, int h, int row) -> bool {
+        if (!mbar_wait(&tail->batch[b & 1u], (b >> 1) & 1u, abort_flag)) return false;
+        load(2u + (b & 1u), &a.tmap_v, h, row);
+        return true;
+      };
+      // the record of the next unit, and the head of its kv list, are fetched while the current one is loaded: the chain
+      // position -> record -> list entry would otherwise sit in front of every unit's first tiles
+      bool q_pending = false;
+      int n_next = 0, t_next = 0, kvb_first = 0, hk_next = 0, q_row_next = 0, kv_row_next = 0, kv_off_next = 0;
+      auto fetch = [&]() {
+        n_next = 0;
+        while (true) {
+          const int pos = src.next();
+          if (pos < 0) return;
+          const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
+          const int4 u0 = up[0], u1 = up[1];
+          if (u0.x <= 0) continue;
+          n_next = u0.x;
+          kv_off_next = u0.y;
+          hk_next = (u0.z & 0xffff) - a.head_begin;   // a unit's head is the kv head; its q tile holds the group's q heads
+          q_row_next = u0.w;                          // of 128 / group tokens, token-major
+          kv_row_next = u1.y;
+          t_next = rot_of(q_row_next >> 7, n_next);
+          kvb_first = a.kv_idx[kv_off_next + t_next];
+          q_pending = true;
+          return;
+        }
+      };
+      auto load_q = [&]() -> bool {  // of the unit fetched last
+        const int qb = unit_no & 1;
+        if (!mbar_wait(&tail->q_empty[qb], (static_cast<uint32_t>(unit_no >> 1) & 1u) ^ 1u, abort_flag)) return false;
+        ++unit_no;
+        uint8_t* dst = smem_q + qb * kTileBytes;
+        mbar_expect_tx(&tail->q_full[qb], kLoadBytes);
+#pragma unroll
+        for (int i = 0; i < kHalves; ++i)
+          tma_load_3d(dst + i * kHalfBytes, &a.tmap_q, &tail->q_full[qb], 64 * i, hk_next * a.group_size, q_row_next);
+        q_pending = false;
+        return true;
+      };
+      fetch();
+      while (ok && n_next > 0) {
+        const int n = n_next, hk = hk_next, kv_row0 = kv_row_next;
+        const int32_t* kv = a.kv_idx + kv_off_next;
+        int t = t_next;
+        int kvb_next = kvb_first;
+        for (int j = 0; j < n && ok; ++j) {
+          const int kvb = kvb_next;
+          if (j + 1 < n) {
+            if (++t == n) t = 0;
+            kvb_next = kv[t];
+          }
+          // (the wait of this V also frees the slot of the K below: both were read by batch (g - 2) >> 1 or before)
+          if (vrow0 >= 0) ok = push_v(g - 2u, vh0, vrow0);
+          vh0 = vh1; vrow0 = vrow1;
+          if (ok && j == 0 && q_pending) ok = load_q();
+          vh1 = hk; vrow1 = kv_row0 + kvb * kBKV;
+          if (ok) load(g & 1u, &a.tmap_k, vh1, vrow1);
+          ++g;
+          // The next unit's Q comes from HBM: it is requested early, to the buffer of the unit before this one, whose last
+          // QK has been issued by now (it is in front of this unit's second K, which is on its way).
+          if (ok && j == (n > 1 ? 1 : 0)) {
+            fetch();
+            if (n > 1 && n_next > 0) ok = load_q();
+          }
+        }
+      }
+      if (ok && vrow0 >= 0) ok = push_v(g - 2u, vh0, vrow0);
+      if (ok && vrow1 >= 0) push_v(g - 1u, vh1, vrow1);
+    }
+  } else if (warp == kWarpMma || warp == kWarpMma + 1) {
+    // ------------------------------------------------------------------ MMA issuers, one per stream
+    // Batch i of a stream is PV of its block i - 1 and QK of its block i, sixteen MMAs behind one set of waits and in front
+    // of ONE commit: its completion says that S of block i is written, that the PV of block i - 1 is done (O may be
+    // rescaled or read), and that the stream's K and V slots are free.
+    if (lane == 0) {
+      constexpr uint32_t idesc_qk = make_idesc_f16(kBQ, kBKV, kBf16, 0, 0);
+      constexpr uint32_t idesc_pv = make_idesc_f16(kBQ, kD, kBf16, 0, 1);
+      const uint32_t X = static_cast<uint32_t>(warp - kWarpMma);
+      // descriptors: constant high words (128-byte swizzle; Q and K K-major, V MN-major with its two 64-column halves
+      // 16 KB apart), low words hold the address
+      const uint64_t dk = make_smem_desc_sw128(smem_u32(smem_ring + X * kTileBytes), 16, 1024);
+      const uint64_t dv = make_smem_desc_sw128(smem_u32(smem_ring + (2u + X) * kTileBytes), kHalfBytes, 1024);
+      const uint32_t hi_k = static_cast<uint32_t>(dk >> 32), hi_v = static_cast<uint32_t>(dv >> 32);
+      const uint32_t q_lo0 = static_cast<uint32_t>(make_smem_desc_sw128(smem_u32(smem_q), 16, 1024));
+      uint32_t lk[8], lv[8], tp[8];
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        // 16 elements further along K: +32 B inside a 64-column half, +16 KB for the second half; 16 kv rows further =
+        // 16 * 128 B in the V tile, 8 columns further in the 16-bit P tile
+        lk[kk] = static_cast<uint32_t>(dk) + static_cast<uint32_t>(((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4);
+        lv[kk] = static_cast<uint32_t>(dv) + static_cast<uint32_t>((kk * 2048) >> 4);
+        tp[kk] = tmem_base + kColS + X * 128u + static_cast<uint32_t>(kk * 8);
+      }
+      const uint32_t tmem_s = tmem_base + kColS + X * 128u, tmem_o = tmem_base + kColO + X * 128u;
+      ItemRead<false> src;
+      src.init(tail, abort_flag);
+      bool ok = true;
+      int n_next = 0;
+      auto fetch = [&]() {  // the block count of the next unit, one unit ahead; 0 at the end
+        do {
+          const int pos = src.next();
+          if (pos < 0) { n_next = 0; return; }
+          n_next = a.units[8 * static_cast<int64_t>(pos)];
+        } while (n_next <= 0);
+      };
+      fetch();
+      int n = 0, j = 0, unit_no = -1;
+      uint32_t g0 = 0;      // blocks in front of the current unit
+      uint32_t i = 0;       // this stream's batches so far
+      uint32_t units_started = 0;
+      uint32_t q_lo = 0;
+      bool pv = false, pv_first = false;   // a PV is pending, and it is its unit's first one
+      while (true) {
+        // ---- the next block of this stream, if there is one
+        j += 2;
+        bool qk = true;
+        bool new_unit = false;
+        while (j >= n) {
+          g0 += static_cast<uint32_t>(n);
+          n = n_next;
+          if (n == 0) { qk = false; break; }
+          ++unit_no;
+          fetch();
+          j = static_cast<int>((g0 ^ X) & 1u);
+          new_unit = true;
+          if (j >= n) {  // a unit of one block, and it is the other stream's: its Q tile is none of this stream's business
+            if (!mbar_wait(&tail->q_full[unit_no & 1], static_cast<uint32_t>(unit_no >> 1) & 1u, abort_flag)) { ok = false; break; }
+            mbar_arrive(&tail->q_empty[unit_no & 1]);
+          }
+        }
+        if (!ok) break;
+        if (!qk && !pv) {  // a stream that had no block at all still passes the turn on
+          if (i == 0u) mbar_arrive(&tail->turn[X ^ 1u]);
+          break;
+        }
+        // ---- everything the batch needs
+        if (pv) {
+          if (!mbar_wait(&tail->full[2u + X], (i - 1u) & 1u, abort_flag)) break;
+          if (pv_first) {  // O must have been read by the epilogue of this stream's previous unit
+            if (units_started > 0u && !mbar_wait(&tail->o_free[X], (units_started - 1u) & 1u, abort_flag)) break;
+            ++units_started;
+          }
+          if (!mbar_wait(&tail->p_most[X], (i - 1u) & 1u, abort_flag)) break;
+        }
+        // the two streams' batches alternate: interleaved in the pipe both would end when the second one does now
+        if ((X != 0u || i != 0u) && !mbar_wait_spin(&tail->turn[X], (i & 1u) ^ (X ^ 1u), abort_flag)) break;
+        tc_fence_after_sync();
+        if (pv) {
+          static_assert(kEarly == 4, "the PV is issued in two halves");
+          umma_ts_x4(tmem_o, hi_v, idesc_pv, pv_first ? 0u : 1u, tp, lv);
+          if (!mbar_wait_spin(&tail->p_full[X], (i - 1u) & 1u, abort_flag)) break;
+          tc_fence_after_sync();
+          umma_ts_x4(tmem_o, hi_v, idesc_pv, 1u, tp + 4, lv + 4);
+        }
+        if (pv && (new_unit || !qk)) umma_commit(&tail->o_full[X]);  // O of the unit is complete
+        if (qk) {
+          if (new_unit) {
+            if (!mbar_wait(&tail->q_full[unit_no & 1], static_cast<uint32_t>(unit_no >> 1) & 1u, abort_flag)) break;
+            q_lo = q_lo0 + static_cast<uint32_t>(((unit_no & 1) * kTileBytes) >> 4);
+          }
+          if (!mbar_wait(&tail->full[X], i & 1u, abort_flag)) break;
+          uint32_t la[8];
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) la[kk] = q_lo + static_cast<uint32_t>(((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4);
+          if constexpr (kD == 128) umma_ss_x8(tmem_s, hi_k, hi_k, idesc_qk, 0u, la, lk);
+          else umma_ss_x4(tmem_s, hi_k, hi_k, idesc_qk, 0u, la, lk);
+        }
+        mbar_arrive(&tail->turn[X ^ 1u]);
+        umma_commit(&tail->batch[X]);
+        if (qk && j + 2 >= n) umma_commit(&tail->q_empty[unit_no & 1]);
+        ++i;
+        pv = qk;
+        pv_first = new_unit;
+      }
+    }
+  }
+  } else if (warp >= kWarpEpilogue) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+    // ------------------------------------------------------------------ epilogue warps: (O0 w0 + O1 w1) / l to global memory
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t tmem_o = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kColO;
+    uint8_t* stg = smem_stage + quad * kOutSlabBytes;
+    const int grp = a.group_size;
+    const int grp_shift = 31 - __clz(grp);   // 1, 2, 4, 8 or 16 q heads share a kv head
+    const int row_tok = row >> grp_shift, row_head = row & (grp - 1), row_tok0 = (quad * 32) >> grp_shift;
+    uint32_t item = 0;
+    uint32_t g = 0;         // blocks in front of the current unit
+    uint32_t units0 = 0, units1 = 0;   // units so far that had blocks of stream 0 / 1
+    ItemRead<true> src;
+    src.init(tail, abort_flag);
+    while (true) {
+      const int pos = src.next();
+      if (pos < 0) break;
+      const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
+      const int4 u0 = up[0], u1 = up[1];
+      const int q_row0 = u0.w, q_valid = u1.x & 0xffff, h = (u0.z & 0xffff) - a.head_begin;
+      // Row r of a tile is token q_row0 + r / group, q head h * group + r % group (group = 1: the row itself).
+      const bool row_ok = row < q_valid * grp;
+      const int64_t grow = static_cast<int64_t>(q_row0) + row_tok;
+      const int hq = h * grp + row_head;
+      uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + grow * a.o_stride_n + static_cast<int64_t>(hq) * a.o_stride_h;
+      float* lse = a.lse != nullptr ? a.lse + grow * a.lse_stride_n + hq : nullptr;
+      if (u0.x <= 0) {  // active q-block that keeps nothing: zeros, lse = -5e4
+        if (row_ok) {
+#pragma unroll 1
+          for (int i = 0; i < kD / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (lse != nullptr) *lse = -5e4f;
+        }
+        continue;
+      }
+      const uint32_t ip = item & 1u;
+      if (!mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag)) break;
+      const float m0 = tail->stats_m[ip][0][row], m1 = tail->stats_m[ip][1][row];
+      const float l0 = tail->stats_l[ip][0][row], l1 = tail->stats_l[ip][1][row];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->stats_free[ip]);
+      const float m_out = fmaxf(m0, m1);
+      // a stream without a visible column has m = -inf, l = 0
+      float w0 = (m0 == m_out) ? 1.f : ex2_approx(m0 - m_out), w1 = (m1 == m_out) ? 1.f : ex2_approx(m1 - m_out);
+      const float l_out = fmaf(l0, w0, l1 * w1);
+      const float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
+      w0 *= inv_out;
+      w1 *= inv_out;
+      // a unit of one block leaves the other stream's O as it was: whatever that is, it does not count
+      const bool has0 = u0.x > 1 || (g & 1u) == 0u, has1 = u0.x > 1 || (g & 1u) == 1u;
+      g += static_cast<uint32_t>(u0.x);
+      if (has0 && !mbar_wait(&tail->o_full[0], units0++ & 1u, abort_flag)) break;
+      if (has1 && !mbar_wait(&tail->o_full[1], units1++ & 1u, abort_flag)) break;
+      tc_fence_after_sync();
+      const bool whole = q_valid * grp == kBQ;   // no row of the q-block is past the request
+      // (an O that nothing wrote may hold anything: the other one stands in for it, with the weight of zero)
+      const uint32_t tmem_o0 = tmem_o + (has0 ? 0u : 128u), tmem_o1 = tmem_o + (has1 ? 128u : 0u);
+      const uint64_t w0p = pack_f32x2(w0, w0), w1p = pack_f32x2(w1, w1);
+#pragma unroll 1
+      for (int half = 0; half < kHalves; ++half) {
+        uint4 out[8];
+        uint32_t* w = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v0[16], v1[16];
+          tmem_ld_x16(tmem_o0 + 64u * half + 16u * c, v0);
+          tmem_ld_x16(tmem_o1 + 64u * half + 16u * c, v1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const uint64_t b2 = ffma2(pack_f32x2(__uint_as_float(v1[2 * t]), __uint_as_float(v1[2 * t + 1])), w1p, 0ull);
+            const uint64_t x2 = ffma2(pack_f32x2(__uint_as_float(v0[2 * t]), __uint_as_float(v0[2 * t + 1])), w0p, b2);
+            float x0, x1;
+            unpack_f32x2(x2, x0, x1);
+            w[8 * c + t] = kBf16 ? pack_bf16x2(x0, x1) : pack_f16x2(x0, x1);
+          }
+        }
+        if (half == kHalves - 1) {  // both O may be overwritten by the next unit
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            if (has0) mbar_arrive(&tail->o_free[0]);
+            if (has1) mbar_arrive(&tail->o_free[1]);
+          }
+        }
+        // Through a staging slab per warp (32 rows x 64 columns in the 128-byte swizzle pattern): a store instruction of
+        // a warp would otherwise write 32 scattered 16-byte pieces. Whole q-blocks leave by one TMA store per slab, the rows
+        // of a partial one with four rows per instruction.
+        if (lane == 0) tma_store_wait_read<0>();  // the slab is free once the store before has read it
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16)) = out[c];
+        if (whole) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&a.tmap_o, stg, 64 * half, h * grp, q_row0 + row_tok0);
+            tma_store_commit();
+          }
+        } else {
+          __syncwarp();
+#pragma unroll 1
+          for (int r = lane >> 3; r < 32; r += 4) {
+            const int tr = quad * 32 + r;   // row of the tile
+            if (tr >= q_valid * grp) break;
+            const int64_t tok = static_cast<int64_t>(q_row0) + (tr >> grp_shift);
+            uint16_t* dst = reinterpret_cast<uint16_t*>(a.o) + tok * a.o_stride_n +
+                            static_cast<int64_t>(h * grp + (tr & (grp - 1))) * a.o_stride_h + 64 * half;
+            reinterpret_cast<uint4*>(dst)[lane & 7] = *reinterpret_cast<const uint4*>(stg + r * 128 + (((lane & 7) ^ (r & 7)) * 16));
+          }
+        }
+      }
+      ++item;
+      if (row_ok && lse != nullptr) *lse = (l_out > 0.f) ? (log2f(l_out) + m_out) : -5e4f;
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
+    // ------------------------------------------------------------------ softmax: one q row per thread
+    const uint32_t X = static_cast<uint32_t>(warp >> 2);
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t tmem_s = tmem_base + lane_base + kColS + X * 128u;
+    const uint32_t tmem_o = tmem_base + lane_base + kColO + X * 128u;
+    uint64_t* s_full = &tail->batch[X];
+    uint64_t* p_full = &tail->p_full[X];
+    ItemRead<true> src;
+    src.init(tail, abort_flag);
+    uint32_t g = 0;          // blocks in front of the current unit
+    uint32_t phase = 0;      // parity of this stream's block count
+    uint32_t item = 0;
+    bool ok = true;
+    const uint64_t scale2 = pack_f32x2(a.sm_scale_log2, a.sm_scale_log2);
+
+    // the record of the next unit is fetched while the current one runs
+    int n_next = -1, qb_next = 0, rag_next = 0;
+    auto fetch = [&]() {
+      n_next = -1;
+      while (true) {
+        const int pos = src.next();
+        if (pos < 0) return;
+        const int32_t* up = a.units + 8 * static_cast<int64_t>(pos);
+        n_next = up[0];
+        if (n_next > 0) { qb_next = up[3] >> 7; rag_next = up[4] >> 16; return; }
+      }
+    };
+    fetch();
+    while (ok && n_next > 0) {
+      const int n = n_next, rag = rag_next;
+      int ragged_j = -1;   // visiting step of the request's partial last kv block
+      if (rag != 0) {
+        ragged_j = n - 1 - rot_of(qb_next, n);
+        if (ragged_j < 0) ragged_j += n;
+      }
+      fetch();
+      float m_ref = -INFINITY;
+      uint64_t l2a = 0, l2b = 0;
+      const int j0 = static_cast<int>((g ^ X) & 1u);
+#pragma unroll 1
+      for (int j = j0; j < n; j += 2) {
+        if (!mbar_wait(s_full, phase, abort_flag)) { ok = false; break; }
+        phase ^= 1u;
+        tc_fence_after_sync();
+        uint32_t s[128];
+        tmem_ld_x32(tmem_s, s);
+        tmem_ld_x32(tmem_s + 32u, s + 32);
+        tmem_wait_ld();
+        tmem_ld_x32(tmem_s + 64u, s + 64);   // ... while the maximum of the first half is taken
+        tmem_ld_x32(tmem_s + 96u, s + 96);
+        const bool ragged = j == ragged_j;
+        float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        auto half_max = [&](int c0) {
+          if (ragged) {
+#pragma unroll
+            for (int c = c0; c < c0 + 64; c += 32) {
+              const int have = rag - c;   // existing columns from here on: as a mask of 32 bits
+              const uint32_t keep = have >= 32 ? 0xffffffffu : (have <= 0 ? 0u : (1u << have) - 1u);
+#pragma unroll
+              for (int t = 0; t < 32; ++t)
+                if (((keep >> t) & 1u) == 0u) s[c + t] = 0xff800000u;  // -inf: exp2 gives 0
+            }
+          }
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              mxs[i] = fmax3(mxs[i], __uint_as_float(s[c0 + 8 * t + 2 * i]), __uint_as_float(s[c0 + 8 * t + 2 * i + 1]));
+          }
+        };
+        half_max(0);
+        tmem_wait_ld_32(s + 64);
+        tmem_wait_ld_32(s + 96);
+        half_max(64);
+        float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
+        // with a soft cap the logit is cap * tanh(s * sm_scale / cap): monotonic, so the maximum is transformed once
+        if constexpr (kSoftCap) mx = (mx == -INFINITY) ? mx : tanh_approx(mx * a.soft_cap_pre);
+        const bool first = j < 2;
+        const float m_prev = m_ref;
+        const float m_new = fmaxf(m_prev, mx * a.sm_scale_log2);
+        const bool need = (m_new - m_prev) > kRescaleThreshold;
+        const bool rescale = !first && __any_sync(0xffffffffu, need);
+        float alpha = 1.f;
+        if (first) {
+          m_ref = m_new;
+        } else if (need) {
+          m_ref = m_new;
+          alpha = ex2_approx(m_prev - m_new);
+          const uint64_t alpha2 = pack_f32x2(alpha, alpha);
+          l2a = ffma2(l2a, alpha2, 0ull);
+          l2b = ffma2(l2b, alpha2, 0ull);
+        }
+        const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
+        const uint64_t negm2 = pack_f32x2(neg_m, neg_m);
+        if (rescale) {  // the PV of this stream's previous block is done: it is in the batch that wrote S
+#pragma unroll 1
+          for (int c = 0; c < kD / 16; ++c) {
+            uint32_t v[16];
+            tmem_ld_x16(tmem_o + 16u * c, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = __float_as_uint(__uint_as_float(v[t]) * alpha);
+            tmem_st_x16(tmem_o + 16u * c, v);
+          }
+        }
+        if constexpr (kSoftCap) {
+#pragma unroll
+          for (int t = 0; t < 128; ++t)  // masked columns stay at -inf
+            if (s[t] != 0xff800000u) s[t] = __float_as_uint(tanh_approx(__uint_as_float(s[t]) * a.soft_cap_pre));
+        }
+        auto hand_over = [&](uint64_t* bar) {
+          tmem_wait_st();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar);
+        };
+        // The sum and the conversion of a pair follow its exponentials by kLag pairs: between two volatile TMEM stores
+        // nothing then waits for the last exponential in front of it.
+#pragma unroll
+        for (int t = 0; t < 64 + kLag; ++t) {
+          if (t < 64) {
+            const uint64_t x2 = ffma2(pack_f32x2(__uint_as_float(s[2 * t]), __uint_as_float(s[2 * t + 1])), scale2, negm2);
+            float x0, x1;
+            unpack_f32x2(x2, x0, x1);
+            s[2 * t] = __float_as_uint(ex2_approx(x0));
+            s[2 * t + 1] = __float_as_uint(ex2_approx(x1));
+          }
+          if (t >= kLag) {
+            const int e = t - kLag;
+            const float p0 = __uint_as_float(s[2 * e]), p1 = __uint_as_float(s[2 * e + 1]);
+            if (e & 1) l2b = fadd2(l2b, pack_f32x2(p0, p1)); else l2a = fadd2(l2a, pack_f32x2(p0, p1));
+            s[e] = kBf16 ? pack_bf16x2(p0, p1) : pack_f16x2(p0, p1);   // (entry e of s is free by now)
+            if ((e & 15) == 15) {   // P over S: this thread has its whole row in registers
+              tmem_st_x16(tmem_s + static_cast<uint32_t>(e - 15), s + e - 15);
+            }
+            // (a few pairs after the store, so that nothing waits for it)
+            if (e == kEarly * 8 + 4) hand_over(&tail->p_most[X]);
+          }
+        }
+        hand_over(p_full);
+      }
+      if (!ok) break;
+      g += static_cast<uint32_t>(n);
+      const uint32_t ip = item & 1u;
+      // the statistics of the unit before the last one must have been read
+      if (item >= 2u && !mbar_wait(&tail->stats_free[ip], ((item >> 1) - 1u) & 1u, abort_flag)) break;
+      float la, lb, lc, ld;
+      unpack_f32x2(l2a, la, lb);
+      unpack_f32x2(l2b, lc, ld);
+      tail->stats_m[ip][X][row] = m_ref;
+      tail->stats_l[ip][X][row] = (la + lb) + (lc + ld);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tail->stats_ready[ip]);
+      ++item;
+    }
+  }
+
+  // ------------------------------------------------------------------ common exit
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+    if (threadIdx.x == 0) atomicExch(a.status, kDevWaitTimeout);
+    __syncthreads();
+  }
+  if (list_bad && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(a.status, kDevOk, kDevBadIndex);
+  if (warp == kWarpMma) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+  // the last CTA to get here puts the cursor and the arrival count back to zero for the next launch
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(a.status + 2, 1) == static_cast<int>(gridDim.x) - 1) {
+      atomicExch(a.status + 1, 0);
+      atomicExch(a.status + 2, 0);
+    }
+  }
+}
+
+template <bool kBf16, bool kSoftCap, int kD>
+cudaError_t launch_one(const AttnArgs& a, int ctas, cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(attention_streams_kernel<kBf16, kSoftCap, kD>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(attention_streams_kernel<kBf16, kSoftCap, kD>, ctas, kThreads, kSmemBytes, stream,
+                          a.after_lists != 0, a);
+}
+template <bool kBf16, bool kSoftCap>
+cudaError_t launch_two(const AttnArgs& a, int ctas, cudaStream_t stream) {
+  return a.head_dim == 64 ? launch_one<kBf16, kSoftCap, 64>(a, ctas, stream) : launch_one<kBf16, kSoftCap, 128>(a, ctas, stream);
+}
+}  // namespace
+
+cudaError_t launch_attention_streams(const AttnArgs& a, int max_ctas, cudaStream_t stream) {
+  if (max_ctas <= 0) return cudaSuccess;
+  const bool cap = a.soft_cap_pre > 0.f;
+  if (a.is_bf16) return cap ? launch_two<true, true>(a, max_ctas, stream) : launch_two<true, false>(a, max_ctas, stream);
+  return cap ? launch_two<false, true>(a, max_ctas, stream) : launch_two<false, false>(a, max_ctas, stream);
+}
+
+}  // namespace fo

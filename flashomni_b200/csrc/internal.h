@@ -199,7 +199,8 @@ struct AttnArgs {
   CUtensorMap tmap_q;              // [D, H, Tq]   box 64 x 1 x 128
   CUtensorMap tmap_k;              // [D, Hkv, Tkv]
   CUtensorMap tmap_v;
-  CUtensorMap tmap_o16;            // [D, Hq, Tq]   box 32 x 1 x 16, no swizzle (stores of whole q-blocks)
+  CUtensorMap tmap_o;              // [D, Hq, Tq], stores of whole q-blocks: box 64 x 1 x 32, 128-byte swizzle (streams kernel)
+                                   // or 32 x 1 x 16, no swizzle (the other one)
   void* o;                         // [Tq, H, D] (strides below, in elements)
   float* lse;                      // [Tq, H] or null
   int64_t o_stride_n, o_stride_h;
@@ -228,7 +229,12 @@ struct AttnArgs {
 };
 // floats of one partial result: O (32 column groups x 128 rows x 4), then the row maxima and the row sums
 constexpr int kPartialFloats = 128 * 128 + 2 * 128;
-// one unit at a time per SM (launches with many units) / two streams of units per SM with split kv lists (few units)
+// whole items without a causal or custom mask, head dimension 64 or 128: attention_streams.cu, which was faster at every
+// shape measured but the one named there; the other launches keep attention.cu
+inline bool attention_streams_applies(const AttnArgs& a) {
+  return a.mask_mode == 0 && a.partial_slots <= 0 && (a.head_dim == 64 || a.head_dim == 128);
+}
+cudaError_t launch_attention_streams(const AttnArgs& a, int max_ctas, cudaStream_t stream);
 cudaError_t launch_attention(const AttnArgs& a, int max_ctas, cudaStream_t stream);
 
 // ------------------------------------------------------------------ host helpers

@@ -1,0 +1,66 @@
+"""GPU: the attention kernel with two streams of kv blocks per SM where it can go wrong: units of one, two and three kv
+blocks in a row (a unit of one block belongs to one stream only), more units than CTAs, partial q-blocks and kv blocks,
+rows whose maximum rises late (rescale), grouped heads, both head dimensions and types, NaN inputs."""
+
+import numpy as np
+import pytest
+import torch
+
+import flashomni_b200 as fo
+from flashomni_b200 import workloads as wl
+from oracle import attention as oa
+from helpers import assert_close_bf16, dev, masks_to_device
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(lens_q, lens_kv, H, Hkv, D, dtype, density, seed, q_scale=1.0):
+    rng = np.random.default_rng(seed)
+    qo = np.concatenate([[0], np.cumsum(lens_q)]); kv = np.concatenate([[0], np.cumsum(lens_kv)])
+    qt = 128 // (H // Hkv)
+    qa = [(rng.random((-(-a // qt), Hkv)) < 0.8).astype(np.uint8) for a in lens_q]
+    kk = [(rng.random((-(-a // qt), Hkv, -(-b // 128))) < density).astype(np.uint8) for a, b in zip(lens_q, lens_kv)]
+    q = (wl.randn_bf16((int(qo[-1]), H, D), seed + 1).float() * q_scale).to(dtype)
+    k = wl.randn_bf16((int(kv[-1]), Hkv, D), seed + 2, dtype=dtype)
+    v = wl.randn_bf16((int(kv[-1]), Hkv, D), seed + 3, dtype=dtype)
+    return qo, kv, wl.pack_masks(qa, kk), q, k, v
+
+
+def _plan(device, qo, kv, H, Hkv, D, dtype):
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=device))
+    w.plan(dev(np.asarray(qo, np.int32), device), dev(np.asarray(kv, np.int32), device), H, Hkv, D, q_data_type=dtype)
+    return w
+
+
+@pytest.mark.parametrize("D,H,Hkv,dtype,q_scale", [
+    (128, 8, 8, torch.bfloat16, 1.0), (128, 8, 8, torch.float16, 3.0), (128, 16, 4, torch.bfloat16, 1.0),
+    (64, 8, 8, torch.bfloat16, 3.0), (64, 6, 3, torch.float16, 1.0)])
+def test_many_short_units_against_the_oracle(cuda_device, D, H, Hkv, dtype, q_scale):
+    """With q_scale 3 the logits are N(0, 9): maxima rise by more than the rescale threshold between blocks. The error
+    of one value is at most two roundings to 16 bits (P and O), 2 * 2^-9 * max|v| < 0.02 for bf16 and |v| < 5."""
+    lens_kv = [128, 77, 256, 1, 129, 128, 384, 300, 500, 64, 128, 128, 1100] * 3
+    lens_q = [128, 77, 300, 1, 128, 200, 129, 64, 333, 127, 65, 500, 260] * 3
+    qo, kv, m, q, k, v = _case(lens_q, lens_kv, H, Hkv, D, dtype, 0.7, 31, q_scale)
+    w = _plan(cuda_device, qo, kv, H, Hkv, D, dtype)
+    prior, lse_prior = wl.randn_bf16(q.shape, 9, dtype=dtype), torch.full((q.shape[0], H), 3.0)
+    for _ in range(2):   # twice: the second launch starts from the cursor that the first one put back
+        o, lse = w.run(dev(q, cuda_device), dev(k, cuda_device), dev(v, cuda_device), *masks_to_device(m, cuda_device),
+                       out=dev(prior, cuda_device).clone(), lse=dev(lse_prior, cuda_device).clone(), return_lse=True)
+        w.check_status()
+    n = w.work_lists()["items"][:, 3]
+    assert len(n) > 148 and {0, 1, 2, 3} <= set(n.tolist())
+    ref, ref_lse = oa.sparse_attention(q, k, v, qo, kv, m.sparse_info, m.sparse_kv_info, m.info_indptr, m.kv_info_indptr,
+                                       out_prior=prior, lse_prior=lse_prior, return_lse=True)
+    assert_close_bf16(o, ref, f"D={D} H={H}/{Hkv} {dtype}", allow_ulp=1.0)
+    assert torch.allclose(lse.cpu(), ref_lse, atol=2e-2, rtol=1e-4)
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 5])
+def test_nan_in_a_key_reaches_every_row_that_attends_to_it(cuda_device, blocks):
+    S, H, D = 128 * blocks, 2, 128
+    q, k, v = (wl.randn_bf16((S, H, D), s) for s in (1, 2, 3))
+    k[S - 20, 1, 7] = float("nan")
+    w = _plan(cuda_device, [0, S], [0, S], H, H, D, torch.bfloat16)
+    o = w.run(dev(q, cuda_device), dev(k, cuda_device), dev(v, cuda_device), is_full=True).cpu()
+    w.check_status()
+    assert torch.isnan(o[:, 1]).all() and torch.isfinite(o[:, 0]).all()
