@@ -32,7 +32,7 @@
 // requests of 77 tokens are slower, 55 -> 64 (one masked block and one partial store per unit).
 //
 // Warps: 0-3 softmax stream 0, 4-7 softmax stream 1 (TMEM lane = q row), 8-11 epilogue, 12 TMA producer and drawer of
-// work-list positions, 13 and 14 MMA issuers; 15 only takes part in the register split.
+// work-list positions, 13 and 14 MMA issuers, 15 writes the q-blocks that keep nothing.
 // Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
 
@@ -52,7 +52,8 @@ constexpr int kWarpEpilogue = kSoftmaxWarps;      // first of four (TMEM lane qu
 constexpr int kEpilogueWarps = 4;
 constexpr int kWarpProducer = kWarpEpilogue + kEpilogueWarps;
 constexpr int kWarpMma = kWarpProducer + 1;
-constexpr int kThreads = (kWarpProducer + 4) * 32;   // 512
+constexpr int kWarpZero = kWarpMma + 2;
+constexpr int kThreads = (kWarpZero + 1) * 32;   // 512
 constexpr int kRegsSoftmax = 184, kRegsEpilogue = 88, kRegsOther = 56;  // setmaxnreg split
 // setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with: a split that asks for more
 // never returns.
@@ -79,7 +80,7 @@ struct Tail {
   uint64_t o_full[2];              // the last PV of a unit on a stream is done
   uint64_t o_free[2];              // the epilogue has read a stream's O
   uint64_t iq_full[kItemQ], iq_empty[kItemQ];  // unit queue: the producer draws work-list positions for the CTA
-  int item_q[kItemQ];
+  int4 item_q[kItemQ][2];          // the units' records; no kv blocks: the end
   uint32_t tmem_base;
   int abort_flag;
   float stats_m[2][2][128];        // [unit parity][stream][row]: the maximum the sum refers to
@@ -95,48 +96,36 @@ __device__ __forceinline__ int rot_of(int qb, int n) {
 }
 
 // Work-list positions: position i < gridDim.x goes to CTA i, the following ones are drawn from a device-wide cursor by
-// the producer and passed to the other roles through a small shared-memory queue (-1 ends the sequence).
+// the producer. It passes the records of the units that have kv blocks on to the other roles through a small shared-memory
+// queue; units without any never enter it, so that no role ever walks past several entries in one go: the producer
+// fetches unit u + 1 when the first two blocks of unit u are on their way, at most seven units ahead of the epilogue, and
+// every reader needs no more than that to finish what it has.
 struct ItemDraw {
   Tail* tail;
   int32_t* cursor;
   volatile int* abort_flag;
-  int n_items, n_pub;
-  int p0, p1, p2;  // current, published next, drawn (still in flight) after next: the atomic never sits between two units
-  bool started, ended;
+  int n_items, n_pub, ahead;  // `ahead` is drawn (and in flight) while the position in front of it is looked at
   __device__ __forceinline__ int draw() {
     const int p = atomicAdd(cursor, 1) + static_cast<int>(gridDim.x);
     return p < n_items ? p : -1;
   }
-  __device__ __forceinline__ bool publish(int v) {
-    if (ended) return true;
+  __device__ __forceinline__ void init(Tail* t, int32_t* cur, volatile int* ab, int n) {
+    tail = t; cursor = cur; abort_flag = ab; n_items = n; n_pub = 0;
+    ahead = static_cast<int>(blockIdx.x) < n ? static_cast<int>(blockIdx.x) : -1;
+  }
+  __device__ __forceinline__ int next() {  // the next position, published or not
+    const int p = ahead;
+    if (p >= 0) ahead = draw();
+    return p;
+  }
+  __device__ __forceinline__ bool publish(const int4& u0, const int4& u1) {
     const int slot = n_pub % kItemQ;
     if (!mbar_wait(&tail->iq_empty[slot], (static_cast<uint32_t>(n_pub / kItemQ) & 1u) ^ 1u, abort_flag)) return false;
-    tail->item_q[slot] = v;
+    tail->item_q[slot][0] = u0;
+    tail->item_q[slot][1] = u1;
     mbar_arrive(&tail->iq_full[slot]);
     ++n_pub;
-    if (v < 0) ended = true;
     return true;
-  }
-  __device__ __forceinline__ void init(Tail* t, int32_t* cur, volatile int* ab, int n) {
-    tail = t; cursor = cur; abort_flag = ab; n_items = n; n_pub = 0; started = false; ended = false;
-    p0 = static_cast<int>(blockIdx.x) < n ? static_cast<int>(blockIdx.x) : -1;
-    p1 = p2 = -1;
-    bool ok = publish(p0);
-    if (ok && p0 >= 0) {
-      p1 = draw();
-      ok = publish(p1);
-      if (ok && p1 >= 0) p2 = draw();
-    }
-    if (!ok) p0 = -1;
-  }
-  __device__ __forceinline__ int next() {
-    if (!started) { started = true; return p0; }
-    p0 = p1;
-    if (p0 < 0) return -1;
-    p1 = p2;
-    if (!publish(p1)) return -1;
-    p2 = p1 >= 0 ? draw() : -1;
-    return p0;
   }
 };
 
@@ -146,10 +135,11 @@ struct ItemRead {  // the reading roles: one thread, or all lanes of a warp
   volatile int* abort_flag;
   int k;
   __device__ __forceinline__ void init(Tail* t, volatile int* ab) { tail = t; abort_flag = ab; k = 0; }
-  __device__ __forceinline__ int next() {
+  __device__ __forceinline__ bool next(int4& u0, int4& u1) {  // false at the end
     const int slot = k % kItemQ;
-    if (!mbar_wait(&tail->iq_full[slot], static_cast<uint32_t>(k / kItemQ) & 1u, abort_flag)) return -1;
-    const int v = tail->item_q[slot];
+    if (!mbar_wait(&tail->iq_full[slot], static_cast<uint32_t>(k / kItemQ) & 1u, abort_flag)) return false;
+    u0 = tail->item_q[slot][0];
+    u1 = tail->item_q[slot][1];
     if (kWholeWarp) {
       __syncwarp();
       if ((threadIdx.x & 31) == 0) mbar_arrive(&tail->iq_empty[slot]);
@@ -157,7 +147,7 @@ struct ItemRead {  // the reading roles: one thread, or all lanes of a warp
       mbar_arrive(&tail->iq_empty[slot]);
     }
     ++k;
-    return v;
+    return u0.x > 0;
   }
 };
 
@@ -258,10 +248,12 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         n_next = 0;
         while (true) {
           const int pos = src.next();
-          if (pos < 0) return;
+          if (pos < 0) { ok = src.publish(make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0)); return; }
           const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
           const int4 u0 = up[0], u1 = up[1];
-          if (u0.x <= 0) continue;
+          if (u0.x <= 0) continue;   // (warp 15 writes its zeros)
+          ok = src.publish(u0, u1);
+          if (!ok) return;
           n_next = u0.x;
           kv_off_next = u0.y;
           hk_next = (u0.z & 0xffff) - a.head_begin;   // a unit's head is the kv head; its q tile holds the group's q heads
@@ -345,11 +337,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       bool ok = true;
       int n_next = 0;
       auto fetch = [&]() {  // the block count of the next unit, one unit ahead; 0 at the end
-        do {
-          const int pos = src.next();
-          if (pos < 0) { n_next = 0; return; }
-          n_next = a.units[8 * static_cast<int64_t>(pos)];
-        } while (n_next <= 0);
+        int4 u0, u1;
+        n_next = src.next(u0, u1) ? u0.x : 0;
       };
       fetch();
       int n = 0, j = 0, unit_no = -1;
@@ -421,6 +410,28 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         pv_first = new_unit;
       }
     }
+  } else if (warp == kWarpZero) {
+    // ------------------------------------------------------------------ active q-blocks that keep nothing: zeros, lse = -5e4
+    // Every CTA looks at its share of the positions, whoever draws them.
+    const int grp = a.group_size, grp_shift = 31 - __clz(grp);
+    for (int base = static_cast<int>(blockIdx.x); base < n_items; base += 32 * static_cast<int>(gridDim.x)) {
+      const int mine = base + lane * static_cast<int>(gridDim.x);
+      uint32_t todo = __ballot_sync(0xffffffffu, mine < n_items && a.units[8 * static_cast<int64_t>(mine)] <= 0);
+      for (; todo != 0u; todo &= todo - 1u) {
+        const int pos = base + (__ffs(static_cast<int>(todo)) - 1) * static_cast<int>(gridDim.x);
+        const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
+        const int4 u0 = up[0], u1 = up[1];
+        const int h = (u0.z & 0xffff) - a.head_begin, rows = (u1.x & 0xffff) * grp;
+        for (int i = lane; i < rows * (kD / 8); i += 32) {
+          const int r = i / (kD / 8);
+          const int64_t tok = static_cast<int64_t>(u0.w) + (r >> grp_shift);
+          const int hq = h * grp + (r & (grp - 1));
+          uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + tok * a.o_stride_n + static_cast<int64_t>(hq) * a.o_stride_h;
+          reinterpret_cast<uint4*>(orow)[i % (kD / 8)] = make_uint4(0u, 0u, 0u, 0u);
+          if (i % (kD / 8) == 0 && a.lse != nullptr) a.lse[tok * a.lse_stride_n + hq] = -5e4f;
+        }
+      }
+    }
   }
   } else if (warp >= kWarpEpilogue) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
@@ -438,25 +449,14 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
     ItemRead<true> src;
     src.init(tail, abort_flag);
     while (true) {
-      const int pos = src.next();
-      if (pos < 0) break;
-      const int4* up = reinterpret_cast<const int4*>(a.units + 8 * static_cast<int64_t>(pos));
-      const int4 u0 = up[0], u1 = up[1];
+      int4 u0, u1;
+      if (!src.next(u0, u1)) break;
       const int q_row0 = u0.w, q_valid = u1.x & 0xffff, h = (u0.z & 0xffff) - a.head_begin;
       // Row r of a tile is token q_row0 + r / group, q head h * group + r % group (group = 1: the row itself).
       const bool row_ok = row < q_valid * grp;
       const int64_t grow = static_cast<int64_t>(q_row0) + row_tok;
       const int hq = h * grp + row_head;
-      uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + grow * a.o_stride_n + static_cast<int64_t>(hq) * a.o_stride_h;
       float* lse = a.lse != nullptr ? a.lse + grow * a.lse_stride_n + hq : nullptr;
-      if (u0.x <= 0) {  // active q-block that keeps nothing: zeros, lse = -5e4
-        if (row_ok) {
-#pragma unroll 1
-          for (int i = 0; i < kD / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0u, 0u, 0u, 0u);
-          if (lse != nullptr) *lse = -5e4f;
-        }
-        continue;
-      }
       const uint32_t ip = item & 1u;
       if (!mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag)) break;
       const float m0 = tail->stats_m[ip][0][row], m1 = tail->stats_m[ip][1][row];
@@ -560,14 +560,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
     // the record of the next unit is fetched while the current one runs
     int n_next = -1, qb_next = 0, rag_next = 0;
     auto fetch = [&]() {
-      n_next = -1;
-      while (true) {
-        const int pos = src.next();
-        if (pos < 0) return;
-        const int32_t* up = a.units + 8 * static_cast<int64_t>(pos);
-        n_next = up[0];
-        if (n_next > 0) { qb_next = up[3] >> 7; rag_next = up[4] >> 16; return; }
-      }
+      int4 u0, u1;
+      n_next = src.next(u0, u1) ? u0.x : -1;
+      qb_next = u0.w >> 7;
+      rag_next = u1.x >> 16;
     };
     fetch();
     while (ok && n_next > 0) {

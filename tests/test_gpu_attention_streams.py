@@ -55,6 +55,33 @@ def test_many_short_units_against_the_oracle(cuda_device, D, H, Hkv, dtype, q_sc
     assert torch.allclose(lse.cpu(), ref_lse, atol=2e-2, rtol=1e-4)
 
 
+@pytest.mark.parametrize("keep", [0.0, 0.02, 0.25])
+def test_long_runs_of_units_that_keep_nothing(cuda_device, keep):
+    """Active q-blocks without a kept kv-block sit at the end of the processing order, several per CTA behind each other."""
+    S, H, D = 4992, 32, 64
+    n = S // 128
+    rng = np.random.default_rng(5)
+    kk = np.zeros((n, H, n), np.uint8)
+    some = rng.random((n, H)) < keep
+    kk[some] = rng.random((int(some.sum()), n)) < 0.2
+    m = wl.pack_masks([np.ones((n, H), np.uint8)], [kk])
+    q, k, v = (wl.randn_bf16((S, H, D), s) for s in (1, 2, 3))
+    w = _plan(cuda_device, [0, S], [0, S], H, H, D, torch.bfloat16)
+    prior = wl.randn_bf16(q.shape, 9)
+    o, lse = w.run(dev(q, cuda_device), dev(k, cuda_device), dev(v, cuda_device), *masks_to_device(m, cuda_device),
+                   out=dev(prior, cuda_device).clone(), return_lse=True)
+    w.check_status()
+    kept = kk.any(2)
+    blocks = o.cpu().view(n, 128, H, D).permute(0, 2, 1, 3)
+    assert (blocks[torch.from_numpy(~kept)] == 0).all()
+    assert (lse.cpu().view(n, 128, H).permute(0, 2, 1)[torch.from_numpy(~kept)] == -5e4).all()
+    for h in np.flatnonzero(kept.any(0))[:6]:
+        one = wl.pack_masks([np.ones((n, 1), np.uint8)], [np.ascontiguousarray(kk[:, h:h + 1])])
+        ref = oa.sparse_attention(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], [0, S], [0, S], one.sparse_info, one.sparse_kv_info,
+                                  one.info_indptr, one.kv_info_indptr)
+        assert_close_bf16(o[:, h:h + 1], ref, f"head {h}")
+
+
 @pytest.mark.parametrize("blocks", [1, 2, 5])
 def test_nan_in_a_key_reaches_every_row_that_attends_to_it(cuda_device, blocks):
     S, H, D = 128 * blocks, 2, 128
