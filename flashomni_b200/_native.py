@@ -13,6 +13,7 @@ from ctypes import c_char_p, c_float, c_int32, c_int64, c_size_t, c_void_p
 _LIB_ENV = "FLASHOMNI_B200_LIB"
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _DEFAULT = os.path.join(_HERE, "lib", "libflashomni_b200.so")
+_HOST = os.path.join(_HERE, "lib", "_fo_host.so")
 
 FO_OK, FO_ERR_INVALID_ARG, FO_ERR_UNSUPPORTED, FO_ERR_CUDA, FO_ERR_WORKSPACE = 0, 1, 2, 3, 4
 FO_DTYPE_F16, FO_DTYPE_BF16 = 0, 1
@@ -95,6 +96,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None   # the Python extension that issues the usual calls (csrc/host.cpp)
 
 
 def lib_path() -> str:
@@ -119,8 +121,33 @@ def load():
         fn.argtypes = args
     if lib.fo_abi_version() != 2:
         raise RuntimeError("flashomni_b200: ABI version mismatch")
+    _load_host(lib)
     _lib = lib
     return lib
+
+
+def _load_host(lib) -> None:
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        if not os.path.exists(_HOST):
+            raise RuntimeError(f"flashomni_b200: Python extension not found at {_HOST}; build it with "
+                               "`python -m flashomni_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_fo_host", _HOST)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fo_host", loader))
+        loader.exec_module(module)
+        module.bind(lib._handle)
+        _host = module
+    else:
+        _host.bind(lib._handle)
+
+
+def host():
+    """The extension of csrc/host.cpp: functions that do a whole call of an op, or return None for what they do not take."""
+    if _lib is None:
+        load()
+    return _host
 
 
 def last_error() -> str:

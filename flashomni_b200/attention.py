@@ -124,6 +124,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         self._side_stream = None
         self._prepared_event = None
         self._prepared_key = None
+        self._fast_plan = self._fast_args = None
 
     @property
     def is_cuda_graph_enabled(self) -> bool:
@@ -386,6 +387,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         # ... and the same as the host array that fo_layer_lists reads
         fixed = (self._qo_indptr_buf.data_ptr(), self._kv_indptr_buf.data_ptr()) + self._list_args
         self._layer_plan = (ctypes.c_int64 * len(fixed))(*fixed)
+        self._fast_plan = None
         pbytes = lib.fo_attn_partial_bytes(self._partial_slots)
         fw = self._float_workspace_buffer
         self._partials = None
@@ -396,6 +398,15 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 self._partials = raw[shift: shift + pbytes]
             else:
                 self._partials = torch.empty(pbytes, dtype=torch.uint8, device=self.device)
+        # ... and the whole plan for the native function that issues the usual call (no causal or custom mask)
+        if not self._causal and self._packed_custom_mask is None:
+            self._fast_args = self._list_args
+            self._fast_plan = _native.host().attn_plan(
+                self.device.index, native_dtype(self._cached_q_data_type),
+                _FP8_KINDS.get(self._cached_kv_data_type, -1), self._total_q, self._num_qo_heads, self._num_kv_heads,
+                self._head_dim, self._total_kv, self._batch_size, 1 if self._kv_layout == "NHD" else 0,
+                1 if self._rows_from_0 and not self._use_cuda_graph else 0, self._qo_indptr_buf.data_ptr(),
+                self._kv_indptr_buf.data_ptr(), *self._list_args, ptrs["status"], _native.ptr(self._partials))
 
     # ------------------------------------------------------------------------------------------ run
     def run(
@@ -419,6 +430,21 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         (zeros when `out` is allocated here). Reference: flashomni/attention.py:709-835."""
         if not self._planned:
             raise RuntimeError("plan() must be called before run()")
+        if self._fast_plan is not None and self._fast_args is self._list_args:
+            # the usual call in one native function; it returns None, having done nothing, for anything else
+            prepared = None
+            if self._prepared_key is not None and (is_full or (sparse_info is not None and sparse_kv_info is not None)):
+                if self._prepared_key == self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr,
+                                                        sparse_kv_info_indptr, is_full):
+                    prepared = self._prepared_event
+            r = _native.host().attn_run(self._fast_plan, q, k, v, sparse_info, sparse_kv_info, sparse_info_indptr,
+                                        sparse_kv_info_indptr, is_full, out, lse, return_lse, self._sm_scale,
+                                        self._logits_soft_cap, prepared)
+            if r is not None:
+                self._prepared_key = None
+                if type(r) is int:
+                    _native.check(r, "BatchFlashOmniFAWithRaggedKVWrapper.run")
+                return r
         _native.require_cuda(q, k, v)
         _check_cached_qkv_data_type(q, k, self._cached_q_data_type, self._cached_kv_data_type)
         if v.dtype != k.dtype:

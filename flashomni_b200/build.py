@@ -2,6 +2,7 @@
 
     python -m flashomni_b200.build [--force] [--verbose]
 
+and, with the host compiler, flashomni_b200/lib/_fo_host.so (csrc/host.cpp), the Python extension that issues the usual calls.
 Each .cu under csrc/ is compiled to an object file (in parallel) and the objects are linked into
 flashomni_b200/lib/libflashomni_b200.so. Objects are rebuilt when their source or any header is
 newer. No GPU is needed to build.
@@ -26,6 +27,22 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
           "--expt-relaxed-constexpr"]
+
+
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_LIB = os.path.join(LIBDIR, "_fo_host.so")
+
+
+def _host_cmd():
+    import sysconfig
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f"-I{t}/include",
+            f"-I{t}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include", HOST_SRC,
+            "-o", HOST_LIB, f"-L{t}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{cuda}/lib64",
+            "-lcudart"]
 
 
 def _headers():
@@ -54,6 +71,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
+    cuda_jobs = len(jobs)
+    if force or _stale(HOST_LIB, [HOST_SRC, os.path.join(HERE, "..", "include", "flashomni_b200.h")]):
+        jobs.append(_host_cmd())
 
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
@@ -65,9 +85,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 if verbose or r.returncode != 0:
                     sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
                 if r.returncode != 0:
-                    raise RuntimeError("nvcc failed for " + cmd[-3])
+                    raise RuntimeError(f"{os.path.basename(cmd[0])} failed: " + " ".join(cmd[-3:]))
     objs = [os.path.join(OBJDIR, s.replace(".cu", ".o")) for s in sources]
-    if force or jobs or _stale(LIB, objs):
+    if force or cuda_jobs or _stale(LIB, objs):
         cmd = [NVCC, *ARCH_FLAGS, "-shared", "-cudart", "shared", "-o", LIB, *objs,
                "-Xlinker", "-rpath", "-Xlinker", "/usr/local/cuda/lib64"]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -977,8 +977,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const __grid_con
 namespace {
 template <bool kBf16, bool kSoftCap, bool kParts, int kD, int kMask = 0>
 cudaError_t launch_one(const AttnArgs& a, int ctas, cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(attention_kernel<kBf16, kSoftCap, kParts, kD, kMask>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  static std::atomic<uint64_t> done{0};
+  const cudaError_t e = allow_smem(attention_kernel<kBf16, kSoftCap, kParts, kD, kMask>, kSmemBytes, done);
   if (e != cudaSuccess) return e;
   return launch_dependent(attention_kernel<kBf16, kSoftCap, kParts, kD, kMask>, ctas, kThreads, kSmemBytes, stream,
                           a.after_lists != 0, a);

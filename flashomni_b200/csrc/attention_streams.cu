@@ -722,8 +722,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
 
 template <bool kBf16, bool kSoftCap, int kD>
 cudaError_t launch_one(const AttnArgs& a, int ctas, cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(attention_streams_kernel<kBf16, kSoftCap, kD>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  static std::atomic<uint64_t> done{0};
+  const cudaError_t e = allow_smem(attention_streams_kernel<kBf16, kSoftCap, kD>, kSmemBytes, done);
   if (e != cudaSuccess) return e;
   return launch_dependent(attention_streams_kernel<kBf16, kSoftCap, kD>, ctas, kThreads, kSmemBytes, stream,
                           a.after_lists != 0, a);

@@ -476,7 +476,8 @@ cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream) {
   if (cap <= 0) return cudaSuccess;
   const int grid = cap < max_ctas ? cap : max_ctas;
   const auto kernel = a.is_bf16 ? gemm_kernel<true> : gemm_kernel<false>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  static std::atomic<uint64_t> done[2] = {{0}, {0}};
+  const cudaError_t e = allow_smem(kernel, kSmemBytes, done[a.is_bf16 ? 1 : 0]);
   if (e != cudaSuccess) return e;
   return launch_dependent(kernel, grid, kThreads, kSmemBytes, stream, g.after_list != 0, g);
 }

@@ -281,7 +281,8 @@ bool gemm_tall_applies(const GemmArgs& a, int sm_count) { return tall_tile_cols(
 namespace {
 template <bool kBf16, int kBN>
 cudaError_t launch_tall(const GemmArgs& a, int grid, cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(gemm_tall_kernel<kBf16, kBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  static std::atomic<uint64_t> done{0};
+  const cudaError_t e = allow_smem(gemm_tall_kernel<kBf16, kBN>, kSmemBytes, done);
   if (e != cudaSuccess) return e;
   gemm_tall_kernel<kBf16, kBN><<<grid, kThreads, kSmemBytes, stream>>>(a);
   return cudaGetLastError();

@@ -6,9 +6,24 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "ptx.cuh"
 
 namespace fo {
+
+// Raises a kernel's limit of dynamic shared memory, once per kernel and device (the call costs about a microsecond).
+template <class Kernel>
+inline cudaError_t allow_smem(Kernel* kernel, int bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_relaxed) & bit) != 0) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 // Launches a kernel whose arguments struct is `args`; with `dependent` it may start while the kernel in front of it in the
 // stream still runs (programmatic dependent launch): it must then wait (griddepcontrol.wait) before it touches memory.

@@ -73,6 +73,13 @@ def flashomni_gemm(
     reference behaviour) let B hold the rows of a head window when heads are split over GPUs. `worklist`
     (extension): a list from `prepare_gemm_q_list` for the same mask and shape, built earlier (e.g. on a side
     stream); the mask arguments are then not read."""
+    # the usual call in one native function; it returns None, having done nothing, for anything else
+    r = _native.host().gemm_q(A, B, num_qo_heads, sparse_info, sparse_info_indptr, num_text_tokens, bias, out, sparse_q_size,
+                              is_full, head_begin, head_dim, worklist, _workspaces)
+    if r is not None:
+        if type(r) is int:
+            _native.check(r, "flashomni_gemm")
+        return r
     _gemm_common(A, B, "flashomni_gemm")
     batch, M, K = A.shape
     N = B.shape[0]
@@ -135,6 +142,12 @@ def flashomni_gemm_reduction(
     active heads (is_for_cache=False, init = the cached [batch, M, N] tensor passed as `bias`) or inactive
     heads (is_for_cache=True, init = 1-D bias) (reference: flashomni/gemm.py:188-216, kernel
     gemm_reduction.cuh:27-276). `head_begin` / `head_dim` / `out` are extensions with reference defaults."""
+    r = _native.host().gemm_o(A, B, num_qo_heads, sparse_info, sparse_info_indptr, num_text_tokens, bias, is_for_cache,
+                              sparse_q_size, head_begin, head_dim, out, worklist, _workspaces)
+    if r is not None:
+        if type(r) is int:
+            _native.check(r, "flashomni_gemm_reduction")
+        return r
     _gemm_common(A, B, "flashomni_gemm_reduction")
     if worklist is None and (sparse_info is None or sparse_info_indptr is None):
         raise ValueError("flashomni_gemm_reduction: sparse_info and sparse_info_indptr are required")

@@ -44,6 +44,12 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
     new_indptr[i+1]-new_indptr[i] == ceil(len_i/8) (reference: flashomni/quantization.py:102-159,
     including its one host synchronisation to size the output)."""
     little = _little(bitorder)
+    # the usual call in one native function; it returns None for anything else
+    r = _native.host().segment_packbits(x, indptr, little)
+    if r is not None:
+        if type(r) is int:
+            _native.check(r, "segment_packbits")
+        return r
     _native.require_cuda(x)
     n_seg = len(indptr) - 1
     refused = False

@@ -33,6 +33,12 @@ def select_blocks(pooled_score: torch.Tensor, num_text_blocks: int, q_threshold:
     q_threshold: scalar or [B]; kv_threshold: scalar or [H] (cumulative softmax mass that may be switched off).
     Returns (sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr): uint8 bit streams
     (little-endian, one segment per request) and int32 byte indptrs."""
+    # the usual call in one native function; it returns None, having done nothing, for anything else
+    r = _native.host().select_blocks(pooled_score, num_text_blocks, q_threshold, kv_threshold, zero_inactive)
+    if r is not None:
+        if type(r) is int:
+            _native.check(r, "select_blocks")
+        return r
     if pooled_score.dim() != 4 or pooled_score.shape[2] != pooled_score.shape[3]:
         raise ValueError("pooled_score must be [B, H, n, n]")
     if pooled_score.dtype != torch.float32:
