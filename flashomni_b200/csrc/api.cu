@@ -89,14 +89,14 @@ thread_local TmapSlot t_tmaps[kTmapSlots];
 }  // namespace
 
 int encode_tmap_16bit(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
-                      const uint64_t* strides_bytes, const uint32_t* box, bool swizzle128) {
+                      const uint64_t* strides_bytes, const uint32_t* box, int swizzle) {
   if (rank < 1 || rank > 5) return -2;
   TmapKey key;
   memset(&key, 0, sizeof(key));
   key.base = base;
   key.rank = rank;
-  key.swizzle = swizzle128 ? 1 : 0;
-  uint64_t h = reinterpret_cast<uint64_t>(base) * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(rank * 2 + key.swizzle);
+  key.swizzle = swizzle;
+  uint64_t h = reinterpret_cast<uint64_t>(base) * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(rank * 128 + key.swizzle);
   for (int i = 0; i < rank; ++i) {
     key.dims[i] = dims[i];
     key.strides[i] = i > 0 ? strides_bytes[i] : 0;
@@ -123,7 +123,7 @@ int encode_tmap_16bit(CUtensorMap* out, const void* base, int rank, const uint64
   }
   const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base),
                         gdim, gstr, bdim, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                        swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE),
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return static_cast<int>(r);
   slot.key = key;
@@ -449,7 +449,7 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     // the output boxes of the kernel that will run (see AttnArgs)
     const bool streams = attention_streams_applies(a);
     const uint32_t obox[3] = {streams ? 64u : 32u, group, (streams ? 32u : 16u) / group};
-    if (r == 0) r = encode_tmap_16bit(&a.tmap_o, o, 3, qd, os, obox, streams);
+    if (r == 0) r = encode_tmap_16bit(&a.tmap_o, o, 3, qd, os, obox, streams ? 128 : 0);
     if (r != 0) {
       char buf[96];
       snprintf(buf, sizeof(buf), "fo_sparse_attn_fwd: cuTensorMapEncodeTiled failed (%d)", r);
@@ -881,6 +881,13 @@ int gemm_o_impl(const void* x, const void* w, void* y, const void* init, int32_t
   g.y = y;
   g.init = init;
   g.init_mode = init == nullptr ? kInitNone : (init_is_full ? kInitFull : kInitBias1D);
+  if (g.init_mode == kInitFull) {
+    const uint32_t box[2] = {32, 128};   // init slabs come in, and result slabs leave, 32 columns at a time
+    const uint64_t cd[2] = {static_cast<uint64_t>(n), static_cast<uint64_t>(batch) * m};
+    const uint64_t cst[2] = {0, static_cast<uint64_t>(n) * 2};
+    if (encode_tmap_16bit(&g.tmap_c, init, 2, cd, cst, box, 64) != 0 || encode_tmap_16bit(&g.tmap_y, y, 2, cd, cst, box, 64) != 0)
+      return fail(FO_ERR_CUDA, "fo_gemm_o: cuTensorMapEncodeTiled failed (init)");
+  }
   g.mode = kGemmO;
   g.is_bf16 = dtype == FO_DTYPE_BF16;
   g.batch = batch;

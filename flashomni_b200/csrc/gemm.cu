@@ -14,8 +14,8 @@
 // the A operand is read from shared memory once per 256 output columns. A leftover single block
 // runs as N = 128.
 //
-// CTA = 192 threads: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer. K step 64 (one
-// 128-byte swizzle atom), 4-stage ring of (A 16 KB + B 32 KB), two 256-column TMEM accumulators so
+// CTA = 192 threads: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer (with a full init tensor warp 6 loads its
+// slabs). K step 64 (one 128-byte swizzle atom), 4-stage (3) ring of (A 16 KB + B 32 KB), two 256-column TMEM accumulators so
 // the epilogue of tile i overlaps the main loop of tile i+1. The epilogue converts 64-column slabs
 // (TMEM -> registers -> +init -> 16-bit) into a swizzled shared-memory slab and hands each slab to a
 // TMA store, so global writes are full 128-byte lines and asynchronous. The tiles of the sparse modes
@@ -29,14 +29,21 @@ namespace fo {
 namespace {
 
 constexpr int kBM = 128, kBNH = 128, kBK = 64;
-constexpr int kStages = 4;
 constexpr int kABytes = kBM * kBK * 2;        // 16 KB
 constexpr int kBHalfBytes = kBNH * kBK * 2;   // 16 KB per 128-column block of W
 constexpr int kStageBytes = kABytes + 2 * kBHalfBytes;
-constexpr int kSlabCols = 64;
-constexpr int kSlabBytes = kBM * kSlabCols * 2;  // 16 KB
-constexpr int kSlabBufs = 2;
-constexpr int kThreads = 192;
+constexpr int kStages = 4;
+constexpr int kSlabsBytes = 2 * kBM * 64 * 2;    // staging of the epilogue: two slabs of 64 columns, or four of 32
+constexpr int kMaxSlabBufs = 4;
+// With a full init tensor (GEMM-O and the cached contribution) the init values of a slab are loaded by TMA into the staging
+// slab that the result leaves from, up to three slabs ahead, by a warp of their own. Loaded by the epilogue threads instead, one
+// slab ahead and a row per thread, they made the epilogue wait for HBM on every slab. GEMM-O with its list, inputs that change
+// from call to call, us on a B200, threads -> TMA: 9216 rows x 3072 with 3 / 6 / 12 / 24 heads 54.7 / 57.0 / 63.9 / 90.7 -> 41.7 /
+// 45.0 / 55.6 / 87.1, 4608 rows 31.5 / 34.5 / 40.6 / 56.5 -> 26.4 / 29.2 / 36.9 / 54.1, 1024 rows with 24 heads 33.3 -> 32.1, 4608 x 5120
+// with 40 heads 125.8 -> 121.6. Slabs of 64 columns would leave three operand stages: 38.0 us with 3 heads of 9216
+// rows, but 91.3 with 24 and 239 against 230 with 40 of 9216 x 5120.
+constexpr int threads_of(bool cache) { return cache ? 224 : 192; }
+constexpr int slabs_of(bool cache) { return cache ? 4 : 2; }
 constexpr int kTmemCols = 512;
 constexpr int kMaxHeadsSmem = 128;
 constexpr int kTileQ = 8;   // entries of the tile queue (the producer runs at most a few tiles ahead of the epilogue)
@@ -44,6 +51,8 @@ constexpr int kTileQ = 8;   // entries of the tile queue (the producer runs at m
 struct Tail {
   uint64_t full[kStages];
   uint64_t empty[kStages];
+  uint64_t slab_full[kMaxSlabBufs];    // init values of a slab have landed
+  uint64_t slab_empty[kMaxSlabBufs];   // the store of the slab has read it
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t tq_full[kTileQ];   // tile queue: the producer warp draws tile numbers and hands them to the other roles
@@ -54,7 +63,8 @@ struct Tail {
   int epi_go;                   // outcome of the epilogue warps' vote of the current round
   int heads[2][kMaxHeadsSmem];  // GEMM-O: head lists of the current and the next tile, staged for the producer
 };
-constexpr int kSmemBytes = kStages * kStageBytes + kSlabBufs * kSlabBytes + 1024 + static_cast<int>(sizeof(Tail));
+constexpr int kSmemBytes = kStages * kStageBytes + kSlabsBytes + 1024 + static_cast<int>(sizeof(Tail));
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 
 struct TileInfo {
@@ -109,13 +119,15 @@ __device__ __forceinline__ TileInfo get_tile(const GemmArgs& a, int t) {
 
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant__ GemmArgs a) {
+template <bool kBf16, bool kCache>
+__global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __grid_constant__ GemmArgs a) {
+  constexpr int kSlabBufs = slabs_of(kCache), kSlabCols = kCache ? 32 : 64, kSlabBytes = kBM * kSlabCols * 2;
+  constexpr int kSlabsPerBlock = kBNH / kSlabCols;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* smem_slab = smem + kStages * kStageBytes;
-  Tail* tail = reinterpret_cast<Tail*>(smem_slab + kSlabBufs * kSlabBytes);
+  Tail* tail = reinterpret_cast<Tail*>(smem_slab + kSlabsBytes);
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5;
@@ -132,7 +144,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     }
     for (int i = 0; i < kTileQ; ++i) {
       mbar_init(&tail->tq_full[i], 1);
-      mbar_init(&tail->tq_empty[i], 5);  // the MMA thread and the four epilogue warps
+      mbar_init(&tail->tq_empty[i], kCache ? 6 : 5);  // the MMA thread, the four epilogue warps, the loader of init slabs
+    }
+    for (int i = 0; i < kSlabBufs; ++i) {
+      mbar_init(&tail->slab_full[i], 1);
+      mbar_init(&tail->slab_empty[i], 1);
     }
     tail->abort_flag = 0;
     fence_barrier_init();
@@ -141,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     tma_prefetch_desc(&a.tmap_a);
     tma_prefetch_desc(&a.tmap_b);
     tma_prefetch_desc(&a.tmap_y);
+    if (kCache) tma_prefetch_desc(&a.tmap_c);
   }
   if (warp == 5) {
     tmem_alloc(&tail->tmem_base, kTmemCols);
@@ -317,6 +334,27 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         if (acc == 0) acc_phase ^= 1u;
       }
     }
+  } else if (kCache && warp == 6) {
+    // ------------------------------------------------------------- loader of init slabs, in the epilogue's order
+    if (lane == 0) {
+      uint32_t count = 0;
+      for (int k_seq = 0;; ++k_seq) {
+        const int t = read_slot(k_seq);
+        if (t < 0) break;
+        const TileInfo ti = get_tile(a, t);
+        const int nslab = ti.w_row1 >= 0 ? 2 * kSlabsPerBlock : kSlabsPerBlock;
+        bool ok = true;
+        for (int s = 0; s < nslab && ok; ++s, ++count) {
+          const uint32_t buf = count % kSlabBufs;
+          ok = mbar_wait(&tail->slab_empty[buf], ((count / kSlabBufs) & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(&tail->slab_full[buf], kSlabBytes);
+          tma_load_2d(smem_slab + buf * kSlabBytes, &a.tmap_c, &tail->slab_full[buf],
+                      (s < kSlabsPerBlock ? ti.w_row0 : ti.w_row1) + (s % kSlabsPerBlock) * kSlabCols, ti.a_row);
+        }
+        if (!ok) break;
+      }
+    }
   } else {
     // ------------------------------------------------------------- epilogue warps 0..3
     int acc = 0;
@@ -324,7 +362,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     uint32_t slab_count = 0;  // slabs handed to TMA stores so far (selects the staging buffer)
     const uint16_t* init16 = reinterpret_cast<const uint16_t*>(a.init);
     const int r_in_tile = warp * 32 + lane;
-    const uint32_t swz = static_cast<uint32_t>(r_in_tile & 7);
+    // 16-byte pieces of a row of the slab: the 128-byte swizzle of 64 columns, the 64-byte one of 32
+    constexpr int kPieces = kSlabCols / 8;
+    const uint32_t swz = static_cast<uint32_t>(kCache ? (r_in_tile >> 1) & 3 : r_in_tile & 7);
     TileInfo nxt;
     nxt.a_row = nxt.w_row0 = nxt.nkb = 0; nxt.w_row1 = -1; nxt.heads = nullptr;
     auto read_slot_warp = [&](int k) -> int {  // lane 0 reads, the warp shares the value
@@ -346,18 +386,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         if (t_nxt >= 0) nxt = get_tile(a, t_nxt);
         t_cur = t_nxt;
       }
-      const int64_t row = static_cast<int64_t>(ti.a_row) + r_in_tile;
-      const int nslab = ti.w_row1 >= 0 ? 4 : 2;
+      const int nslab = ti.w_row1 >= 0 ? 2 * kSlabsPerBlock : kSlabsPerBlock;
       // init values of slab 0 are fetched before the accumulator is waited for
-      uint4 initv[8];
+      uint4 initv[kPieces];
       auto load_init = [&](int s) {
-        const int col0 = ((s >> 1) == 0 ? ti.w_row0 : ti.w_row1) + (s & 1) * kSlabCols;
+        const int col0 = (s < kSlabsPerBlock ? ti.w_row0 : ti.w_row1) + (s % kSlabsPerBlock) * kSlabCols;
         if (a.init_mode == kInitBias1D) {
           const uint4* p = reinterpret_cast<const uint4*>(init16 + col0);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) initv[i] = __ldg(p + i);
-        } else if (a.init_mode == kInitFull) {
-          const uint4* p = reinterpret_cast<const uint4*>(init16 + row * a.n + col0);
 #pragma unroll
           for (int i = 0; i < 8; ++i) initv[i] = __ldg(p + i);
         }
@@ -375,29 +410,37 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(acc * 2 * kBNH);
 #pragma unroll 1
       for (int s = 0; s < nslab; ++s) {
-        const int col0 = ((s >> 1) == 0 ? ti.w_row0 : ti.w_row1) + (s & 1) * kSlabCols;
-        uint32_t v0[32], v1[32];
+        const int col0 = (s < kSlabsPerBlock ? ti.w_row0 : ti.w_row1) + (s % kSlabsPerBlock) * kSlabCols;
+        uint32_t v[kSlabCols];
         if (ti.nkb > 0) {
-          tmem_ld_x32(taddr + static_cast<uint32_t>(s * kSlabCols), v0);
-          tmem_ld_x32(taddr + static_cast<uint32_t>(s * kSlabCols + 32), v1);
+          tmem_ld_x32(taddr + static_cast<uint32_t>(s * kSlabCols), v);
+          if constexpr (kSlabCols == 64) tmem_ld_x32(taddr + static_cast<uint32_t>(s * kSlabCols + 32), v + 32);
           tmem_wait_ld();
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) { v0[i] = 0u; v1[i] = 0u; }
+          for (int i = 0; i < kSlabCols; ++i) v[i] = 0u;
         }
         if (s == nslab - 1) {  // accumulator fully read: hand it back to the MMA warp
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tail->acc_empty[acc]);
         }
-        uint4 outv[8];
+        uint8_t* buf = smem_slab + (slab_count % kSlabBufs) * kSlabBytes;
+        uint8_t* rowp = buf + r_in_tile * kSlabCols * 2;
+        bool ok = true;
+        if constexpr (kCache) {  // this thread's row of the slab
+          ok = __all_sync(0xffffffffu, mbar_wait(&tail->slab_full[slab_count % kSlabBufs], (slab_count / kSlabBufs) & 1u, abort_flag) ? 1 : 0) != 0;
+#pragma unroll
+          for (int c = 0; c < kPieces; ++c) initv[c] = *reinterpret_cast<const uint4*>(rowp + ((static_cast<uint32_t>(c) ^ swz) << 4));
+        }
+        uint4 outv[kPieces];
         uint32_t* o32 = reinterpret_cast<uint32_t*>(outv);
         const uint32_t* a32 = reinterpret_cast<const uint32_t*>(initv);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float lo = __uint_as_float(i < 16 ? v0[2 * i] : v1[2 * i - 32]);
-          float hi = __uint_as_float(i < 16 ? v0[2 * i + 1] : v1[2 * i - 31]);
-          if (a.init_mode != kInitNone) {
+        for (int i = 0; i < kSlabCols / 2; ++i) {
+          float lo = __uint_as_float(v[2 * i]);
+          float hi = __uint_as_float(v[2 * i + 1]);
+          if (kCache || a.init_mode != kInitNone) {
             if (kBf16) {
               lo += __uint_as_float(a32[i] << 16);
               hi += __uint_as_float(a32[i] & 0xFFFF0000u);
@@ -409,20 +452,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
           }
           o32[i] = kBf16 ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
         }
-        if (s + 1 < nslab) load_init(s + 1);  // next slab's init loads fly during the store hand-off
-        // staging buffer of this slab must no longer be read by the store issued two slabs ago
-        uint8_t* buf = smem_slab + (slab_count & 1u) * kSlabBytes;
-        if (threadIdx.x == 0) tma_store_wait_read<1>();
-        epi_bar();
-        uint8_t* rowp = buf + r_in_tile * 128;
+        if constexpr (!kCache) {
+          if (s + 1 < nslab) load_init(s + 1);  // next slab's init loads fly during the store hand-off
+          // staging buffer of this slab must no longer be read by the store issued two slabs ago
+          if (threadIdx.x == 0) tma_store_wait_read<1>();
+          epi_bar();
+        }
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
+        for (int c = 0; c < kPieces; ++c)
           *reinterpret_cast<uint4*>(rowp + ((static_cast<uint32_t>(c) ^ swz) << 4)) = outv[c];
         fence_proxy_async_smem();
         epi_bar();
         if (threadIdx.x == 0) {
-          tma_store_2d(&a.tmap_y, buf, col0, ti.a_row);
+          if (ok) tma_store_2d(&a.tmap_y, buf, col0, ti.a_row);
           tma_store_commit();
+          if constexpr (kCache) {  // the slab before this one has been read: its buffer takes the next init values
+            tma_store_wait_read<1>();
+            if (slab_count > 0u) mbar_arrive(&tail->slab_empty[(slab_count - 1u) % kSlabBufs]);
+          }
         }
         ++slab_count;
       }
@@ -475,11 +522,13 @@ cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream) {
   const int cap = listed || g.single ? blocks : a.batch * (a.m / kBM) * ((a.n / kBNH + 1) / 2);
   if (cap <= 0) return cudaSuccess;
   const int grid = cap < max_ctas ? cap : max_ctas;
-  const auto kernel = a.is_bf16 ? gemm_kernel<true> : gemm_kernel<false>;
-  static std::atomic<uint64_t> done[2] = {{0}, {0}};
-  const cudaError_t e = allow_smem(kernel, kSmemBytes, done[a.is_bf16 ? 1 : 0]);
+  const bool cache = a.init_mode == kInitFull;
+  const auto kernel = a.is_bf16 ? (cache ? gemm_kernel<true, true> : gemm_kernel<true, false>)
+                                : (cache ? gemm_kernel<false, true> : gemm_kernel<false, false>);
+  static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
+  const cudaError_t e = allow_smem(kernel, kSmemBytes, done[(a.is_bf16 ? 1 : 0) + (cache ? 2 : 0)]);
   if (e != cudaSuccess) return e;
-  return launch_dependent(kernel, grid, kThreads, kSmemBytes, stream, g.after_list != 0, g);
+  return launch_dependent(kernel, grid, threads_of(cache), kSmemBytes, stream, g.after_list != 0, g);
 }
 
 }  // namespace fo

@@ -134,6 +134,7 @@ struct GemmArgs {
   CUtensorMap tmap_a;              // X as [batch*m, k], box 64 x 128, 128B swizzle
   CUtensorMap tmap_b;              // W as [n, k],       box 64 x 128, 128B swizzle
   CUtensorMap tmap_y;              // Y as [batch*m, n], box 64 x 128, 128B swizzle (TMA stores)
+  CUtensorMap tmap_c;              // kInitFull: init as [batch*m, n]; it and Y with a box of 32 x 128, 64B swizzle
   CUtensorMap tmap_b64;            // W with a box of 64 x 64 (the 192-column tiles of gemm_tall.cu)
   void* y;                         // [batch, m, n]
   const void* init;                // bias [n] or cache [batch, m, n] or null
@@ -253,9 +254,9 @@ cudaError_t launch_attention_streams(const AttnArgs& a, int max_ctas, cudaStream
 cudaError_t launch_attention(const AttnArgs& a, int max_ctas, cudaStream_t stream);
 
 // ------------------------------------------------------------------ host helpers
-// Encodes a tiled tensor map (bf16/f16 elements, 128-byte swizzle or none). dims/strides innermost first;
+// Encodes a tiled tensor map (bf16/f16 elements; swizzle of 128 or 64 bytes, or 0 for none). dims/strides innermost first;
 // strides in bytes for dims 1..rank-1. Returns 0 on success.
 int encode_tmap_16bit(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
-                      const uint64_t* strides_bytes, const uint32_t* box, bool swizzle128 = true);
+                      const uint64_t* strides_bytes, const uint32_t* box, int swizzle = 128);
 
 }  // namespace fo
