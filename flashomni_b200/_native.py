@@ -39,6 +39,7 @@ SIGNATURES = {
     "fo_packbits": (c_int32, [_P, c_int64, c_int32, _P, _P]),
     "fo_segment_packbits": (c_int32, [_P, _P, _P, c_int32, c_int64, c_int32, _P, _P]),
     "fo_segment_packbits_within": (c_int32, [_P, c_int64, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
+    "fo_segment_packbits_early": (c_int32, [_P, c_int64, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
     "fo_segment_packbits_sized": (c_int32, [_P, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
     "fo_mask_compact_scratch_bytes": (c_size_t, [c_int64, c_int32]),
     "fo_mask_compact": (c_int32, [_P, c_int64, _P, c_int64, _P, _P, _P, _P,

@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <chrono>
 #include <string>
 
 #include "../../include/flashomni_b200.h"
@@ -171,19 +172,51 @@ int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32_t indp
                                     total_bytes, stream);
 }
 
-int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
-                               int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
-                               void* stream) {
+namespace {
+constexpr int64_t kNotYet = -2;   // total_bytes before the kernel has written it
+// Waits until the kernel has written *total: polls for it for up to a millisecond, then waits for the stream, as it also does
+// under capture, where nothing runs (and the wait is the error that the caller expects).
+cudaError_t wait_total(const int64_t* total, cudaStream_t st) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &capture);
+  if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return cudaStreamSynchronize(st);
+  const volatile int64_t* t = total;
+  const auto t0 = std::chrono::steady_clock::now();
+  for (uint32_t i = 0;; ++i) {
+    if (*t != kNotYet) return cudaSuccess;
+    if ((i & 255u) == 255u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1)) return cudaStreamSynchronize(st);
+  }
+}
+
+int segment_packbits_impl(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes, bool early,
+                          void* stream) {
   if (n < 0 || num_segments < 0 || capacity < 0) return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: negative size");
   if (num_segments > 1024) return fail(FO_ERR_UNSUPPORTED, "fo_segment_packbits_sized: at most 1024 segments");
   if (x == nullptr || y == nullptr || indptr == nullptr || new_indptr == nullptr || total_bytes == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: null pointer");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (early) *static_cast<volatile int64_t*>(total_bytes) = kNotYet;
   cudaError_t e = launch_segment_packbits_sized(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr,
                                                 reinterpret_cast<long long*>(total_bytes), st);
   count_launches(1);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = early ? wait_total(total_bytes, st) : cudaStreamSynchronize(st);
   return e == cudaSuccess ? FO_OK : fail_cuda("fo_segment_packbits_sized", e);
+}
+}  // namespace
+
+int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                               int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
+                               void* stream) {
+  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, total_bytes, false,
+                               stream);
+}
+
+int fo_segment_packbits_early(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                              int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
+                              void* stream) {
+  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, total_bytes, true,
+                               stream);
 }
 
 // ------------------------------------------------------------------------------------------ compaction

@@ -136,8 +136,9 @@ cudaError_t launch_segment_packbits(const uint8_t* x, const int32_t* indptr, con
 // The same without a byte indptr in hand: every CTA derives it from the element indptr (a few segments: one scan in shared
 // memory) and packs its share; CTA 0 also writes the byte indptr and, to host memory that the device can write, the
 // total (-1: an indptr that decreases or leaves the n values of x, nothing is packed). What bounds the step is the
-// caller's wait for that total; the byte indptr, its last element and the packing used to be ten launches and a copy:
-// two calls for the masks of 2 x 36 q-blocks x 24 heads took 191.5 us on a B200, 66.0 us now.
+// caller's wait for that total, so it is written first, and a caller who only needs it polls for it instead of waiting for the
+// stream (fo_segment_packbits_early): two calls for the masks of 2 x 36 q-blocks x 24 heads 33.9 -> 24.8 us on a B200 (ten
+// launches and a copy in place of this kernel: 191.5 us).
 constexpr int kPackSegs = 1024;
 template <typename Idx>
 __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8_t* __restrict__ x, int64_t n,
@@ -171,7 +172,10 @@ __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8
     if (tid == 0) {
       s_new[0] = 0;
       s_bad = bad ? 1 : 0;
-      if (blockIdx.x == 0) *total_out = bad ? -1ll : static_cast<long long>(carry);
+      if (blockIdx.x == 0) {  // the host may be polling for it
+        *static_cast<volatile long long*>(total_out) = bad ? -1ll : static_cast<long long>(carry);
+        __threadfence_system();
+      }
     }
   }
   __syncthreads();

@@ -174,3 +174,19 @@ def test_masks_forms_and_refusals(cuda_device, monkeypatch):
     for i, c in enumerate(calls):
         a, b = _both(monkeypatch, c)
         assert _same(a, b), f"call {i}: {a} {b}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("work_in_front", [False, True])
+def test_packed_size_is_waited_for_whatever_is_queued(cuda_device, work_in_front):
+    """The size is polled for and, behind some milliseconds of other work, waited for with the stream."""
+    rng = np.random.default_rng(8)
+    x = (rng.random(3000) < 0.5).astype(np.uint8)
+    ip = [0, 13, 1500, 3000]
+    a = torch.randn(8192, 8192, device=cuda_device)
+    for _ in range(3):
+        if work_in_front:
+            a @ a
+        y, new = fo.segment_packbits(torch.from_numpy(x).to(cuda_device), torch.tensor(ip, dtype=torch.int32, device=cuda_device), "little")
+        want = np.concatenate([np.packbits(x[i:j], bitorder="little") for i, j in zip(ip, ip[1:])])
+        assert np.array_equal(y.cpu().numpy(), want) and new.tolist() == [0, 2, 188, 376]
