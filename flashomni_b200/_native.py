@@ -51,6 +51,7 @@ SIGNATURES = {
     "fo_attn_lists": (c_int32, [_P, c_int64, _P, c_int64, _P, _P, c_int32, _P, c_int64, c_int32, c_int64, _P, _P, c_int32,
                                 c_int32, c_int32, c_int32, c_int32, c_int32, c_int64, c_int32, c_int64, c_int64,
                                 _P, _P, _P, _P, _P, _P, c_size_t, c_int32, c_int32, c_int32, c_int64, c_int64, _P, _P, _P, _P]),
+    "fo_attn_run": (c_int32, [_P, _P]),
     "fo_attn_partial_bytes": (c_size_t, [c_int64]),
     "fo_cast_fp8": (c_int32, [_P, c_int64, c_int32, c_int32, _P, _P]),
     "fo_cast_fp8_pair": (c_int32, [_P, _P, c_int64, c_int32, c_int32, _P, _P, _P]),

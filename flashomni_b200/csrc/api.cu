@@ -397,7 +397,7 @@ int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const u
   z.token_bytes = zero_token_bytes;
   z.head_bytes = zero_head_bytes;
   if (attn_lists_small_applies(a, u, z)) {
-    const cudaError_t e = launch_attn_lists_small(a, u, z, st);
+    const cudaError_t e = launch_attn_lists_small(a, u, z, ZeroLater(), CastArgs(), st);
     count_launches(1);
     t_lists_pending = e == cudaSuccess;
     t_lists_stream = st;
@@ -427,7 +427,7 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
                      float* partials, int64_t partial_slots, int32_t head_begin, float sm_scale,
                      float logits_soft_cap, int32_t mask_mode, const uint8_t* custom_mask, int64_t custom_mask_bytes,
                      const int32_t* mask_indptr, const int32_t* qo_indptr, const int32_t* kv_indptr, int32_t* status,
-                     void* stream) {
+                     void* stream, const int2* zero_rec = nullptr, const int32_t* zero_count = nullptr) {
   if (mask_mode == 2 && (custom_mask == nullptr || mask_indptr == nullptr || qo_indptr == nullptr || kv_indptr == nullptr ||
                          custom_mask_bytes <= 0))
     return fail(FO_ERR_INVALID_ARG, "fo_sparse_attn_fwd_custom_mask: mask, its indptr and the request indptrs are required");
@@ -516,6 +516,8 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
     a.sm_scale_log2 = sm_scale * 1.4426950408889634f;
   }
   a.status = status;
+  a.zero_rec = zero_rec;
+  a.zero_count = zero_count;
   a.after_lists = t_lists_pending && t_lists_stream == static_cast<cudaStream_t>(stream);
   t_lists_pending = false;
   int64_t ctas = static_cast<int64_t>(sm_count());  // one persistent CTA per SM
@@ -607,6 +609,87 @@ int fo_cast_fp8(const void* src, int64_t n, int32_t fp8_kind, int32_t dtype, voi
 int fo_cast_fp8_pair(const void* src0, const void* src1, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst0, void* dst1,
                      void* stream) {
   return cast_fp8_impl("fo_cast_fp8_pair", src0, src1, n, fp8_kind, dtype, dst0, dst1, true, stream);
+}
+
+// ------------------------------------------------------------------------------------------ a whole attention call
+int fo_attn_run(const fo_attn_call* c, void* stream) {
+  if (c == nullptr || c->plan == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_attn_run: null call or plan");
+  const int64_t* p = c->plan;
+  auto i32 = [&](int i) { return static_cast<int32_t>(p[i]); };
+  auto ptr = [&](int i) { return reinterpret_cast<int32_t*>(p[i]); };
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool cast = c->fp8_kind >= 0 && c->kv_values > 0;
+  ZeroLater later = ZeroLater();
+  bool cast_done = false;
+  if (!c->lists_ready) {
+    CompactArgs a;
+    int rc = make_compact_args(a, c->sparse_info, c->sparse_info_bytes, c->sparse_kv_info, c->sparse_kv_info_bytes,
+                               c->sparse_info_indptr, c->sparse_kv_info_indptr, ptr(0), ptr(1), i32(2), i32(3), i32(4), i32(5),
+                               i32(6), i32(7), c->is_full, p[8], i32(9), p[10], p[11], ptr(12), ptr(13), ptr(14), ptr(15),
+                               ptr(16), reinterpret_cast<void*>(p[17]), static_cast<size_t>(p[18]));
+    if (rc != FO_OK) return rc;
+    UnitArgs u;
+    rc = make_unit_args(u, ptr(12), ptr(13), ptr(14), ptr(15), ptr(16), ptr(0), ptr(1), p[10], i32(9), i32(6), i32(7), i32(19),
+                        i32(20), i32(21), p[22], p[23], ptr(24), ptr(25), ptr(26));
+    if (rc != FO_OK) return rc;
+    ZeroArgs z = ZeroArgs();
+    z.out = c->zero_inactive ? static_cast<uint8_t*>(c->o) : nullptr;
+    const bool small = attn_lists_small_applies(a, u, z);
+    if (small) {
+      // One launch builds the lists and casts fp8 K and V beside that. The attention kernel with streams zeroes the inactive
+      // q-blocks itself, from a list in the scratch that this path does not use otherwise.
+      AttnArgs probe;
+      memset(&probe, 0, sizeof(probe));
+      probe.head_dim = c->head_dim;
+      probe.partial_slots = static_cast<int>(p[23] > 0x7fffffffLL ? 0x7fffffffLL : p[23]);
+      if (z.out != nullptr && (!aligned16(c->o) || c->o_stride_n % 8 != 0 || c->o_stride_n <= 0))
+        return fail(FO_ERR_INVALID_ARG, "fo_attn_run: an output to zero must be aligned to 16 bytes");
+      if (z.out != nullptr && !c->is_full && attention_streams_applies(probe) && c->total_q > 0 && c->total_kv > 0) {
+        later.rec = reinterpret_cast<int2*>(a.kv_off);
+        later.count = a.hist;
+        z.out = nullptr;
+      } else if (z.out != nullptr) {
+        z.token_bytes = c->o_stride_n * 2;
+        z.head_bytes = c->num_qo_heads / c->num_kv_heads * c->head_dim * 2;
+      }
+      CastArgs ca = CastArgs();
+      if (cast) {
+        if (c->k == nullptr || c->v == nullptr || c->k16 == nullptr || c->v16 == nullptr || !aligned16(c->k) || !aligned16(c->v) ||
+            !aligned16(c->k16) || !aligned16(c->v16) || c->fp8_kind > 1)
+          return fail(FO_ERR_INVALID_ARG, "fo_attn_run: fp8 k / v and their copies must be aligned to 16 bytes");
+        ca.src[0] = static_cast<const uint8_t*>(c->k);
+        ca.src[1] = static_cast<const uint8_t*>(c->v);
+        ca.dst[0] = static_cast<uint16_t*>(c->k16);
+        ca.dst[1] = static_cast<uint16_t*>(c->v16);
+        ca.n = c->kv_values;
+        ca.e5m2 = c->fp8_kind;
+        ca.is_bf16 = c->dtype == FO_DTYPE_BF16;
+        cast_done = true;
+      }
+      const cudaError_t e = launch_attn_lists_small(a, u, z, later, ca, st);
+      count_launches(1);
+      if (e != cudaSuccess) return fail_cuda("fo_attn_run (work lists)", e);
+    } else {
+      cudaError_t e = cudaSuccess;
+      if (z.out != nullptr && !c->is_full) e = cudaMemsetAsync(c->o, 0, static_cast<size_t>(c->total_q * c->o_stride_n) * 2, st);
+      if (e == cudaSuccess) e = launch_attn_compact(a, st);
+      if (e == cudaSuccess) e = launch_attn_units(u, st);
+      count_launches(a.n_cand > 0 ? 4 : 1);
+      if (e != cudaSuccess) return fail_cuda("fo_attn_run (work lists)", e);
+    }
+    t_lists_pending = small;   // the attention launch below may set itself up while the lists are built
+    t_lists_stream = st;
+  }
+  if (cast && !cast_done) {
+    t_lists_pending = false;
+    const int rc = cast_fp8_impl("fo_attn_run", c->k, c->v, c->kv_values, c->fp8_kind, c->dtype, c->k16, c->v16, true, stream);
+    if (rc != FO_OK) return rc;
+  }
+  return sparse_attn_impl(c->q, cast ? c->k16 : c->k, cast ? c->v16 : c->v, c->o, c->lse, c->dtype, c->total_q, c->total_kv,
+                          c->num_qo_heads, c->num_kv_heads, c->head_dim, c->q_stride_n, c->q_stride_h, c->k_stride_n, c->k_stride_h,
+                          c->v_stride_n, c->v_stride_h, c->o_stride_n, c->o_stride_h, i32(7), i32(7), ptr(14), ptr(24), ptr(25), p[22],
+                          ptr(26), c->partials, p[23], i32(4), c->sm_scale, c->logits_soft_cap, 0, nullptr, 0, nullptr, nullptr,
+                          nullptr, c->status, stream, later.rec, later.count);
 }
 
 // ------------------------------------------------------------------------------------------ GEMMs

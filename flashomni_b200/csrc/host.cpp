@@ -25,10 +25,7 @@
 namespace {
 
 struct Api {
-  decltype(&fo_attn_lists) attn_lists;
-  decltype(&fo_sparse_attn_fwd) attn;
-  decltype(&fo_sparse_attn_fwd_softcap) attn_softcap;
-  decltype(&fo_cast_fp8_pair) cast_fp8_pair;
+  decltype(&fo_attn_run) attn_run;
   decltype(&fo_gemm_q) gemm_q;
   decltype(&fo_gemm_o) gemm_o;
   decltype(&fo_gemm_q_prepared) gemm_q_prepared;
@@ -89,7 +86,7 @@ bool wait_event(void* stream, PyObject* event) {
 // ------------------------------------------------------------------------------------------------ attention
 struct AttnPlan {
   int64_t dev, is_bf16, fp8_kind /* -1: k and v have the type of q */, total_q, hq, hkv, d, total_kv, batch, nhd, fresh_out,
-      qo_indptr, kv_indptr, list[25], status, partials;
+      lists[27] /* the plan array of fo_layer_lists */, status, partials;
 };
 constexpr int kPlanWords = sizeof(AttnPlan) / sizeof(int64_t);
 
@@ -168,49 +165,58 @@ PyObject* attn_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (p->fp8_kind >= 0 && (k->numel() % 8 != 0 || k->numel() == 0 || !k->is_contiguous() || !v->is_contiguous())) NOT_HERE;
 
   void* stream = current_stream(dev);
-  int rc = FO_OK;
-  at::Tensor kv16, out, lse;
-  const void *kd = k->data_ptr(), *vd = v->data_ptr();
-  const int64_t kn = k->stride(tok), kh = k->stride(hd), vn = v->stride(tok), vh = v->stride(hd);   // (the copies are laid out alike)
-  if (p->fp8_kind >= 0) {  // cast both in one launch, into one allocation
+  at::Tensor kv16, lse;
+  fo_attn_call c;
+  memset(&c, 0, sizeof(c));
+  c.fp8_kind = i32(p->fp8_kind);
+  if (p->fp8_kind >= 0) {  // both copies in one allocation
     kv16 = at::empty({2, k->size(0), k->size(1), k->size(2)}, q->options());
-    char* dst = static_cast<char*>(kv16.data_ptr());
-    rc = g_api.cast_fp8_pair(kd, vd, k->numel(), i32(p->fp8_kind), dtype_code(*q), dst, dst + 2 * k->numel(), stream);
-    if (rc != FO_OK) return PyLong_FromLong(rc);
-    kd = dst;
-    vd = dst + 2 * k->numel();
+    c.kv_values = k->numel();
+    c.k16 = kv16.data_ptr();
+    c.v16 = static_cast<char*>(c.k16) + 2 * k->numel();
   }
   if (return_lse) lse = lse_in != nullptr ? *lse_in : at::empty({q->size(0), q->size(1)}, q->options().dtype(at::kFloat));
-  out = fresh ? at::empty(q->sizes(), q->options()) : *out_in;
-  const int64_t* L = p->list;
-  {
-    pybind11::gil_scoped_release no_gil;
-    if (!prepared) {
-      // an output allocated here reads as zero in q-blocks that are not computed: the list builder zeroes them
-      void* zero = fresh ? out.data_ptr() : nullptr;
-      rc = g_api.attn_lists(
-          si != nullptr ? si->data_ptr<uint8_t>() : nullptr, si != nullptr ? si->numel() : 0,
-          skv != nullptr ? skv->data_ptr<uint8_t>() : nullptr, skv != nullptr ? skv->numel() : 0,
-          ip != nullptr ? ip->data_ptr<int32_t>() : nullptr, kp != nullptr ? kp->data_ptr<int32_t>() : nullptr, full, zero,
-          fresh ? out.stride(0) * 2 : 0, fresh ? i32(p->hq / p->hkv * p->d * 2) : 0, fresh ? out.numel() * 2 : 0,
-          ptr<const int32_t>(p->qo_indptr), ptr<const int32_t>(p->kv_indptr), i32(L[0]), i32(L[1]), i32(L[2]), i32(L[3]), i32(L[4]),
-          i32(L[5]), L[6], i32(L[7]), L[8], L[9], ptr<int32_t>(L[10]), ptr<int32_t>(L[11]), ptr<int32_t>(L[12]), ptr<int32_t>(L[13]),
-          ptr<int32_t>(L[14]), ptr<void>(L[15]), static_cast<size_t>(L[16]), i32(L[17]), i32(L[18]), i32(L[19]), L[20], L[21],
-          ptr<int32_t>(L[22]), ptr<int32_t>(L[23]), ptr<int32_t>(L[24]), stream);
-    }
+  const at::Tensor out = fresh ? at::empty(q->sizes(), q->options()) : *out_in;
+  c.plan = p->lists;
+  if (!full) {
+    c.sparse_info = si->data_ptr<uint8_t>();
+    c.sparse_info_bytes = si->numel();
+    c.sparse_kv_info = skv->data_ptr<uint8_t>();
+    c.sparse_kv_info_bytes = skv->numel();
+    c.sparse_info_indptr = ip->data_ptr<int32_t>();
+    c.sparse_kv_info_indptr = kp->data_ptr<int32_t>();
   }
-  if (rc != FO_OK) return PyLong_FromLong(rc);
+  c.is_full = full;
+  c.lists_ready = prepared ? 1 : 0;
+  c.zero_inactive = fresh ? 1 : 0;   // an output allocated here reads as zero in q-blocks that are not computed
+  c.dtype = dtype_code(*q);
+  c.q = q->data_ptr();
+  c.k = k->data_ptr();
+  c.v = v->data_ptr();
+  c.o = out.data_ptr();
+  c.lse = return_lse ? lse.data_ptr<float>() : nullptr;
+  c.total_q = p->total_q;
+  c.total_kv = p->total_kv;
+  c.num_qo_heads = i32(p->hq);
+  c.num_kv_heads = i32(p->hkv);
+  c.head_dim = i32(p->d);
+  c.q_stride_n = q->stride(0);
+  c.q_stride_h = q->stride(1);
+  c.k_stride_n = k->stride(tok);   // (fp8: contiguous, and the copies are laid out alike)
+  c.k_stride_h = k->stride(hd);
+  c.v_stride_n = v->stride(tok);
+  c.v_stride_h = v->stride(hd);
+  c.o_stride_n = out.stride(0);
+  c.o_stride_h = out.stride(1);
+  c.partials = ptr<float>(p->partials);
+  c.sm_scale = static_cast<float>(scale);
+  c.logits_soft_cap = static_cast<float>(cap);
+  c.status = ptr<int32_t>(p->status);
   if (prepared && !wait_event(stream, args[14])) return PyErr_Format(PyExc_RuntimeError, "waiting for the prepared work lists failed");
+  int rc;
   {
     pybind11::gil_scoped_release no_gil;
-    auto call = [&](auto fn, auto... tail) {
-      return fn(q->data_ptr(), kd, vd, out.data_ptr(), return_lse ? lse.data_ptr<float>() : nullptr, dtype_code(*q), p->total_q,
-                p->total_kv, i32(p->hq), i32(p->hkv), i32(p->d), q->stride(0), q->stride(1), kn, kh, vn, vh, out.stride(0),
-                out.stride(1), 128, 128,
-                ptr<const int32_t>(L[12]), ptr<const int32_t>(L[22]), ptr<const int32_t>(L[23]), L[20], ptr<int32_t>(L[24]),
-                ptr<float>(p->partials), L[21], i32(L[2]), static_cast<float>(scale), tail..., ptr<int32_t>(p->status), stream);
-    };
-    rc = cap > 0.0 ? call(g_api.attn_softcap, static_cast<float>(cap)) : call(g_api.attn);
+    rc = g_api.attn_run(&c, stream);
   }
   if (rc != FO_OK) return PyLong_FromLong(rc);
   PyObject* o = fresh ? THPVariable_Wrap(out) : (Py_INCREF(args[9]), args[9]);
@@ -474,10 +480,7 @@ PyObject* bind(PyObject*, PyObject* arg) {
     fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(h, name));
     if (fn == nullptr) missing = name;
   };
-  get(a.attn_lists, "fo_attn_lists");
-  get(a.attn, "fo_sparse_attn_fwd");
-  get(a.attn_softcap, "fo_sparse_attn_fwd_softcap");
-  get(a.cast_fp8_pair, "fo_cast_fp8_pair");
+  get(a.attn_run, "fo_attn_run");
   get(a.gemm_q, "fo_gemm_q");
   get(a.gemm_o, "fo_gemm_o");
   get(a.gemm_q_prepared, "fo_gemm_q_prepared");

@@ -109,6 +109,16 @@ struct UnitArgs {
   int32_t* arrive;           // [max_slots]
 };
 cudaError_t launch_attn_units(const UnitArgs& a, cudaStream_t stream);
+struct ZeroLater {           // output rows of inactive q-blocks that the list builder only lists, for the attention kernel (rec null: none)
+  int2* rec;                 // [n_cand] (first row in the output, valid rows << 16 | head inside the tensors)
+  int32_t* count;
+};
+struct CastArgs {            // fp8 K and V to cast in the same launch (src null: none)
+  const uint8_t* src[2];
+  uint16_t* dst[2];
+  int64_t n;                 // values of each
+  int e5m2, is_bf16;
+};
 struct ZeroArgs {            // output rows of inactive q-blocks that the list builder zeroes (out null: none)
   uint8_t* out;              // first byte of token 0, first head of the mask window
   int64_t token_bytes;       // bytes between tokens
@@ -116,7 +126,8 @@ struct ZeroArgs {            // output rows of inactive q-blocks that the list b
 };
 bool attn_lists_small_fits(const CompactArgs& a, const UnitArgs& u);
 bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z);
-cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream);
+cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, const ZeroLater& later,
+                                    const CastArgs& cast, cudaStream_t stream);
 // src1 / dst1: a second tensor of the same size, or null
 cudaError_t launch_cast_fp8(const void* src0, const void* src1, int64_t n, int e5m2, int is_bf16, void* dst0, void* dst1,
                             int sm_count, cudaStream_t stream);
@@ -240,6 +251,8 @@ struct AttnArgs {
   int is_bf16;
   float sm_scale_log2;             // sm_scale * log2(e); with a soft cap: cap * log2(e)
   int after_lists;                 // the launch in front of this one builds the lists (dependent launch)
+  const int2* zero_rec;            // q-blocks to zero (ZeroLater), or null; streams kernel only
+  const int32_t* zero_count;
   float soft_cap_pre;              // 0: no soft cap; else sm_scale / cap (logits = cap * tanh(q.k * sm_scale / cap))
   int32_t* status;
 };

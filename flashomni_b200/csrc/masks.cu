@@ -9,6 +9,7 @@
 // All kernels here are integer / byte work bound by HBM and launch latency; they never touch
 // memory outside the extents given (reads are clamped to the packed buffers' byte sizes) and
 // report malformed input through a status word instead of faulting.
+#include "cast_fp8.cuh"
 #include "internal.h"
 
 namespace fo {
@@ -975,8 +976,8 @@ cudaError_t launch_attn_units(const UnitArgs& a, cudaStream_t stream) {
 constexpr int kSmallThreads = 512, kSmallBatch = 64;
 constexpr int64_t kSmallCand = 4096, kSmallBits = 1 << 18;
 
-__device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, int by_length,
-                                                      int heads_per_group, int cta) {
+__device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z,
+                                                      const ZeroLater& later, int by_length, int heads_per_group, int cta) {
   extern __shared__ __align__(16) uint32_t s_dyn[];   // [n_cand] keys, then [n_cand] counts
   __shared__ int s_first[kSmallBatch + 1];            // first candidate of a request
   __shared__ int s_q0[kSmallBatch], s_ql[kSmallBatch], s_k0[kSmallBatch], s_kl[kSmallBatch];
@@ -1074,6 +1075,7 @@ __device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, cons
     u.unit_counters[1] = 0;
     u.unit_counters[2] = 0x7fffffff;
     u.unit_counters[3] = (status != kDevOk || tot_items > u.max_units) ? kDevBadIndex : kDevOk;
+    if (later.rec != nullptr) *later.count = status != kDevOk || tot_items > u.max_units ? n_real : n_real - tot_items;
   }
   if (c >= n_real) return;
   const int b = request_of(c);
@@ -1081,7 +1083,10 @@ __device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, cons
   int q_valid = s_ql[b] - qb * a.sbq;
   q_valid = q_valid > a.sbq ? a.sbq : q_valid;
   // a q-block that nobody computes: not active, or in lists that do not fit (the attention ignores all of those)
-  if (z.out != nullptr && (kept < 0 || status != kDevOk || tot_items > u.max_units)) {
+  const bool fits = status == kDevOk && tot_items <= u.max_units;
+  if (later.rec != nullptr && (kept < 0 || !fits) && lane == 0)
+    later.rec[fits ? c - pos : c] = make_int2(s_q0[b] + qb * a.sbq, (q_valid << 16) | hl);
+  if (z.out != nullptr && (kept < 0 || !fits)) {
     const int vecs = z.head_bytes >> 4;   // 16-byte words of one token's share of this mask head
     uint8_t* dst = z.out + static_cast<int64_t>(s_q0[b] + qb * a.sbq) * z.token_bytes + static_cast<int64_t>(hl) * z.head_bytes;
     for (int i = lane; i < q_valid * vecs; i += 32) {
@@ -1139,10 +1144,19 @@ __device__ __forceinline__ void attn_lists_small_body(const CompactArgs& a, cons
   }
 }
 
-__global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(CompactArgs a, UnitArgs u, ZeroArgs z, int by_length,
-                                                                         int heads_per_group) {
+// kCast: the CTAs past the list builders cast fp8 K and V (0: there are none; else 1 + e5m2 + 2 * bf16). The lists are pure
+// latency and the cast pure bandwidth; one behind the other they took 17 us in front of the attention of 3959 tokens with 8
+// kv heads on a B200, together 9.8.
+template <int kCast>
+__global__ void __launch_bounds__(kSmallThreads) attn_lists_small_kernel(CompactArgs a, UnitArgs u, ZeroArgs z, ZeroLater later, CastArgs cast,
+                                                                         int list_ctas, int by_length, int heads_per_group) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention kernel may set itself up meanwhile
-  attn_lists_small_body(a, u, z, by_length, heads_per_group, static_cast<int>(blockIdx.x));
+  if (kCast != 0 && static_cast<int>(blockIdx.x) >= list_ctas) {
+    const int i = static_cast<int>(blockIdx.x) - list_ctas, ctas = (static_cast<int>(gridDim.x) - list_ctas) / 2, t = i < ctas ? 0 : 1;
+    cast_fp8_body<((kCast - 1) & 1) != 0, ((kCast - 1) & 2) != 0>(cast.src[t], cast.n, cast.dst[t], i - t * ctas, ctas);
+    return;
+  }
+  attn_lists_small_body(a, u, z, later, by_length, heads_per_group, static_cast<int>(blockIdx.x));
 }
 
 // What the kernel can take: keys have 12 bits for the candidate, and every CTA reads the whole mask (kSmallBits = 32 KB).
@@ -1162,12 +1176,26 @@ bool attn_lists_small_applies(const CompactArgs& a, const UnitArgs& u, const Zer
   return attn_lists_small_fits(a, u) && (a.n_cand <= 2560 || a.batch >= 16 || a.is_full || z.out != nullptr);
 }
 
-cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, cudaStream_t stream) {
+cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, const ZeroArgs& z, const ZeroLater& later,
+                                    const CastArgs& cast, cudaStream_t stream) {
   int by_length, hpg;
   order_rule(a, &by_length, &hpg);
   const int wpb = kSmallThreads / 32;
   const int blocks = static_cast<int>((a.n_cand + wpb - 1) / wpb);
-  attn_lists_small_kernel<<<blocks, kSmallThreads, static_cast<size_t>(a.n_cand) * 8, stream>>>(a, u, z, by_length, hpg);
+  const size_t smem = static_cast<size_t>(a.n_cand) * 8;
+  if (cast.src[0] == nullptr) {
+    attn_lists_small_kernel<0><<<blocks, kSmallThreads, smem, stream>>>(a, u, z, later, cast, blocks, by_length, hpg);
+  } else {
+    int64_t per = (cast.n / 16 + kSmallThreads - 1) / kSmallThreads;   // cast CTAs for each of K and V
+    per = per > 148 * 2 ? 148 * 2 : (per < 1 ? 1 : per);
+    const int grid = blocks + 2 * static_cast<int>(per);
+    switch (1 + (cast.e5m2 ? 1 : 0) + (cast.is_bf16 ? 2 : 0)) {
+      case 1: attn_lists_small_kernel<1><<<grid, kSmallThreads, smem, stream>>>(a, u, z, later, cast, blocks, by_length, hpg); break;
+      case 2: attn_lists_small_kernel<2><<<grid, kSmallThreads, smem, stream>>>(a, u, z, later, cast, blocks, by_length, hpg); break;
+      case 3: attn_lists_small_kernel<3><<<grid, kSmallThreads, smem, stream>>>(a, u, z, later, cast, blocks, by_length, hpg); break;
+      default: attn_lists_small_kernel<4><<<grid, kSmallThreads, smem, stream>>>(a, u, z, later, cast, blocks, by_length, hpg); break;
+    }
+  }
   return cudaGetLastError();
 }
 
@@ -1469,7 +1497,10 @@ __global__ void __launch_bounds__(kSmallThreads) layer_lists_kernel(CompactArgs 
     z.out = nullptr;
     z.token_bytes = 0;
     z.head_bytes = 16;
-    attn_lists_small_body(a, u, z, by_length, heads_per_group, static_cast<int>(blockIdx.x) - 2);
+    ZeroLater later;
+    later.rec = nullptr;
+    later.count = nullptr;
+    attn_lists_small_body(a, u, z, later, by_length, heads_per_group, static_cast<int>(blockIdx.x) - 2);
   }
 }
 

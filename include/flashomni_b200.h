@@ -249,6 +249,36 @@ FO_API int fo_cast_fp8(const void* src, int64_t n, int32_t fp8_kind, int32_t dty
 FO_API int fo_cast_fp8_pair(const void* src0, const void* src1, int64_t n, int32_t fp8_kind, int32_t dtype, void* dst0,
                             void* dst1, void* stream);
 
+/* ---- a whole attention call ---------------------------------------------------------------------
+ * fo_attn_lists (unless lists_ready), fo_cast_fp8_pair (fp8_kind >= 0: k and v hold kv_values 8-bit values each and are cast to
+ * k16 and v16, whose strides are k_stride_* and v_stride_*) and fo_sparse_attn_fwd (with logits_soft_cap > 0: _softcap) in
+ * one call, with the lists and the cast in one launch for small masks. zero_inactive: rows of q-blocks that are not computed
+ * are zeroed in o, which is then contiguous. `plan` is the array of fo_layer_lists. */
+typedef struct fo_attn_call {
+  const int64_t* plan;
+  const uint8_t* sparse_info;
+  const uint8_t* sparse_kv_info;
+  int64_t sparse_info_bytes, sparse_kv_info_bytes;
+  const int32_t* sparse_info_indptr;
+  const int32_t* sparse_kv_info_indptr;
+  int32_t is_full, lists_ready, zero_inactive, dtype;
+  const void* q;
+  const void* k;
+  const void* v;
+  void* o;
+  float* lse;
+  int64_t total_q, total_kv;
+  int32_t num_qo_heads, num_kv_heads, head_dim, fp8_kind;
+  int64_t q_stride_n, q_stride_h, k_stride_n, k_stride_h, v_stride_n, v_stride_h, o_stride_n, o_stride_h;
+  void* k16;
+  void* v16;
+  int64_t kv_values;
+  float* partials;
+  float sm_scale, logits_soft_cap;
+  int32_t* status;
+} fo_attn_call;
+FO_API int fo_attn_run(const fo_attn_call* call, void* stream);
+
 /* ---- GEMM-Q / GEMM-O ---------------------------------------------------------------------------
  * Workspace (device, caller-owned, 16-byte aligned) of fo_gemm_workspace_bytes(...) bytes, laid out
  * as int32 words: [0..3] counters (count, aux, list status, two-block records), [4] kernel status (FO_DEV_*,
