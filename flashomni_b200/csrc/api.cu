@@ -911,6 +911,7 @@ int gemm_q_impl(const void* x, const void* w, void* y, const void* bias, int32_t
     e = prepared ? cudaSuccess : launch_gemm_q_tiles(la, st);
     if (e != cudaSuccess) return fail_cuda("fo_gemm_q (work list)", e);
     g.after_list = prepared ? 0 : 1;
+    g.list = la;
     count_launches(prepared ? 0 : 1);
     g.tiles = la.tiles;
     g.n_tiles_ptr = la.counters;
@@ -993,6 +994,7 @@ int gemm_o_impl(const void* x, const void* w, void* y, const void* init, int32_t
   cudaError_t e = prepared ? cudaSuccess : launch_gemm_o_rows(la, st);
   if (e != cudaSuccess) return fail_cuda("fo_gemm_o (work list)", e);
   g.after_list = prepared ? 0 : 1;
+  g.list = la;
   count_launches(prepared ? 1 : 2);
   g.y = y;
   g.init = init;

@@ -24,6 +24,7 @@
 #include <cuda_fp16.h>
 
 #include "internal.h"
+#include "mask_bits.cuh"
 
 namespace fo {
 namespace {
@@ -47,17 +48,18 @@ constexpr int slabs_of(bool cache) { return cache ? 4 : 2; }
 constexpr int kTmemCols = 512;
 constexpr int kMaxHeadsSmem = 128;
 constexpr int kTileQ = 8;   // entries of the tile queue (the producer runs at most a few tiles ahead of the epilogue)
+constexpr int kFirstRows = 192;   // own_first: row blocks, one per thread of the smaller CTA
 
-struct Tail {
+struct alignas(16) Tail {
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t slab_full[kMaxSlabBufs];    // init values of a slab have landed
   uint64_t slab_empty[kMaxSlabBufs];   // the store of the slab has read it
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
-  uint64_t tq_full[kTileQ];   // tile queue: the producer warp draws tile numbers and hands them to the other roles
+  uint64_t tq_full[kTileQ];   // tile queue: the producer warp draws tiles, looks them up and hands them to the other roles
   uint64_t tq_empty[kTileQ];
-  int tile_q[kTileQ];
+  int4 tile_q[kTileQ];        // (a_row, w_row0, w_row1, nkb); a_row -1 ends the sequence
   uint32_t tmem_base;
   int abort_flag;
   int epi_go;                   // outcome of the epilogue warps' vote of the current round
@@ -117,6 +119,136 @@ __device__ __forceinline__ TileInfo get_tile(const GemmArgs& a, int t) {
   return ti;
 }
 
+// What the list kernel in front of this one writes for tile blockIdx.x, worked out from the mask by the whole CTA: one row block
+// per thread, at most kFirstRows of them and 64 column blocks (GEMM-Q, heads of 128) or heads (GEMM-O). With the list the first
+// operands of a 4608 x 24 heads GEMM-Q arrive 9.6 us after its launch, with the mask after 4.4; what is left of that in the
+// whole call is less, since the operands of the first round come from HBM in either case. GEMM-Q / GEMM-O with list kernel,
+// inputs that change from call to call, us on a B200: 512 rows x 6 heads 12.5 / 13.6 -> 12.0 / 12.5, 1024 x 8 14.3 / 15.4 -> 13.6 /
+// 14.3, 1280 x 24 32.8 / 31.0 -> 30.7 / 28.9, 2560 x 12 21.5 / 22.3 -> 20.0 / 20.2, 4608 x 24 51.6 / 52.2 -> 50.2 / 51.0, 9216 x 24
+// 84.2 / 84.7 -> 83.2 / 84.0. More row blocks than that take 150 us and more, of which the list is a few percent.
+struct FirstScratch {   // in the staging slabs, which nothing uses yet
+  int sums[8];
+  int hist[65];
+  int best;
+  int2 tile;            // GEMM-Q: (row block, column blocks ix0 | ix1 << 8, ix1 255 for a single one); GEMM-O: (row block, -)
+  unsigned long long bits;
+};
+__device__ __forceinline__ TileInfo first_tile(const GemmArgs& a, FirstScratch& s, int* heads) {
+  const GemmListArgs& l = a.list;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, warp = tid >> 5, warps = static_cast<int>(blockDim.x) >> 5;
+  const int mt = a.m / kBM, rows = a.batch * mt, t = static_cast<int>(blockIdx.x);
+  const bool q = a.mode == kGemmQ;
+  const int nbits = q ? a.n / kBNH : l.k / l.head_dim;
+  TileInfo ti;
+  ti.a_row = -1; ti.w_row0 = ti.nkb = 0; ti.w_row1 = -1; ti.heads = nullptr;
+
+  for (int i = tid; i <= 64; i += static_cast<int>(blockDim.x)) s.hist[i] = 0;
+  if (tid == 0) { s.best = 0x7fffffff; s.tile = make_int2(-1, 0); }
+  uint64_t bits = 0;
+  if (tid < rows) {
+    const int b = tid / mt, iy = tid % mt;
+    const int64_t ioff = l.info_indptr[b];
+    const uint32_t qb = (static_cast<uint32_t>(l.num_text_tokens) + static_cast<uint32_t>(iy) * 128u) / static_cast<uint32_t>(l.sparse_q_size);
+    bits = load_bits64(l.sparse_info + ioff, static_cast<int64_t>(qb) * l.num_heads + l.head_begin, l.info_bytes - ioff, nbits);
+    if (!q && l.is_for_cache) bits = ~bits & (nbits < 64 ? (1ull << nbits) - 1ull : ~0ull);
+  }
+  const int cnt = __popcll(bits);
+  if (q) {
+    const int npair = cnt >> 1, nsingle = cnt & 1;
+    int x = npair << 16 | nsingle;   // inclusive scans of both kinds of record in one word: at most 192 * 32 and 192
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s.sums[warp] = x;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < warps; ++w) {
+      if (w == warp) before = total;
+      total += s.sums[w];
+    }
+    x += before;
+    const int P = total >> 16, S = total & 0xffff, n = l.n_ctas > 0 ? l.n_ctas : 1;
+    for (int k = tid; k <= P && k <= n && k < 1024 && P + S + k <= l.max_tiles; k += static_cast<int>(blockDim.x)) {
+      const int e = gemm_q_makespan(P - k, S + 2 * k, n);
+      atomicMin(&s.best, ((e < 32767 ? e : 32767) << 16) | k);
+    }
+    __syncthreads();
+    const int n_split = s.best == 0x7fffffff ? 0 : s.best & 0xffff, kept = P - n_split;
+    const int p0 = (x >> 16) - npair, s0 = (x & 0xffff) - nsingle;   // numbers of this row's first records
+    const int cut = t - kept, single = t - P - n_split;
+    int skip = -1, take = 0;   // active column blocks of this row in front of the tile, and its own
+    if (t < kept) {
+      if (t >= p0 && t < p0 + npair) { skip = 2 * (t - p0); take = 2; }
+    } else if (cut < 2 * n_split) {
+      const int p = kept + (cut >> 1);
+      if (p >= p0 && p < p0 + npair) { skip = 2 * (p - p0) + (cut & 1); take = 1; }
+    } else if (nsingle && single == s0) {
+      skip = cnt - 1; take = 1;
+    }
+    if (take) {
+      uint64_t rest = bits;
+      for (int i = 0; i < skip; ++i) rest &= rest - 1;
+      const int ix0 = __ffsll(static_cast<long long>(rest)) - 1;
+      rest &= rest - 1;
+      s.tile = make_int2(tid, ix0 | (take == 2 ? __ffsll(static_cast<long long>(rest)) - 1 : 255) << 8);
+    }
+    __syncthreads();
+    const int2 rec = s.tile;
+    if (rec.x < 0) return ti;
+    ti.a_row = rec.x * kBM;
+    ti.w_row0 = (rec.y & 255) * kBNH;
+    ti.w_row1 = (rec.y >> 8) == 255 ? -1 : (rec.y >> 8) * kBNH;
+    ti.nkb = (a.k + kBK - 1) / kBK;
+    return ti;
+  }
+  // GEMM-O: the row block that comes (t / tiles of a row)-th when they are sorted by falling head count, stable
+  __syncthreads();
+  if (tid < rows) atomicAdd(&s.hist[cnt], 1);
+  __syncthreads();
+  const int npr = tiles_per_row(a), want = t / npr, j = t % npr;
+  // counts from 64 down, two a lane: the bucket that holds the row and how many rows of that count come before it
+  const int h1 = s.hist[64 - 2 * lane], h2 = s.hist[63 - 2 * lane];
+  int x = h1 + h2;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const unsigned past = __ballot_sync(0xffffffffu, x > want);
+  int bucket = 0, nth = want - __shfl_sync(0xffffffffu, x, 31);   // no lane: the rows without a head
+  if (past != 0u) {
+    const int src = __ffs(past) - 1;
+    const int start = __shfl_sync(0xffffffffu, x - h1 - h2, src), first = __shfl_sync(0xffffffffu, h1, src);
+    const bool lower = want >= start + first;
+    bucket = 64 - 2 * src - (lower ? 1 : 0);
+    nth = want - start - (lower ? first : 0);
+  }
+  const unsigned mine = __ballot_sync(0xffffffffu, tid < rows && cnt == bucket);
+  if (lane == 0) s.sums[warp] = __popc(mine);
+  __syncthreads();
+  int before = __popc(mine & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) before += s.sums[w];
+  if (tid < rows && cnt == bucket && before == nth) {
+    s.tile = make_int2(tid, 0);
+    s.bits = bits;
+  }
+  __syncthreads();
+  const int row = s.tile.x;
+  if (row < 0) return ti;
+  const uint64_t hb = s.bits;
+  if (tid < 64 && (hb >> tid & 1ull)) heads[__popcll(hb & ((1ull << tid) - 1ull))] = tid;
+  fence_proxy_async_smem();   // the first init slabs land on the scratch
+  __syncthreads();
+  ti.a_row = row * kBM;
+  ti.w_row0 = (a.single ? j : 2 * j) * kBNH;
+  ti.w_row1 = (!a.single && 2 * j + 1 < a.n / kBNH) ? (2 * j + 1) * kBNH : -1;
+  ti.nkb = __popcll(hb) * a.kb_per_head;
+  ti.heads = heads;
+  return ti;
+}
+
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 template <bool kBf16, bool kCache>
@@ -167,19 +299,24 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
-  if (a.after_list) asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the list in front of it was built
+  // launched while the list in front of it was built: waits for it now, or before the second tile (every CTA, also one without)
+  if (a.after_list && !a.own_first) asm volatile("griddepcontrol.wait;" ::: "memory");
+  TileInfo first;
+  if (a.own_first) first = first_tile(a, *reinterpret_cast<FirstScratch*>(smem_slab), tail->heads[0]);
 
-  const int n_tiles = num_tiles(a);
   // Tiles are handed out in list order through a device-wide cursor (the GEMM-O rows are sorted
   // longest first, the GEMM-Q list ends with its half-size tiles), so that a CTA that finishes early
   // takes the next tile instead of idling at the end of a fixed share. Tile i < gridDim.x goes to CTA i; the cursor counts the tiles after those.
-  // Entry k of a CTA's sequence travels through slot k % kTileQ; -1 ends the sequence.
-  auto read_slot = [&](int k) -> int {  // one thread of a consumer role; -2 when the wait gave up
+  // Entry k of a CTA's sequence travels through slot k % kTileQ.
+  auto read_slot = [&](int k) -> TileInfo {  // one thread of a consumer role; a_row -1 ends the sequence, -2 when the wait gave up
     const int slot = k % kTileQ;
-    if (!mbar_wait(&tail->tq_full[slot], static_cast<uint32_t>(k / kTileQ) & 1u, abort_flag)) return -2;
-    const int t = tail->tile_q[slot];
+    TileInfo ti;
+    ti.a_row = -2; ti.w_row0 = ti.nkb = 0; ti.w_row1 = -1; ti.heads = nullptr;
+    if (!mbar_wait(&tail->tq_full[slot], static_cast<uint32_t>(k / kTileQ) & 1u, abort_flag)) return ti;
+    const int4 rec = tail->tile_q[slot];
     mbar_arrive(&tail->tq_empty[slot]);
-    return t;
+    ti.a_row = rec.x; ti.w_row0 = rec.y; ti.w_row1 = rec.z; ti.nkb = rec.w;
+    return ti;
   };
 
   if (warp == 4) {
@@ -191,8 +328,6 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
     int stage = 0;
     uint32_t phase = 0;
     int ok = 1;
-    TileInfo nxt;
-    nxt.a_row = nxt.w_row0 = nxt.nkb = 0; nxt.w_row1 = -1; nxt.heads = nullptr;
     int hreg[kMaxHeadsSmem / 32];
     auto fetch_heads = [&](const TileInfo& ti) {
       if (ti.heads == nullptr) return;
@@ -205,15 +340,15 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
       for (int i = 0; i < kMaxHeadsSmem / 32; ++i) tail->heads[par][lane + 32 * i] = hreg[i];
     };
     int n_pub = 0;  // entries published so far (lane 0)
-    auto publish = [&](int t) -> bool {  // lane 0
+    auto publish = [&](const TileInfo& ti) -> bool {  // lane 0
       const int slot = n_pub % kTileQ;
       if (!mbar_wait(&tail->tq_empty[slot], (static_cast<uint32_t>(n_pub / kTileQ) & 1u) ^ 1u, abort_flag)) return false;
-      tail->tile_q[slot] = t;
+      tail->tile_q[slot] = make_int4(ti.a_row, ti.w_row0, ti.w_row1, ti.nkb);
       mbar_arrive(&tail->tq_full[slot]);
       ++n_pub;
       return true;
     };
-    int n_drawn = 0;
+    int n_tiles = 0, n_drawn = 0;
     auto draw = [&]() -> int {  // lane 0: the next tile of the device-wide sequence
       // equal tiles (dense: no cursor) keep the fixed round-robin share and skip the atomic
       ++n_drawn;
@@ -221,42 +356,37 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
                                         : static_cast<int>(blockIdx.x) + n_drawn * static_cast<int>(gridDim.x);
       return t < n_tiles ? t : -1;
     };
-    // t_cur is being loaded, t_n1 is known and published, t_n2 is drawn while t_cur runs (two tiles of
-    // lead, so that the atomic's round trip never sits between two tiles)
-    int t_cur = static_cast<int>(blockIdx.x) < n_tiles ? static_cast<int>(blockIdx.x) : -1;
+    TileInfo none;
+    none.a_row = -1; none.w_row0 = none.nkb = 0; none.w_row1 = -1; none.heads = nullptr;
+    // `cur` is being loaded, t_n1 is known, t_n2 is drawn while `cur` runs, so that the atomic's round trip never sits
+    // between two tiles. The next tile's record goes to the other roles before the rest of `cur` is loaded.
+    TileInfo cur = none;
     int t_n1 = -1;
-    if (lane == 0) {
-      ok = publish(t_cur) ? 1 : 0;
-      if (ok && t_cur >= 0) {
-        t_n1 = draw();
-        ok = publish(t_n1) ? 1 : 0;
-      }
+    if (a.own_first) {
+      cur = first;
+    } else {
+      n_tiles = num_tiles(a);
+      if (static_cast<int>(blockIdx.x) < n_tiles) cur = get_tile(a, static_cast<int>(blockIdx.x));
     }
+    if (lane == 0) ok = publish(cur) ? 1 : 0;
     ok = __shfl_sync(0xffffffffu, ok, 0);
-    t_n1 = __shfl_sync(0xffffffffu, t_n1, 0);
-    if (t_cur >= 0) {
-      nxt = get_tile(a, t_cur);
-      fetch_heads(nxt);
+    if (!a.own_first && cur.a_row >= 0) {
+      fetch_heads(cur);
       stash_heads(0);
     }
     __syncwarp();
+    bool is_first = true;
+    bool list_due = a.own_first != 0;   // the list is still to be waited for
     int par = 0;
-    while (t_cur >= 0 && ok) {
-      int t_n2 = -1;
-      if (lane == 0 && t_n1 >= 0) t_n2 = draw();
-      TileInfo ti = nxt;
+    while (cur.a_row >= 0 && ok) {
+      TileInfo ti = cur;
       if (ti.heads != nullptr && ti.nkb / a.kb_per_head <= kMaxHeadsSmem) ti.heads = tail->heads[par];
-      const bool more = t_n1 >= 0;
-      if (more) {
-        nxt = get_tile(a, t_n1);
-        fetch_heads(nxt);
-      }
-      if (lane == 0) {
+      // K columns are generated without divisions: (head list entry, K block inside the head)
+      int hh = 0, sub = 0;
+      int kcol = (ti.heads != nullptr && ti.nkb > 0) ? ti.heads[0] * a.kb_per_head * kBK : 0;
+      auto load = [&](int j0, int j1) {   // lane 0
         const uint32_t bytes = ti.w_row1 >= 0 ? kStageBytes : (kABytes + kBHalfBytes);
-        // K columns are generated without divisions: (head list entry, K block inside the head)
-        int hh = 0, sub = 0;
-        int kcol = (ti.heads != nullptr && ti.nkb > 0) ? ti.heads[0] * a.kb_per_head * kBK : 0;
-        for (int j = 0; j < ti.nkb; ++j) {
+        for (int j = j0; j < j1; ++j) {
           if (!mbar_wait(&tail->empty[stage], phase ^ 1u, abort_flag)) { ok = 0; break; }
           uint8_t* sa = smem + stage * kStageBytes;
           mbar_expect_tx(&tail->full[stage], bytes);
@@ -276,18 +406,43 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
             if (j + 1 < ti.nkb) kcol = ti.heads[hh] * a.kb_per_head * kBK;
           }
         }
-        if (ok && more && !publish(t_n2)) ok = 0;
+      };
+      int head = 0;   // K blocks loaded before the next tile is looked up
+      if (is_first) {
+        head = ti.nkb < kStages ? ti.nkb : kStages;
+        if (lane == 0) load(0, head);
+        __syncwarp();
+        is_first = false;
+        if (list_due) {
+          asm volatile("griddepcontrol.wait;" ::: "memory");
+          list_due = false;
+          n_tiles = num_tiles(a);
+        }
+        if (lane == 0) t_n1 = draw();
+      }
+      t_n1 = __shfl_sync(0xffffffffu, t_n1, 0);
+      int t_n2 = -1;
+      if (lane == 0 && t_n1 >= 0) t_n2 = draw();
+      TileInfo nxt = none;
+      if (t_n1 >= 0) {
+        nxt = get_tile(a, t_n1);
+        fetch_heads(nxt);
+      }
+      if (lane == 0) {
+        if (ok && !publish(nxt)) ok = 0;
+        if (ok) load(head, ti.nkb);
       }
       __syncwarp();
-      if (more) stash_heads(par ^ 1);
+      if (t_n1 >= 0) stash_heads(par ^ 1);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       stage = __shfl_sync(0xffffffffu, stage, 0);
       phase = __shfl_sync(0xffffffffu, phase, 0);
-      t_n2 = __shfl_sync(0xffffffffu, t_n2, 0);
-      t_cur = t_n1;
       t_n1 = t_n2;
+      cur = nxt;
       par ^= 1;
+      __syncwarp();
     }
+    if (list_due) asm volatile("griddepcontrol.wait;" ::: "memory");
   } else if (warp == 5) {
     // ------------------------------------------------------------- MMA issuer
     if (lane == 0) {
@@ -301,17 +456,9 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
       // every operand tile is K-major with 128-byte swizzle: same descriptor high word, low word = address
       const uint64_t desc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
       const uint32_t desc_hi = static_cast<uint32_t>(desc0 >> 32), desc_lo0 = static_cast<uint32_t>(desc0);
-      TileInfo nxt;
-      nxt.a_row = nxt.w_row0 = nxt.nkb = 0; nxt.w_row1 = -1; nxt.heads = nullptr;
-      int k_seq = 0;
-      int t_cur = read_slot(0);
-      if (t_cur >= 0) nxt = get_tile(a, t_cur);
-      for (; t_cur >= 0 && ok; ++k_seq) {
-        const TileInfo ti = nxt;  // the next tile's record is fetched while this one runs
-        const int t_nxt = read_slot(k_seq + 1);
-        if (t_nxt >= 0) nxt = get_tile(a, t_nxt);
-        if (t_nxt == -2) ok = false;
-        t_cur = t_nxt;
+      for (int k_seq = 0; ok; ++k_seq) {
+        const TileInfo ti = read_slot(k_seq);
+        if (ti.a_row < 0) break;
         const uint32_t idesc = ti.w_row1 >= 0 ? idesc256 : idesc128;
         if (!mbar_wait(&tail->acc_empty[acc], acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
@@ -339,9 +486,8 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
     if (lane == 0) {
       uint32_t count = 0;
       for (int k_seq = 0;; ++k_seq) {
-        const int t = read_slot(k_seq);
-        if (t < 0) break;
-        const TileInfo ti = get_tile(a, t);
+        const TileInfo ti = read_slot(k_seq);
+        if (ti.a_row < 0) break;
         const int nslab = ti.w_row1 >= 0 ? 2 * kSlabsPerBlock : kSlabsPerBlock;
         bool ok = true;
         for (int s = 0; s < nslab && ok; ++s, ++count) {
@@ -365,27 +511,22 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
     // 16-byte pieces of a row of the slab: the 128-byte swizzle of 64 columns, the 64-byte one of 32
     constexpr int kPieces = kSlabCols / 8;
     const uint32_t swz = static_cast<uint32_t>(kCache ? (r_in_tile >> 1) & 3 : r_in_tile & 7);
-    TileInfo nxt;
-    nxt.a_row = nxt.w_row0 = nxt.nkb = 0; nxt.w_row1 = -1; nxt.heads = nullptr;
-    auto read_slot_warp = [&](int k) -> int {  // lane 0 reads, the warp shares the value
-      int t = 0;
-      if (lane == 0) t = read_slot(k);
-      return __shfl_sync(0xffffffffu, t, 0);
+    auto read_slot_warp = [&](int k) -> TileInfo {  // lane 0 reads, the warp shares the record
+      TileInfo ti;
+      ti.a_row = ti.w_row0 = ti.w_row1 = ti.nkb = 0; ti.heads = nullptr;
+      if (lane == 0) ti = read_slot(k);
+      ti.a_row = __shfl_sync(0xffffffffu, ti.a_row, 0);
+      ti.w_row0 = __shfl_sync(0xffffffffu, ti.w_row0, 0);
+      ti.w_row1 = __shfl_sync(0xffffffffu, ti.w_row1, 0);
+      ti.nkb = __shfl_sync(0xffffffffu, ti.nkb, 0);
+      return ti;
     };
-    int k_seq = 0;
-    int t_cur = read_slot_warp(0);
-    if (t_cur >= 0) nxt = get_tile(a, t_cur);
     // The four warps leave this loop together: every round ends in a vote (two CTA-local barriers around one
     // shared word), so a wait that ran out in one warp can never leave the others behind at `epi_bar`.
-    for (;; ++k_seq) {
-      const TileInfo ti = nxt;
-      const int t_this = t_cur;
+    for (int k_seq = 0;; ++k_seq) {
+      const TileInfo ti = read_slot_warp(k_seq);
+      const int t_this = ti.a_row;
       bool fail = t_this == -2;
-      if (t_this >= 0) {
-        const int t_nxt = read_slot_warp(k_seq + 1);
-        if (t_nxt >= 0) nxt = get_tile(a, t_nxt);
-        t_cur = t_nxt;
-      }
       const int nslab = ti.w_row1 >= 0 ? 2 * kSlabsPerBlock : kSlabsPerBlock;
       // init values of slab 0 are fetched before the accumulator is waited for
       uint4 initv[kPieces];
@@ -523,6 +664,9 @@ cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream) {
   if (cap <= 0) return cudaSuccess;
   const int grid = cap < max_ctas ? cap : max_ctas;
   const bool cache = a.init_mode == kInitFull;
+  const int rows = a.batch * (a.m / kBM);
+  g.own_first = a.after_list && rows <= kFirstRows &&
+                (listed ? a.list.head_dim == kBNH && a.n / kBNH <= 64 && a.list.is_full == 0 : a.list.k / a.list.head_dim <= 64);
   const auto kernel = a.is_bf16 ? (cache ? gemm_kernel<true, true> : gemm_kernel<true, false>)
                                 : (cache ? gemm_kernel<false, true> : gemm_kernel<false, false>);
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};

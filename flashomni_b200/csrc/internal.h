@@ -163,6 +163,8 @@ struct GemmArgs {
   int32_t* cursor;                 // device-wide tile cursor, zero when the kernel starts
   int single;                      // no tile list: tiles of one column block instead of two (set by launch_gemm)
   int after_list;                  // the launch in front of this one builds the list (dependent launch)
+  int own_first;                   // a CTA finds its first tile in the mask itself (set by launch_gemm); needs `list`
+  GemmListArgs list;               // after_list: what that launch got
 };
 cudaError_t launch_gemm(const GemmArgs& a, int max_ctas, cudaStream_t stream);
 // dense projections whose shape divides into 256x256 tiles take the tall-tile kernel (gemm_tall.cu)

@@ -11,6 +11,7 @@
 // report malformed input through a status word instead of faulting.
 #include "cast_fp8.cuh"
 #include "internal.h"
+#include "mask_bits.cuh"
 
 namespace fo {
 
@@ -219,46 +220,6 @@ cudaError_t launch_segment_packbits_sized(const uint8_t* x, int64_t n, const voi
     segment_packbits_sized_kernel<int32_t><<<static_cast<int>(blocks), 256, 0, stream>>>(
         x, n, static_cast<const int32_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
   return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------------------------
-// Bit-stream helpers
-// ---------------------------------------------------------------------------------------------
-// 32 bits of the little-endian bit stream `seg` starting at bit `pos`; bytes at or beyond `limit`
-// (the number of readable bytes from `seg`) read as zero.
-__device__ __forceinline__ uint32_t load_bits32(const uint8_t* seg, int64_t pos, int64_t limit) {
-  const int64_t byte0 = pos >> 3;
-  const int sh = static_cast<int>(pos & 7);
-  uint64_t acc = 0;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    const int64_t bi = byte0 + i;
-    const uint64_t v = (bi < limit) ? seg[bi] : 0u;
-    acc |= v << (8 * i);
-  }
-  return static_cast<uint32_t>(acc >> sh);
-}
-__device__ __forceinline__ int get_bit(const uint8_t* seg, int64_t pos, int64_t limit) {
-  const int64_t bi = pos >> 3;
-  if (bi >= limit) return 0;
-  return (seg[bi] >> (pos & 7)) & 1;
-}
-
-// up to 64 bits of the stream starting at bit `pos` (9 independent byte loads, clamped like load_bits32)
-__device__ __forceinline__ uint64_t load_bits64(const uint8_t* seg, int64_t pos, int64_t limit, int nbits) {
-  const int64_t byte0 = pos >> 3;
-  const int sh = static_cast<int>(pos & 7);
-  uint64_t lo = 0, hi = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t bi = byte0 + i;
-    const uint64_t v = (bi < limit) ? seg[bi] : 0u;
-    lo |= v << (8 * i);
-  }
-  if (byte0 + 8 < limit) hi = seg[byte0 + 8];
-  uint64_t r = sh ? ((lo >> sh) | (hi << (64 - sh))) : lo;
-  if (nbits < 64) r &= (1ull << nbits) - 1ull;
-  return r;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1213,30 +1174,6 @@ cudaError_t launch_attn_lists_small(const CompactArgs& a, const UnitArgs& u, con
 // per thread (the usual case) the second walk has everything in registers.
 // Both list kernels are all latency and sit in front of the GEMM when the caller did not prepare the list: they let it
 // start its set-up at once (programmatic dependent launch; the GEMM waits for the list before reading it).
-constexpr int kPairCost = 20, kSingleCost = 13;
-
-// Time at which the last CTA ends when `n` CTAs draw `pairs` two-block tiles and then `singles` single-block tiles
-// in list order, every tile going to the CTA that is free first.
-__device__ __forceinline__ int gemm_q_makespan(int pairs, int singles, int n) {
-  const int full = pairs / n, r = pairs % n;
-  int t_a = full * kPairCost, c_a = n - r;        // CTAs free after the full rounds
-  int t_b = (full + 1) * kPairCost, c_b = r;      // CTAs that run one more two-block tile
-  int end = (full + (r ? 1 : 0)) * kPairCost;
-  int m = singles;
-  while (m > 0) {
-    if (c_a > 0 && (c_b == 0 || t_a <= t_b)) {
-      m -= c_a;
-      t_a += kSingleCost;
-      end = end > t_a ? end : t_a;
-    } else {
-      m -= c_b;
-      t_b += kSingleCost;
-      end = end > t_b ? end : t_b;
-    }
-  }
-  return end;
-}
-
 __device__ __forceinline__ void gemm_q_tiles_body(const GemmListArgs& a) {
   __shared__ int s_warp[32];
   __shared__ int s_warp_t[32];
