@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
     const int row_tok = row >> grp_shift, row_head = row & (grp - 1), row_tok0 = (quad * 32) >> grp_shift;
     uint32_t item = 0;
     uint32_t g = 0;         // blocks in front of the current unit
-    uint32_t units0 = 0, units1 = 0;   // units so far that had blocks of stream 0 / 1
+    uint32_t o_phase = 0;   // bit X: parity of the units so far that had blocks of stream X
     ItemRead<true> src;
     src.init(tail, abort_flag);
     while (true) {
@@ -470,8 +470,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       float* lse = a.lse != nullptr ? a.lse + grow * a.lse_stride_n + hq : nullptr;
       const uint32_t ip = item & 1u;
       if (!mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag)) break;
-      const float m0 = tail->stats_m[ip][0][row], m1 = tail->stats_m[ip][1][row];
-      const float l0 = tail->stats_l[ip][0][row], l1 = tail->stats_l[ip][1][row];
+      // 0 and 1 are the streams of the unit's first and second block from here on: which of the two that is depends on the
+      // units that this CTA drew before, the rounding of the sums must not
+      const uint32_t f = g & 1u;
+      const float m0 = tail->stats_m[ip][f][row], m1 = tail->stats_m[ip][f ^ 1u][row];
+      const float l0 = tail->stats_l[ip][f][row], l1 = tail->stats_l[ip][f ^ 1u][row];
       __syncwarp();
       if (lane == 0) mbar_arrive(&tail->stats_free[ip]);
       const float m_out = fmaxf(m0, m1);
@@ -482,14 +485,15 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       w0 *= inv_out;
       w1 *= inv_out;
       // a unit of one block leaves the other stream's O as it was: whatever that is, it does not count
-      const bool has0 = u0.x > 1 || (g & 1u) == 0u, has1 = u0.x > 1 || (g & 1u) == 1u;
+      const bool has1 = u0.x > 1;
       g += static_cast<uint32_t>(u0.x);
-      if (has0 && !mbar_wait(&tail->o_full[0], units0++ & 1u, abort_flag)) break;
-      if (has1 && !mbar_wait(&tail->o_full[1], units1++ & 1u, abort_flag)) break;
+      if (!mbar_wait(&tail->o_full[f], (o_phase >> f) & 1u, abort_flag)) break;
+      if (has1 && !mbar_wait(&tail->o_full[f ^ 1u], (o_phase >> (f ^ 1u)) & 1u, abort_flag)) break;
+      o_phase ^= has1 ? 3u : 1u << f;
       tc_fence_after_sync();
       const bool whole = q_valid * grp == kBQ;   // no row of the q-block is past the request
       // (an O that nothing wrote may hold anything: the other one stands in for it, with the weight of zero)
-      const uint32_t tmem_o0 = tmem_o + (has0 ? 0u : 128u), tmem_o1 = tmem_o + (has1 ? 128u : 0u);
+      const uint32_t tmem_o0 = tmem_o + 128u * f, tmem_o1 = has1 ? tmem_o + 128u * (f ^ 1u) : tmem_o0;
       const uint64_t w0p = pack_f32x2(w0, w0), w1p = pack_f32x2(w1, w1);
 #pragma unroll 1
       for (int half = 0; half < kHalves; ++half) {
@@ -514,8 +518,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            if (has0) mbar_arrive(&tail->o_free[0]);
-            if (has1) mbar_arrive(&tail->o_free[1]);
+            mbar_arrive(&tail->o_free[f]);
+            if (has1) mbar_arrive(&tail->o_free[f ^ 1u]);
           }
         }
         // Through a staging slab per warp (32 rows x 64 columns in the 128-byte swizzle pattern): a store instruction of

@@ -55,6 +55,22 @@ def test_many_short_units_against_the_oracle(cuda_device, D, H, Hkv, dtype, q_sc
     assert torch.allclose(lse.cpu(), ref_lse, atol=2e-2, rtol=1e-4)
 
 
+def test_the_same_bits_from_call_to_call(cuda_device):
+    """Which units a CTA draws, and with them which stream a unit's first block belongs to, changes from call to call; sums and
+    their rounding do not."""
+    lens = [128, 700, 333, 1, 900, 77, 512, 1300]
+    qo, kv, m, q, k, v = _case(lens, lens[::-1], 16, 16, 128, torch.bfloat16, 0.6, 5)
+    w = _plan(cuda_device, qo, kv, 16, 16, 128, torch.bfloat16)
+    args = [dev(t, cuda_device) for t in (q, k, v)] + list(masks_to_device(m, cuda_device))
+    fresh = lambda: torch.full((q.shape[0], 16), 3.0, device=cuda_device)   # rows of skipped q-blocks keep what they hold
+    first, first_lse = w.run(*args, lse=fresh(), return_lse=True)
+    first = first.clone()
+    for _ in range(20):
+        o, lse = w.run(*args, lse=fresh(), return_lse=True)
+        assert torch.equal(o.view(torch.int16), first.view(torch.int16)) and torch.equal(lse, first_lse)
+    w.check_status()
+
+
 @pytest.mark.parametrize("keep", [0.0, 0.02, 0.25])
 def test_long_runs_of_units_that_keep_nothing(cuda_device, keep):
     """Active q-blocks without a kept kv-block sit at the end of the processing order, several per CTA behind each other."""
