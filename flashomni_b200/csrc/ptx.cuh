@@ -140,6 +140,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// 4 bytes from global to shared memory without a register in between; cp_async_wait_all: this thread's copies have landed
+__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // TMA tiled loads (no multicast anywhere in this library)
 // ---------------------------------------------------------------------------------------------

@@ -16,7 +16,11 @@
 // most 32 entries lie in the bracket each lane takes one and ranks it against the others. Equal masses that never get
 // below 32 are cut by index directly.
 // Measured on a B200 at 40 heads x 604 blocks, thresholds 0.2 / 0.3 (the text-to-image scores switch most q-blocks off):
-// whole call 82.4 us with four launches, a memset and threshold arrays, 25.5 us with these two launches.
+// whole call 82.4 us with four launches, a memset and threshold arrays, 25.5 us with these two launches; on the device
+// 21.1 -> 19.1 us with the score values as asynchronous copies, a byte of sparse_info from at most two flags and the rows'
+// flag addresses worked out before the first kernel ends (every row computed 87 -> 83, 24 heads x 2048 blocks 53.6 -> 49).
+// Both kernels run their code once per thread, so length of code counts: four masses at a time and unrolled, the ranking of
+// the image blocks took 4.0 us instead of 2.4. Rows computed ahead of their flags cost more than they saved (19 -> 28 us).
 #include <cooperative_groups.h>
 
 #include <utility>
@@ -210,7 +214,8 @@ __device__ __forceinline__ void select_row(const float* __restrict__ x, int len,
 // First launch. Cluster b < batch (eight CTAs): which image q-blocks of request b stay on, sparse_info and the indptrs;
 // the other clusters zero the kv bit stream, into which the rows of the second launch are written.
 // The text-to-image score of a block is sum over heads (outer) and text rows (inner) of score[b][h][q][t2t + j] in
-// sequential fp32: a CTA fetches the values of its eighth of the blocks with every thread into shared memory, one thread
+// sequential fp32: a CTA fetches the values of its eighth of the blocks with every thread into shared memory (asynchronous
+// copies, a warp per score row, so that no thread holds values or divides per value), one thread
 // per block adds them up. The scores then go to all eight CTAs (distributed shared memory), which compute the masses
 // redundantly and rank an eighth of the blocks each, eight lanes per block, against all of them: no sort, no search.
 // Shared memory of another CTA may only be touched once that CTA runs: each announces itself at the cluster barrier on
@@ -245,12 +250,12 @@ __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelQThrea
     float acc = 0.f;
     for (int p0 = 0; p0 < pairs; p0 += per_pass) {
       const int np = pairs - p0 < per_pass ? pairs - p0 : per_pass;
-#pragma unroll 8
-      for (int i = tid; i < np * cols; i += kSelQThreads) {
-        const int p = i / cols, pair = p0 + p;
-        const int h = pair / a.t2t, q = pair - h * a.t2t;
-        s_val[i] = score[(static_cast<int64_t>(h) * a.n + q) * a.n + (i - p * cols)];
+      for (int p = warp; p < np; p += kSelQThreads / 32) {   // all of them in flight at once
+        const int pair = p0 + p, h = pair / a.t2t, q = pair - h * a.t2t;
+        const float* src = score + (static_cast<int64_t>(h) * a.n + q) * a.n;
+        for (int c = lane; c < cols; c += 32) cp_async_4(s_val + p * cols + c, src + c);
       }
+      cp_async_wait_all();
       __syncthreads();
       if (tid < cols) {
 #pragma unroll 8
@@ -316,10 +321,17 @@ __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelQThrea
   const int64_t nbits = static_cast<int64_t>(a.n) * a.heads;
   for (int64_t i = t0; i < a.info_seg_bytes; i += kSelCluster * kSelQThreads) {
     uint32_t v = 0;
-    int qb = static_cast<int>(i * 8 / a.heads), h = static_cast<int>(i * 8 - static_cast<int64_t>(qb) * a.heads);
-    for (int t = 0; t < 8; ++t) {
-      if (i * 8 + t < nbits && kept(qb)) v |= 1u << t;
-      if (++h == a.heads) { h = 0; ++qb; }
+    int qb = i < (1 << 28) ? static_cast<int>(i) * 8 / a.heads : static_cast<int>(i * 8 / a.heads);
+    int h = static_cast<int>(i * 8 - static_cast<int64_t>(qb) * a.heads);
+    if (a.heads >= 8) {   // one or two q-blocks in the byte
+      const int left = a.heads - h, own = left < 8 ? left : 8;
+      if (kept(qb)) v = (1u << own) - 1u;
+      if (own < 8 && qb + 1 < a.n && kept(qb + 1)) v |= 0xffu << own & 0xffu;
+    } else {
+      for (int t = 0; t < 8; ++t) {
+        if (i * 8 + t < nbits && kept(qb)) v |= 1u << t;
+        if (++h == a.heads) { h = 0; ++qb; }
+      }
     }
     a.sparse_info[b * a.info_seg_bytes + i] = static_cast<uint8_t>(v);
   }
@@ -343,12 +355,14 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_kv_kernel(SelectArgs a)
   const int64_t rows = static_cast<int64_t>(a.batch) * a.heads * a.n;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * kSelWarps + warp, step = static_cast<int64_t>(gridDim.x) * kSelWarps;
   uint32_t* words = s_words[warp];
+  auto keep_of = [&](int64_t row) { return a.q_keep + row / (static_cast<int64_t>(a.n) * a.heads) * a.n + row % a.n; };
+  const uint8_t* keep = keep_of(first + lane * step < rows ? first + lane * step : 0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int64_t base = first; base < rows; base += 32 * step) {
     const int64_t mine = base + lane * step;
     bool on = mine < rows;
-    if (on && a.zero_inactive)
-      on = __ldcg(a.q_keep + mine / (static_cast<int64_t>(a.n) * a.heads) * a.n + mine % a.n) != 0;
+    if (base != first && on) keep = keep_of(mine);
+    if (on && a.zero_inactive) on = __ldcg(keep) != 0;
     for (unsigned left = __ballot_sync(0xffffffffu, on); left != 0u; left &= left - 1u) {
       const int64_t row = base + (__ffs(left) - 1) * step;
       const int q = static_cast<int>(row % a.n);

@@ -32,6 +32,16 @@ def test_bit_exact(cuda_device, B, H, n, t2t, zero_inactive):
     assert np.array_equal(kv, rkv)
 
 
+@pytest.mark.parametrize("H", [7, 8, 9, 13, 65])
+@pytest.mark.parametrize("n,t2t", [(9, 2), (17, 9), (44, 3)])
+def test_bytes_that_two_blocks_share(cuda_device, H, n, t2t):
+    """A byte of sparse_info holds bits of one, two (8 heads and more) or several q-blocks, and ends short in the last one."""
+    s = (np.random.default_rng(H * n).standard_normal((2, H, n, n)) * 1.5).astype(np.float32)
+    got = _run(s, t2t, 0.35, 0.3, True, cuda_device)
+    want = osel.pack_selection(*osel.select_blocks(s, t2t, 0.35, 0.3))
+    assert all(np.array_equal(g, w) for g, w in zip(got, (want[0], want[1], want[2], want[3])))
+
+
 def test_ties_and_extremes(cuda_device):
     n = 64
     s = np.zeros((1, 2, n, n), dtype=np.float32)          # all scores equal: ties broken by block index
