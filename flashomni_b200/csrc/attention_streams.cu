@@ -492,8 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       o_phase ^= has1 ? 3u : 1u << f;
       tc_fence_after_sync();
       const bool whole = q_valid * grp == kBQ;   // no row of the q-block is past the request
-      // (an O that nothing wrote may hold anything: the other one stands in for it, with the weight of zero)
-      const uint32_t tmem_o0 = tmem_o + 128u * f, tmem_o1 = has1 ? tmem_o + 128u * (f ^ 1u) : tmem_o0;
+      const uint32_t tmem_o0 = tmem_o + 128u * f, tmem_o1 = tmem_o + 128u * (f ^ 1u);
       const uint64_t w0p = pack_f32x2(w0, w0), w1p = pack_f32x2(w1, w1);
 #pragma unroll 1
       for (int half = 0; half < kHalves; ++half) {
@@ -503,7 +502,12 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         for (int c = 0; c < 4; ++c) {
           uint32_t v0[16], v1[16];
           tmem_ld_x16(tmem_o0 + 64u * half + 16u * c, v0);
-          tmem_ld_x16(tmem_o1 + 64u * half + 16u * c, v1);
+          if (has1) {
+            tmem_ld_x16(tmem_o1 + 64u * half + 16u * c, v1);
+          } else {  // an O that nothing wrote may hold anything, and no value times its weight of zero need be zero
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v1[t] = 0u;
+          }
           tmem_wait_ld();
 #pragma unroll
           for (int t = 0; t < 8; ++t) {

@@ -107,3 +107,30 @@ def test_nan_in_a_key_reaches_every_row_that_attends_to_it(cuda_device, blocks):
     o = w.run(dev(q, cuda_device), dev(k, cuda_device), dev(v, cuda_device), is_full=True).cpu()
     w.check_status()
     assert torch.isnan(o[:, 1]).all() and torch.isfinite(o[:, 0]).all()
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 3])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("kind", ["bf16", "f16", "e5m2"])
+def test_infinities_in_v_reach_the_output_as_infinities(cuda_device, kind, D, blocks):
+    """A row of V with +inf, -inf or both in a column: every weight is positive (|logit| < 8, so P > 2^-24 also in f16), so
+    the column is +inf, -inf or NaN in every row that attends to it, and nothing else changes."""
+    S, H = 128 * blocks, 2
+    dtype = torch.float16 if kind == "f16" else torch.bfloat16
+    q, k, v = (wl.randn_bf16((S, H, D), s).to(dtype) for s in (1, 2, 3))
+    v[S - 20, 1, 7], v[3, 1, 9] = float("inf"), -float("inf")
+    v[5, 1, D - 1], v[S - 1, 1, D - 1] = float("inf"), -float("inf")
+    kv_dtype = torch.float8_e5m2 if kind == "e5m2" else dtype
+    k, v = k.to(kv_dtype), v.to(kv_dtype)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device))
+    ip = torch.tensor([0, S], dtype=torch.int32, device=cuda_device)
+    w.plan(ip, ip, H, H, D, q_data_type=dtype, kv_data_type=kv_dtype)
+    o = w.run(dev(q, cuda_device), dev(k, cuda_device), dev(v, cuda_device), is_full=True).float().cpu()
+    w.check_status()
+    qf, kf, vf = (t.float().transpose(0, 1) for t in (q, k, v))
+    p = torch.softmax(qf @ kf.transpose(1, 2) / D ** 0.5, 2)
+    ref = (p @ vf).transpose(0, 1)
+    assert torch.isposinf(o[:, 1, 7]).all() and torch.isneginf(o[:, 1, 9]).all() and torch.isnan(o[:, 1, D - 1]).all()
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(o), fin)
+    assert_close_bf16(o[fin], ref[fin], f"{kind} D={D} blocks={blocks}", allow_ulp=1.0)
