@@ -17,6 +17,7 @@ _HOST = os.path.join(_HERE, "lib", "_fo_host.so")
 
 FO_OK, FO_ERR_INVALID_ARG, FO_ERR_UNSUPPORTED, FO_ERR_CUDA, FO_ERR_WORKSPACE = 0, 1, 2, 3, 4
 FO_DTYPE_F16, FO_DTYPE_BF16 = 0, 1
+PACK_WORDS = 148   # words of fo_segment_packbits_polled: one block per SM
 FO_DEV_OK, FO_DEV_WAIT_TIMEOUT, FO_DEV_BAD_INDEX = 0, 1, 2
 
 # name -> (restype, argtypes); mirrors include/flashomni_b200.h one to one
@@ -39,7 +40,7 @@ SIGNATURES = {
     "fo_packbits": (c_int32, [_P, c_int64, c_int32, _P, _P]),
     "fo_segment_packbits": (c_int32, [_P, _P, _P, c_int32, c_int64, c_int32, _P, _P]),
     "fo_segment_packbits_within": (c_int32, [_P, c_int64, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
-    "fo_segment_packbits_early": (c_int32, [_P, c_int64, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
+    "fo_segment_packbits_polled": (c_int32, [_P, c_int64, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, c_int32, _P]),
     "fo_segment_packbits_sized": (c_int32, [_P, _P, c_int32, c_int32, c_int64, c_int32, _P, _P, _P, _P]),
     "fo_mask_compact_scratch_bytes": (c_size_t, [c_int64, c_int32]),
     "fo_mask_compact": (c_int32, [_P, c_int64, _P, c_int64, _P, _P, _P, _P,

@@ -173,34 +173,38 @@ int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32_t indp
 }
 
 namespace {
-constexpr int64_t kNotYet = -2;   // total_bytes before the kernel has written it
-// Waits until the kernel has written *total: polls for it for up to a millisecond, then waits for the stream, as it also does
+constexpr int64_t kNotYet = -2;   // a word before its block has written it
+// Waits until all blocks have written their words: polls for up to a millisecond, then waits for the stream, as it also does
 // under capture, where nothing runs (and the wait is the error that the caller expects).
-cudaError_t wait_total(const int64_t* total, cudaStream_t st) {
+cudaError_t wait_words(const int64_t* words, int n, cudaStream_t st) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   const cudaError_t e = cudaStreamIsCapturing(st, &capture);
   if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return cudaStreamSynchronize(st);
-  const volatile int64_t* t = total;
+  const volatile int64_t* w = words;
   const auto t0 = std::chrono::steady_clock::now();
+  int done = 0;
   for (uint32_t i = 0;; ++i) {
-    if (*t != kNotYet) return cudaSuccess;
+    while (done < n && w[done] != kNotYet) ++done;
+    if (done == n) return cudaSuccess;
     if ((i & 255u) == 255u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(1)) return cudaStreamSynchronize(st);
   }
 }
 
 int segment_packbits_impl(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
-                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes, bool early,
+                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* words, int32_t num_words,
                           void* stream) {
   if (n < 0 || num_segments < 0 || capacity < 0) return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: negative size");
   if (num_segments > 1024) return fail(FO_ERR_UNSUPPORTED, "fo_segment_packbits_sized: at most 1024 segments");
-  if (x == nullptr || y == nullptr || indptr == nullptr || new_indptr == nullptr || total_bytes == nullptr)
+  if (x == nullptr || y == nullptr || indptr == nullptr || new_indptr == nullptr || words == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_sized: null pointer");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (early) *static_cast<volatile int64_t*>(total_bytes) = kNotYet;
+  const int blocks = segment_packbits_sized_blocks(capacity);
+  const bool poll = blocks <= num_words;
+  for (int i = 0; poll && i < blocks; ++i) static_cast<volatile int64_t*>(words)[i] = kNotYet;
   cudaError_t e = launch_segment_packbits_sized(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr,
-                                                reinterpret_cast<long long*>(total_bytes), st);
+                                                reinterpret_cast<long long*>(words), poll ? 1 : 0, st);
   count_launches(1);
-  if (e == cudaSuccess) e = early ? wait_total(total_bytes, st) : cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = poll ? wait_words(words, blocks, st) : cudaStreamSynchronize(st);
   return e == cudaSuccess ? FO_OK : fail_cuda("fo_segment_packbits_sized", e);
 }
 }  // namespace
@@ -208,14 +212,15 @@ int segment_packbits_impl(const uint8_t* x, int64_t n, const void* indptr, int32
 int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
                                int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
                                void* stream) {
-  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, total_bytes, false,
+  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, total_bytes, 0,
                                stream);
 }
 
-int fo_segment_packbits_early(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
-                              int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* total_bytes,
-                              void* stream) {
-  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, total_bytes, true,
+int fo_segment_packbits_polled(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64, int32_t num_segments,
+                               int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, int64_t* words,
+                               int32_t num_words, void* stream) {
+  if (num_words < 1) return fail(FO_ERR_INVALID_ARG, "fo_segment_packbits_polled: at least one word");
+  return segment_packbits_impl(x, n, indptr, indptr_is_64, num_segments, capacity, little, y, new_indptr, words, num_words,
                                stream);
 }
 

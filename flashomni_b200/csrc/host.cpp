@@ -31,7 +31,7 @@ struct Api {
   decltype(&fo_gemm_q_prepared) gemm_q_prepared;
   decltype(&fo_gemm_o_prepared) gemm_o_prepared;
   decltype(&fo_gemm_workspace_bytes) gemm_workspace_bytes;
-  decltype(&fo_segment_packbits_early) segment_packbits_early;
+  decltype(&fo_segment_packbits_polled) segment_packbits_polled;
   decltype(&fo_select_blocks_uniform) select_blocks_uniform;
   decltype(&fo_select_blocks_scratch_bytes) select_scratch_bytes;
   decltype(&fo_layer_lists) layer_lists;
@@ -407,17 +407,18 @@ PyObject* segment_packbits(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t capacity = (n + 7 * nseg) / 8;
   at::Tensor y = at::empty({capacity}, x->options().dtype(at::kByte));
   at::Tensor bytes_indptr = at::empty({nseg + 1}, x->options().dtype(at::kInt));
-  const at::Tensor total = at::empty({1}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  constexpr int kWords = 148;   // (one block per SM: beyond that the wait for the stream is a small part of the call)
+  const at::Tensor words = at::empty({kWords}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
   void* stream = current_stream(dev);
   int rc;
   {
-    pybind11::gil_scoped_release no_gil;   // (this call waits for the size, not for the packing)
-    rc = g_api.segment_packbits_early(static_cast<const uint8_t*>(x->data_ptr()), n, ip->data_ptr(), it == at::kLong ? 1 : 0, i32(nseg),
+    pybind11::gil_scoped_release no_gil;   // (this call waits)
+    rc = g_api.segment_packbits_polled(static_cast<const uint8_t*>(x->data_ptr()), n, ip->data_ptr(), it == at::kLong ? 1 : 0, i32(nseg),
                                        capacity, little, y.data_ptr<uint8_t>(), bytes_indptr.data_ptr<int32_t>(),
-                                       total.data_ptr<int64_t>(), stream);
+                                       words.data_ptr<int64_t>(), kWords, stream);
   }
   if (rc != FO_OK) return PyLong_FromLong(rc);
-  const int64_t nbytes = *total.data_ptr<int64_t>();
+  const int64_t nbytes = *words.data_ptr<int64_t>();
   // (refused, or a copy pays: the Python code does the call again)
   if (nbytes < 0 || capacity - nbytes > (nbytes > (1 << 20) ? nbytes : (1 << 20))) NOT_HERE;
   PyObject* a = THPVariable_Wrap(y.narrow(0, 0, nbytes));
@@ -486,7 +487,7 @@ PyObject* bind(PyObject*, PyObject* arg) {
   get(a.gemm_q_prepared, "fo_gemm_q_prepared");
   get(a.gemm_o_prepared, "fo_gemm_o_prepared");
   get(a.gemm_workspace_bytes, "fo_gemm_workspace_bytes");
-  get(a.segment_packbits_early, "fo_segment_packbits_early");
+  get(a.segment_packbits_polled, "fo_segment_packbits_polled");
   get(a.select_blocks_uniform, "fo_select_blocks_uniform");
   get(a.select_scratch_bytes, "fo_select_blocks_scratch_bytes");
   get(a.layer_lists, "fo_layer_lists");

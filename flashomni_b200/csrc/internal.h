@@ -89,9 +89,11 @@ cudaError_t launch_packbits(const uint8_t* x, int64_t n, int little, uint8_t* y,
 cudaError_t launch_segment_packbits(const uint8_t* x, const int32_t* indptr, const int32_t* new_indptr,
                                     int num_segments, int64_t out_bytes, int little, uint8_t* y,
                                     cudaStream_t stream);
+int segment_packbits_sized_blocks(int64_t capacity);
+// every_block: each block writes the total to its own word when it is done (else block 0 to words[0])
 cudaError_t launch_segment_packbits_sized(const uint8_t* x, int64_t n, const void* indptr, int indptr_is_64, int num_segments,
-                                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, long long* total_out,
-                                          cudaStream_t stream);
+                                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, long long* words,
+                                          int every_block, cudaStream_t stream);
 cudaError_t launch_attn_compact(const CompactArgs& a, cudaStream_t stream);
 
 struct UnitArgs {

@@ -138,15 +138,16 @@ cudaError_t launch_segment_packbits(const uint8_t* x, const int32_t* indptr, con
 // The same without a byte indptr in hand: every CTA derives it from the element indptr (a few segments: one scan in shared
 // memory) and packs its share; CTA 0 also writes the byte indptr and, to host memory that the device can write, the
 // total (-1: an indptr that decreases or leaves the n values of x, nothing is packed). What bounds the step is the
-// caller's wait for that total, so it is written first, and a caller who only needs it polls for it instead of waiting for the
-// stream (fo_segment_packbits_early): two calls for the masks of 2 x 36 q-blocks x 24 heads 33.9 -> 24.8 us on a B200 (ten
-// launches and a copy in place of this kernel: 191.5 us).
+// caller's wait. With at most one CTA per SM each reports to a word of its own when its bytes are written, and the caller polls
+// these words instead of waiting for the stream: two calls for the masks of 2 x 36 q-blocks x 24 heads 33.3 -> 31.2 us on a
+// B200, of 604 q-blocks x 40 heads 38.2 -> 36.0 (ten launches and a copy in place of this kernel: 191.5 us). Returning when
+// CTA 0 knows the total would take 24.8, but the caller's other streams would then read bytes that are still being written.
 constexpr int kPackSegs = 1024;
 template <typename Idx>
 __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8_t* __restrict__ x, int64_t n,
                                                                      const Idx* __restrict__ indptr, int num_segments, int64_t capacity, int little,
                                                                      uint8_t* __restrict__ y, int32_t* __restrict__ new_indptr,
-                                                                     long long* __restrict__ total_out) {
+                                                                     long long* __restrict__ words, int every_block) {
   __shared__ int64_t s_in[kPackSegs + 1];
   __shared__ int32_t s_new[kPackSegs + 1];
   __shared__ int s_bad;
@@ -174,17 +175,12 @@ __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8
     if (tid == 0) {
       s_new[0] = 0;
       s_bad = bad ? 1 : 0;
-      if (blockIdx.x == 0) {  // the host may be polling for it
-        *static_cast<volatile long long*>(total_out) = bad ? -1ll : static_cast<long long>(carry);
-        __threadfence_system();
-      }
     }
   }
   __syncthreads();
-  if (s_bad) return;
-  if (blockIdx.x == 0)
+  const int64_t out_bytes = s_bad ? 0 : s_new[num_segments];
+  if (blockIdx.x == 0 && !s_bad)
     for (int i = tid; i <= num_segments; i += 256) new_indptr[i] = s_new[i];
-  const int64_t out_bytes = s_new[num_segments];
   const int64_t nwords = (out_bytes + 3) >> 2;
   const bool y4 = (reinterpret_cast<uintptr_t>(y) & 3u) == 0;
   for (int64_t w = blockIdx.x * 256ll + tid; w < nwords; w += static_cast<int64_t>(gridDim.x) * 256) {
@@ -204,21 +200,29 @@ __global__ void __launch_bounds__(256) segment_packbits_sized_kernel(const uint8
       y[i] = static_cast<uint8_t>(pack8(x + src, avail, little != 0, aligned));
     }
   }
+  __syncthreads();
+  if (tid == 0 && (every_block || blockIdx.x == 0)) {  // the host may be polling: what this block has written comes first
+    __threadfence_system();
+    static_cast<volatile long long*>(words)[blockIdx.x] = s_bad ? -1ll : static_cast<long long>(out_bytes);
+  }
+}
+
+int segment_packbits_sized_blocks(int64_t capacity) {
+  const int64_t blocks = ((capacity >> 2) + 255) / 256;
+  return blocks > 148 * 8 ? 148 * 8 : (blocks < 1 ? 1 : static_cast<int>(blocks));
 }
 
 cudaError_t launch_segment_packbits_sized(const uint8_t* x, int64_t n, const void* indptr, int indptr_is_64, int num_segments,
-                                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, long long* total_out,
-                                          cudaStream_t stream) {
+                                          int64_t capacity, int little, uint8_t* y, int32_t* new_indptr, long long* words,
+                                          int every_block, cudaStream_t stream) {
   if (num_segments > kPackSegs) return cudaErrorInvalidValue;
-  int64_t blocks = ((capacity >> 2) + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  if (blocks < 1) blocks = 1;
+  const int blocks = segment_packbits_sized_blocks(capacity);
   if (indptr_is_64)
-    segment_packbits_sized_kernel<int64_t><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        x, n, static_cast<const int64_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
+    segment_packbits_sized_kernel<int64_t><<<blocks, 256, 0, stream>>>(x, n, static_cast<const int64_t*>(indptr), num_segments, capacity, little,
+                                                                      y, new_indptr, words, every_block);
   else
-    segment_packbits_sized_kernel<int32_t><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        x, n, static_cast<const int32_t*>(indptr), num_segments, capacity, little, y, new_indptr, total_out);
+    segment_packbits_sized_kernel<int32_t><<<blocks, 256, 0, stream>>>(x, n, static_cast<const int32_t*>(indptr), num_segments, capacity, little,
+                                                                      y, new_indptr, words, every_block);
   return cudaGetLastError();
 }
 

@@ -42,7 +42,7 @@ def packbits(x: torch.Tensor, bitorder: str = "big") -> torch.Tensor:
 def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big") -> Tuple[torch.Tensor, torch.Tensor]:
     """Packs each segment x[indptr[i]:indptr[i+1]] separately; returns (y, new_indptr) with
     new_indptr[i+1]-new_indptr[i] == ceil(len_i/8) (reference: flashomni/quantization.py:102-159,
-    including its one wait of the host, for the size of the output; the bytes themselves are complete in stream order)."""
+    including its one wait of the host, which here is for the packed bytes as well as for their number)."""
     little = _little(bitorder)
     # the usual call in one native function; it returns None for anything else
     r = _native.host().segment_packbits(x, indptr, little)
@@ -62,13 +62,13 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
         capacity = (xb.numel() + 7 * n_seg) // 8
         y = torch.empty(capacity, dtype=torch.uint8, device=device)
         indptr_new = torch.empty(n_seg + 1, dtype=torch.int32, device=device)
-        total = torch.empty(1, dtype=torch.int64, pin_memory=True)
+        words = torch.empty(_native.PACK_WORDS, dtype=torch.int64, pin_memory=True)
         with torch.cuda.device(device):
-            rc = _native.load().fo_segment_packbits_early(
+            rc = _native.load().fo_segment_packbits_polled(
                 xb.data_ptr(), xb.numel(), ip.data_ptr(), int(ip.dtype == torch.int64), n_seg, capacity, little, y.data_ptr(),
-                indptr_new.data_ptr(), total.data_ptr(), _native.current_stream(device))
+                indptr_new.data_ptr(), words.data_ptr(), words.numel(), _native.current_stream(device))
         _native.check(rc, "segment_packbits")
-        nbytes = int(total[0])
+        nbytes = int(words[0])
         if nbytes >= 0:
             y = y.narrow(0, 0, nbytes)
             # segments that cover little of x: the result does not keep the rest of the allocation alive (below a megabyte,

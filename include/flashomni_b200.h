@@ -85,11 +85,12 @@ FO_API int fo_segment_packbits_sized(const uint8_t* x, const void* indptr, int32
 FO_API int fo_segment_packbits_within(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64,
                                       int32_t num_segments, int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
                                       int64_t* total_bytes, void* stream);
-/* The same, but it returns as soon as total_bytes is known: y and new_indptr are complete in stream order, like the results of
- * every other op. */
-FO_API int fo_segment_packbits_early(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64,
-                                     int32_t num_segments, int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
-                                     int64_t* total_bytes, void* stream);
+/* The same without a wait for the stream where the launch has at most num_words blocks: every block writes the total to its
+ * own one of num_words >= 1 words of pinned host memory when its part of y is complete, and the call returns when all of them
+ * have; words[0] is total_bytes. y and new_indptr are complete on return, as above. */
+FO_API int fo_segment_packbits_polled(const uint8_t* x, int64_t n, const void* indptr, int32_t indptr_is_64,
+                                      int32_t num_segments, int64_t capacity, int little, uint8_t* y, int32_t* new_indptr,
+                                      int64_t* words, int32_t num_words, void* stream);
 
 /* ---- attention mask compaction (new step; no counterpart op in the reference, which re-reads
  * the bits in the kernel: prefill.cuh:1284-1294,1380-1460) -------------------------------------

@@ -460,3 +460,54 @@ def test_attention_work_units_bit_exact(cuda_device, case, monkeypatch):
     if case == "few_items_cut":
         assert slots > 0
     assert got["n_units"] <= w._max_units and slots <= w._partial_slots
+
+
+@pytest.mark.parametrize("n", [3000, 147 * 8192, 149 * 8192, 40_000_000])
+def test_packed_bytes_are_complete_on_return(cuda_device, n):
+    """Whatever reads them next, on any stream: here a stream that is not ordered behind the packing, which itself waits behind
+    other work. One block, a block short of and past one per SM (the words that are polled), more than eight per SM."""
+    side = torch.cuda.Stream(cuda_device)
+    a = torch.randn(4096, 4096, device=cuda_device)
+    for seed in range(3):
+        x = torch.from_numpy(np.random.default_rng(seed).random(n) < 0.5).to(cuda_device)
+        ip = torch.tensor([0, 5, n // 2, n], dtype=torch.int32, device=cuda_device)
+        a @ a
+        y, new = fo.segment_packbits(x, ip, "little")
+        x.zero_()   # (in stream order behind the packing)
+        with torch.cuda.stream(side):
+            y, new = y.clone(), new.clone()
+        side.synchronize()
+        want = np.random.default_rng(seed).random(n) < 0.5
+        want = np.concatenate([np.packbits(want[i:j], bitorder="little") for i, j in ((0, 5), (5, n // 2), (n // 2, n))])
+        assert np.array_equal(y.cpu().numpy(), want) and int(new[-1]) == len(want)
+
+
+def test_lists_on_a_side_stream_are_built_from_masks_packed_after_the_event(cuda_device):
+    """`prepare_masks(stream=, after=)` is ordered behind that event alone, and a GEMM list in storage of its own behind nothing:
+    masks packed since then must be complete."""
+    B, S, H, D = 2, 1024, 8, 128
+    nb = S // 128
+    side = torch.cuda.Stream(cuda_device)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device))
+    ip = torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * S
+    w.plan(ip, ip, H, H, D, q_data_type=torch.bfloat16)
+    q, k, v = (torch.randn(B * S, H, D, device=cuda_device).bfloat16() for _ in range(3))
+    x, wq = torch.randn(B, S, 256, device=cuda_device).bfloat16(), torch.randn(H * D, 256, device=cuda_device).bfloat16()
+    busy = torch.randn(4096, 4096, device=cuda_device)
+    wl_q = None
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        qa, kk = (torch.from_numpy(rng.random(s) < 0.5).to(cuda_device) for s in ((B, nb, H), (B, nb, H, nb)))
+        qi, ki = (torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * t[0].numel() for t in (qa, kk))
+        after = torch.cuda.Event()
+        after.record()
+        busy @ busy
+        si, sp = fo.segment_packbits(qa.view(-1), qi, "little")
+        sk, kp = fo.segment_packbits(kk.view(-1), ki, "little")
+        w.prepare_masks(si, sk, sp, kp, stream=side, after=after)
+        wl_q = fo.gemm.prepare_gemm_q_list(B, S, H * D, H, si, sp, 0, into=wl_q, stream=side)
+        o = w.run(q, k, v, si, sk, sp, kp, out=torch.zeros_like(q))
+        y = fo.flashomni_gemm(x, wq, H, si, sp, 0, out=torch.zeros(B, S, H * D, dtype=x.dtype, device=cuda_device), worklist=wl_q)
+        assert torch.equal(o, w.run(q, k, v, si, sk, sp, kp, out=torch.zeros_like(q)))
+        assert torch.equal(y, fo.flashomni_gemm(x, wq, H, si, sp, 0, out=torch.zeros_like(y)))
+        w.check_status()
