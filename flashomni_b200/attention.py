@@ -427,7 +427,8 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         """q [qo_indptr[-1], H, D]; k, v [kv_indptr[-1], H, D] (NHD) or [H, kv_indptr[-1], D] (HND).
         `sparse_info` / `sparse_kv_info` are the packed uint8 masks and their *byte* indptrs as returned
         by `segment_packbits(..., bitorder="little")`. q-blocks whose bit is 0 keep the contents of `out`
-        (zeros when `out` is allocated here). Reference: flashomni/attention.py:709-835."""
+        (zeros when `out` is allocated here), and so do their rows of `lse` (float32 [qo_indptr[-1], H], any strides).
+        Reference: flashomni/attention.py:709-835."""
         if not self._planned:
             raise RuntimeError("plan() must be called before run()")
         if self._fast_plan is not None and self._fast_args is self._list_args:
@@ -456,11 +457,16 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             sm_scale = 1.0 / math.sqrt(q.size(-1))
         if q.dim() != 3 or q.size(0) != self._total_q or q.size(1) != self._num_qo_heads or q.size(2) != self._head_dim:
             raise ValueError(f"q has shape {tuple(q.shape)}, planned [{self._total_q}, {self._num_qo_heads}, {self._head_dim}]")
-        if return_lse:
-            if lse is None:
-                lse = torch.empty((q.size(0), q.size(1)), dtype=torch.float32, device=q.device)
-            else:
-                _check_shape_dtype_device(lse, (q.size(0), q.size(1)), torch.float32, q.device, "lse")
+        caller_lse = None
+        if lse is not None:
+            _check_shape_dtype_device(lse, (q.size(0), q.size(1)), torch.float32, q.device, "lse")
+            if not lse.is_contiguous():
+                # the kernels write rows of num_qo_heads values; rows of skipped q-blocks keep what the caller's tensor holds
+                if any(st == 0 and n > 1 for st, n in zip(lse.stride(), lse.shape)):
+                    raise ValueError("lse must not be an expanded tensor")
+                caller_lse, lse = lse, lse.contiguous()
+        elif return_lse:
+            lse = torch.empty((q.size(0), q.size(1)), dtype=torch.float32, device=q.device)
         fresh_out = out is None
         if not fresh_out:
             _check_shape_dtype_device(out, q.shape[:-1] + v.shape[-1:], q.dtype, q.device, "out")
@@ -531,6 +537,8 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             else:
                 rc = lib.fo_sparse_attn_fwd(*head, _native.ptr(ws["status"]), stream)
             _native.check(rc, "BatchFlashOmniFAWithRaggedKVWrapper.run")
+            if caller_lse is not None:
+                lse = caller_lse.copy_(lse)
         if _native.debug_checks():
             self.check_status()
         return (out, lse) if return_lse else out

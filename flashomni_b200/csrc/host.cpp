@@ -151,7 +151,7 @@ PyObject* attn_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (args[10] != Py_None) {
     lse_in = plain(args[10], dev);
     if (!return_lse || lse_in == nullptr || lse_in->scalar_type() != at::kFloat || lse_in->dim() != 2 ||
-        lse_in->size(0) != p->total_q || lse_in->size(1) != p->hq) NOT_HERE;
+        lse_in->size(0) != p->total_q || lse_in->size(1) != p->hq || !lse_in->is_contiguous()) NOT_HERE;
   }
   double scale = 0.0, cap = 0.0;
   if (args[12] == Py_None) scale = 1.0 / std::sqrt(static_cast<double>(q->size(2)));

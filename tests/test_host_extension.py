@@ -190,3 +190,28 @@ def test_packed_size_is_waited_for_whatever_is_queued(cuda_device, work_in_front
         y, new = fo.segment_packbits(torch.from_numpy(x).to(cuda_device), torch.tensor(ip, dtype=torch.int32, device=cuda_device), "little")
         want = np.concatenate([np.packbits(x[i:j], bitorder="little") for i, j in zip(ip, ip[1:])])
         assert np.array_equal(y.cpu().numpy(), want) and new.tolist() == [0, 2, 188, 376]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["columns", "transposed", "rows", "expanded"])
+def test_log_sum_exp_into_a_strided_buffer(cuda_device, monkeypatch, form):
+    """The values land where the caller's view says, nothing beside it changes, and an expanded view is refused."""
+    w, q, k, v, masks = _attn(cuda_device)
+    T, H = q.shape[:2]
+    want = torch.full((T, H), 3.0, device=cuda_device)
+    w.run(q, k, v, *masks, lse=want, return_lse=True)
+    buf = torch.full({"columns": (T, 2 * H), "transposed": (H, T), "rows": (2 * T, H), "expanded": (T, 1)}[form], 3.0, device=cuda_device)
+    view = {"columns": lambda b: b[:, 1:H + 1], "transposed": lambda b: b.t(), "rows": lambda b: b[::2], "expanded": lambda b: b.expand(T, H)}[form]
+    for return_lse in (True, False):
+        def call():
+            b = buf.clone()
+            r = w.run(q, k, v, *masks, lse=view(b), return_lse=return_lse)
+            return (b, *r) if return_lse else (b, r)
+        a, b = _both(monkeypatch, call)
+        assert _same(a, b)
+        if form == "expanded":
+            assert a[0] is ValueError
+            continue
+        full = buf.clone()
+        view(full).copy_(want)
+        assert torch.equal(a[0], full) and (not return_lse or torch.equal(a[2], want))
