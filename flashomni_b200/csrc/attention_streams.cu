@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       if (lane == 0) mbar_arrive(&tail->stats_free[ip]);
       const float m_out = fmaxf(m0, m1);
       // a stream without a visible column has m = -inf, l = 0
-      float w0 = (m0 == m_out) ? 1.f : ex2_approx(m0 - m_out), w1 = (m1 == m_out) ? 1.f : ex2_approx(m1 - m_out);
+      const float w_min = exp2_series(fminf(m0, m1) - m_out);
+      float w0 = (m0 == m_out) ? 1.f : w_min, w1 = (m1 == m_out) ? 1.f : w_min;
       const float l_out = fmaf(l0, w0, l1 * w1);
       const float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
       w0 *= inv_out;
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         if (ragged_j < 0) ragged_j += n;
       }
       float m_ref = -INFINITY;
-      uint64_t l2a = 0, l2b = 0;
+      float l_sum = 0.f;
       const int j0 = static_cast<int>((g ^ X) & 1u);
 #pragma unroll 1
       for (int j = j0; j < n; j += 2) {
@@ -636,9 +637,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         } else if (need) {
           m_ref = m_new;
           alpha = ex2_approx(m_prev - m_new);
-          const uint64_t alpha2 = pack_f32x2(alpha, alpha);
-          l2a = ffma2(l2a, alpha2, 0ull);
-          l2b = ffma2(l2b, alpha2, 0ull);
+          l_sum *= alpha;
         }
         const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
         const uint64_t negm2 = pack_f32x2(neg_m, neg_m);
@@ -665,7 +664,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
           if (lane == 0) mbar_arrive(bar);
         };
         // The sum and the conversion of a pair follow its exponentials by kLag pairs: between two volatile TMEM stores
-        // nothing then waits for the last exponential in front of it.
+        // nothing then waits for the last exponential in front of it. A block is summed up for itself: added one by one to the
+        // sum of all blocks, small values fall below its last bit (log-sum-exp of 9216 tokens, logits N(0, 4^2): rms error
+        // against 64 bits 4.0e-6, here 2.3e-6, at the same time; with four accumulators 2.2e-6, and 1.5 % slower).
+        uint64_t l2[2];
 #pragma unroll
         for (int t = 0; t < 64 + kLag; ++t) {
           if (t < 64) {
@@ -678,7 +680,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
           if (t >= kLag) {
             const int e = t - kLag;
             const float p0 = __uint_as_float(s[2 * e]), p1 = __uint_as_float(s[2 * e + 1]);
-            if (e & 1) l2b = fadd2(l2b, pack_f32x2(p0, p1)); else l2a = fadd2(l2a, pack_f32x2(p0, p1));
+            const uint64_t p2 = pack_f32x2(p0, p1);
+            l2[e & 1] = e < 2 ? p2 : fadd2(l2[e & 1], p2);
             s[e] = kBf16 ? pack_bf16x2(p0, p1) : pack_f16x2(p0, p1);   // (entry e of s is free by now)
             if ((e & 15) == 15) {   // P over S: this thread has its whole row in registers
               tmem_st_x16(tmem_s + static_cast<uint32_t>(e - 15), s + e - 15);
@@ -688,17 +691,17 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
           }
         }
         hand_over(p_full);
+        float la, lb;
+        unpack_f32x2(fadd2(l2[0], l2[1]), la, lb);
+        l_sum += la + lb;
       }
       if (!ok) break;
       g += static_cast<uint32_t>(n);
       const uint32_t ip = item & 1u;
       // the statistics of the unit before the last one must have been read
       if (item >= 2u && !mbar_wait(&tail->stats_free[ip], ((item >> 1) - 1u) & 1u, abort_flag)) break;
-      float la, lb, lc, ld;
-      unpack_f32x2(l2a, la, lb);
-      unpack_f32x2(l2b, lc, ld);
       tail->stats_m[ip][X][row] = m_ref;
-      tail->stats_l[ip][X][row] = (la + lb) + (lc + ld);
+      tail->stats_l[ip][X][row] = l_sum;
       __syncwarp();
       if (lane == 0) mbar_arrive(&tail->stats_ready[ip]);
       ++item;

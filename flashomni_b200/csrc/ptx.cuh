@@ -483,6 +483,22 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 2^d for d <= 0 (0 below -126.5) with a relative error of at most 1.3 * 2^-24: 2^n times the Taylor series of
+// 2^f = exp(f ln 2), abs(f) <= 1/2, whose next term is 5e-9. For factors that scale whole sums, where the error of ex2.approx
+// would be the largest error (ex2.approx: 4 * 2^-24).
+__device__ __forceinline__ float exp2_series(float d) {
+  d = fmaxf(d, -127.f);
+  const float n = rintf(d), f = d - n;
+  float p = 1.5252734e-5f;                 // (ln 2)^7 / 7!
+  p = fmaf(p, f, 1.5403530e-4f);
+  p = fmaf(p, f, 1.3333558e-3f);
+  p = fmaf(p, f, 9.6181291e-3f);
+  p = fmaf(p, f, 5.5504109e-2f);
+  p = fmaf(p, f, 2.4022651e-1f);
+  p = fmaf(p, f, 6.9314718e-1f);
+  p = fmaf(p, f, 1.f);
+  return p * __int_as_float((static_cast<int>(n) + 127) << 23);
+}
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

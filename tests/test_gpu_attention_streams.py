@@ -134,3 +134,24 @@ def test_infinities_in_v_reach_the_output_as_infinities(cuda_device, kind, D, bl
     fin = torch.isfinite(ref)
     assert torch.equal(torch.isfinite(o), fin)
     assert_close_bf16(o[fin], ref[fin], f"{kind} D={D} blocks={blocks}", allow_ulp=1.0)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_small_weights_add_up_in_the_row_sum(cuda_device, dtype, D):
+    """One block of logits 0 and 71 blocks of logits -21, in base 2: 2^-21 is below the last bit of a sum that has reached 32, but
+    the 9 088 of them are 3.4e-5 of the whole. The log-sum-exp is known to a few units of its last place: log2 and
+    the sum with the maximum 2^-21 each at a magnitude below 8, the scaled logit 21 * 2^-23 times a weight of 3.4e-5."""
+    blocks, H = 72, 1
+    S = 128 * blocks
+    q, k, v = torch.zeros(S, H, D), torch.zeros(S, H, D), torch.ones(S, H, D)
+    q[:, :, 0] = 1.0
+    k[128:, :, 0] = -21.0
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device))
+    ip = torch.tensor([0, S], dtype=torch.int32, device=cuda_device)
+    w.plan(ip, ip, H, H, D, q_data_type=dtype, sm_scale=float(np.log(2.0)))
+    o, lse = w.run(*(dev(t.to(dtype), cuda_device) for t in (q, k, v)), is_full=True, return_lse=True)
+    w.check_status()
+    want = np.log2(128 + (S - 128) * 2.0 ** -21)
+    assert (lse.cpu().double() - want).abs().max() <= 2.0 ** -20
+    assert (o == 1).all()
