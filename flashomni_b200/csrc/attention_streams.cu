@@ -28,8 +28,9 @@
 //   P handed over after three quarters (a quarter) instead of half                                               109 / 263 (109 / 258)
 //   each stream with units of its own instead of alternate blocks of one unit                                    125 / 261
 // Other shapes, device time of a call from a graph, attention.cu -> here: one request of 4608 tokens with 12 heads 76 -> 68, at
-// density 0.2 67 -> 59; 64 requests of 128 tokens 60 -> 50, 32 of 256 60 -> 50, 8 of 1024 118 -> 108; only 64
-// requests of 77 tokens are slower, 55 -> 64 (one masked block and one partial store per unit).
+// density 0.2 67 -> 59; 32 requests of 256 tokens 60 -> 50, 8 of 1024 118 -> 108; 64 requests of 128 tokens 59.5 -> 50.9, of 100
+// 55.4 -> 48.4, of 77 50.8 -> 48.0, of 33 46.6 -> 44.3, of 20 46.0 -> 47.3. Rows of a slab that is not whole leave from the thread
+// that has them: staged like the others, four rows an instruction, 64 requests of 77 / 33 / 20 tokens took 55.8 / 53.8 / 50.5.
 //
 // Warps: 0-3 softmax stream 0, 4-7 softmax stream 1 (TMEM lane = q row), 8-11 epilogue, 12 TMA producer and drawer of
 // work-list positions, 13 and 14 MMA issuers, 15 writes the q-blocks without work.
@@ -483,17 +484,19 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       float w0 = (m0 == m_out) ? 1.f : w_min, w1 = (m1 == m_out) ? 1.f : w_min;
       const float l_out = fmaf(l0, w0, l1 * w1);
       const float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
-      w0 *= inv_out;
-      w1 *= inv_out;
-      // a unit of one block leaves the other stream's O as it was: whatever that is, it does not count
+      // A unit of one block leaves the other stream's O as it was, which may be anything: O of the stream with the block stands in
+      // for it, with a weight that rounds away beside w0 (at least 2^-40) and, unlike zero, leaves an infinity one.
       const bool has1 = u0.x > 1;
+      w0 *= inv_out;
+      w1 = has1 ? w1 * inv_out : 0x1p-126f;
       g += static_cast<uint32_t>(u0.x);
       if (!mbar_wait(&tail->o_full[f], (o_phase >> f) & 1u, abort_flag)) break;
       if (has1 && !mbar_wait(&tail->o_full[f ^ 1u], (o_phase >> (f ^ 1u)) & 1u, abort_flag)) break;
       o_phase ^= has1 ? 3u : 1u << f;
       tc_fence_after_sync();
-      const bool whole = q_valid * grp == kBQ;   // no row of the q-block is past the request
-      const uint32_t tmem_o0 = tmem_o + 128u * f, tmem_o1 = tmem_o + 128u * (f ^ 1u);
+      const int rows = q_valid * grp - quad * 32;   // rows of this warp that are not past the request: all from 32 on
+      const bool whole = rows >= 32;
+      const uint32_t tmem_o0 = tmem_o + 128u * f, tmem_o1 = has1 ? tmem_o + 128u * (f ^ 1u) : tmem_o0;
       const uint64_t w0p = pack_f32x2(w0, w0), w1p = pack_f32x2(w1, w1);
 #pragma unroll 1
       for (int half = 0; half < kHalves; ++half) {
@@ -503,12 +506,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         for (int c = 0; c < 4; ++c) {
           uint32_t v0[16], v1[16];
           tmem_ld_x16(tmem_o0 + 64u * half + 16u * c, v0);
-          if (has1) {
-            tmem_ld_x16(tmem_o1 + 64u * half + 16u * c, v1);
-          } else {  // an O that nothing wrote may hold anything, and no value times its weight of zero need be zero
-#pragma unroll
-            for (int t = 0; t < 16; ++t) v1[t] = 0u;
-          }
+          tmem_ld_x16(tmem_o1 + 64u * half + 16u * c, v1);
           tmem_wait_ld();
 #pragma unroll
           for (int t = 0; t < 8; ++t) {
@@ -527,31 +525,24 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
             if (has1) mbar_arrive(&tail->o_free[f ^ 1u]);
           }
         }
-        // Through a staging slab per warp (32 rows x 64 columns in the 128-byte swizzle pattern): a store instruction of
-        // a warp would otherwise write 32 scattered 16-byte pieces. Whole q-blocks leave by one TMA store per slab, the rows
-        // of a partial one with four rows per instruction.
-        if (lane == 0) tma_store_wait_read<0>();  // the slab is free once the store before has read it
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16)) = out[c];
         if (whole) {
+          // Through a staging slab per warp (32 rows x 64 columns in the 128-byte swizzle pattern) and one TMA store: a store
+          // instruction of a warp would write 32 scattered 16-byte pieces.
+          if (lane == 0) tma_store_wait_read<0>();  // the slab is free once the store before has read it
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16)) = out[c];
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             tma_store_3d(&a.tmap_o, stg, 64 * half, h * grp, q_row0 + row_tok0);
             tma_store_commit();
           }
-        } else {
-          __syncwarp();
-#pragma unroll 1
-          for (int r = lane >> 3; r < 32; r += 4) {
-            const int tr = quad * 32 + r;   // row of the tile
-            if (tr >= q_valid * grp) break;
-            const int64_t tok = static_cast<int64_t>(q_row0) + (tr >> grp_shift);
-            uint16_t* dst = reinterpret_cast<uint16_t*>(a.o) + tok * a.o_stride_n +
-                            static_cast<int64_t>(h * grp + (tr & (grp - 1))) * a.o_stride_h + 64 * half;
-            reinterpret_cast<uint4*>(dst)[lane & 7] = *reinterpret_cast<const uint4*>(stg + r * 128 + (((lane & 7) ^ (r & 7)) * 16));
-          }
+        } else if (row_ok) {  // rows past the request must not be written
+          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.o) + grow * a.o_stride_n +
+                                                static_cast<int64_t>(hq) * a.o_stride_h + 64 * half);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) dst[c] = out[c];
         }
       }
       ++item;
