@@ -34,7 +34,8 @@
 //
 // Warps: 0-3 softmax stream 0, 4-7 softmax stream 1 (TMEM lane = q row), 8-11 epilogue, 12 TMA producer and drawer of
 // work-list positions, 13 and 14 MMA issuers, 15 writes the q-blocks without work.
-// Every mbarrier wait is bounded.
+// Every mbarrier wait is bounded. A wait that runs out may do so for some lanes of a warp only: the softmax and epilogue warps go
+// on together to a vote and leave there, the former behind the block, the latter before anything is stored.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -55,7 +56,9 @@ constexpr int kWarpProducer = kWarpEpilogue + kEpilogueWarps;
 constexpr int kWarpMma = kWarpProducer + 1;
 constexpr int kWarpZero = kWarpMma + 2;
 constexpr int kThreads = (kWarpZero + 1) * 32;   // 512
-constexpr int kRegsSoftmax = 184, kRegsEpilogue = 88, kRegsOther = 56;  // setmaxnreg split
+// setmaxnreg split. 184 / 88 / 56 gave the epilogue too few: image layer 95.2 us instead of 94.5, 64 requests of 90 / 20 tokens 51.5 /
+// 47.8 instead of 47.5 / 43.9 (device time of a call from a graph).
+constexpr int kRegsSoftmax = 168, kRegsEpilogue = 120, kRegsOther = 56;
 // setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with: a split that asks for more
 // never returns.
 constexpr int kRegsAtLaunch = (65536 / kThreads) / 8 * 8;
@@ -139,7 +142,8 @@ struct ItemRead {  // the reading roles: one thread, or all lanes of a warp
   __device__ __forceinline__ void init(Tail* t, volatile int* ab) { tail = t; abort_flag = ab; k = 0; }
   __device__ __forceinline__ bool next(int4& u0, int4& u1) {  // false at the end
     const int slot = k % kItemQ;
-    if (!mbar_wait(&tail->iq_full[slot], static_cast<uint32_t>(k / kItemQ) & 1u, abort_flag)) return false;
+    const uint32_t phase = static_cast<uint32_t>(k / kItemQ) & 1u;
+    if (!(kWholeWarp ? mbar_wait_all(&tail->iq_full[slot], phase, abort_flag) : mbar_wait(&tail->iq_full[slot], phase, abort_flag))) return false;
     u0 = tail->item_q[slot][0];
     u1 = tail->item_q[slot][1];
     if (kWholeWarp) {
@@ -470,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       const int hq = h * grp + row_head;
       float* lse = a.lse != nullptr ? a.lse + grow * a.lse_stride_n + hq : nullptr;
       const uint32_t ip = item & 1u;
-      if (!mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag)) break;
+      bool got = mbar_wait(&tail->stats_ready[ip], (item >> 1) & 1u, abort_flag);
       // 0 and 1 are the streams of the unit's first and second block from here on: which of the two that is depends on the
       // units that this CTA drew before, the rounding of the sums must not
       const uint32_t f = g & 1u;
@@ -490,8 +494,9 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       w0 *= inv_out;
       w1 = has1 ? w1 * inv_out : 0x1p-126f;
       g += static_cast<uint32_t>(u0.x);
-      if (!mbar_wait(&tail->o_full[f], (o_phase >> f) & 1u, abort_flag)) break;
-      if (has1 && !mbar_wait(&tail->o_full[f ^ 1u], (o_phase >> (f ^ 1u)) & 1u, abort_flag)) break;
+      got = mbar_wait(&tail->o_full[f], (o_phase >> f) & 1u, abort_flag) && got;
+      if (has1) got = mbar_wait(&tail->o_full[f ^ 1u], (o_phase >> (f ^ 1u)) & 1u, abort_flag) && got;
+      if (!__all_sync(0xffffffffu, got)) break;
       o_phase ^= has1 ? 3u : 1u << f;
       tc_fence_after_sync();
       const int rows = q_valid * grp - quad * 32;   // rows of this warp that are not past the request: all from 32 on
@@ -581,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       const int j0 = static_cast<int>((g ^ X) & 1u);
 #pragma unroll 1
       for (int j = j0; j < n; j += 2) {
-        if (!mbar_wait(s_full, phase, abort_flag)) { ok = false; break; }
+        const bool got = mbar_wait(s_full, phase, abort_flag);
         phase ^= 1u;
         tc_fence_after_sync();
         uint32_t s[128];
@@ -685,12 +690,14 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         float la, lb;
         unpack_f32x2(fadd2(l2[0], l2[1]), la, lb);
         l_sum += la + lb;
+        ok = __all_sync(0xffffffffu, got);
+        if (!ok) break;
       }
       if (!ok) break;
       g += static_cast<uint32_t>(n);
       const uint32_t ip = item & 1u;
       // the statistics of the unit before the last one must have been read
-      if (item >= 2u && !mbar_wait(&tail->stats_free[ip], ((item >> 1) - 1u) & 1u, abort_flag)) break;
+      if (item >= 2u && !mbar_wait_all(&tail->stats_free[ip], ((item >> 1) - 1u) & 1u, abort_flag)) break;
       tail->stats_m[ip][X][row] = m_ref;
       tail->stats_l[ip][X][row] = l_sum;
       __syncwarp();

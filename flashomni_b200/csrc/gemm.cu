@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
         uint8_t* rowp = buf + r_in_tile * kSlabCols * 2;
         bool ok = true;
         if constexpr (kCache) {  // this thread's row of the slab
-          ok = __all_sync(0xffffffffu, mbar_wait(&tail->slab_full[slab_count % kSlabBufs], (slab_count / kSlabBufs) & 1u, abort_flag) ? 1 : 0) != 0;
+          ok = mbar_wait_all(&tail->slab_full[slab_count % kSlabBufs], (slab_count / kSlabBufs) & 1u, abort_flag);
 #pragma unroll
           for (int c = 0; c < kPieces; ++c) initv[c] = *reinterpret_cast<const uint4*>(rowp + ((static_cast<uint32_t>(c) ^ swz) << 4));
         }

@@ -131,7 +131,13 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, v
   }
 }
 
-// The same for a whole warp that goes on to warp-collective instructions (tcgen05.ld, __syncwarp): lane 0
+// The same for all lanes of a warp that goes on to warp-collective instructions: every lane waits (and sees what was written
+// before the arrivals), and the warp leaves with one outcome. All 32 lanes must call it.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
+}
+
+// Another one for a whole warp that goes on to warp-collective instructions (tcgen05.ld, __syncwarp): lane 0
 // waits and the outcome is broadcast, so that a wait that runs out never leaves the lanes of a warp on
 // different sides of it. All 32 lanes must call it.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
