@@ -423,6 +423,7 @@ int fo_attn_lists(const uint8_t* sparse_info, int64_t sparse_info_bytes, const u
 
 // ------------------------------------------------------------------------------------------ attention
 namespace {
+// `check_only`: the arguments are looked at, nothing is launched.
 int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float* lse, int32_t dtype,
                      int64_t total_q, int64_t total_kv, int32_t num_qo_heads, int32_t num_kv_heads,
                      int32_t head_dim, int64_t q_stride_n, int64_t q_stride_h, int64_t k_stride_n,
@@ -432,7 +433,7 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
                      float* partials, int64_t partial_slots, int32_t head_begin, float sm_scale,
                      float logits_soft_cap, int32_t mask_mode, const uint8_t* custom_mask, int64_t custom_mask_bytes,
                      const int32_t* mask_indptr, const int32_t* qo_indptr, const int32_t* kv_indptr, int32_t* status,
-                     void* stream, const int2* zero_rec = nullptr, const int32_t* zero_count = nullptr) {
+                     void* stream, const int2* zero_rec = nullptr, const int32_t* zero_count = nullptr, bool check_only = false) {
   if (mask_mode == 2 && (custom_mask == nullptr || mask_indptr == nullptr || qo_indptr == nullptr || kv_indptr == nullptr ||
                          custom_mask_bytes <= 0))
     return fail(FO_ERR_INVALID_ARG, "fo_sparse_attn_fwd_custom_mask: mask, its indptr and the request indptrs are required");
@@ -467,6 +468,7 @@ int sparse_attn_impl(const void* q, const void* k, const void* v, void* o, float
   const uint32_t group = static_cast<uint32_t>(num_qo_heads / num_kv_heads);
   if (group > 16 || (16 % group) != 0)
     return fail(FO_ERR_UNSUPPORTED, "fo_sparse_attn_fwd: num_qo_heads / num_kv_heads must be 1, 2, 4, 8 or 16");
+  if (check_only) return FO_OK;
   AttnArgs a;
   memset(&a, 0, sizeof(a));
   a.head_dim = head_dim;
@@ -625,6 +627,23 @@ int fo_attn_run(const fo_attn_call* c, void* stream) {
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool cast = c->fp8_kind >= 0 && c->kv_values > 0;
   ZeroLater later = ZeroLater();
+  auto attention = [&](bool check_only) {
+    return sparse_attn_impl(c->q, cast ? c->k16 : c->k, cast ? c->v16 : c->v, c->o, c->lse, c->dtype, c->total_q, c->total_kv,
+                            c->num_qo_heads, c->num_kv_heads, c->head_dim, c->q_stride_n, c->q_stride_h, c->k_stride_n, c->k_stride_h,
+                            c->v_stride_n, c->v_stride_h, c->o_stride_n, c->o_stride_h, i32(7), i32(7), ptr(14), ptr(24), ptr(25), p[22],
+                            ptr(26), c->partials, p[23], i32(4), c->sm_scale, c->logits_soft_cap, 0, nullptr, 0, nullptr, nullptr,
+                            nullptr, c->status, stream, later.rec, later.count, check_only);
+  };
+  // everything is looked at before the first launch: a call that is refused leaves the output and the lists as they are
+  const int refused = attention(true);
+  if (refused != FO_OK) return refused;
+  if (cast && (c->k == nullptr || c->v == nullptr || c->k16 == nullptr || c->v16 == nullptr || !aligned16(c->k) || !aligned16(c->v) ||
+               !aligned16(c->k16) || !aligned16(c->v16) || c->fp8_kind > 1))
+    return fail(FO_ERR_INVALID_ARG, "fo_attn_run: fp8 k / v and their copies must be aligned to 16 bytes, of kind 0 or 1");
+  if (c->zero_inactive && c->total_q > 0 &&
+      (c->o == nullptr || !aligned16(c->o) || c->o_stride_h != c->head_dim ||
+       c->o_stride_n != static_cast<int64_t>(c->num_qo_heads) * c->head_dim))
+    return fail(FO_ERR_INVALID_ARG, "fo_attn_run: an output to zero must be contiguous and aligned to 16 bytes");
   bool cast_done = false;
   if (!c->lists_ready) {
     CompactArgs a;
@@ -647,8 +666,6 @@ int fo_attn_run(const fo_attn_call* c, void* stream) {
       memset(&probe, 0, sizeof(probe));
       probe.head_dim = c->head_dim;
       probe.partial_slots = static_cast<int>(p[23] > 0x7fffffffLL ? 0x7fffffffLL : p[23]);
-      if (z.out != nullptr && (!aligned16(c->o) || c->o_stride_n % 8 != 0 || c->o_stride_n <= 0))
-        return fail(FO_ERR_INVALID_ARG, "fo_attn_run: an output to zero must be aligned to 16 bytes");
       if (z.out != nullptr && !c->is_full && attention_streams_applies(probe) && c->total_q > 0 && c->total_kv > 0) {
         later.rec = reinterpret_cast<int2*>(a.kv_off);
         later.count = a.hist;
@@ -659,9 +676,6 @@ int fo_attn_run(const fo_attn_call* c, void* stream) {
       }
       CastArgs ca = CastArgs();
       if (cast) {
-        if (c->k == nullptr || c->v == nullptr || c->k16 == nullptr || c->v16 == nullptr || !aligned16(c->k) || !aligned16(c->v) ||
-            !aligned16(c->k16) || !aligned16(c->v16) || c->fp8_kind > 1)
-          return fail(FO_ERR_INVALID_ARG, "fo_attn_run: fp8 k / v and their copies must be aligned to 16 bytes");
         ca.src[0] = static_cast<const uint8_t*>(c->k);
         ca.src[1] = static_cast<const uint8_t*>(c->v);
         ca.dst[0] = static_cast<uint16_t*>(c->k16);
@@ -690,11 +704,7 @@ int fo_attn_run(const fo_attn_call* c, void* stream) {
     const int rc = cast_fp8_impl("fo_attn_run", c->k, c->v, c->kv_values, c->fp8_kind, c->dtype, c->k16, c->v16, true, stream);
     if (rc != FO_OK) return rc;
   }
-  return sparse_attn_impl(c->q, cast ? c->k16 : c->k, cast ? c->v16 : c->v, c->o, c->lse, c->dtype, c->total_q, c->total_kv,
-                          c->num_qo_heads, c->num_kv_heads, c->head_dim, c->q_stride_n, c->q_stride_h, c->k_stride_n, c->k_stride_h,
-                          c->v_stride_n, c->v_stride_h, c->o_stride_n, c->o_stride_h, i32(7), i32(7), ptr(14), ptr(24), ptr(25), p[22],
-                          ptr(26), c->partials, p[23], i32(4), c->sm_scale, c->logits_soft_cap, 0, nullptr, 0, nullptr, nullptr,
-                          nullptr, c->status, stream, later.rec, later.count);
+  return attention(false);
 }
 
 // ------------------------------------------------------------------------------------------ GEMMs

@@ -254,7 +254,8 @@ FO_API int fo_cast_fp8_pair(const void* src0, const void* src1, int64_t n, int32
  * fo_attn_lists (unless lists_ready), fo_cast_fp8_pair (fp8_kind >= 0: k and v hold kv_values 8-bit values each and are cast to
  * k16 and v16, whose strides are k_stride_* and v_stride_*) and fo_sparse_attn_fwd (with logits_soft_cap > 0: _softcap) in
  * one call, with the lists and the cast in one launch for small masks. zero_inactive: rows of q-blocks that are not computed
- * are zeroed in o, which is then contiguous. `plan` is the array of fo_layer_lists. */
+ * are zeroed in o, which must then be contiguous. `plan` is the array of fo_layer_lists. A call whose arguments are refused
+ * launches nothing. */
 typedef struct fo_attn_call {
   const int64_t* plan;
   const uint8_t* sparse_info;

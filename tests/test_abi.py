@@ -51,3 +51,39 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_native, "_lib", None)
     with pytest.raises(RuntimeError, match="native library not found"):
         _native.load()
+
+
+class _AttnCall(ctypes.Structure):   # fo_attn_call
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("plan", "sparse_info", "sparse_kv_info")]
+                + [(n, ctypes.c_int64) for n in ("sparse_info_bytes", "sparse_kv_info_bytes")]
+                + [(n, ctypes.c_void_p) for n in ("sparse_info_indptr", "sparse_kv_info_indptr")]
+                + [(n, ctypes.c_int32) for n in ("is_full", "lists_ready", "zero_inactive", "dtype")]
+                + [(n, ctypes.c_void_p) for n in ("q", "k", "v", "o", "lse")]
+                + [(n, ctypes.c_int64) for n in ("total_q", "total_kv")]
+                + [(n, ctypes.c_int32) for n in ("num_qo_heads", "num_kv_heads", "head_dim", "fp8_kind")]
+                + [(n, ctypes.c_int64) for n in ("q_stride_n", "q_stride_h", "k_stride_n", "k_stride_h", "v_stride_n", "v_stride_h",
+                                                 "o_stride_n", "o_stride_h")]
+                + [(n, ctypes.c_void_p) for n in ("k16", "v16")] + [("kv_values", ctypes.c_int64), ("partials", ctypes.c_void_p)]
+                + [(n, ctypes.c_float) for n in ("sm_scale", "logits_soft_cap")] + [("status", ctypes.c_void_p)])
+
+
+@pytest.mark.parametrize("small", [True, False])
+@pytest.mark.parametrize("bad", [
+    dict(num_kv_heads=0), dict(num_kv_heads=-1), dict(num_kv_heads=3), dict(dtype=7), dict(head_dim=96), dict(sm_scale=0.0), dict(logits_soft_cap=-1.0),
+    dict(q=None), dict(q=0x1008), dict(status=None), dict(q_stride_n=4), dict(k_stride_h=0), dict(o_stride_n=1024), dict(o_stride_h=256),
+    dict(o=0x1008), dict(fp8_kind=2), dict(fp8_kind=0, k16=None), dict(fp8_kind=0, k=0x1004), dict(fp8_kind=1, v16=0x1008)])
+def test_attention_call_is_refused_before_anything_is_launched(bad, small):
+    """On a machine without a GPU a launch is an error of CUDA, so an argument error says that none was tried (and num_kv_heads = 0
+    divides nothing). Nothing is read or written behind the pointers, small numbers that only have to be aligned."""
+    n_cand, P = 4 if small else 40000, 0x1000
+    plan = (ctypes.c_int64 * 27)(P, P, 1, 4, 0, 4, 128, 128, n_cand, 1, n_cand, n_cand, P, P, P, P, P, P, 1 << 30, 148, 1, 16, n_cand, 0, P, P, P)
+    c = _AttnCall(plan=ctypes.addressof(plan), sparse_info=P, sparse_kv_info=P, sparse_info_bytes=1, sparse_kv_info_bytes=1, sparse_info_indptr=P,
+                  sparse_kv_info_indptr=P, zero_inactive=1, dtype=1, q=P, k=P, v=P, o=P, total_q=128, total_kv=128, num_qo_heads=4, num_kv_heads=4,
+                  head_dim=128, fp8_kind=-1, q_stride_n=512, q_stride_h=128, k_stride_n=512, k_stride_h=128, v_stride_n=512, v_stride_h=128,
+                  o_stride_n=512, o_stride_h=128, k16=P, v16=P, kv_values=65536, sm_scale=1.0, status=P)
+    for k, v in bad.items():
+        setattr(c, k, v)
+    lib = _native.load()
+    before = lib.fo_launch_count()
+    assert lib.fo_attn_run(ctypes.byref(c), None) in (_native.FO_ERR_INVALID_ARG, _native.FO_ERR_UNSUPPORTED)
+    assert lib.fo_launch_count() == before
