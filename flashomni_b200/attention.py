@@ -124,6 +124,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         self._side_stream = None
         self._prepared_event = None
         self._prepared_key = None
+        self._prepared_in_capture = False
         self._fast_plan = self._fast_args = None
 
     @property
@@ -370,6 +371,9 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if buf is None or buf.numel() * buf.element_size() < need or buf.device != self.device:
             buf = torch.zeros(need, dtype=torch.uint8, device=self.device)
             self._int_workspace_buffer = buf
+        # lists prepared under an earlier plan are not those of this one, and may still be on their way into this buffer
+        self._after_prepared(torch.cuda.current_stream(self.device))
+        self._prepared_key = None
         words = buf.view(torch.uint8)[: need].view(torch.int32)
         words[offs["counters"]: offs["counters"] + 12].zero_()  # counters, status / cursor words start from zero
         words[offs["arrive"]: offs["arrive"] + max(self._partial_slots, 1)].zero_()
@@ -438,6 +442,8 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 if self._prepared_key == self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr,
                                                         sparse_kv_info_indptr, is_full):
                     prepared = self._prepared_event
+                else:
+                    self._after_prepared(torch.cuda.current_stream(self.device))
             r = _native.host().attn_run(self._fast_plan, q, k, v, sparse_info, sparse_kv_info, sparse_info_indptr,
                                         sparse_kv_info_indptr, is_full, out, lse, return_lse, self._sm_scale,
                                         self._logits_soft_cap, prepared)
@@ -513,6 +519,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 # the lists were built by prepare_masks() on the side stream: just order after it
                 torch.cuda.current_stream(self.device).wait_event(self._prepared_event)
             else:
+                self._after_prepared(torch.cuda.current_stream(self.device))
                 self._compact(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full, stream,
                               zero_out)
             self._prepared_key = None
@@ -553,6 +560,12 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         return tuple((t.data_ptr(), t._version) for t in (sparse_info, sparse_kv_info, sparse_info_indptr,
                                                           sparse_kv_info_indptr))
 
+    def _after_prepared(self, stream) -> None:
+        """Orders `stream`, which is about to rebuild the lists, behind a prepare_masks() whose lists no run() has taken: it may
+        still be writing them. (Not from a capture into a stream outside of it or the other way round.)"""
+        if self._prepared_key is not None and self._prepared_in_capture == torch.cuda.is_current_stream_capturing():
+            stream.wait_event(self._prepared_event)
+
     def _check_masks(self, sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr) -> None:
         # the reference dereferences null masks (csrc/batch_sparseFA.cu:123-131); raise instead
         if sparse_info is None or sparse_kv_info is None or sparse_info_indptr is None \
@@ -588,6 +601,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if not self._planned:
             raise RuntimeError("plan() must be called before build_work_lists()")
         with torch.cuda.device(self.device):
+            self._after_prepared(torch.cuda.current_stream(self.device))
             self._compact(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full,
                           _native.current_stream(self.device))
         self._prepared_key = None
@@ -620,9 +634,11 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
                 side.wait_event(after)
             else:
                 side.wait_stream(torch.cuda.current_stream(self.device))
+            self._after_prepared(side)
             self._compact(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, is_full,
                           side.cuda_stream)
             self._prepared_event.record(side)
+            self._prepared_in_capture = torch.cuda.is_current_stream_capturing()
         self._prepared_key = self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr,
                                             is_full)
 
@@ -658,12 +674,14 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             if self._prepared_event is None:
                 self._prepared_event = torch.cuda.Event()
             stream.wait_event(after)
+            self._after_prepared(stream)
             rc = _native.load().fo_layer_lists(
                 p(sparse_info), sparse_info.numel(), p(sparse_kv_info), sparse_kv_info.numel(), p(sparse_info_indptr),
                 p(sparse_kv_info_indptr), self._layer_plan, m, n_local, self._head_dim, 0, p(q_list.ws), q_list.ws.numel(),
                 p(o_list.ws), o_list.ws.numel(), stream.cuda_stream)
             _native.check(rc, "prepare_layer_lists")
             self._prepared_event.record(stream)
+            self._prepared_in_capture = torch.cuda.is_current_stream_capturing()
         q_list.event = o_list.event = self._prepared_event
         self._prepared_key = self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr, sparse_kv_info_indptr, False)
 

@@ -758,3 +758,32 @@ def test_split_rule_follows_the_planned_shape(cuda_device, monkeypatch):
     assert few._partial_slots > 0 and few._max_units == few._n_cand + streams
     assert many._partial_slots == 0 and many._max_units == many._n_cand and many._partials is None
     assert one_per_sm._partial_slots == 0
+
+
+def test_prepared_lists_that_no_run_takes(cuda_device):
+    """Other masks, or another plan, while the preparation is still waiting or at work on its stream: the lists are built again,
+    behind it."""
+    H, S = 4, 1024
+    a, b = (wl.attention_inputs(1, H, S, 128, d, seed=s) for d, s in ((0.5, 91), (0.3, 92)))
+    w, fresh = (_wrapper(cuda_device, a.qo_indptr, a.kv_indptr, H) for _ in range(2))
+    ma, mb = masks_to_device(a.masks, cuda_device), masks_to_device(b.masks, cuda_device)
+    q, k, v = (dev(t, cuda_device) for t in (a.q, a.k, a.v))
+    busy = torch.randn(4096, 4096, device=cuda_device)
+    side = torch.cuda.Stream(cuda_device)
+    want = fresh.run(q, k, v, *mb).clone()
+    for other in ("masks", "lists", "preparation", "plan"):
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                busy @ busy
+        w.prepare_masks(*ma, stream=side)
+        if other == "lists":
+            w.build_work_lists(*mb)
+        elif other == "preparation":
+            w.prepare_masks(*mb)
+        elif other == "plan":
+            ip = dev(np.asarray([0, S], np.int32), cuda_device)
+            w.plan(ip, ip, H, H, 128, q_data_type=q.dtype)
+            assert w._prepared_key is None
+        assert torch.equal(w.run(q, k, v, *mb), want), other
+        w.check_status()
+        torch.cuda.synchronize()

@@ -68,3 +68,40 @@ def test_dense_gemm_tile_choice_fills_whole_waves():
     assert q(1, 128, 256, 64) == 128              # a single row block
     assert q(2, 4608, 3072, 3072, full=1) == 128  # a full-tensor init is the other kernel's
     assert q(0, 4608, 3072, 3072) == 0
+
+
+@pytest.mark.parametrize("captured,capturing,waits", [(False, False, True), (True, True, True), (True, False, False), (False, True, False)])
+def test_lists_are_not_rebuilt_beside_a_preparation_that_nobody_took(monkeypatch, captured, capturing, waits):
+    """run() with other masks than the prepared ones orders its stream behind the preparation, which may still write the lists
+    (unless one of the two is recorded in a capture and the other is not); a new plan() drops the prepared lists."""
+    from flashomni_b200 import _native
+    from flashomni_b200.attention import BatchFlashOmniFAWithRaggedKVWrapper as W
+    waited = []
+
+    class Stream:
+        def wait_event(self, e):
+            waited.append(e)
+
+    class Host:
+        @staticmethod
+        def attn_run(*args):
+            return ("done", args[-1])
+
+    w = W.__new__(W)
+    w._planned, w._fast_plan, w.device = True, object(), torch.device("cpu")
+    w._list_args = w._fast_args = ()
+    w._sm_scale = w._logits_soft_cap = None
+    w._prepared_event, w._prepared_in_capture = "event", captured
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    monkeypatch.setattr(_native, "host", lambda: Host)
+    masks = [torch.zeros(4, dtype=torch.uint8), torch.zeros(4, dtype=torch.uint8), torch.zeros(2, dtype=torch.int32),
+             torch.zeros(2, dtype=torch.int32)]
+    q = torch.zeros(1)
+    w._prepared_key = W._mask_key(*masks, False)
+    assert w.run(q, q, q, *masks) == ("done", "event") and waited == []    # the prepared masks: the native call waits
+    w._prepared_key = W._mask_key(*masks, False)
+    masks[0].fill_(1)
+    assert w.run(q, q, q, *masks) == ("done", None) and waited == ["event"] * waits
+    assert w._prepared_key is None
+    assert w.run(q, q, q, *masks) == ("done", None) and waited == ["event"] * waits
