@@ -129,25 +129,47 @@ def load():
     return lib
 
 
+def host_abi() -> str:
+    """What the Python extension's binary interface depends on."""
+    import sysconfig
+    import torch
+    return f"torch {torch.__version__} {sysconfig.get_config_var('SOABI')}"
+
+
+class _NoHost:
+    """In place of the extension: every function leaves the call to the Python code."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def _load_host(lib) -> None:
     global _host
-    if _host is None:
-        import importlib.machinery
-        import importlib.util
+    try:
         if not os.path.exists(_HOST):
-            raise RuntimeError(f"flashomni_b200: Python extension not found at {_HOST}; build it with "
-                               "`python -m flashomni_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_fo_host", _HOST)
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fo_host", loader))
-        loader.exec_module(module)
+            raise ImportError("not built")
+        if _host is None or isinstance(_host, _NoHost):
+            import importlib.machinery
+            import importlib.util
+            loader = importlib.machinery.ExtensionFileLoader("_fo_host", _HOST)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fo_host", loader))
+            loader.exec_module(module)
+        else:
+            module = _host
+        if module.abi() != host_abi():
+            raise ImportError(f"built for {module.abi()}, this is {host_abi()}")
         module.bind(lib._handle)
         _host = module
-    else:
-        _host.bind(lib._handle)
+    except (ImportError, AttributeError, OSError, RuntimeError) as e:
+        import warnings
+        warnings.warn(f"flashomni_b200: {_HOST} is not used ({e}); calls take longer on the host. Build it with "
+                      "`python -m flashomni_b200.build`", RuntimeWarning, stacklevel=3)
+        _host = _NoHost()
 
 
 def host():
-    """The extension of csrc/host.cpp: functions that do a whole call of an op, or return None for what they do not take."""
+    """The extension of csrc/host.cpp: functions that do a whole call of an op, or return None for what they do not take (all
+    of them do where it could not be loaded)."""
     if _lib is None:
         load()
     return _host

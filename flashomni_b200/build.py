@@ -16,6 +16,8 @@ import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
 
+from . import _native
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
@@ -31,6 +33,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 
 HOST_SRC = os.path.join(CSRC, "host.cpp")
 HOST_LIB = os.path.join(LIBDIR, "_fo_host.so")
+HOST_STAMP = os.path.join(OBJDIR, "_fo_host.stamp")   # the command it was built with
 
 
 def _host_cmd():
@@ -39,10 +42,26 @@ def _host_cmd():
     t = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(NVCC))
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f'-DFO_HOST_ABI="{_native.host_abi()}"',
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f"-I{t}/include",
             f"-I{t}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include", HOST_SRC,
             "-o", HOST_LIB, f"-L{t}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{cuda}/lib64",
             "-lcudart"]
+
+
+def _host_stamp() -> str:
+    return " ".join(_host_cmd()) + "\n"
+
+
+def _host_stale() -> bool:
+    """The extension depends on the C++ interfaces of torch and Python, which change without any source here getting newer."""
+    if _stale(HOST_LIB, [HOST_SRC, os.path.join(HERE, "..", "include", "flashomni_b200.h")]):
+        return True
+    try:
+        with open(HOST_STAMP) as f:
+            return f.read() != _host_stamp()
+    except OSError:
+        return True
 
 
 def _headers():
@@ -72,7 +91,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
     cuda_jobs = len(jobs)
-    if force or _stale(HOST_LIB, [HOST_SRC, os.path.join(HERE, "..", "include", "flashomni_b200.h")]):
+    host = force or _host_stale()
+    if host:
+        if os.path.exists(HOST_STAMP):
+            os.remove(HOST_STAMP)
         jobs.append(_host_cmd())
 
     def run(cmd):
@@ -86,6 +108,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
                     sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
                 if r.returncode != 0:
                     raise RuntimeError(f"{os.path.basename(cmd[0])} failed: " + " ".join(cmd[-3:]))
+    if host:
+        with open(HOST_STAMP, "w") as f:
+            f.write(_host_stamp())
     objs = [os.path.join(OBJDIR, s.replace(".cu", ".o")) for s in sources]
     if force or cuda_jobs or _stale(LIB, objs):
         cmd = [NVCC, *ARCH_FLAGS, "-shared", "-cudart", "shared", "-o", LIB, *objs,

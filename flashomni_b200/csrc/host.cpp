@@ -496,9 +496,12 @@ PyObject* bind(PyObject*, PyObject* arg) {
   Py_RETURN_NONE;
 }
 
+// What it was compiled for, as flashomni_b200._native.host_abi() names it: the caller compares before any other function is used.
+PyObject* abi(PyObject*, PyObject*) { return PyUnicode_FromString(FO_HOST_ABI); }
+
 #define FAST(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(attn_plan), FAST(attn_run), FAST(gemm_q), FAST(gemm_o), FAST(segment_packbits), FAST(select_blocks),
-                          {"bind", bind, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                          {"bind", bind, METH_O, nullptr}, {"abi", abi, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fo_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

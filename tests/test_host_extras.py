@@ -1,5 +1,6 @@
 """Host-side checks of the extensions (no GPU): argument validation, CPU refusal, list bookkeeping."""
 
+import os
 import numpy as np
 import pytest
 import torch
@@ -105,3 +106,32 @@ def test_lists_are_not_rebuilt_beside_a_preparation_that_nobody_took(monkeypatch
     assert w.run(q, q, q, *masks) == ("done", None) and waited == ["event"] * waits
     assert w._prepared_key is None
     assert w.run(q, q, q, *masks) == ("done", None) and waited == ["event"] * waits
+
+
+@pytest.mark.parametrize("how", ["missing", "other torch", "not a library"])
+def test_the_python_code_does_every_call_without_the_extension(monkeypatch, tmp_path, how):
+    """An extension that is not built, or for another torch or Python, is left alone with a warning; the ops still work."""
+    from flashomni_b200 import _native
+    so = tmp_path / "_fo_host.so"
+    if how == "not a library":
+        so.write_bytes(b"no shared object")
+    if how == "other torch":
+        monkeypatch.setattr(_native, "host_abi", lambda: "torch 1.0 cpython-27")
+    for name, value in (("_HOST", _native._HOST if how == "other torch" else str(so)), ("_host", None), ("_lib", None)):
+        monkeypatch.setattr(_native, name, value)
+    with pytest.warns(RuntimeWarning, match="is not used"):
+        h = _native.host()
+    assert h.attn_plan(1, 2) is None and h.gemm_q() is None
+    assert _native.load().fo_gemm_workspace_bytes(1, 128, 128, 128, 128) >= 64
+    with pytest.raises(RuntimeError, match="CUDA device"):
+        import flashomni_b200 as fo
+        fo.flashomni_gemm(torch.zeros(1, 128, 128), torch.zeros(128, 128), 1, is_full=True)
+
+
+def test_the_extension_is_rebuilt_for_another_torch(monkeypatch):
+    from flashomni_b200 import _native, build
+    if not os.path.exists(build.HOST_LIB):
+        pytest.skip("not built")
+    assert not build._host_stale()
+    monkeypatch.setattr(_native, "host_abi", lambda: "torch 1.0 cpython-27")
+    assert build._host_stale()
