@@ -419,9 +419,16 @@ PyObject* segment_packbits(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   if (rc != FO_OK) return PyLong_FromLong(rc);
   const int64_t nbytes = *words.data_ptr<int64_t>();
-  // (refused, or a copy pays: the Python code does the call again)
-  if (nbytes < 0 || capacity - nbytes > (nbytes > (1 << 20) ? nbytes : (1 << 20))) NOT_HERE;
-  PyObject* a = THPVariable_Wrap(y.narrow(0, 0, nbytes));
+  if (nbytes < 0) NOT_HERE;   // (refused: the Python code finds the reason)
+  at::Tensor packed = y.narrow(0, 0, nbytes);
+  // segments that cover little of x: the result does not keep the rest of the allocation alive (below a megabyte, the
+  // allocator's own granularity, the copy would cost more than it frees)
+  if (capacity - nbytes > (nbytes > (1 << 20) ? nbytes : (1 << 20))) {
+    pybind11::gil_scoped_release no_gil;
+    packed = packed.clone();
+    c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev)).synchronize();
+  }
+  PyObject* a = THPVariable_Wrap(packed);
   PyObject* b = THPVariable_Wrap(bytes_indptr);
   PyObject* t = a != nullptr && b != nullptr ? PyTuple_New(2) : nullptr;
   if (t == nullptr) { Py_XDECREF(a); Py_XDECREF(b); return nullptr; }

@@ -73,7 +73,10 @@ def segment_packbits(x: torch.Tensor, indptr: torch.Tensor, bitorder: str = "big
             y = y.narrow(0, 0, nbytes)
             # segments that cover little of x: the result does not keep the rest of the allocation alive (below a megabyte,
             # the allocator's own granularity, the copy would cost more than it frees)
-            return y.clone() if capacity - nbytes > max(nbytes, 1 << 20) else y, indptr_new
+            if capacity - nbytes > max(nbytes, 1 << 20):
+                y = y.clone()
+                torch.cuda.current_stream(device).synchronize()
+            return y, indptr_new
         refused = True
     seglen = indptr[1:] - indptr[:-1]
     packed_len = (seglen + 7) // 8

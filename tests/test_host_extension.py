@@ -215,3 +215,21 @@ def test_log_sum_exp_into_a_strided_buffer(cuda_device, monkeypatch, form):
         full = buf.clone()
         view(full).copy_(want)
         assert torch.equal(a[0], full) and (not return_lse or torch.equal(a[2], want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("indptr", [[0, 7, 5000], [0, 10_000_000]])
+def test_flags_are_packed_once(cuda_device, monkeypatch, indptr):
+    """Also where the packed bytes of a few segments are copied out of an allocation for all of x."""
+    x = torch.from_numpy((np.random.default_rng(1).random(20_000_000) < 0.5).astype(np.uint8)).to(cuda_device)
+    ip = torch.tensor(indptr, dtype=torch.int32, device=cuda_device)
+    lib = _native.load()
+
+    def call():
+        before = lib.fo_launch_count()
+        y, new = fo.segment_packbits(x, ip, "little")
+        return y, new, torch.tensor(lib.fo_launch_count() - before), torch.tensor(y.untyped_storage().nbytes())
+    a, b = _both(monkeypatch, call)
+    assert _same(a, b) and int(a[2]) == 1 and int(a[3]) <= a[0].numel() + (2 << 20)
+    want = np.concatenate([np.packbits(x[i:j].cpu().numpy(), bitorder="little") for i, j in zip(indptr, indptr[1:])])
+    assert np.array_equal(a[0].cpu().numpy(), want)
