@@ -438,7 +438,8 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         if self._fast_plan is not None and self._fast_args is self._list_args:
             # the usual call in one native function; it returns None, having done nothing, for anything else
             prepared = None
-            if self._prepared_key is not None and (is_full or (sparse_info is not None and sparse_kv_info is not None)):
+            if self._prepared_key is not None and (is_full or not (sparse_info is None or sparse_kv_info is None or
+                                                                   sparse_info_indptr is None or sparse_kv_info_indptr is None)):
                 if self._prepared_key == self._mask_key(sparse_info, sparse_kv_info, sparse_info_indptr,
                                                         sparse_kv_info_indptr, is_full):
                     prepared = self._prepared_event

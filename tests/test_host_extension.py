@@ -233,3 +233,16 @@ def test_flags_are_packed_once(cuda_device, monkeypatch, indptr):
     assert _same(a, b) and int(a[2]) == 1 and int(a[3]) <= a[0].numel() + (2 << 20)
     want = np.concatenate([np.packbits(x[i:j].cpu().numpy(), bitorder="little") for i, j in zip(indptr, indptr[1:])])
     assert np.array_equal(a[0].cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("missing", [0, 1, 2, 3])
+def test_missing_masks_are_refused_after_a_preparation_too(cuda_device, monkeypatch, missing):
+    w, q, k, v, masks = _attn(cuda_device)
+    some = [None if i == missing else m for i, m in enumerate(masks)]
+
+    def call():
+        w.prepare_masks(*masks)
+        return w.run(q, k, v, *some)
+    a, b = _both(monkeypatch, call)
+    assert a == b and a[0] is ValueError and "required unless is_full=True" in a[1]
