@@ -15,9 +15,9 @@
 // runs as N = 128.
 //
 // CTA = 192 threads: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer (with a full init tensor warp 6 loads its
-// slabs). K step 64 (one 128-byte swizzle atom), 4-stage (3) ring of (A 16 KB + B 32 KB), two 256-column TMEM accumulators so
-// the epilogue of tile i overlaps the main loop of tile i+1. The epilogue converts 64-column slabs
-// (TMEM -> registers -> +init -> 16-bit) into a swizzled shared-memory slab and hands each slab to a
+// slabs). K step 64 (one 128-byte swizzle atom), 4-stage ring of (A 16 KB + B 32 KB), two 256-column TMEM accumulators so
+// the epilogue of tile i overlaps the main loop of tile i+1. The epilogue converts slabs of 64 columns, or 32 with a full init
+// tensor (TMEM -> registers -> +init -> 16-bit) into a swizzled shared-memory slab and hands each slab to a
 // TMA store, so global writes are full 128-byte lines and asynchronous. The tiles of the sparse modes
 // (unequal lengths) are handed to the persistent CTAs through a device-wide cursor, in list order; the
 // equal tiles of a dense launch keep fixed round-robin shares.
@@ -532,10 +532,12 @@ __global__ void __launch_bounds__(threads_of(kCache), 1) gemm_kernel(const __gri
       uint4 initv[kPieces];
       auto load_init = [&](int s) {
         const int col0 = (s < kSlabsPerBlock ? ti.w_row0 : ti.w_row1) + (s % kSlabsPerBlock) * kSlabCols;
-        if (a.init_mode == kInitBias1D) {
-          const uint4* p = reinterpret_cast<const uint4*>(init16 + col0);
+        if constexpr (!kCache) {
+          if (a.init_mode == kInitBias1D) {
+            const uint4* p = reinterpret_cast<const uint4*>(init16 + col0);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) initv[i] = __ldg(p + i);
+            for (int i = 0; i < kPieces; ++i) initv[i] = __ldg(p + i);
+          }
         }
       };
       if (t_this >= 0) {

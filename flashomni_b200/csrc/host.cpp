@@ -34,7 +34,6 @@ struct Api {
   decltype(&fo_segment_packbits_polled) segment_packbits_polled;
   decltype(&fo_select_blocks_uniform) select_blocks_uniform;
   decltype(&fo_select_blocks_scratch_bytes) select_scratch_bytes;
-  decltype(&fo_layer_lists) layer_lists;
 };
 Api g_api;
 PyObject *s_kind, *s_key, *s_ws, *s_event, *s_cuda_event;
@@ -497,7 +496,6 @@ PyObject* bind(PyObject*, PyObject* arg) {
   get(a.segment_packbits_polled, "fo_segment_packbits_polled");
   get(a.select_blocks_uniform, "fo_select_blocks_uniform");
   get(a.select_scratch_bytes, "fo_select_blocks_scratch_bytes");
-  get(a.layer_lists, "fo_layer_lists");
   if (missing != nullptr) return PyErr_Format(PyExc_RuntimeError, "flashomni_b200: the native library has no %s", missing);
   g_api = a;
   Py_RETURN_NONE;

@@ -173,12 +173,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* t
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-// Brings a tile into L2.
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* tmap, int x, int y, int z) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(tmap)),
-               "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
 // TMA tiled store (shared -> global), bulk-group completion.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, const void* smem_src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
@@ -408,21 +402,6 @@ __device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t b_hi, uint3
       : "memory");
 }
 
-// 2 x (D[tmem] += A[tmem] * B[smem]); the first instruction accumulates iff `acc_first`.
-__device__ __forceinline__ void umma_ts_x2(uint32_t d_tmem, uint32_t b_hi, uint32_t idesc, uint32_t acc_first,
-                                           const uint32_t* ta, const uint32_t* lb) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p0, p1;\n"
-      ".reg .b64 db;\n"
-      "setp.ne.b32 p0, %3, 0;\n"
-      "setp.eq.b32 p1, 0, 0;\n"
-      FO_MMA_TS("%4", "%6", "p0") FO_MMA_TS("%5", "%7", "p1")
-      "}\n" ::"r"(d_tmem),
-      "r"(b_hi), "r"(idesc), "r"(acc_first), "r"(ta[0]), "r"(ta[1]), "r"(lb[0]), "r"(lb[1])
-      : "memory");
-}
-
 // Arrive (count 1) on `bar` once every tcgen05 op issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -473,12 +452,6 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t* r) {
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
       "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
-}
-
-__device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
