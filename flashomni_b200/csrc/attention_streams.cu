@@ -28,8 +28,8 @@
 //   P handed over after three quarters (a quarter) instead of half                                               109 / 263 (109 / 258)
 //   each stream with units of its own instead of alternate blocks of one unit                                    125 / 261
 // Other shapes, device time of a call from a graph, attention.cu -> here: one request of 4608 tokens with 12 heads 76 -> 68, at
-// density 0.2 67 -> 59; 32 requests of 256 tokens 60 -> 50, 8 of 1024 118 -> 108; 64 requests of 128 tokens 59.5 -> 50.9, of 100
-// 55.4 -> 48.4, of 77 50.8 -> 48.0, of 33 46.6 -> 44.3, of 20 46.0 -> 47.3. Rows of a slab that is not whole leave from the thread
+// density 0.2 67 -> 59; 32 requests of 256 tokens 60 -> 50, 8 of 1024 118 -> 108; 64 requests of 128 tokens 59.5 -> 50.8, of 100
+// 55.4 -> 46.8, of 77 50.8 -> 45.6, of 33 46.6 -> 43.1, of 20 46.0 -> 43.9. Rows of a slab that is not whole leave from the thread
 // that has them: staged like the others, four rows an instruction, 64 requests of 77 / 33 / 20 tokens took 55.8 / 53.8 / 50.5.
 //
 // Warps: 0-3 softmax stream 0, 4-7 softmax stream 1 (TMEM lane = q row), 8-11 epilogue, 12 TMA producer and drawer of
@@ -56,7 +56,8 @@ constexpr int kWarpProducer = kWarpEpilogue + kEpilogueWarps;
 constexpr int kWarpMma = kWarpProducer + 1;
 constexpr int kWarpZero = kWarpMma + 2;
 constexpr int kThreads = (kWarpZero + 1) * 32;   // 512
-// setmaxnreg split. 184 / 88 / 56 gave the epilogue too few: image layer 95.2 us instead of 94.5, 64 requests of 90 / 20 tokens 51.5 /
+// setmaxnreg split. The 60 bytes that are spilled at head dimension 128 are descriptor words of the issuers (14.6 local loads of one
+// warp per kv block); 184 / 88 / 56 gave the epilogue too few: image layer 95.2 us instead of 94.5, 64 requests of 90 / 20 tokens 51.5 /
 // 47.8 instead of 47.5 / 43.9 (device time of a call from a graph).
 constexpr int kRegsSoftmax = 168, kRegsEpilogue = 120, kRegsOther = 56;
 // setmaxnreg.inc waits until the registers are free in the pool the CTA was launched with: a split that asks for more
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
       // a stream without a visible column has m = -inf, l = 0
       const float w_min = exp2_series(fminf(m0, m1) - m_out);
       float w0 = (m0 == m_out) ? 1.f : w_min, w1 = (m1 == m_out) ? 1.f : w_min;
-      const float l_out = fmaf(l0, w0, l1 * w1);
+      const float l_out = m0 == m_out ? fmaf(l1, w1, l0) : fmaf(l0, w0, l1);   // (the other weight is 1: one rounding)
       const float inv_out = l_out > 0.f ? __frcp_rn(l_out) : 0.f;
       // A unit of one block leaves the other stream's O as it was, which may be anything: O of the stream with the block stands in
       // for it, with a weight that rounds away beside w0 (at least 2^-40) and, unlike zero, leaves an infinity one.
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_streams_kernel(const __
         }
       }
       ++item;
-      if (row_ok && lse != nullptr) *lse = (l_out > 0.f) ? (log2f(l_out) + m_out) : -5e4f;
+      if (row_ok && lse != nullptr) *lse = (l_out > 0.f) ? add_log2(m_out, l_out) : -5e4f;
     }
     if (lane == 0) tma_store_wait_all<0>();
   } else {

@@ -462,6 +462,15 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// m + log2(l) for a normal l > 0 with one rounding of its size: the exponent of l joins m in a sum whose error is kept (the
+// two-sum of Knuth), and the logarithm is of a number in [1, 2). log2f(l) + m rounds twice.
+__device__ __forceinline__ float add_log2(float m, float l) {
+  const int bits = __float_as_int(l);
+  const float e = static_cast<float>((bits >> 23) - 127), lg = log2f(__int_as_float((bits & 0x007fffff) | 0x3f800000));
+  const float sum = m + e, b = sum - m;
+  const float err = (m - (sum - b)) + (e - b);
+  return sum + (err + lg);
+}
 // 2^d for d <= 0 (0 below -126.5) with a relative error of at most 1.3 * 2^-24: 2^n times the Taylor series of
 // 2^f = exp(f ln 2), abs(f) <= 1/2, whose next term is 5e-9. For factors that scale whole sums, where the error of ex2.approx
 // would be the largest error (ex2.approx: 4 * 2^-24).

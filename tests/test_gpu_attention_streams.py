@@ -155,3 +155,25 @@ def test_small_weights_add_up_in_the_row_sum(cuda_device, dtype, D):
     want = np.log2(128 + (S - 128) * 2.0 ** -21)
     assert (lse.cpu().double() - want).abs().max() <= 2.0 ** -20
     assert (o == 1).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S", [128, 333, 1024])
+def test_log_sum_exp_of_exact_sums_is_rounded_once(cuda_device, S, D):
+    """Integer logits from -4 to 4 in base 2 (sm_scale * log2(e) is 1 in float32): exponentials, merge weights and sums (at most 19
+    bits) are exact, so what is left is the rounding of the result, half a unit in its last place, and one unit of a logarithm
+    below 1 (2^-24) with its addition (2^-25)."""
+    H = 8
+    g = torch.Generator().manual_seed(S + D)
+    q, k = torch.zeros(S, H, D), torch.zeros(S, H, D)
+    q[..., :4] = torch.randint(0, 2, (S, H, 4), generator=g).float()
+    k[..., :4] = torch.randint(-1, 2, (S, H, 4), generator=g).float()
+    v = torch.randn(S, H, D, generator=g)
+    w = fo.BatchFlashOmniFAWithRaggedKVWrapper(torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device))
+    ip = torch.tensor([0, S], dtype=torch.int32, device=cuda_device)
+    w.plan(ip, ip, H, H, D, q_data_type=torch.bfloat16, sm_scale=float(np.log(2.0)))
+    _, lse = w.run(*(dev(t.bfloat16(), cuda_device) for t in (q, k, v)), is_full=True, return_lse=True)
+    w.check_status()
+    want = torch.log2(torch.exp2(torch.einsum("qhd,khd->qhk", q.double(), k.double())).sum(2))
+    half_ulp = torch.exp2(torch.floor(torch.log2(want)) - 24)
+    assert ((lse.cpu().double() - want).abs() <= half_ulp + 1.5 * 2.0 ** -24).all()
