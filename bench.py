@@ -40,7 +40,7 @@ HID, H, D, S, B, DENSITY, SEED = 3072, 24, 128, 4608, 2, 0.5, 2024
 FL_ATTN_TILE = 4 * 128 * 128 * 128
 FL_GEMM_TILE = 2 * 128 * 128 * HID
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, from the ncu captures summarised under profiles/
-NCU_TRAFFIC = {"attention_kernel": 169.2e6, "gemm_kernel": 120.8e6, "gemm_tall_kernel": 232.8e6}
+NCU_TRAFFIC = {"attention_streams_kernel": 169.1e6, "gemm_kernel": 120.7e6, "gemm_tall_kernel": 234.1e6}
 
 
 # ---------------------------------------------------------------------------------------------- helpers
@@ -633,7 +633,7 @@ def run_flux(ctx, args, peaks):
                 "avg_launch_ms": r4(t / launches), "flops_per_step": float(flops), "achieved_tflops": round(tf(flops, t), 1),
                 "frac_of_peak": r4(tf(flops, t) / peaks["burst"]), "share_of_step": r4(t / step_sum_ms)}
 
-    kernels = [kentry("attention_kernel<bf16>", "attention", fl["attention"], 1),
+    kernels = [kentry("attention_streams_kernel<bf16>", "attention", fl["attention"], 1),
                kentry("gemm_kernel<bf16> (GEMM-Q, active tiles)", "gemm_q", fl["gemm_q"], 1),
                kentry("gemm_kernel<bf16> (GEMM-O, active heads)", "gemm_o", fl["gemm_o"], 1),
                kentry(dense_name + "<bf16> (dense K/V projection)", "gemm_kv", fl["gemm_kv"], kv_launches)]

@@ -263,7 +263,7 @@ struct AttnArgs {
 // floats of one partial result: O (32 column groups x 128 rows x 4), then the row maxima and the row sums
 constexpr int kPartialFloats = 128 * 128 + 2 * 128;
 // whole items without a causal or custom mask, head dimension 64 or 128: attention_streams.cu, which was faster at every
-// shape measured but the one named there; the other launches keep attention.cu
+// shape measured (named there); the other launches keep attention.cu
 inline bool attention_streams_applies(const AttnArgs& a) {
   return a.mask_mode == 0 && a.partial_slots <= 0 && (a.head_dim == 64 || a.head_dim == 128);
 }
