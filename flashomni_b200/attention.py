@@ -616,7 +616,7 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
         any other `run()` compacts as usual. Masks only depend on the block selection, not on q/k/v.
         `stream` replaces the wrapper's own side stream; with `after` the side stream is ordered after that
         event instead of after everything enqueued on the current stream so far (the caller guarantees that
-        the previous `run()` of this wrapper precedes the event)."""
+        the previous `run()` of this wrapper precedes the event, and that the masks are complete or written before it)."""
         if not self._planned:
             raise RuntimeError("plan() must be called before prepare_masks()")
         if not is_full:

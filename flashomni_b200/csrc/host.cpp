@@ -6,7 +6,7 @@
 // indptrs, ...). An int is the error code of the C ABI. What it replaces is one Python expression per argument and ctypes
 // conversions of up to 45 of them, which took longer than the kernels of small calls. Host time to issue a call, us, before ->
 // here: attention of a short request 48 -> 14, of the image layer 40 -> 9, GEMM-Q 31 -> 11, GEMM-O 34 -> 10, a layer step 141-157 ->
-// 59, block selection 26 -> 11, packing of both masks (two calls, each waiting for its size) 72 -> 34.
+// 59, block selection 26 -> 11, packing of both masks (two calls, each waiting for its bytes) 72 -> 31.
 #include <Python.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>

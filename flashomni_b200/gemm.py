@@ -262,7 +262,8 @@ def prepare_gemm_q_list(batch: int, M: int, N: int, num_qo_heads: int, sparse_in
                         head_dim: Optional[int] = None, into: Optional[GemmWorklist] = None,
                         stream: Optional[torch.cuda.Stream] = None) -> GemmWorklist:
     """Builds the GEMM-Q work list for a [batch, M, *] x [N, *] product from the mask, on `stream` (default: the
-    current stream). `into` re-uses the workspace of an earlier list of the same shape."""
+    current stream). `into` re-uses the workspace of an earlier list of the same shape. The masks must be complete, or `stream`
+    be ordered behind what writes them, and with `into` behind the last call that used the list."""
     hd = N // num_qo_heads if head_dim is None else head_dim
     return _prepare("q", batch, M, N, hd, num_qo_heads, hd, sparse_info, sparse_info_indptr, num_text_tokens,
                     sparse_q_size, head_begin, False, into, stream)
