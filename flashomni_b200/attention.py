@@ -372,8 +372,9 @@ class BatchFlashOmniFAWithRaggedKVWrapper:
             buf = torch.zeros(need, dtype=torch.uint8, device=self.device)
             self._int_workspace_buffer = buf
         # lists prepared under an earlier plan are not those of this one, and may still be on their way into this buffer
-        self._after_prepared(torch.cuda.current_stream(self.device))
-        self._prepared_key = None
+        if self._prepared_key is not None:
+            self._after_prepared(torch.cuda.current_stream(self.device))
+            self._prepared_key = None
         words = buf.view(torch.uint8)[: need].view(torch.int32)
         words[offs["counters"]: offs["counters"] + 12].zero_()  # counters, status / cursor words start from zero
         words[offs["arrive"]: offs["arrive"] + max(self._partial_slots, 1)].zero_()
